@@ -449,58 +449,152 @@ int exclusive_scan_u32(Ctx* c, const uint32_t* in, uint32_t* out, uint64_t n, ui
 }
 
 // --------------------------------------------------------------------------
-// LSD radix sort of (u64 key, u32 value) pairs, 8-bit digits, stable.
-// Upsweep: per-block digit histogram (digit-major). Scan. Downsweep: warps rank
-// items with __match_any_sync in input order and scatter.
+// LSD radix sort of (u64 key, u32 value) pairs, stable (radix.cuh).
 // --------------------------------------------------------------------------
+__global__ void __launch_bounds__(OS_T) radix_hist_kernel(const uint64_t* __restrict__ keys, uint64_t n, OsPlan plan,
+                                                          uint32_t* __restrict__ hist, uint32_t* __restrict__ done,
+                                                          uint4* __restrict__ status, uint64_t status_vec) {
+  extern __shared__ uint32_t s_hist[];  // [pass][digit][copy]
+  __shared__ uint32_t s_wsum[OS_WARPS];
+  __shared__ bool s_last;
+  const int words = plan.passes * OS_BINS * OS_COPIES;
+  for (int i = threadIdx.x; i < words; i += OS_T) s_hist[i] = 0;
+  const uint64_t gid = (uint64_t)blockIdx.x * OS_T + threadIdx.x, stride = (uint64_t)gridDim.x * OS_T;
+  for (uint64_t i = gid; i < status_vec; i += stride) status[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  const unsigned copy = threadIdx.x & (OS_COPIES - 1);
+  constexpr int U = 4;  // keys in flight per thread
+  for (uint64_t b = gid; b < n; b += U * stride) {
+    uint64_t k[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) k[u] = b + u * stride < n ? keys[b + u * stride] : 0ULL;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (b + u * stride >= n) continue;
+#pragma unroll
+      for (int p = 0; p < OS_MAX_PASSES; ++p)
+        if (p < plan.passes)
+          atomicAdd(&s_hist[((uint32_t)p * OS_BINS + ((uint32_t)(k[u] >> plan.shift[p]) & plan.mask[p])) * OS_COPIES + copy],
+                  1u);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < plan.passes * OS_BINS; i += OS_T) {
+    uint32_t v = 0;
+#pragma unroll
+    for (int k = 0; k < OS_COPIES; ++k) v += s_hist[i * OS_COPIES + k];
+    if (v) atomicAdd(hist + i, v);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int p = 0; p < plan.passes; ++p) {
+    const uint32_t v = __ldcg(hist + p * OS_BINS + threadIdx.x);
+    hist[p * OS_BINS + threadIdx.x] = os_block_prefix<OS_T>(v, s_wsum);
+    __syncthreads();
+  }
+}
+
+// Sorts of up to 8,192 keys run in one block (one launch); up to 2^19 keys in tiles of
+// 2,048, which spread them over the SMs (60,000 keys: 55 us, in 4,096-key tiles 64); above in
+// tiles of 8,192, whose runs of a digit average 16 keys (128 bytes) and whose status rows are
+// few (1 M keys: 114 us, in tiles of 2,048 141 us).
+constexpr uint64_t kOsSmallMax = 1ULL << 19;
+
+template <int IPT, bool VALS, class ST>
+static void onesweep_launch(Ctx* c, unsigned tiles, const uint64_t* kin, const uint32_t* vin, uint64_t n, int shift,
+                            uint32_t mask, const uint32_t* doff, uint32_t* ticket, void* st, void* st_next,
+                            uint64_t* kout, uint32_t* vout) {
+  auto fn = radix_onesweep_kernel<IPT, VALS, ST>;
+  if (os_smem<IPT>() > 40 * 1024)  // with the static part past the 48 KB default
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)os_smem<IPT>());
+  fn<<<tiles, OS_T, os_smem<IPT>(), c->stream>>>(kin, vin, n, shift, mask, doff, ticket, (ST*)st, (ST*)st_next, kout, vout);
+}
+
+template <int IPT, bool VALS>
+static void block_sort_launch(Ctx* c, const uint64_t* keys, const uint32_t* vals, uint64_t n, const OsPlan& plan,
+                              uint64_t* kout, uint32_t* vout) {
+  auto fn = radix_block_kernel<IPT, VALS>;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)os_block_smem<IPT>());
+  fn<<<1, OS_BLOCK_T, os_block_smem<IPT>(), c->stream>>>(keys, vals, (uint32_t)n, plan, kout, vout);
+}
 
 int radix_sort_pairs(Ctx* c, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                      uint64_t n, int bits, bool* result_in_alt) {
   *result_in_alt = false;
   if (n <= 1 || bits <= 0) return CYTOM_OK;
-  const bool small = n < (1ULL << 24);
-  const uint64_t tile = (uint64_t)RS_T * (small ? RS_IPT_SMALL : RS_IPT_LARGE);
-  uint64_t nb = (n + tile - 1) / tile;
-  uint32_t* hist = nullptr;
-  // histogram, its scan and the scan's scratch in one allocation for every pass
-  const uint64_t sw = scan_scratch_words(nb * 256);
-  cudaError_t e = cy_malloc_async((void**)&hist, (nb * 256 * 2 + sw) * 4, c->stream);
-  if (e != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "radix histogram");
-  uint32_t* offs = hist + nb * 256;
-  uint32_t* sscr = offs + nb * 256;
+  const OsPlan plan = os_plan(bits);
+  const double bytes = (double)n * (vals ? 12.0 : 8.0);
+  if (n <= (uint64_t)OS_BLOCK_T * OS_BLOCK_IPT_LARGE) {
+    int slot = prof_begin(c, KC_SORT);
+    if (n <= (uint64_t)OS_BLOCK_T * OS_BLOCK_IPT_SMALL) {
+      if (vals) block_sort_launch<OS_BLOCK_IPT_SMALL, true>(c, keys, vals, n, plan, keys_alt, vals_alt);
+      else block_sort_launch<OS_BLOCK_IPT_SMALL, false>(c, keys, vals, n, plan, keys_alt, vals_alt);
+    } else {
+      if (vals) block_sort_launch<OS_BLOCK_IPT_LARGE, true>(c, keys, vals, n, plan, keys_alt, vals_alt);
+      else block_sort_launch<OS_BLOCK_IPT_LARGE, false>(c, keys, vals, n, plan, keys_alt, vals_alt);
+    }
+    c->launches++;
+    prof_end(c, slot, bytes * 2.0);
+    *result_in_alt = true;
+    return cuda_err(c, cudaGetLastError(), "radix");
+  }
+  const bool small = n <= kOsSmallMax, wide = n >= (1ULL << 30);
+  const uint64_t tile = (uint64_t)OS_T * (small ? OS_IPT_SMALL : OS_IPT_LARGE);
+  const uint64_t tiles = (n + tile - 1) / tile;
+  // digit counts and tickets (cleared), then two sets of status rows: a pass clears the rows
+  // of the next one
+  const size_t head = ((size_t)plan.passes * OS_BINS + 16 + 3) / 4 * 16;
+  const size_t rows = (size_t)tiles * OS_BINS * (wide ? 8 : 4);
+  char* tmp = nullptr;
+  if (cy_malloc_async((void**)&tmp, head + 2 * rows, c->stream) != cudaSuccess)
+    return set_err(c, CYTOM_ERR_OOM, "radix histogram");
+  uint32_t* hist = (uint32_t*)tmp;
+  uint32_t* tickets = hist + (size_t)plan.passes * OS_BINS;  // one per pass, then the counting kernel's block count
+  char* st[2] = {tmp + head, tmp + head + rows};
+  int slot = prof_begin(c, KC_SORT);
+  cudaError_t e = cudaMemsetAsync(tmp, 0, head, c->stream);
+  const size_t hsm = (size_t)plan.passes * OS_BINS * OS_COPIES * 4;
+  if (e == cudaSuccess && hsm > 40 * 1024)
+    e = cudaFuncSetAttribute(radix_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
+  if (e == cudaSuccess) {
+    radix_hist_kernel<<<grid_for(c, (n + 7) / 8, OS_T, 3), OS_T, hsm, c->stream>>>(
+        keys, n, plan, hist, tickets + OS_MAX_PASSES, (uint4*)st[0], rows / 16);
+    c->launches++;
+    e = cudaGetLastError();
+  }
+  prof_end(c, slot, bytes);
   uint64_t *kin = keys, *kout = keys_alt;
   uint32_t *vin = vals, *vout = vals_alt;
-  bool alt = false;
-  for (int shift = 0; shift < bits; shift += 8) {
-    int slot = prof_begin(c, KC_SORT);
-    if (small) radix_upsweep_kernel<RS_IPT_SMALL><<<(unsigned)nb, RS_T, 0, c->stream>>>(kin, n, shift, hist, (uint32_t)nb);
-    else radix_upsweep_kernel<RS_IPT_LARGE><<<(unsigned)nb, RS_T, 0, c->stream>>>(kin, n, shift, hist, (uint32_t)nb);
-    c->launches++;
-    int rc = scan_into(c, hist, offs, nb * 256, nullptr, sscr);
-    if (rc) {
-      cudaFreeAsync(hist, c->stream);
-      return rc;
+  for (int p = 0; p < plan.passes && e == cudaSuccess; ++p) {
+    slot = prof_begin(c, KC_SORT);
+    const uint32_t* doff = hist + (size_t)p * OS_BINS;
+    void *sa = st[p & 1], *sb = st[(p & 1) ^ 1];
+#define CYTOM_OS(IPT, V, ST) \
+  onesweep_launch<IPT, V, ST>(c, (unsigned)tiles, kin, vin, n, plan.shift[p], plan.mask[p], doff, tickets + p, sa, sb, kout, vout)
+    if (small) {
+      if (vals) CYTOM_OS(OS_IPT_SMALL, true, uint32_t);
+      else CYTOM_OS(OS_IPT_SMALL, false, uint32_t);
+    } else if (!wide) {
+      if (vals) CYTOM_OS(OS_IPT_LARGE, true, uint32_t);
+      else CYTOM_OS(OS_IPT_LARGE, false, uint32_t);
+    } else {
+      if (vals) CYTOM_OS(OS_IPT_LARGE, true, unsigned long long);
+      else CYTOM_OS(OS_IPT_LARGE, false, unsigned long long);
     }
-    if (small)
-      radix_downsweep_kernel<RS_IPT_SMALL><<<(unsigned)nb, RS_T, 0, c->stream>>>(kin, vin, n, shift, offs, (uint32_t)nb,
-                                                                               kout, vout);
-    else
-      radix_downsweep_kernel<RS_IPT_LARGE><<<(unsigned)nb, RS_T, 0, c->stream>>>(kin, vin, n, shift, offs, (uint32_t)nb,
-                                                                               kout, vout);
+#undef CYTOM_OS
     c->launches++;
-    prof_end(c, slot, (double)n * (vals ? 12.0 : 8.0) * 3.0);
+    prof_end(c, slot, bytes * 2.0);
     e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      cudaFreeAsync(hist, c->stream);
-      return cuda_err(c, e, "radix");
-    }
     std::swap(kin, kout);
     std::swap(vin, vout);
-    alt = !alt;
   }
-  cudaFreeAsync(hist, c->stream);
-  *result_in_alt = alt;
-  return CYTOM_OK;
+  cudaFreeAsync(tmp, c->stream);
+  *result_in_alt = (plan.passes & 1) != 0;
+  return cuda_err(c, e, "radix");
 }
 
 // --------------------------------------------------------------------------
