@@ -272,7 +272,8 @@ static int job_prepare(Ctx* c, Job* j) {
 static int job_finish(Ctx* c, Job* j, const LoopState& ls, cudaEvent_t ev_a, cudaEvent_t ev_b,
                       cytom_run_stats* st) {
   if (ls.err) return set_err(c, CYTOM_ERR_TIMEOUT, "a bounded device wait gave up");
-  if (j->last_run_graph) c->launches += 4ULL * ls.iter;  // per round: two gathers, chunk pass, apply
+  // passes of the captured loop (the seeding apply counts one): small rounds, two gathers, chunk pass, apply
+  if (j->last_run_graph && ls.sel_rounds) c->launches += 5ULL * (ls.sel_rounds - 1);
   if (st) {
     memset(st, 0, sizeof(*st));
     st->iterations = ls.iter;

@@ -84,7 +84,7 @@ struct LoopState {
   unsigned int err;
   unsigned int active[2];  // vertices activated for the next round (by parity)
   unsigned int nact_words[2];  // non-zero frontier words listed for the next round
-  unsigned int mode;       // gather of the current round: 0 dense (stream), 1 sparse (directory)
+  unsigned int mode;       // current round: 0 dense (stream), 1 sparse (directory), 2 small (one cluster)
   unsigned int spq_count;  // heavy-item chunks queued in this round
   unsigned long long teps[2];  // edges of newly active tile rows (by parity)
   unsigned long long count_edges;   // reference counting rule, summed
@@ -103,6 +103,7 @@ struct LoopState {
   unsigned int sel_rounds;  // rounds started by the captured loop (bounds it independently)
   unsigned int pad2;
   unsigned long long items_read;  // sparse rounds: (word, column) items whose directory was read
+  unsigned int est[2];  // out-edges of the vertices in the first listed frontier words (by parity)
 };
 
 struct JobDesc {

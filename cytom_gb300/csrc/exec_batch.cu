@@ -125,12 +125,13 @@ __device__ void unit_apply(const BJob* J, bool initial, uint32_t unit) {
   const uint64_t nwords = (sd->n + 31) >> 5;
   unsigned cnt = 0;
   unsigned long long teps = 0;
+  unsigned est = 0;  // small rounds are the one-job loops'
   const uint64_t base0 = (uint64_t)unit * BU_APPLY_WORDS;
   for (uint32_t k = 0; k < BU_APPLY_WORDS / BT; ++k) {
     const uint64_t base = base0 + (uint64_t)k * BT;
-    if (base < nwords) apply_step<true>(jd, sd, pw, base, cnt, teps);
+    if (base < nwords) apply_step<true>(jd, sd, pw, base, cnt, teps, est);
   }
-  apply_flush(jd->ls, pw, cnt, teps);
+  apply_flush<BT>(jd->ls, pw, cnt, teps, est);
 }
 
 template <int ALGO>
@@ -660,7 +661,7 @@ __device__ void advance(const BJob* J, BSched* S, BCtl* ctl, unsigned phase) {
       s_next = nq ? PH_CHUNKS : PH_APPLY;
       s_total = nq ? ceil_div(nq, BU_CHUNKS) : 0;
     } else {
-      s_cont = control_step(jd, sd, phase == PH_APPLY0 ? 1 : 0);
+      s_cont = control_step(jd, sd, phase == PH_APPLY0 ? 1 : 0, 0);
     }
   }
   __syncthreads();

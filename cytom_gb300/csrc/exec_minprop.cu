@@ -65,29 +65,108 @@ __global__ void __launch_bounds__(APPLY_T) apply_minprop_kernel(const JobDesc* _
       cudaGraphSetConditional(h, 0u);
     }
   }
-  if (!ls->cont) return;
+  // (mode 2 here: the cluster stopped at its round limit, the next body pass goes on)
+  if (!ls->cont || (!initial && ls->mode == 2)) return;
   const unsigned pw = initial ? 0u : ((ls->iter & 1u) ^ 1u);
   const uint64_t nwords = (sd->n + 31) >> 5;
-  unsigned cnt = 0;
+  unsigned cnt = 0, est = 0;
   unsigned long long teps = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nwords; base += stride)
-    apply_step<false>(jd, sd, pw, base, cnt, teps);
-  apply_flush(ls, pw, cnt, teps);
+    apply_step<false>(jd, sd, pw, base, cnt, teps, est);
+  apply_flush<APPLY_T>(ls, pw, cnt, teps, est);
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicAdd(&ls->apply_done, 1u) == gridDim.x - 1) {
       __threadfence();
       atomicExch(&ls->apply_done, 0u);
-      const unsigned cont = control_step(jd, sd, initial);
+      const unsigned cont = control_step(jd, sd, initial, 1);
       if (use_handle) cudaGraphSetConditional(h, cont);
     }
   }
 }
 
-// Gather for BFS (ALGO 0), CC (1), SSSP (2). A warp owns a 128-edge chunk: lane l
-// loads edges [4l, 4l+4) of it with one 128-bit load. The tile of an edge is found
-// from the chunk's first tile and tile_ptr (edges are tile-major).
+// Chunk c of a dense round for the calling warp, BFS (ALGO 0), CC (1), SSSP (2), SSWP (3):
+// lane l takes edges [4l, 4l+4) of it with one 128-bit load. The tile of an edge is found
+// from the chunk's first tile and tile_ptr (edges are tile-major). Returns the edges scanned
+// (lane 0).
+template <int ALGO, bool PERSIST>
+__device__ __forceinline__ uint32_t dense_chunk(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                                uint64_t c, unsigned p, int adaptive) {
+  const uint64_t T = sd->T;
+  const unsigned* rows_cur = jd->rows + p * T;
+  const unsigned long long* __restrict__ tile_ptr = sd->tile_ptr;
+  const bool async = jd->async != 0;
+  uint32_t* next = jd->next;
+  const uint64_t E = sd->E;
+  const uint32_t lT = sd->lT, lvpt = sd->lvpt;
+  const uint32_t ymask = (uint32_t)(T - 1);
+  const unsigned lane = threadIdx.x & 31;
+  const uint64_t e0 = c * kChunk + (uint64_t)lane * 4;
+  const bool in = e0 < E;
+  const uint4 ev = in ? *reinterpret_cast<const uint4*>(sd->edges + e0) : make_uint4(0, 0, 0, 0);
+  uint4 wv = make_uint4(0, 0, 0, 0);
+  if (mp_weighted<ALGO>() && in) wv = *reinterpret_cast<const uint4*>(sd->wts + e0);
+  const uint32_t t0 = sd->chunk_tile[c], t1 = sd->chunk_tile[c + 1];
+  if (adaptive) {
+    bool any = false;
+    for (uint32_t x = t0 >> lT; x <= (t1 >> lT); ++x) any |= ld_plain<PERSIST>(rows_cur + x) != 0;
+    if (!any) return 0;
+  }
+  const uint32_t scanned =
+      lane == 0 ? (uint32_t)((E - c * kChunk < (uint64_t)kChunk) ? (E - c * kChunk) : kChunk) : 0u;
+  if (!in) return scanned;
+  // locate the tile of e0: last t in [t0, t1] with tile_ptr[t] <= e0
+  uint32_t t = t0;
+  if (tile_ptr[t + 1] <= e0) {
+    uint32_t lo = t0, hi = t1;
+    while (lo < hi) {
+      uint32_t mid = lo + ((hi - lo + 1) >> 1);
+      if (tile_ptr[mid] <= e0) lo = mid;
+      else hi = mid - 1;
+    }
+    t = lo;
+  }
+  unsigned long long tend = tile_ptr[t + 1];
+  const uint32_t evk[4] = {ev.x, ev.y, ev.z, ev.w};
+  const uint32_t wvk[4] = {wv.x, wv.y, wv.z, wv.w};
+  uint32_t u[4], v[4], cand[4], nv[4];
+  bool on[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint64_t e = e0 + k;
+    on[k] = e < E;
+    if (on[k]) {
+      while (tend <= e) {
+        ++t;
+        tend = tile_ptr[t + 1];
+      }
+    }
+    const uint32_t x = t >> lT, y = t & ymask;
+    u[k] = (x << lvpt) | (evk[k] >> 16);
+    v[k] = (y << lvpt) | (evk[k] & 0xFFFFu);
+    if (adaptive && on[k] && ld_plain<PERSIST>(rows_cur + x) == 0) on[k] = false;
+  }
+  // every edge's frontier word, source value and target value in flight together
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    nv[k] = on[k] ? __ldcg(next + v[k]) : 0u;
+    const uint32_t fw = (adaptive && on[k]) ? ld_state<PERSIST>(jd->fa + (u[k] >> 5)) : 0xFFFFFFFFu;
+    cand[k] = on[k] ? ld_src<PERSIST>(jd, async, u[k]) : kInf;
+    if (!((fw >> (u[k] & 31)) & 1u)) cand[k] = kInf;
+    if (cand[k] != kInf) cand[k] = mp_cand<ALGO>(cand[k], wvk[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (cand[k] != kInf && cand[k] < nv[k]) {
+      atomicMin(next + v[k], cand[k]);
+      atomicOr(jd->ch + (v[k] >> 5), 1u << (v[k] & 31));
+    }
+  }
+  return scanned;
+}
+
+// Unstaged dense gather: one chunk per warp.
 template <int ALGO>
 __global__ void __launch_bounds__(GATHER_T) gather_minprop_kernel(const JobDesc* __restrict__ jd,
                                                                   const StoreDesc* __restrict__ sd,
@@ -95,80 +174,16 @@ __global__ void __launch_bounds__(GATHER_T) gather_minprop_kernel(const JobDesc*
   LoopState* ls = jd->ls;
   if (!ls->cont || ls->mode != 0) return;
   const unsigned p = ls->iter & 1u;
-  const uint64_t T = sd->T;
-  const unsigned* __restrict__ rows_cur = jd->rows + p * T;
   round_open<false>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
-  const uint32_t* __restrict__ edges = sd->edges;
-  const uint32_t* __restrict__ wts = sd->wts;
-  const unsigned long long* __restrict__ tile_ptr = sd->tile_ptr;
-  const uint32_t* __restrict__ chunk_tile = sd->chunk_tile;
-  const uint32_t* __restrict__ fa = jd->fa;
-  const uint32_t* __restrict__ cur = jd->cur;
-  const bool async = jd->async != 0;
-  uint32_t* next = jd->next;
-  uint32_t* ch = jd->ch;
-  const uint64_t E = sd->E, nchunks = sd->nchunks;
-  const uint32_t lT = sd->lT, lvpt = sd->lvpt;
-  const uint32_t ymask = (uint32_t)(T - 1);
-  const unsigned lane = threadIdx.x & 31;
+  const uint64_t nchunks = sd->nchunks;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long scanned = 0;
-  for (uint64_t c = warp; c < nchunks; c += nwarps) {
-    const uint32_t t0 = chunk_tile[c];
-    const uint32_t t1 = chunk_tile[c + 1];
-    if (adaptive) {
-      bool any = false;
-      for (uint32_t x = t0 >> lT; x <= (t1 >> lT); ++x) any |= rows_cur[x] != 0;
-      if (!any) continue;
-    }
-    const uint64_t e0 = c * kChunk + (uint64_t)lane * 4;
-    if (lane == 0) scanned += (E - c * kChunk < (uint64_t)kChunk) ? (E - c * kChunk) : kChunk;
-    if (e0 >= E) continue;
-    const uint4 ev = *reinterpret_cast<const uint4*>(edges + e0);
-    uint4 wv = make_uint4(0, 0, 0, 0);
-    if (mp_weighted<ALGO>()) wv = *reinterpret_cast<const uint4*>(wts + e0);
-    // locate the tile of e0: last t in [t0, t1] with tile_ptr[t] <= e0
-    uint32_t t = t0;
-    if (tile_ptr[t + 1] <= e0) {
-      uint32_t lo = t0, hi = t1;
-      while (lo < hi) {
-        uint32_t mid = lo + ((hi - lo + 1) >> 1);
-        if (tile_ptr[mid] <= e0) lo = mid;
-        else hi = mid - 1;
-      }
-      t = lo;
-    }
-    unsigned long long tend = tile_ptr[t + 1];
-    const uint32_t evk[4] = {ev.x, ev.y, ev.z, ev.w};
-    const uint32_t wvk[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t e = e0 + k;
-      if (e >= E) break;
-      while (tend <= e) {
-        ++t;
-        tend = tile_ptr[t + 1];
-      }
-      const uint32_t x = t >> lT, y = t & ymask;
-      if (adaptive && rows_cur[x] == 0) continue;
-      const uint32_t u = (x << lvpt) | (evk[k] >> 16);
-      if (adaptive && !((fa[u >> 5] >> (u & 31)) & 1u)) continue;
-      const uint32_t uv = async ? __ldcg(next + u) : cur[u];
-      if (uv == kInf) continue;
-      const uint32_t cand = mp_cand<ALGO>(uv, wvk[k]);
-      if (cand == kInf) continue;
-      const uint32_t v = (y << lvpt) | (evk[k] & 0xFFFFu);
-      if (cand < __ldcg(next + v)) {
-        uint32_t old = atomicMin(next + v, cand);
-        if (cand < old) atomicOr(ch + (v >> 5), 1u << (v & 31));
-      }
-    }
-  }
+  for (uint64_t c = warp; c < nchunks; c += nwarps) scanned += dense_chunk<ALGO, false>(jd, sd, c, p, adaptive);
   // edges-scanned counter
   __shared__ unsigned long long s_sc[GATHER_T / 32];
-  if (lane == 0) s_sc[threadIdx.x >> 5] = scanned;
+  if ((threadIdx.x & 31) == 0) s_sc[threadIdx.x >> 5] = scanned;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long s = 0;
@@ -801,17 +816,301 @@ __global__ void __launch_bounds__(256, 4) gather_sparse_chunks(const JobDesc* __
   if (lane == 0 && scanned) atomicAdd(&ls->edges_scanned, scanned);
 }
 
+// ---- small rounds in one cluster ---------------------------------------------------
+// Rounds whose work is small next to the launches of a grid-wide round (pick_mode: mode 2)
+// run back to back in one launch of one thread-block cluster: gather, apply and control
+// steps are separated by cluster barriers instead of kernel boundaries, and the kernel
+// goes on until the run ends or a round is no longer small. Same rounds, values and
+// counters as the grid-wide kernels. The time of such a round is its chain of dependent
+// L2 accesses (about 0.6 us each), so loads that do not depend on one another are issued
+// together, the directory searches probe eight ways (sp_narrow_wide), the items are spread
+// over every warp, the changed words are first collected in shared memory so that each is
+// applied by a thread of its own, and the round's totals live in CTA 0's shared memory. A
+// round reads what other CTAs wrote in the same launch through L2 (the PERSIST load policy).
+// SM_ROUNDS bounds one launch.
+constexpr int SM_CL = 16, SM_T = 512;  // CTAs (8 where a cluster of 16 does not fit)
+constexpr int SM_ILP = 4;
+constexpr uint32_t SM_LIST = 2048;
+constexpr uint32_t SM_ROUNDS = 1u << 14;
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// The address of CTA 0's copy of a shared variable.
+template <class T>
+__device__ __forceinline__ T* cta0(T* p) {
+  T* r;
+  asm volatile("mapa.u64 %0, %1, 0;" : "=l"(r) : "l"(p));
+  return r;
+}
+
+// A small round's totals, by the parity of the round they open.
+struct SmallTotals {
+  unsigned long long teps[2];
+  unsigned active[2], nact[2], est[2];
+};
+
+// One changed word of a small round: copies its values, lists it and counts its row.
+__device__ __forceinline__ void small_word(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                           unsigned pw, uint32_t i, uint32_t w, unsigned slot, unsigned& cnt,
+                                           unsigned long long& teps, unsigned& est) {
+  const uint32_t lvpt = sd->lvpt, lT = sd->lT;
+  const uint64_t v0 = (uint64_t)i << 5;
+  const unsigned pc = __popc(w);
+  const unsigned long long* cm = (sd->cmask && pc <= 4) ? sd->cmask + v0 : nullptr;
+  // the values, degrees and masks of up to four vertices and the row's count in flight
+  // together; a word with more copies its 32 values (unchanged vertices hold next == current)
+  const bool wide = pc > 4 && v0 + 32 <= sd->n;
+  uint32_t b[4], nv[4], od[4];
+  unsigned long long cols[4];
+  uint32_t bits = wide ? 0u : w;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    b[k] = bits ? (uint32_t)(__ffs(bits) - 1) : 32u;
+    bits &= bits - 1;
+    nv[k] = b[k] < 32 ? __ldcg(jd->next + v0 + b[k]) : 0u;
+    od[k] = b[k] < 32 ? __ldcg(sd->out_deg + v0 + b[k]) : 0u;
+    cols[k] = (cm && b[k] < 32) ? cm[b[k]] : 0ULL;
+  }
+  unsigned* rows_w = jd->rows + pw * sd->T;
+  if (lvpt >= 5) {  // the word lies in one row
+    const uint64_t x = v0 >> lvpt;
+    const unsigned long long r0 = sd->tile_ptr[x << lT], r1 = sd->tile_ptr[(x + 1) << lT];
+    if (atomicAdd(&rows_w[x], pc) == 0) teps += r1 - r0;
+  } else {
+    for (uint32_t m = w; m;) {
+      const uint64_t x = (v0 + (__ffs(m) - 1)) >> lvpt;
+      const uint32_t last = (uint32_t)(((x + 1) << lvpt) - v0);  // the word's bits below it lie in rows <= x
+      const uint32_t mrow = last < 32 ? m & ((1u << last) - 1u) : m;
+      m &= ~mrow;
+      if (atomicAdd(&rows_w[x], (unsigned)__popc(mrow)) == 0) teps += row_edges(sd, x);
+    }
+  }
+  jd->fa[i] = w;
+  jd->ch[i] = 0;
+  unsigned long long e = 0;
+  if (wide) {
+    const uint4* src = reinterpret_cast<const uint4*>(jd->next + v0);
+    uint4* dst = reinterpret_cast<uint4*>(jd->cur + v0);
+    uint4 q[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) q[k] = __ldcg(src + k);
+    e = word_edges(sd, i, w);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) dst[k] = q[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (b[k] < 32) jd->cur[v0 + b[k]] = nv[k];
+    e += od[k];
+  }
+  while (bits) {  // fewer than 32 vertices
+    const uint32_t c = (uint32_t)(__ffs(bits) - 1);
+    bits &= bits - 1;
+    const uint32_t val = __ldcg(jd->next + v0 + c);
+    e += __ldcg(sd->out_deg + v0 + c);
+    jd->cur[v0 + c] = val;
+  }
+  jd->aw[slot] = i;
+  jd->awm[slot] = cm ? (cols[0] | cols[1] | cols[2] | cols[3]) : ~0ULL;
+  est = (unsigned)(est + e < EST_MAX ? est + e : EST_MAX);
+  cnt += pc;
+}
+
+template <int ALGO>
+__global__ void __launch_bounds__(SM_T, 1)
+    small_rounds_kernel(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd, int adaptive,
+                        unsigned max_rounds, int initial, unsigned max_iter_arg, cudaGraphConditionalHandle h,
+                        int use_handle) {
+  __shared__ uint32_t s_word[SM_LIST], s_bits[SM_LIST];
+  __shared__ unsigned s_n, s_cnt, s_est;
+  __shared__ unsigned long long s_teps;
+  __shared__ SmallTotals s_tot;  // CTA 0's is the cluster's
+  LoopState* ls = jd->ls;
+  volatile LoopState* vls = ls;
+  // a whole run (initial) starts here, with the seeding apply; else the same exit in every
+  // CTA: nothing writes these words before the first barrier
+  if (!initial && (!vls->cont || vls->mode != 2)) return;
+  SmallTotals* tot = cta0(&s_tot);
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank(), ncta = cluster_size();
+  const uint32_t tid = rank * SM_T + threadIdx.x, nthr = ncta * SM_T;
+  const uint32_t warp = tid >> 5, nwarps = nthr / 32;
+  // frontier words are dealt out by sectors of 8, so that few words still spread over the CTAs
+  const uint32_t wtid = ((threadIdx.x >> 3) * ncta + rank) * 8 + (threadIdx.x & 7u);
+  const uint32_t nwords = (uint32_t)((sd->n + 31) >> 5);
+  const uint64_t E = sd->E, T = sd->T;
+  const unsigned max_iter = initial ? max_iter_arg : vls->max_iter;
+  const bool listed = sd->dir_ok && sd->adaptive;
+  unsigned iter = initial ? 0u : vls->iter;
+  if (initial) {
+    for (uint32_t i = tid; i < 2 * T; i += nthr) jd->rows[i] = 0;
+    if (tid == 0) {
+      minprop_begin_state(ls, max_iter);
+      s_tot.active[0] = s_tot.nact[0] = s_tot.est[0] = 0;
+      s_tot.teps[0] = 0;
+    }
+  } else if (tid == 0) {
+    const unsigned p = iter & 1u;
+    s_tot.active[p] = vls->active[p];
+    s_tot.nact[p] = vls->nact_words[p];
+    s_tot.est[p] = vls->est[p];
+    s_tot.teps[p] = vls->teps[p];
+  }
+  unsigned long long scanned = 0, active_total = 0, count_edges = 0;
+  uint32_t nread = 0, rounds = 0;
+  unsigned cont = 1, mode = 2;
+  cluster_barrier();  // the totals are there, and every CTA has read the loop state
+  unsigned nact = 0, est0 = 0;
+  if (!initial) {
+    nact = *(volatile unsigned*)&tot->nact[iter & 1u];
+    est0 = *(volatile unsigned*)&tot->est[iter & 1u];
+  }
+  bool seeding = initial != 0;
+  do {
+    const unsigned p = iter & 1u, pw = seeding ? 0u : p ^ 1u;
+    if (seeding) {
+      // no gather before the seeding apply
+    } else {
+      // opens the round: the next round's row counts and totals start at zero
+      for (uint32_t i = tid; i < T; i += nthr) jd->rows[pw * T + i] = 0;
+      if (tid == 0) {
+        count_edges += adaptive ? s_tot.teps[p] : E;
+        s_tot.active[pw] = s_tot.nact[pw] = s_tot.est[pw] = 0;
+        s_tot.teps[pw] = 0;
+      }
+      if (listed && (E > SMALL_E || (uint64_t)est0 * 8 <= E)) {
+        const uint64_t items = (uint64_t)nact << sd->lT;
+        const uint32_t groups = (uint32_t)((items + 31) / 32);
+        uint32_t nslice = 1;
+        while (nslice < 8 && groups * nslice * 2 <= nwarps) nslice *= 2;
+        const uint32_t slice = warp % nslice;
+        for (uint64_t g = (uint64_t)(warp / nslice) * 32; g < items; g += (uint64_t)(nwarps / nslice) * 32)
+          scanned += sparse_group<ALGO, true, SM_ILP, true>(jd, sd, g, items, nread, slice, nslice);
+        cluster_barrier();
+        uint64_t nq = __ldcg(&ls->spq_count);
+        if (nq) {  // the same in every CTA: the queue is complete and CTA 0 resets it past the next barrier
+          if (nq > jd->spq_cap) nq = jd->spq_cap;
+          for (uint64_t q = warp; q < nq; q += nwarps) scanned += sparse_chunk<ALGO, true>(jd, sd, q, items);
+          cluster_barrier();
+          if (tid == 0) ls->spq_count = 0;
+        }
+      } else {
+        for (uint64_t c = warp; c < sd->nchunks; c += nwarps)
+          scanned += dense_chunk<ALGO, true>(jd, sd, c, p, adaptive);
+        cluster_barrier();
+      }
+    }
+    // apply: the changed words, and the words of the old frontier that did not change
+    if (threadIdx.x == 0) s_n = s_cnt = s_est = 0, s_teps = 0;
+    __syncthreads();
+    unsigned cnt = 0, est = 0;
+    unsigned long long teps = 0;
+    for (uint32_t base = wtid; base < nwords; base += 8 * nthr) {
+      uint32_t w[8], f[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t i = base + (uint32_t)k * nthr;
+        w[k] = i < nwords ? __ldcg(jd->ch + i) : 0u;
+        f[k] = i < nwords ? __ldcg(jd->fa + i) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t i = base + (uint32_t)k * nthr;
+        if (w[k]) {
+          const unsigned at = atomicAdd(&s_n, 1u);
+          if (at < SM_LIST) {
+            s_word[at] = i;
+            s_bits[at] = w[k];
+          } else {  // more changed words than the list holds: applied here
+            small_word(jd, sd, pw, i, w[k], atomicAdd(&tot->nact[pw], 1u), cnt, teps, est);
+          }
+        } else if (f[k]) {
+          jd->fa[i] = 0;
+        }
+      }
+    }
+    __syncthreads();
+    const unsigned nlist = min(s_n, SM_LIST);
+    for (unsigned base = 0; base < nlist; base += SM_T) {
+      const unsigned k = base + threadIdx.x;
+      const bool mine = k < nlist;
+      const unsigned m = __ballot_sync(0xFFFFFFFFu, mine);
+      unsigned slot = 0;
+      if (m && lane == 0) slot = atomicAdd(&tot->nact[pw], (unsigned)__popc(m));
+      slot = __shfl_sync(0xFFFFFFFFu, slot, 0) + lane;
+      if (mine) small_word(jd, sd, pw, s_word[k], s_bits[k], slot, cnt, teps, est);
+    }
+    if (cnt) {
+      atomicAdd(&s_cnt, cnt);
+      atomicAdd(&s_est, est);  // at most SM_T * EST_MAX
+      if (teps) atomicAdd(&s_teps, teps);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_cnt) {
+      atomicAdd(&tot->active[pw], s_cnt);
+      atomicAdd(&tot->est[pw], min(s_est, EST_MAX));
+      if (s_teps) atomicAdd(&tot->teps[pw], s_teps);
+    }
+    cluster_barrier();
+    // control (control_step), decided alike by every thread; thread 0 records it at the end
+    iter += seeding ? 0u : 1u;
+    seeding = false;
+    ++rounds;
+    const unsigned active = *(volatile unsigned*)&tot->active[pw];
+    nact = *(volatile unsigned*)&tot->nact[pw];
+    est0 = *(volatile unsigned*)&tot->est[pw];
+    mode = pick_mode(jd, sd, nact, est0, 1);
+    active_total += active;
+    cont = (active > 0 && iter < max_iter) ? 1u : 0u;
+  } while (cont && mode == 2 && rounds < max_rounds);
+  cluster_barrier();  // CTA 0's totals stay until every CTA has read them
+  if (tid == 0) {
+    const unsigned p = iter & 1u;
+    ls->iter = iter;
+    ls->active[p] = s_tot.active[p];
+    ls->nact_words[p] = s_tot.nact[p];
+    ls->est[p] = s_tot.est[p];
+    ls->teps[p] = s_tot.teps[p];
+    ls->count_edges += count_edges;
+    ls->active_total += active_total;
+    ls->cont = cont;
+    ls->mode = mode;
+    if (use_handle) cudaGraphSetConditional(h, cont);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    scanned += __shfl_xor_sync(0xFFFFFFFFu, scanned, o);
+    nread += __shfl_xor_sync(0xFFFFFFFFu, nread, o);
+  }
+  if (lane == 0 && scanned) atomicAdd(&ls->edges_scanned, scanned);
+  if (lane == 0 && nread) atomicAdd(&ls->items_read, (unsigned long long)nread);
+}
+
 // ---- job state -----------------------------------------------------------
 
+// The start vertex of BFS / SSSP / SSWP: next = 0 and changed, so the seeding apply activates
+// it (examples/bfs.cc:193-196; for SSSP the start distance the reference never sets,
+// examples/sssp.cc:197-202).
 __global__ void init_minprop_kernel(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                    int algo) {
+                                    int algo, unsigned long long start) {
   const uint64_t n = sd->n;
   const uint64_t nwords = (n + 31) >> 5;
   uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     uint32_t val = (algo == CYTOM_ALGO_CC) ? (uint32_t)v : kInf;
     jd->cur[v] = val;
-    jd->next[v] = val;
+    jd->next[v] = (algo != CYTOM_ALGO_CC && v == start) ? 0u : val;
   }
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nwords; i += stride) {
     jd->fa[i] = 0;
@@ -819,17 +1118,11 @@ __global__ void init_minprop_kernel(const JobDesc* __restrict__ jd, const StoreD
     if (algo == CYTOM_ALGO_CC) {
       uint64_t rem = n - (i << 5);
       m = rem >= 32 ? 0xFFFFFFFFu : ((1u << rem) - 1u);
+    } else if (i == (start >> 5)) {
+      m = 1u << (start & 31);
     }
     jd->ch[i] = m;
   }
-}
-
-// BFS / SSSP start vertex: next = 0 and changed, so the seeding apply activates it
-// (examples/bfs.cc:193-196; for SSSP the start distance the reference never sets,
-// examples/sssp.cc:197-202).
-__global__ void init_start_kernel(const JobDesc* __restrict__ jd, unsigned long long s) {
-  jd->next[s] = 0;
-  jd->ch[s >> 5] |= 1u << (s & 31);
 }
 
 // edgeChanged(INSERT) for a batch (examples/bfs.cc:115-140, cc.cc:113-131,
@@ -977,12 +1270,8 @@ int minprop_alloc(Ctx* c, Job* j) {
 
 int minprop_init(Ctx* c, Job* j) {
   int algo = j->algo;
-  init_minprop_kernel<<<grid_persistent(c, 8), 256, 0, c->stream>>>(j->d, c->dsd, algo);
+  init_minprop_kernel<<<grid_persistent(c, 8), 256, 0, c->stream>>>(j->d, c->dsd, algo, j->params.start_vertex);
   c->launches++;
-  if (algo != CYTOM_ALGO_CC) {
-    init_start_kernel<<<1, 1, 0, c->stream>>>(j->d, j->params.start_vertex);
-    c->launches++;
-  }
   return cuda_err(c, cudaGetLastError(), "init_minprop");
 }
 
@@ -1115,6 +1404,54 @@ static GatherLaunch gather_launch(Ctx* c, int algo) {
   return stream_launch(c, a, sg_variant(c, algo));
 }
 
+static void* small_fn(int algo) {
+  return algo == CYTOM_ALGO_BFS    ? (void*)small_rounds_kernel<0>
+         : algo == CYTOM_ALGO_CC   ? (void*)small_rounds_kernel<1>
+         : algo == CYTOM_ALGO_SSWP ? (void*)small_rounds_kernel<3>
+                                   : (void*)small_rounds_kernel<2>;
+}
+
+// CTAs of the cluster: SM_CL where the device can hold one such cluster of `fn`, else 8.
+static unsigned small_cluster(void* fn) {
+  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = SM_CL;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(SM_CL);
+  cfg.blockDim = dim3(SM_T);
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) return SM_CL;
+  cudaGetLastError();
+  return 8;
+}
+
+static cudaError_t launch_small(Ctx* c, Job* j, int adaptive, unsigned max_rounds, int initial, unsigned max_iter) {
+  void* fn = small_fn(j->algo);
+  const unsigned cl = small_cluster(fn);
+  const JobDesc* jd = j->d;
+  const StoreDesc* sd = c->dsd;
+  cudaGraphConditionalHandle h{};
+  int zero = 0;
+  void* args[] = {(void*)&jd,      (void*)&sd,       (void*)&adaptive, (void*)&max_rounds,
+                  (void*)&initial, (void*)&max_iter, (void*)&h,        (void*)&zero};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cl;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cl);
+  cfg.blockDim = dim3(SM_T);
+  cfg.stream = c->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  c->launches++;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 static int launch_gather(Ctx* c, Job* j, int adaptive) {
   GatherLaunch g = gather_launch(c, j->algo);
   const JobDesc* jd = j->d;
@@ -1135,6 +1472,15 @@ static int resident_grid(Ctx* c, void* fn, int threads) {
     per_sm = 1;
   }
   return c->num_sms * per_sm;
+}
+
+// The apply's grid: one wave of resident blocks, and no more than the frontier has words for
+// (every block counts itself in at the round's end: 2^18 vertices need 32 blocks, and with
+// one wave of 1,216 an apply took 8 us there).
+static int apply_grid(Ctx* c) {
+  const uint64_t nwords = (c->n + 31) / 32;
+  const uint64_t need = std::max<uint64_t>((nwords + APPLY_T - 1) / APPLY_T, 1);
+  return (int)std::min<uint64_t>((uint64_t)resident_grid(c, (void*)apply_minprop_kernel, APPLY_T), need);
 }
 
 static void* sparse_fn(int algo) {
@@ -1164,9 +1510,13 @@ static cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGr
   return cudaGraphAddKernelNode(node, g, deps, ndeps, &kp);
 }
 
-// Graph: begin -> seeding apply + control -> while(cont) { dense gather -> sparse gather ->
-// chunk pass -> apply + control }. Dense and sparse are picked on the device per round;
-// the kernels not needed exit at once (measured cheaper than conditional IF nodes around
+// A run on a graph of at most SMALL_E edges is one launch of the cluster, begin and seeding
+// apply included: pick_mode keeps every round of it small.
+static bool whole_run_small(const Ctx* c) { return c->E <= SMALL_E && (c->n + 31) / 32 <= SMALL_WORDS; }
+
+// Graph: begin -> seeding apply + control -> while(cont) { small rounds -> dense gather ->
+// sparse gather -> chunk pass -> apply + control }. The kind of round is picked on the device
+// per round (pick_mode); the kernels not needed exit at once (measured cheaper than conditional IF nodes around
 // them: 182-189 vs 166 GTEPS on the RMAT-22 stream).
 static int build_minprop_graph(Ctx* c, Job* j) {
   cudaGraph_t g = nullptr;
@@ -1179,10 +1529,10 @@ static int build_minprop_graph(Ctx* c, Job* j) {
   unsigned max_iter = (unsigned)std::min<uint64_t>(j->params.max_iterations, 0xFFFFFFFFu);
   int adaptive = c->cfg.enable_adaptive_scheduling;
   int zero = 0, one = 1;
-  const int g_apply = resident_grid(c, (void*)apply_minprop_kernel, APPLY_T);
+  const int g_apply = apply_grid(c);
   const int g_sparse = resident_grid(c, sparse_fn(j->algo), 256);
   const int g_chunks = resident_grid(c, chunks_fn(j->algo), 256);
-  cudaGraphNode_t n_begin, n_apply0, n_while, b_apply, d_gather, s_sparse, c_chunks;
+  cudaGraphNode_t n_begin, n_apply0, n_while, b_small, b_apply, d_gather, s_sparse, c_chunks;
   void* a_begin[] = {(void*)&jd, (void*)&sd, (void*)&max_iter};
   if (e == cudaSuccess)
     e = add_kernel(g, &n_begin, nullptr, 0, (void*)begin_kernel, dim3(std::max(1, c->num_sms)), dim3(256), a_begin);
@@ -1197,9 +1547,20 @@ static int build_minprop_graph(Ctx* c, Job* j) {
   if (e == cudaSuccess) e = cudaGraphAddNode(&n_while, g, &n_apply0, nullptr, 1, &cp);
   if (e == cudaSuccess) {
     cudaGraph_t body = cp.conditional.phGraph_out[0];
+    unsigned max_rounds = SM_ROUNDS;
+    void* a_s[] = {(void*)&jd,   (void*)&sd,       (void*)&adaptive, (void*)&max_rounds,
+                   (void*)&zero, (void*)&max_iter, (void*)&h,        (void*)&one};
+    const unsigned cl = small_cluster(small_fn(j->algo));
+    e = add_kernel(body, &b_small, nullptr, 0, small_fn(j->algo), dim3(cl), dim3(SM_T), a_s);
+    if (e == cudaSuccess) {
+      cudaLaunchAttributeValue av{};
+      av.clusterDim.x = cl;
+      av.clusterDim.y = av.clusterDim.z = 1;
+      e = cudaGraphKernelNodeSetAttribute(b_small, cudaLaunchAttributeClusterDimension, &av);
+    }
     void* a_g[] = {(void*)&jd, (void*)&sd, (void*)&adaptive};
     GatherLaunch gl = gather_launch(c, j->algo);
-    e = add_kernel(body, &d_gather, nullptr, 0, gl.fn, gl.grid, gl.block, a_g, gl.smem);
+    if (e == cudaSuccess) e = add_kernel(body, &d_gather, &b_small, 1, gl.fn, gl.grid, gl.block, a_g, gl.smem);
     if (e == cudaSuccess)
       e = add_kernel(body, &s_sparse, &d_gather, 1, sparse_fn(j->algo), dim3(g_sparse), dim3(256), a_g);
     void* a_q[] = {(void*)&jd, (void*)&sd};
@@ -1249,6 +1610,12 @@ static double round_bytes(const Ctx* c, const LoopState& a, const LoopState& b, 
 int minprop_run(Ctx* c, Job* j) {
   int adaptive = c->cfg.enable_adaptive_scheduling;
   unsigned max_iter = (unsigned)std::min<uint64_t>(j->params.max_iterations, 0xFFFFFFFFu);
+  if (!c->profiling && use_graphs() && whole_run_small(c)) {
+    j->last_run_graph = false;
+    // a run converges within n rounds, each of them bounded
+    cudaError_t e = launch_small(c, j, adaptive, 0xFFFFFFFFu, 1, max_iter);
+    return cuda_err(c, e, "small run");
+  }
   if (!c->profiling && use_graphs() && !j->graph_failed) {
     if (j->loop_exec && j->graph_epoch != c->tune_epoch) {
       cudaGraphExecDestroy(j->loop_exec);
@@ -1268,7 +1635,7 @@ int minprop_run(Ctx* c, Job* j) {
   }
   // host-driven loop (profiling mode or no graph support)
   j->last_run_graph = false;
-  const int g_apply = resident_grid(c, (void*)apply_minprop_kernel, APPLY_T);
+  const int g_apply = apply_grid(c);
   const int g_sparse = resident_grid(c, sparse_fn(j->algo), 256);
   const int g_chunks = resident_grid(c, chunks_fn(j->algo), 256);
   begin_kernel<<<std::max(1, c->num_sms), 256, 0, c->stream>>>(j->d, c->dsd, max_iter);
@@ -1295,6 +1662,16 @@ int minprop_run(Ctx* c, Job* j) {
       prev_slot = -1;
       if (!snap.cont) break;
       prev = snap;
+      if (snap.mode == 2) {
+        // a small round with its apply and control: one launch, one round
+        int s1 = prof_begin(c, KC_OTHER);
+        e = launch_small(c, j, adaptive, 1, 0, max_iter);
+        prof_end(c, s1, 0.0);
+        prev_slot = s1;
+        if (e != cudaSuccess) return cuda_err(c, e, "small round");
+        ++round;
+        continue;
+      }
       if (snap.mode == 0) {
         int s1 = prof_begin(c, KC_GATHER);
         int rc = launch_gather(c, j, adaptive);
@@ -1320,6 +1697,8 @@ int minprop_run(Ctx* c, Job* j) {
     }
     // launch a few rounds before checking: kernels are no-ops once the run ended
     for (int k = 0; k < 4 && round < max_iter; ++k, ++round) {
+      e = launch_small(c, j, adaptive, SM_ROUNDS, 0, max_iter);
+      if (e != cudaSuccess) return cuda_err(c, e, "small rounds");
       int rc = launch_gather(c, j, adaptive);
       if (rc) return rc;
       e = cudaLaunchKernel(sparse_fn(j->algo), dim3(g_sparse), dim3(256), a_g, 0, c->stream);
@@ -1497,7 +1876,7 @@ int minprop_autotune(Ctx* c) {
     c->tune_div[cls] = 0;
     if (e == cudaSuccess && c->hsd.dir_ok && c->cfg.enable_adaptive_scheduling && !sparse_div_from_env()) {
       GatherLaunch gd = stream_launch(c, algo, best);
-      const int g_apply = resident_grid(c, (void*)apply_minprop_kernel, APPLY_T);
+      const int g_apply = apply_grid(c);
       const int g_sparse = resident_grid(c, sparse_fn(algo), 256);
       const int g_chunks = resident_grid(c, chunks_fn(algo), 256);
       void* a_q[] = {(void*)&jd, (void*)&sd};

@@ -100,6 +100,7 @@ __device__ __forceinline__ void round_open(const JobDesc* __restrict__ jd, const
     ls->active[p ^ 1u] = 0;
     ls->nact_words[p ^ 1u] = 0;
     ls->teps[p ^ 1u] = 0;
+    ls->est[p ^ 1u] = 0;
     atomicAdd(&ls->count_edges, adaptive ? ld_plain<PERSIST>(&ls->teps[p]) : sd->E);
   }
 }
@@ -123,6 +124,61 @@ __device__ __forceinline__ unsigned long long word_columns(const StoreDesc* __re
   return m;
 }
 
+// ---- small rounds --------------------------------------------------------
+// A round is small when one thread-block cluster finishes it sooner than the grid-wide
+// kernels, whose four launches cost about 20 us whatever the frontier holds: a graph of at
+// most SMALL_E edges, or a sparse round of at most SMALL_ITEMS (word, column) items whose
+// active vertices have at most SMALL_EDGES out-edges (LoopState::est). The cluster scans the
+// changed bitmap every round, which bounds the vertices (SMALL_WORDS).
+constexpr uint32_t SMALL_E = 1u << 16;
+constexpr uint32_t SMALL_ITEMS = 1u << 13;
+constexpr uint32_t SMALL_EDGES = 1u << 16;
+constexpr uint32_t SMALL_WORDS = 1u << 19;
+constexpr uint32_t EST_MAX = 1u << 20;  // est saturates per block here
+
+// Out-edges of the active vertices of frontier word i (bits w), their degrees in flight
+// together; words past the vertex count (fewer than 32 vertices) one by one.
+__device__ __forceinline__ unsigned word_edges(const StoreDesc* __restrict__ sd, uint64_t i, uint32_t w) {
+  const uint32_t* deg = sd->out_deg + (i << 5);
+  unsigned long long e = 0;
+  if (__popc(w) > 4 && ((i + 1) << 5) <= sd->n) {
+    uint4 q[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) q[k] = __ldcg(reinterpret_cast<const uint4*>(deg) + k);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t m = w >> (4 * k);
+      e += (m & 1u ? q[k].x : 0u);
+      e += (m & 2u ? q[k].y : 0u);
+      e += (m & 4u ? q[k].z : 0u);
+      e += (m & 8u ? q[k].w : 0u);
+    }
+  } else {
+    uint32_t d[4];
+    do {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        d[k] = w ? __ldcg(deg + (__ffs(w) - 1)) : 0u;
+        w &= w - 1;
+      }
+      e += (unsigned long long)d[0] + d[1] + d[2] + d[3];
+    } while (w);
+  }
+  return (unsigned)(e < EST_MAX ? e : EST_MAX);
+}
+
+// The gather of a round with `nact` listed frontier words.
+__device__ __forceinline__ unsigned pick_mode(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                              unsigned nact, unsigned est, int allow_small) {
+  const uint64_t nwords = (sd->n + 31) >> 5;
+  const bool listed = sd->dir_ok && sd->adaptive;
+  if (allow_small && nwords <= SMALL_WORDS &&
+      (sd->E <= SMALL_E || (listed && ((uint64_t)nact << sd->lT) <= SMALL_ITEMS && est <= SMALL_EDGES)))
+    return 2u;
+  const uint32_t div = jd->sparse_div ? jd->sparse_div : sd->sparse_div;
+  return (listed && (uint64_t)nact * div <= nwords) ? 1u : 0u;
+}
+
 // ---- apply ---------------------------------------------------------------
 // One apply step of a block: thread t handles frontier word base + t (base a multiple
 // of 32). `initial` apply = the seeding apply before round 0 (writes parity 0).
@@ -133,7 +189,8 @@ __device__ __forceinline__ unsigned long long word_columns(const StoreDesc* __re
 // words are listed (warp-ballot compaction) for sparse rounds.
 template <bool PERSIST>
 __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                           unsigned pw, uint64_t base, unsigned& cnt, unsigned long long& teps) {
+                                           unsigned pw, uint64_t base, unsigned& cnt, unsigned long long& teps,
+                                           unsigned& est) {
   LoopState* ls = jd->ls;
   const uint64_t n = sd->n, T = sd->T;
   const uint32_t lvpt = sd->lvpt;
@@ -186,6 +243,8 @@ __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const
         const unsigned slot = slot0 + __popc(nz & ((1u << lane) - 1u));
         jd->aw[slot] = (uint32_t)i;
         jd->awm[slot] = word_columns(sd, i, w);
+        // past this many words the round is not a small one whatever the estimate
+        if (!PERSIST && slot < (SMALL_ITEMS >> sd->lT) + 1u) est = min(est + word_edges(sd, i, w), EST_MAX);
       }
     }
   }
@@ -214,29 +273,35 @@ __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const
 }
 
 // Block reduction of the apply counters into the loop state (every thread calls it).
-__device__ __forceinline__ void apply_flush(LoopState* ls, unsigned pw, unsigned cnt, unsigned long long teps) {
-  __shared__ unsigned s_cnt[APPLY_T / 32];
-  __shared__ unsigned long long s_teps[APPLY_T / 32];
+template <int T>
+__device__ __forceinline__ void apply_flush(LoopState* ls, unsigned pw, unsigned cnt, unsigned long long teps,
+                                            unsigned est) {
+  __shared__ unsigned s_cnt[T / 32], s_est[T / 32];
+  __shared__ unsigned long long s_teps[T / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
     teps += __shfl_xor_sync(0xFFFFFFFFu, teps, o);
+    est = min(est + __shfl_xor_sync(0xFFFFFFFFu, est, o), EST_MAX);
   }
   const unsigned wid = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     s_cnt[wid] = cnt;
     s_teps[wid] = teps;
+    s_est[wid] = est;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned c = 0;
+    unsigned c = 0, e = 0;
     unsigned long long t = 0;
-    for (int k = 0; k < APPLY_T / 32; ++k) {
+    for (int k = 0; k < T / 32; ++k) {
       c += s_cnt[k];
       t += s_teps[k];
+      e = min(e + s_est[k], EST_MAX);
     }
     if (c) atomicAdd(&ls->active[pw], c);
     if (t) atomicAdd(&ls->teps[pw], t);
+    if (e) atomicAdd(&ls->est[pw], e);
   }
   __syncthreads();
 }
@@ -246,26 +311,30 @@ __device__ __forceinline__ void apply_flush(LoopState* ls, unsigned pw, unsigned
 // run when nothing changed or max_iterations rounds ran, and picks the next round's
 // gather: sparse (directory, only the listed frontier words) while at most 1/sparse_div
 // of the frontier words are non-zero, dense (stream every active row) above.
+// The one-job loops (allow_small) run small rounds in one cluster (pick_mode).
 __device__ __forceinline__ unsigned control_step(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                                 int initial) {
-  volatile LoopState* ls = jd->ls;
-  if (ls->cont) {
-    unsigned iter = ls->iter;
-    unsigned p = 0;
-    if (!initial) {
-      iter += 1;
-      ls->iter = iter;
-      p = iter & 1u;
-    }
-    const unsigned a = ls->active[p];
-    ls->active_total = ls->active_total + a;
-    ls->cont = (a > 0 && iter < ls->max_iter && ls->err == 0) ? 1u : 0u;
-    const uint64_t nwords = (sd->n + 31) >> 5;
-    const uint32_t div = jd->sparse_div ? jd->sparse_div : sd->sparse_div;
-    ls->mode = (sd->dir_ok && sd->adaptive && (uint64_t)ls->nact_words[p] * div <= nwords) ? 1u : 0u;
-    ls->spq_count = 0;
-  }
-  return ls->cont;
+                                                 int initial, int allow_small) {
+  // every word the step reads is loaded before any is used (one L2 round trip); the other
+  // blocks' totals are complete and visible when it runs
+  LoopState* ls = jd->ls;
+  const unsigned was = __ldcg(&ls->cont), it0 = __ldcg(&ls->iter), max_iter = __ldcg(&ls->max_iter);
+  const unsigned err = __ldcg(&ls->err);
+  const unsigned act[2] = {__ldcg(&ls->active[0]), __ldcg(&ls->active[1])};
+  const unsigned nact[2] = {__ldcg(&ls->nact_words[0]), __ldcg(&ls->nact_words[1])};
+  const unsigned est[2] = {__ldcg(&ls->est[0]), __ldcg(&ls->est[1])};
+  const unsigned long long total = __ldcg(&ls->active_total);
+  if (!was) return 0u;
+  const unsigned iter = initial ? it0 : it0 + 1;
+  const unsigned p = initial ? 0u : (iter & 1u);
+  const unsigned a = act[p];
+  const unsigned cont = (a > 0 && iter < max_iter && err == 0) ? 1u : 0u;
+  volatile LoopState* vls = ls;
+  vls->iter = iter;
+  vls->active_total = total + a;
+  vls->cont = cont;
+  vls->mode = pick_mode(jd, sd, nact[p], est[p], allow_small);
+  vls->spq_count = 0;
+  return cont;
 }
 
 // The loop state of a BFS / CC / SSSP / SSWP run before its first round (one thread).
@@ -285,6 +354,7 @@ __device__ __forceinline__ void minprop_begin_state(LoopState* ls, unsigned max_
   ls->apply_done = 0;
   ls->sel_rounds = 0;
   ls->items_read = 0;
+  ls->est[0] = ls->est[1] = 0;
 }
 
 // ---- dense gather: one stage of SG_T * EPT edges ---------------------------
@@ -526,35 +596,38 @@ __device__ __forceinline__ SpItem sp_item(const JobDesc* __restrict__ jd, const 
   return sp_item_at<PERSIST>(jd, sd, w, (uint32_t)(it & (sd->T - 1)));
 }
 
-// Relaxes SP_ILP edges per lane whose sources are in their item's frontier word; the
-// loads of all SP_ILP edges are issued before any of them is used.
-template <int ALGO, bool PERSIST>
+// Relaxes ILP edges per lane whose sources are in their item's frontier word; the
+// loads of all ILP edges are issued before any of them is used.
+// LAT: a target's value is loaded beside the source's, for every edge with an active source
+// (one dependent step less; otherwise only for edges that offer a value).
+template <int ALGO, bool PERSIST, int ILP, bool LAT = false>
 __device__ __forceinline__ void sp_batch(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                         const uint32_t (&xs)[SP_ILP], const uint32_t (&ys)[SP_ILP],
-                                         const uint32_t (&bits)[SP_ILP], const unsigned long long (&pos)[SP_ILP],
+                                         const uint32_t (&xs)[ILP], const uint32_t (&ys)[ILP],
+                                         const uint32_t (&bits)[ILP], const unsigned long long (&pos)[ILP],
                                          uint32_t valid) {
   const uint32_t lvpt = sd->lvpt;
   const bool async = jd->async != 0;
-  uint32_t pk[SP_ILP], wv[SP_ILP], cand[SP_ILP], nv[SP_ILP];
+  uint32_t pk[ILP], wv[ILP], cand[ILP], nv[ILP];
 #pragma unroll
-  for (int k = 0; k < SP_ILP; ++k) pk[k] = ((valid >> k) & 1u) ? sd->edges[pos[k]] : 0u;
+  for (int k = 0; k < ILP; ++k) pk[k] = ((valid >> k) & 1u) ? sd->edges[pos[k]] : 0u;
   // the weight is read only for an edge whose source is in the frontier, beside its
   // source value (one dependent step, as before; most listed edges have inactive sources)
 #pragma unroll
-  for (int k = 0; k < SP_ILP; ++k) {
+  for (int k = 0; k < ILP; ++k) {
     const uint32_t sl = pk[k] >> 16;
     const bool act = ((valid >> k) & 1u) && ((bits[k] >> (sl & 31)) & 1u);
     cand[k] = act ? ld_src<PERSIST>(jd, async, (xs[k] << lvpt) | sl) : kInf;
     wv[k] = (mp_weighted<ALGO>() && act) ? sd->wts[pos[k]] : 0u;
+    if (LAT) nv[k] = act ? ld_next<PERSIST>(jd->next + ((ys[k] << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
   }
 #pragma unroll
-  for (int k = 0; k < SP_ILP; ++k)
+  for (int k = 0; k < ILP; ++k)
     if (cand[k] != kInf) cand[k] = mp_cand<ALGO>(cand[k], wv[k]);
 #pragma unroll
-  for (int k = 0; k < SP_ILP; ++k)
+  for (int k = 0; k < ILP && !LAT; ++k)
     nv[k] = (cand[k] != kInf) ? ld_next<PERSIST>(jd->next + ((ys[k] << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
 #pragma unroll
-  for (int k = 0; k < SP_ILP; ++k) {
+  for (int k = 0; k < ILP; ++k) {
     if (cand[k] != kInf && cand[k] < nv[k]) {
       const uint32_t v = (ys[k] << lvpt) | (pk[k] & 0xFFFFu);
       atomicMin(jd->next + v, cand[k]);
@@ -593,13 +666,53 @@ __device__ __forceinline__ void sp_narrow(const StoreDesc* __restrict__ sd, SpIt
   m.hi = top ? m.hi : c0;
 }
 
+// sp_narrow with seven probes of each search per step: a third of the dependent loads, for
+// rounds whose time is their latency.
+__device__ __forceinline__ void sp_narrow_wide(const StoreDesc* __restrict__ sd, SpItem& m) {
+  const uint32_t smin = (m.b << 5) + (uint32_t)(__ffs(m.bits) - 1);
+  const uint32_t smax = (m.b << 5) + (31u - (uint32_t)__clz(m.bits));
+  const uint32_t klo = smin << 16;
+  const bool top = smax == 0xFFFFu;
+  const uint32_t khi = top ? 0u : (smax + 1u) << 16;
+  const uint32_t* e = sd->edges + m.base;
+  uint32_t a0 = m.lo, a1 = m.hi, c0 = m.lo, c1 = top ? m.lo : m.hi;
+  while (a0 < a1 || c0 < c1) {
+    const uint32_t la = a1 - a0, lc = c1 - c0;
+    uint32_t va[7], vc[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      va[k] = la ? e[a0 + ((la * (uint32_t)(k + 1)) >> 3)] : 0u;
+      vc[k] = lc ? e[c0 + ((lc * (uint32_t)(k + 1)) >> 3)] : 0u;
+    }
+    // the probes ascend: the span after the last one below the key, up to the first at or above it
+    uint32_t na = 0, nc = 0;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      na += va[k] < klo ? 1u : 0u;
+      nc += vc[k] < khi ? 1u : 0u;
+    }
+    if (la) {
+      const uint32_t b = a0;
+      if (na < 7) a1 = b + ((la * (na + 1)) >> 3);
+      if (na > 0) a0 = b + ((la * na) >> 3) + 1;
+    }
+    if (lc) {
+      const uint32_t b = c0;
+      if (nc < 7) c1 = b + ((lc * (nc + 1)) >> 3);
+      if (nc > 0) c0 = b + ((lc * nc) >> 3) + 1;
+    }
+  }
+  m.lo = a0;
+  m.hi = top ? m.hi : c0;
+}
+
 // One group of 32 items [g, g + 32) for the calling warp; returns the light edges walked
 // and adds the items whose directory entries it read to `nread` (slice 0 only).
 // With nslice > 1 several warps share the group: each reads the group's items, slice 0
-// alone queues the heavy ones, and the light edges are dealt out in steps of 32 * SP_ILP
+// alone queues the heavy ones, and the light edges are dealt out in steps of 32 * ILP
 // (slice k takes steps k, k + nslice, ...); if the queue overflowed, slice 0 walks every
 // light edge itself (the others' share is then walked twice, which changes nothing).
-template <int ALGO, bool PERSIST>
+template <int ALGO, bool PERSIST, int ILP = SP_ILP, bool WIDE = false>
 __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                                  uint64_t g, uint64_t items, uint32_t& nread,
                                                  uint32_t slice = 0, uint32_t nslice = 1) {
@@ -621,7 +734,8 @@ __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd,
       m = sp_item_at<PERSIST>(jd, sd, w, y);
       len = m.hi > m.lo ? m.hi - m.lo : 0u;
       if (len > SP_NARROW && len <= SP_HEAVY) {
-        sp_narrow(sd, m);
+        if (WIDE) sp_narrow_wide(sd, m);
+        else sp_narrow(sd, m);
         len = m.hi > m.lo ? m.hi - m.lo : 0u;
       }
     }
@@ -644,7 +758,7 @@ __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd,
   }
   const bool walk_all = nslice > 1 && slice == 0 && __any_sync(0xFFFFFFFFu, overflow);
   // light items: the group's edges are numbered 0..total-1 (warp prefix sum over the
-  // items' lengths); lanes take SP_ILP of them per step and find their item by a
+  // items' lengths); lanes take ILP of them per step and find their item by a
   // binary search over the prefix sums held in the lanes
   const uint32_t mine = (len > 0 && !queued) ? len : 0u;
   uint32_t incl = mine;
@@ -655,12 +769,12 @@ __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd,
   }
   const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
   const uint32_t step0 = walk_all ? 0u : slice, nstep = walk_all ? 1u : nslice;
-  for (uint32_t f0 = step0 * 32 * SP_ILP; f0 < total; f0 += nstep * 32 * SP_ILP) {
-    uint32_t xs[SP_ILP], ys[SP_ILP], bits[SP_ILP];
-    unsigned long long pos[SP_ILP];
+  for (uint32_t f0 = step0 * 32 * ILP; f0 < total; f0 += nstep * 32 * ILP) {
+    uint32_t xs[ILP], ys[ILP], bits[ILP];
+    unsigned long long pos[ILP];
     uint32_t valid = 0;
 #pragma unroll
-    for (int k = 0; k < SP_ILP; ++k) {
+    for (int k = 0; k < ILP; ++k) {
       const uint32_t f = f0 + lane + 32u * k;
       // item j holding flattened edge f: the least j with incl[j] > f
       uint32_t j = 0;
@@ -679,7 +793,7 @@ __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd,
       pos[k] = base_j + lo_j + (f - (incl_j - mine_j));
       valid |= (f < total) ? (1u << k) : 0u;
     }
-    sp_batch<ALGO, PERSIST>(jd, sd, xs, ys, bits, pos, valid);
+    sp_batch<ALGO, PERSIST, ILP, WIDE>(jd, sd, xs, ys, bits, pos, valid);
   }
   return slice == 0 ? mine : 0u;
 }
@@ -725,7 +839,7 @@ __device__ __forceinline__ uint32_t sparse_chunk(const JobDesc* __restrict__ jd,
       pos[k] = m.base + ek;
       valid |= (ek < e1) ? (1u << k) : 0u;
     }
-    sp_batch<ALGO, PERSIST>(jd, sd, xs, ys, bits, pos, valid);
+    sp_batch<ALGO, PERSIST, SP_ILP>(jd, sd, xs, ys, bits, pos, valid);
   }
   return lane == 0 ? e1 - e0 : 0u;
 }
