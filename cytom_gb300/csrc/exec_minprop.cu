@@ -198,14 +198,21 @@ __global__ void __launch_bounds__(GATHER_T) gather_minprop_kernel(const JobDesc*
 // its threads resolve the dependent frontier / value / atomic loads of EPT edges each
 // in batches.
 //  - Stages are SG_T * EPT-edge slices of the tile-major edge array. A block owns
-//    groups of 128 / EPT consecutive stages (group g, g + gridDim.x, ...), so
+//    groups of up to 128 / EPT consecutive stages (group g, g + gridDim.x, ...), so
 //    consecutive stages of a block usually lie in one tile row and its frontier words
-//    stay in L1.
+//    stay in L1. A store of few stages is cut into smaller groups, at least
+//    SG_GROUPS_PER_BLOCK for every block.
 //  - A stage whose tile rows are all inactive is skipped without being copied.
 //  - Single-row stages (the common case at large vertices-per-tile) take the source
 //    row from the stage: the frontier test needs no per-edge tile lookup, and only
 //    edges with an active source look up their target tile.
 // The shape (EPT, NST, blocks per SM) is a variant picked by the autotuner.
+// Groups per block from which a block keeps consecutive stages together. Full groups left
+// most blocks without work below some ten million edges (a million edges are 29 groups of 8
+// stages for 304 blocks): sliding-window update 1,731 -> 1,497 us, four programs on 16 M
+// edges 2,561 -> 2,445, RMAT-22 stream 75.2 -> 72.0 ms; 1 group per block 73.4, 4 72.5, 16
+// 72.5, single stages everywhere 72.1 but 11.4 for 10.8 ms on 268 M edges.
+constexpr uint64_t SG_GROUPS_PER_BLOCK = 8;
 template <int ALGO, int EPT, int NST>
 __host__ __device__ constexpr size_t gather_stream_smem() {
   return (size_t)NST * SG_T * EPT * 4 * (mp_weighted<ALGO>() ? 2 : 1) + NST * sizeof(uint64_t);
@@ -216,7 +223,6 @@ __global__ void __launch_bounds__(SG_T, MINB) gather_stream_kernel(const JobDesc
                                                                     const StoreDesc* __restrict__ sd,
                                                                     int adaptive) {
   constexpr uint32_t SE = SG_T * EPT;
-  constexpr int SG_GROUP = 128 / EPT;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   uint32_t* ebuf = reinterpret_cast<uint32_t*>(smem_raw);
   uint32_t* wbuf = ebuf + NST * SE;
@@ -232,12 +238,15 @@ __global__ void __launch_bounds__(SG_T, MINB) gather_stream_kernel(const JobDesc
   const uint64_t E = sd->E;
   const uint64_t nst = (E + SE - 1) / SE;
   const uint64_t G = gridDim.x;
+  int lgrp = 31 - __clz(128 / EPT);  // log2 of the stages per group
+  while (lgrp > 0 && (nst >> lgrp) < G * SG_GROUPS_PER_BLOCK) --lgrp;
+  const uint64_t gmask = (1ULL << lgrp) - 1ULL;
 
-  // the block's stage sequence: groups blockIdx.x, blockIdx.x + G, ... of SG_GROUP stages
+  // the block's stage sequence: groups blockIdx.x, blockIdx.x + G, ... of 2^lgrp stages
   auto advance = [&](uint64_t s) -> uint64_t {
     uint64_t n1 = s + 1;
-    if ((n1 % SG_GROUP) != 0 && n1 < nst) return n1;
-    return (s / SG_GROUP + G) * SG_GROUP;
+    if ((n1 & gmask) != 0 && n1 < nst) return n1;
+    return ((s >> lgrp) + G) << lgrp;
   };
   auto next_active = [&](uint64_t s) -> uint64_t {
     while (s < nst && !stage_active<false, EPT>(jd, sd, s, p, adaptive)) s = advance(s);
@@ -269,7 +278,7 @@ __global__ void __launch_bounds__(SG_T, MINB) gather_stream_kernel(const JobDesc
   uint64_t stq[NST];
   uint64_t s_next = nst;
   if (threadIdx.x == 0) {
-    const uint64_t first = (uint64_t)blockIdx.x * SG_GROUP;
+    const uint64_t first = (uint64_t)blockIdx.x << lgrp;
     uint64_t s0 = next_active(first < nst ? first : nst);
 #pragma unroll
     for (int k = 0; k < NST; ++k) {
