@@ -85,12 +85,14 @@ struct PrState {
   uint64_t seen_version = ~0ULL;
   // WPAGERANK
   double* tele = nullptr;     // teleport vector (NULL = uniform 1/n)
+  float2* tele2 = nullptr;    // the same as float pairs (FP32 form)
   // WPAGERANK adjoint (allocated by the first adjoint call)
   float* lam = nullptr;       // FP32: lambda, double-buffered (2 x n)
   double* lam64 = nullptr;    // FP64: lambda, double-buffered (2 x n)
   float* pt = nullptr;        // (P^T lambda) of the last round
   double* pt64 = nullptr;
-  double* cvec = nullptr;     // loss weights c
+  double* cvec = nullptr;     // loss weights c (FP64 form)
+  float2* cvec2 = nullptr;    // the same as float pairs (FP32 form)
   LoopState* adj_ls = nullptr;
   // captured round loops (one per round kind), rebuilt when their launch arguments change
   cudaGraphExec_t loop_exec[8] = {};
@@ -107,6 +109,7 @@ struct WGraph {
   float* out_w = nullptr;
   uint64_t in_wcap = 0, out_wcap = 0;
   double* wsum = nullptr;
+  float2* wsum2 = nullptr;  // the same as float pairs (FP32 forms)
   uint64_t built_version = ~0ULL;
 };
 
@@ -566,6 +569,16 @@ __global__ void permute_kernel(const T* __restrict__ in, const uint32_t* __restr
   }
 }
 
+// out[perm[v]] = in[v] as an unevaluated float pair
+__global__ void permute_ff_kernel(const double* __restrict__ in, const uint32_t* __restrict__ perm, uint64_t n,
+                                  float2* __restrict__ out) {
+  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+    const FF f = ff_from_double(in[v]);
+    out[perm[v]] = make_float2(f.hi, f.lo);
+  }
+}
+
 // The renumbering, made once per context from the out-degrees of the graph at that time
 // (a later graph keeps it: any numbering gives the same results, this one only packs
 // the sources most edges read into few cache lines).
@@ -815,7 +828,7 @@ void pagerank_ctx_free(Ctx* c) {
   if (g) {
     csc_free(&g->in);
     csc_free(&g->out);
-    void* ptrs[] = {g->in_w, g->out_w, g->wsum};
+    void* ptrs[] = {g->in_w, g->out_w, g->wsum, g->wsum2};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     delete g;
@@ -860,7 +873,7 @@ void pagerank_free(Job* j) {
   for (auto& g : s->loop_exec)
     if (g) cudaGraphExecDestroy(g);
   void* ptrs[] = {s->rank, s->comp, s->delta, s->contrib, s->r64,  s->r64n, s->contrib64, s->lo,
-                  s->tele, s->lam,  s->lam64, s->pt,      s->pt64, s->cvec, s->adj_ls};
+                  s->tele, s->tele2, s->lam,  s->lam64, s->pt,   s->pt64, s->cvec, s->cvec2, s->adj_ls};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete s;
@@ -953,11 +966,11 @@ static unsigned pull_grid(Ctx* c, const Csc& q) {
 }
 
 // Whether a round of this form opens with a contribution pass: every round of the
-// unfused forms, PageRank-delta's residual round (its delta rounds take the previous
-// pull's contributions).
+// unfused forms but the adjoint's, which gathers lambda itself, and PageRank-delta's
+// residual round (its delta rounds take the previous pull's contributions).
 template <int MODE>
 static constexpr bool pr_opens_with_contrib() {
-  return !pr_fused<MODE>() || MODE == PR_DELTA_RESIDUAL;
+  return (!pr_fused<MODE>() && !pr_adj<MODE>()) || MODE == PR_DELTA_RESIDUAL;
 }
 
 // One round (first: the run's first round). Fused form: the pull alone (its last block
@@ -967,7 +980,7 @@ template <int MODE>
 static int launch_round(Ctx* c, const PrArgs& base_args, const Csc& q, bool first) {
   PrArgs a = base_args;
   int launched = 0;
-  if (!pr_fused<MODE>() || (first && pr_opens_with_contrib<MODE>())) {
+  if (pr_opens_with_contrib<MODE>() && (!pr_fused<MODE>() || first)) {
     pr_contrib_kernel<MODE><<<grid_n(c, c->n), 256, 0, c->stream>>>(a);
     ++launched;
   }
@@ -1030,9 +1043,11 @@ static int build_round_graph(Ctx* c, const PrArgs& base, const Csc& q, cudaGraph
       cudaGraphNode_t n_c, n_p, n_ctl;
       int zero = 0;
       void* a_p0[] = {(void*)&a, (void*)&blp, (void*)&h, (void*)&zero};
-      e = pr_add_kernel(body, &n_c, nullptr, 0, (void*)pr_contrib_kernel<MODE>, dim3(grid_n(c, c->n)), dim3(256), a_c);
+      const bool con = pr_opens_with_contrib<MODE>();
+      if (con)
+        e = pr_add_kernel(body, &n_c, nullptr, 0, (void*)pr_contrib_kernel<MODE>, dim3(grid_n(c, c->n)), dim3(256), a_c);
       if (e == cudaSuccess)
-        e = pr_add_kernel(body, &n_p, &n_c, 1, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p0);
+        e = pr_add_kernel(body, &n_p, con ? &n_c : nullptr, con ? 1 : 0, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p0);
       void* a_ctl[] = {(void*)&ls, (void*)&mode, (void*)&h, (void*)&one};
       if (e == cudaSuccess)
         e = pr_add_kernel(body, &n_ctl, &n_p, 1, (void*)pr_control_kernel, dim3(1), dim3(1), a_ctl);
@@ -1289,7 +1304,7 @@ int pagerank_result64(Ctx* c, Job* j, double* out, int where) {
 
 // s_u = sum of u's out-weights, one warp per source in CSR order (deterministic).
 __global__ void wsum_kernel(const uint32_t* __restrict__ ptr, const float* __restrict__ w, uint64_t n,
-                            double* __restrict__ wsum) {
+                            double* __restrict__ wsum, float2* __restrict__ wsum2) {
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -1298,7 +1313,11 @@ __global__ void wsum_kernel(const uint32_t* __restrict__ ptr, const float* __res
     for (uint32_t e = ptr[u] + lane; e < ptr[u + 1]; e += 32) s += (double)w[e];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) wsum[u] = s;
+    if (lane == 0) {
+      wsum[u] = s;
+      const FF f = ff_from_double(s);
+      wsum2[u] = make_float2(f.hi, f.lo);
+    }
   }
 }
 
@@ -1307,8 +1326,10 @@ static int build_wgraph(Ctx* c, WGraph& g) {
   int rc = build_csx(c, g.in, 0, &g.in_w, &g.in_wcap);
   if (!rc) rc = build_csx(c, g.out, 1, &g.out_w, &g.out_wcap);
   if (rc) return rc;
-  if (!g.wsum && cy_malloc(&g.wsum, c->n * 8) != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "weight sums");
-  wsum_kernel<<<grid_n(c, c->n * 32), 256, 0, c->stream>>>(g.out.ptr, g.out_w, c->n, g.wsum);
+  if ((!g.wsum && cy_malloc(&g.wsum, c->n * 8) != cudaSuccess) ||
+      (!g.wsum2 && cy_malloc(&g.wsum2, c->n * 8) != cudaSuccess))
+    return set_err(c, CYTOM_ERR_OOM, "weight sums");
+  wsum_kernel<<<grid_n(c, c->n * 32), 256, 0, c->stream>>>(g.out.ptr, g.out_w, c->n, g.wsum, g.wsum2);
   c->launches++;
   g.built_version = c->version;
   return cuda_err(c, cudaGetLastError(), "weight sums");
@@ -1322,7 +1343,9 @@ static PrArgs wargs(Ctx* c, Job* j, const WGraph& g) {
   a.bins = g.in.bins;
   a.csc_w = g.in_w;
   a.wsum = g.wsum;
+  a.wsum2 = g.wsum2;
   a.tele = s->tele;
+  a.tele2 = s->tele2;
   a.rank = s->rank;
   a.comp = s->comp;
   a.lo0 = s->lo;
@@ -1359,13 +1382,25 @@ int pagerank_set_teleport(Ctx* c, Job* j, const double* t, int where) {
     if (s->tele) {
       cudaStreamSynchronize(c->stream);
       cudaFree(s->tele);
+      cudaFree(s->tele2);
     }
     s->tele = nullptr;
+    s->tele2 = nullptr;
     return CYTOM_OK;
   }
   int prc = pr_ensure_perm(c);
   if (prc) return prc;
-  if (!s->tele && cy_malloc(&s->tele, c->n * 8) != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "teleport");
+  if (!s->tele) {
+    float2* t2 = nullptr;
+    double* t1 = nullptr;
+    if (cy_malloc(&t1, c->n * 8) != cudaSuccess || cy_malloc(&t2, c->n * 8) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(t1);
+      return set_err(c, CYTOM_ERR_OOM, "teleport");
+    }
+    s->tele = t1;
+    s->tele2 = t2;
+  }
   // kept in the renumbering
   double* tmp = nullptr;
   if (cy_malloc_async((void**)&tmp, c->n * 8, c->stream) != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "teleport");
@@ -1373,25 +1408,38 @@ int pagerank_set_teleport(Ctx* c, Job* j, const double* t, int where) {
                                   where == CYTOM_PTR_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                   c->stream);
   permute_kernel<double><<<grid_n(c, c->n), 256, 0, c->stream>>>(tmp, c->pr_perm, c->n, 1, s->tele);
-  c->launches++;
+  permute_ff_kernel<<<grid_n(c, c->n), 256, 0, c->stream>>>(tmp, c->pr_perm, c->n, s->tele2);
+  c->launches += 2;
   cudaFreeAsync(tmp, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   return cuda_err(c, e, "teleport upload");
 }
 
-__global__ void adj_init_kernel(const double* __restrict__ cvec, uint64_t n, float* lam32, double* lam64,
-                                LoopState* ls) {
-  double l1 = 0.0;
+// lambda_0 = c, |c|_1 and t . lambda_0 (FP32 form: c as float pairs, lambda its high word).
+template <typename T>
+__global__ void adj_init_kernel(const double* __restrict__ cvec, const float2* __restrict__ cvec2,
+                                const double* __restrict__ tele, uint64_t n, T* __restrict__ lam, LoopState* ls) {
+  double l1 = 0.0, td = 0.0;
+  const double tu = 1.0 / (double)n;
   uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
-    const double cv = cvec[v];
-    if (lam32) lam32[v] = (float)cv;
-    if (lam64) lam64[v] = cv;
+    double cv;
+    if (cvec2) cv = isfinite(cvec2[v].x) ? (double)cvec2[v].x + (double)cvec2[v].y : (double)cvec2[v].x;
+    else cv = cvec[v];
+    const T l = (T)cv;
+    lam[v] = l;
     l1 += fabs(cv);
+    td += (tele ? tele[v] : tu) * (double)l;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, o);
-  if ((threadIdx.x & 31) == 0 && l1 != 0.0) atomicAdd(&ls->base_sum, l1);
+  for (int o = 16; o > 0; o >>= 1) {
+    l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, o);
+    td += __shfl_xor_sync(0xFFFFFFFFu, td, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (l1 != 0.0) atomicAdd(&ls->base_sum, l1);
+    if (td != 0.0) atomicAdd(&ls->dangling[0], td);
+  }
 }
 
 // The adjoint stops at an L1 change <= rel * |c|_1.
@@ -1410,12 +1458,49 @@ __global__ void dangling_sum_kernel(const T* __restrict__ r, const double* __res
   if ((threadIdx.x & 31) == 0 && d != 0.0) atomicAdd(out, d);
 }
 
+// What dL/dw needs of vertex v, in vertex order: alpha r_v / s_v as a float pair and
+// (P^T lambda)_v in g, lambda_v. One FP64 division per vertex instead of one per edge.
+__global__ void grad_prep_kernel(const uint32_t* __restrict__ perm, const float* __restrict__ r,
+                                 const float* __restrict__ lam, const float* __restrict__ pt,
+                                 const double* __restrict__ wsum, uint64_t n, double alpha, float4* __restrict__ g,
+                                 float* __restrict__ lamv) {
+  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+    const uint32_t q = perm[v];
+    const FF f = ff_from_double(alpha * (double)r[q] / wsum[q]);
+    g[v] = make_float4(f.hi, f.lo, pt[q], 0.f);
+    lamv[v] = lam[q];
+  }
+}
+
 // dL/dw of every stored edge u -> k, in store order:
-// alpha * r_u / s_u * (lambda_k - (P^T lambda)_u), evaluated in FP64.
-template <typename T>
-__global__ void grad_w_kernel(const StoreDesc* __restrict__ sd, const uint32_t* __restrict__ perm,
-                              const T* __restrict__ r, const T* __restrict__ lam, const T* __restrict__ pt,
-                              const double* __restrict__ wsum, double alpha, float* __restrict__ gw) {
+// alpha * r_u / s_u * (lambda_k - (P^T lambda)_u). FP32 form: the factor of u and the
+// difference as float pairs (each exact to about 44 bits), their product rounded once. Bound
+// by the gather of lambda_k; in FP64 with a division per edge it was bound by the FP64 pipe.
+__global__ void grad_w32_kernel(const StoreDesc* __restrict__ sd, const float4* __restrict__ g,
+                                const float* __restrict__ lamv, float* __restrict__ gw) {
+  const uint64_t E = sd->E;
+  const uint32_t lT = sd->lT, lvpt = sd->lvpt;
+  const uint32_t ymask = (uint32_t)(sd->T - 1);
+  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
+    uint32_t t = sd->chunk_tile[e >> 7];
+    while (sd->tile_ptr[t + 1] <= e) ++t;
+    const uint32_t p = sd->edges[e];
+    const float4 gu = g[((t >> lT) << lvpt) | (p >> 16)];
+    const float lk = lamv[((t & ymask) << lvpt) | (p & 0xFFFFu)];
+    const FF d = ff_two_sum(lk, -gu.z);
+    const float y = ff_mul(FF{gu.x, gu.y}, d).hi;
+    // an infinity makes the float pairs NaN; its plain product is what FP64 gives
+    gw[e] = isfinite(y) ? y : gu.x * (lk - gu.z);
+  }
+}
+
+// The FP64 form: every factor and the result's last rounding in FP64.
+__global__ void grad_w64_kernel(const StoreDesc* __restrict__ sd, const uint32_t* __restrict__ perm,
+                                const double* __restrict__ r, const double* __restrict__ lam,
+                                const double* __restrict__ pt, const double* __restrict__ wsum, double alpha,
+                                float* __restrict__ gw) {
   const uint64_t E = sd->E;
   const uint32_t lT = sd->lT, lvpt = sd->lvpt;
   const uint32_t ymask = (uint32_t)(sd->T - 1);
@@ -1426,7 +1511,7 @@ __global__ void grad_w_kernel(const StoreDesc* __restrict__ sd, const uint32_t* 
     const uint32_t p = sd->edges[e];
     const uint32_t u = perm[((t >> lT) << lvpt) | (p >> 16)];
     const uint32_t k = perm[((t & ymask) << lvpt) | (p & 0xFFFFu)];
-    gw[e] = (float)(alpha * (double)r[u] / wsum[u] * ((double)lam[k] - (double)pt[u]));
+    gw[e] = (float)(alpha * r[u] / wsum[u] * (lam[k] - pt[u]));
   }
 }
 
@@ -1455,11 +1540,12 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   const bool f32 = j->params.kahan != 0;
   cudaError_t e = cudaSuccess;
   if (!s->adj_ls) e = cy_malloc(&s->adj_ls, sizeof(LoopState));
-  if (e == cudaSuccess && !s->cvec) e = cy_malloc(&s->cvec, n * 8);
   if (f32) {
+    if (e == cudaSuccess && !s->cvec2) e = cy_malloc(&s->cvec2, n * 8);
     if (e == cudaSuccess && !s->lam) e = cy_malloc(&s->lam, 2 * n * 4);
     if (e == cudaSuccess && !s->pt) e = cy_malloc(&s->pt, n * 4);
   } else {
+    if (e == cudaSuccess && !s->cvec) e = cy_malloc(&s->cvec, n * 8);
     if (e == cudaSuccess && !s->lam64) e = cy_malloc(&s->lam64, 2 * n * 8);
     if (e == cudaSuccess && !s->pt64) e = cy_malloc(&s->pt64, n * 8);
   }
@@ -1477,7 +1563,8 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
     e = cudaMemcpyAsync(ctmp, cv, n * 8, cwhere == CYTOM_PTR_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                         c->stream);
   if (e == cudaSuccess) {
-    permute_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(ctmp, c->pr_perm, n, 1, s->cvec);
+    if (f32) permute_ff_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(ctmp, c->pr_perm, n, s->cvec2);
+    else permute_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(ctmp, c->pr_perm, n, 1, s->cvec);
     c->launches++;
   }
   if (ctmp) cudaFreeAsync(ctmp, c->stream);
@@ -1490,8 +1577,10 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   cudaEventRecord(c->run_a, c->stream);
   unsigned max_iter = (unsigned)std::min<uint64_t>(j->params.max_iterations, 0xFFFFFFFFu);
   pr_begin_kernel<<<1, 1, 0, c->stream>>>(s->adj_ls, max_iter, 0.0, (unsigned long long)g->out.E);
-  adj_init_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(s->cvec, n, f32 ? s->lam : nullptr, f32 ? nullptr : s->lam64,
-                                                        s->adj_ls);
+  if (f32)
+    adj_init_kernel<float><<<grid_n(c, n), 256, 0, c->stream>>>(nullptr, s->cvec2, s->tele, n, s->lam, s->adj_ls);
+  else
+    adj_init_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(s->cvec, nullptr, s->tele, n, s->lam64, s->adj_ls);
   adj_tol_kernel<<<1, 1, 0, c->stream>>>(s->adj_ls, j->params.tolerance);
   c->launches += 3;
   PrArgs a{};
@@ -1501,15 +1590,16 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   a.csc_w = g->out_w;
   a.wsum = g->wsum;
   a.tele = s->tele;
+  a.wsum2 = g->wsum2;
+  a.tele2 = s->tele2;
   a.cvec = s->cvec;
+  a.cvec2 = s->cvec2;
   a.pt = s->pt;
   a.pt64 = s->pt64;
   a.rank = f32 ? s->lam : nullptr;
   a.comp = f32 ? s->lam + n : nullptr;
   a.r64 = f32 ? nullptr : s->lam64;
   a.r64n = f32 ? nullptr : s->lam64 + n;
-  a.contrib = s->contrib;  // the forward's contribution buffer is free once it has converged
-  a.contrib64 = s->contrib64;
   a.ls = s->adj_ls;
   a.n = n;
   a.alpha = j->params.alpha;
@@ -1522,11 +1612,13 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   if (e != cudaSuccess) return cuda_err(c, e, "adjoint run");
   const unsigned pa = als.iter & 1u;  // buffer holding the newest lambda
   // gradients into device scratch, then to the caller
-  // layout (256-byte aligned regions): D (one double), dL/dw (E floats), dL/dt (n floats)
+  // layout (256-byte aligned regions): D (one double), dL/dw (E floats), dL/dt (n floats),
+  // and for the FP32 form the vertices' factors (n float4) and lambda (n floats)
   char* tmp = nullptr;
   auto align256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t wbytes = align256(std::max<uint64_t>(E, 1) * 4), tbytes = align256(n * 4);
-  if (cy_malloc_async((void**)&tmp, 256 + wbytes + tbytes, c->stream) != cudaSuccess)
+  const size_t gbytes = f32 ? align256(n * 16) : 0;
+  if (cy_malloc_async((void**)&tmp, 256 + wbytes + tbytes + gbytes + (f32 ? n * 4 : 0), c->stream) != cudaSuccess)
     return set_err(c, CYTOM_ERR_OOM, "adjoint outputs");
   double* dang = (double*)tmp;
   float* gw = (owhere == CYTOM_PTR_DEVICE && d_w) ? d_w : (float*)(tmp + 256);
@@ -1535,14 +1627,17 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   if (f32) {
     const float* lam = (pa == 0) ? s->lam : s->lam + n;
     dangling_sum_kernel<float><<<grid_n(c, n), 256, 0, c->stream>>>(r32, g->wsum, n, dang);
-    if (E)
-      grad_w_kernel<float><<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, c->pr_perm, r32, lam, s->pt, g->wsum, a.alpha, gw);
+    float4* gv = (float4*)(tmp + 256 + wbytes + tbytes);
+    float* lamv = (float*)(tmp + 256 + wbytes + tbytes + gbytes);
+    grad_prep_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(c->pr_perm, r32, lam, s->pt, g->wsum, n, a.alpha, gv, lamv);
+    c->launches++;
+    if (E) grad_w32_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, gv, lamv, gw);
     grad_t_kernel<float><<<grid_n(c, n), 256, 0, c->stream>>>(lam, c->pr_perm, n, dang, a.alpha, gt);
   } else {
     const double* lam = (pa == 0) ? s->lam64 : s->lam64 + n;
     dangling_sum_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(r64, g->wsum, n, dang);
     if (E)
-      grad_w_kernel<double><<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, c->pr_perm, r64, lam, s->pt64, g->wsum, a.alpha, gw);
+      grad_w64_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, c->pr_perm, r64, lam, s->pt64, g->wsum, a.alpha, gw);
     grad_t_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(lam, c->pr_perm, n, dang, a.alpha, gt);
   }
   c->launches += 3;

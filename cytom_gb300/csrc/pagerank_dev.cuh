@@ -64,6 +64,17 @@ template <int MODE>
 __host__ __device__ constexpr bool pr_fused() {
   return MODE == PR_DELTA_RESIDUAL || MODE == PR_DELTA_PUSH;
 }
+// FP32 forms that carry float-float arithmetic per target (FF below).
+template <int MODE>
+__host__ __device__ constexpr bool pr_ff() {
+  return MODE == PR_NORM32 || MODE == PR_W32 || MODE == PR_ADJ32;
+}
+// The adjoint gathers lambda itself, so it has no contribution pass: its pull also adds up
+// t . lambda for the next round.
+template <int MODE>
+__host__ __device__ constexpr bool pr_adj() {
+  return MODE == PR_ADJ32 || MODE == PR_ADJ64;
+}
 // Value type of the contributions (and of a lane's partial sums before the merge).
 template <int MODE>
 using pr_val_t = typename std::conditional<pr_is64<MODE>(), double, float>::type;
@@ -100,8 +111,10 @@ struct Acc64 {
 // Float-float numbers: an unevaluated pair hi + lo of FP32 values (about 44 significant
 // bits), built from error-free transformations -- Knuth's two-sum, Dekker's fast two-sum
 // (|a| >= |b|) and the FMA-exact product. GB300 runs FP64 at a small fraction of its FP32
-// rate, so the FP32-compensated PageRank keeps its per-target arithmetic (update, change,
-// dangling mass) in this form instead of FP64. The _rn intrinsics keep the compiler from
+// rate, and a warp in which one lane of a group finishes its target pays for all 32, so the
+// FP32-compensated forms keep their per-target arithmetic (update, change, dangling mass) in
+// this form instead of FP64 (RMAT-20, 16.8 M weighted edges: adjoint pull @ADJ@, forward pull
+// @FWD@). The _rn intrinsics keep the compiler from
 // contracting the transformations' products and sums into FMAs.
 struct FF {
   float hi, lo;
@@ -125,6 +138,12 @@ __device__ __forceinline__ FF ff_mul(FF a, FF b) {
   const float p = __fmul_rn(a.hi, b.hi);
   const float e = __fmaf_rn(a.hi, b.hi, -p);
   return ff_fast_two_sum(p, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, e)));
+}
+// a / b by one correction of the quotient of the high words (Dekker's division).
+__device__ __forceinline__ FF ff_div(FF a, FF b) {
+  const float q = a.hi / b.hi;
+  const FF r = ff_add(a, ff_mul(FF{-q, 0.f}, b));
+  return ff_fast_two_sum(q, r.hi / b.hi);
 }
 __device__ __forceinline__ FF ff_abs(FF a) { return a.hi < 0.f ? FF{-a.hi, -a.lo} : a; }
 __host__ __device__ inline FF ff_from_double(double x) {
@@ -151,6 +170,9 @@ struct PrArgs {
   const double* wsum;       // weighted modes: out-weight sum s_u of each vertex
   const double* tele;       // weighted modes: teleport vector (NULL = uniform 1/n)
   const double* cvec;       // adjoint: the loss weights c
+  const float2* wsum2;      // the FP32 weighted forms' wsum, tele and cvec as float pairs
+  const float2* tele2;
+  const float2* cvec2;
   float* pt;                // adjoint FP32: (P^T lambda)_u of the last round
   double* pt64;             // adjoint FP64
   LoopState* ls;
@@ -166,10 +188,10 @@ inline void pr_args_ff(PrArgs& a) {
   a.inv_n_ff = ff_from_double(a.n ? 1.0 / (double)a.n : 0.0);
 }
 
-// A round's sums and the dangling term: float-float in the FP32-compensated form, FP64
+// A round's sums and the dangling term: float-float in the FP32-compensated forms, FP64
 // in the others.
 template <int MODE>
-using pr_ff_t = typename std::conditional<MODE == PR_NORM32, FF, double>::type;
+using pr_ff_t = typename std::conditional<pr_ff<MODE>(), FF, double>::type;
 
 template <bool PERSIST, class T>
 __device__ __forceinline__ T pr_ld(const T* p) {
@@ -177,9 +199,12 @@ __device__ __forceinline__ T pr_ld(const T* p) {
   else return *p;
 }
 
-// The contributions round p reads (fused form: half p; the others: the one vector).
+// The contributions round p reads (fused form: half p; the adjoint: lambda before the round;
+// the others: the one vector).
 template <int MODE>
 __device__ __forceinline__ const pr_val_t<MODE>* pr_cread(const PrArgs& a, unsigned p) {
+  if constexpr (MODE == PR_ADJ32) return (p == 0) ? a.rank : a.comp;
+  if constexpr (MODE == PR_ADJ64) return (p == 0) ? a.r64 : a.r64n;
   const uint64_t off = pr_fused<MODE>() ? (uint64_t)p * a.n : 0;
   if constexpr (pr_is64<MODE>()) return a.contrib64 + off;
   else return a.contrib + off;
@@ -225,10 +250,10 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_contrib_range(const PrArgs& a, unsig
     const float* r = (p == 0) ? a.rank : a.comp;
     const float* rl = (p == 0) ? a.lo0 : a.lo1;
     for (uint64_t u = lo + tid; u < hi; u += nthr) {
-      const double s = a.wsum[u];
+      const float s = a.wsum2[u].x;
       const float rh = pr_ld<PERSIST>(r + u);
-      a.contrib[u] = s > 0.0 ? rh / (float)s : 0.f;
-      if (!(s > 0.0)) dangling += (double)rh + (double)pr_ld<PERSIST>(rl + u);
+      a.contrib[u] = s > 0.f ? rh / s : 0.f;
+      if (!(s > 0.f)) dangling = ff_add(dangling, FF{rh, pr_ld<PERSIST>(rl + u)});
     }
   } else if constexpr (MODE == PR_W64) {
     const double* r = (p == 0) ? a.r64 : a.r64n;
@@ -238,23 +263,8 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_contrib_range(const PrArgs& a, unsig
       a.contrib64[u] = s > 0.0 ? rv / s : 0.0;
       if (!(s > 0.0)) dangling += rv;
     }
-  } else if constexpr (MODE == PR_ADJ32) {
-    // gather source = lambda itself; the returned sum is t . lambda
-    const float* l = (p == 0) ? a.rank : a.comp;
-    const double tu = 1.0 / (double)a.n;
-    for (uint64_t u = lo + tid; u < hi; u += nthr) {
-      const float lv = pr_ld<PERSIST>(l + u);
-      a.contrib[u] = lv;
-      dangling += (a.tele ? a.tele[u] : tu) * (double)lv;
-    }
-  } else if constexpr (MODE == PR_ADJ64) {
-    const double* l = (p == 0) ? a.r64 : a.r64n;
-    const double tu = 1.0 / (double)a.n;
-    for (uint64_t u = lo + tid; u < hi; u += nthr) {
-      const double lv = pr_ld<PERSIST>(l + u);
-      a.contrib64[u] = lv;
-      dangling += (a.tele ? a.tele[u] : tu) * lv;
-    }
+  } else if constexpr (pr_adj<MODE>()) {
+    // no pass
   } else {
     const double* r = (p == 0) ? a.r64 : a.r64n;
     double* cw = a.contrib64;
@@ -271,7 +281,7 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_contrib_range(const PrArgs& a, unsig
 // Warp-reduced dangling mass into the loop state (every lane calls it).
 template <int MODE>
 __device__ __forceinline__ void pr_dangling_flush(LoopState* ls, unsigned p, pr_ff_t<MODE> dangling) {
-  if constexpr (MODE == PR_NORM32) {
+  if constexpr (pr_ff<MODE>()) {
     // float-float warp sum; one conversion per warp
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -287,11 +297,16 @@ __device__ __forceinline__ void pr_dangling_flush(LoopState* ls, unsigned p, pr_
 }
 
 // The round's dangling term as pr_finish takes it: D / n (normalised PageRank), D
-// (weighted: scaled by t_v in pr_finish), t . lambda (adjoint), none (PageRank-delta).
+// (weighted FP64: scaled by t_v in pr_finish), (1 - alpha) + alpha D (weighted FP32),
+// t . lambda (adjoint), none (PageRank-delta).
 template <int MODE, bool PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_dang_arg(const PrArgs& a, const LoopState* ls, unsigned p) {
   if constexpr (MODE == PR_NORM32) {
     return ff_mul(ff_from_double(pr_ld<PERSIST>(&ls->dangling[p])), a.inv_n_ff);
+  } else if constexpr (MODE == PR_W32) {
+    return ff_from_double((1.0 - a.alpha) + a.alpha * pr_ld<PERSIST>(&ls->dangling[p]));
+  } else if constexpr (MODE == PR_ADJ32) {
+    return ff_from_double(pr_ld<PERSIST>(&ls->dangling[p]));
   } else {
     if (MODE < PR_NORM32) return 0.0;
     const double d = pr_ld<PERSIST>(&ls->dangling[p]);
@@ -321,47 +336,24 @@ __device__ __forceinline__ PrOld pr_load_old(const PrArgs& a, uint64_t v, unsign
 template <int MODE, bool PERSIST>
 __device__ __forceinline__ double pr_apply(const PrArgs& a, uint64_t v, double sum, unsigned p, double dang,
                                            double* rsum, unsigned* nact) {
-  if (MODE == PR_W32 || MODE == PR_W64) {
+  if (MODE == PR_W64) {
     const double tv = a.tele ? a.tele[v] : 1.0 / (double)a.n;
     const double nv = tv * ((1.0 - a.alpha) + a.alpha * dang) + a.alpha * sum;
-    if (MODE == PR_W32) {
-      const float* r = (p == 0) ? a.rank : a.comp;
-      const float* rl = (p == 0) ? a.lo0 : a.lo1;
-      float* rn = (p == 0) ? a.comp : a.rank;
-      float* rnl = (p == 0) ? a.lo1 : a.lo0;
-      const float hi = (float)nv;
-      rn[v] = hi;
-      rnl[v] = (float)(nv - (double)hi);
-      *rsum += nv;
-      return fabs(nv - ((double)pr_ld<PERSIST>(r + v) + (double)pr_ld<PERSIST>(rl + v)));
-    } else {
-      const double* r = (p == 0) ? a.r64 : a.r64n;
-      double* rn = (p == 0) ? a.r64n : a.r64;
-      rn[v] = nv;
-      *rsum += nv;
-      return fabs(nv - pr_ld<PERSIST>(r + v));
-    }
-  } else if (MODE == PR_ADJ32 || MODE == PR_ADJ64) {
+    const double* r = (p == 0) ? a.r64 : a.r64n;
+    double* rn = (p == 0) ? a.r64n : a.r64;
+    rn[v] = nv;
+    return fabs(nv - pr_ld<PERSIST>(r + v));
+  } else if (MODE == PR_ADJ64) {
     // v is a source here: lambda'_v = c_v + alpha ((P^T lambda)_v + a_v (t . lambda))
     const double s = a.wsum[v];
     const double ptv = s > 0.0 ? sum / s : 0.0;
     const double nl = a.cvec[v] + a.alpha * (ptv + (s > 0.0 ? 0.0 : dang));
-    if (MODE == PR_ADJ32) {
-      const float* l = (p == 0) ? a.rank : a.comp;
-      float* ln = (p == 0) ? a.comp : a.rank;
-      const float nf = (float)nl;
-      ln[v] = nf;
-      a.pt[v] = (float)ptv;
-      *rsum += (double)nf;
-      return fabs((double)nf - (double)pr_ld<PERSIST>(l + v));
-    } else {
-      const double* l = (p == 0) ? a.r64 : a.r64n;
-      double* ln = (p == 0) ? a.r64n : a.r64;
-      ln[v] = nl;
-      a.pt64[v] = ptv;
-      *rsum += nl;
-      return fabs(nl - pr_ld<PERSIST>(l + v));
-    }
+    const double* l = (p == 0) ? a.r64 : a.r64n;
+    double* ln = (p == 0) ? a.r64n : a.r64;
+    ln[v] = nl;
+    a.pt64[v] = ptv;
+    *rsum += (a.tele ? a.tele[v] : 1.0 / (double)a.n) * nl;  // t . lambda of the next round
+    return fabs(nl - pr_ld<PERSIST>(l + v));
   } else {
     // PageRank-delta: residual round or delta round, rank += change (compensated)
     const float rank_v = pr_ld<PERSIST>(a.rank + v);
@@ -393,9 +385,10 @@ __device__ __forceinline__ double pr_apply(const PrArgs& a, uint64_t v, double s
 // (pr_tally_flush).
 struct PrTally {
   double resid, rsum;
-  FF fres;  // FP32-compensated form: the residual in float-float
+  FF fres;  // FP32-compensated forms: the residual in float-float
+  FF ftd;   // FP32 adjoint: t . lambda in float-float (FP64 adjoint: rsum)
   unsigned nact;
-  __device__ __forceinline__ void init() { resid = rsum = 0.0, fres = FF{0.f, 0.f}, nact = 0u; }
+  __device__ __forceinline__ void init() { resid = rsum = 0.0, fres = ftd = FF{0.f, 0.f}, nact = 0u; }
 };
 
 // The normalised forms' update of v from its sum and its rank before the round; the
@@ -420,6 +413,57 @@ __device__ __forceinline__ void pr_apply_norm(const PrArgs& a, uint64_t v, pr_ff
   }
 }
 
+// The FP32 weighted forms' update of v in float-float.
+// PR_W32: r'_v = t_v ((1-alpha) + alpha D) + alpha sum (dang holds the bracket), kept as a
+// float pair. PR_ADJ32 (v is a source): lambda'_v = c_v + alpha ((P^T lambda)_v + a_v (t . lambda)),
+// kept as a float; its share of the next round's t . lambda joins the tally. Float pairs
+// turn an infinity into NaN, so a result that is not finite is taken in FP64 instead.
+template <int MODE, bool PERSIST>
+__device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum, unsigned p, FF dang, PrTally& t) {
+  FF tv = a.inv_n_ff;
+  if (a.tele2) {
+    const float2 q = a.tele2[v];
+    tv = FF{q.x, q.y};
+  }
+  FF change;
+  if constexpr (MODE == PR_W32) {
+    const PrOld o{0.0, pr_ld<PERSIST>(((p == 0) ? a.rank : a.comp) + v), pr_ld<PERSIST>(((p == 0) ? a.lo0 : a.lo1) + v)};
+    float* rn = (p == 0) ? a.comp : a.rank;
+    float* rnl = (p == 0) ? a.lo1 : a.lo0;
+    FF nv = ff_add(ff_mul(tv, dang), ff_mul(a.alpha_ff, sum));
+    if (!isfinite(nv.hi)) {
+      const double d = (a.tele ? a.tele[v] : 1.0 / (double)a.n) * ((double)dang.hi + (double)dang.lo) +
+                       a.alpha * ((double)sum.hi + (double)sum.lo);
+      nv = ff_from_double(d);
+    }
+    rn[v] = nv.hi;
+    rnl[v] = nv.lo;
+    change = ff_add(nv, FF{-o.hi, -o.lo});
+    if (!isfinite(change.hi)) change = FF{(nv.hi + nv.lo) - (o.hi + o.lo), 0.f};
+  } else {
+    const float old = pr_ld<PERSIST>(((p == 0) ? a.rank : a.comp) + v);
+    const float2 s = a.wsum2[v], c = a.cvec2[v];
+    FF ptv{0.f, 0.f}, add = dang;
+    if (s.x > 0.f) ptv = add = ff_div(sum, FF{s.x, s.y});
+    float nl = ff_add(FF{c.x, c.y}, ff_mul(a.alpha_ff, add)).hi, pv = ptv.hi;
+    if (!isfinite(nl) || !isfinite(pv)) {
+      const double sv = a.wsum[v];
+      const double ptd = sv > 0.0 ? ((double)sum.hi + (double)sum.lo) / sv : 0.0;
+      const double cd = isfinite(c.x) ? (double)c.x + (double)c.y : (double)c.x;
+      pv = (float)ptd;
+      nl = (float)(cd + a.alpha * (ptd + (sv > 0.0 ? 0.0 : (double)dang.hi + (double)dang.lo)));
+    }
+    ((p == 0) ? a.comp : a.rank)[v] = nl;
+    a.pt[v] = pv;
+    change = isfinite(nl - old) ? ff_two_sum(nl, -old) : FF{nl - old, 0.f};
+    const FF td = ff_mul(tv, FF{nl, 0.f});
+    if (isfinite(td.hi)) t.ftd = ff_add(t.ftd, td);
+    else t.rsum += (double)(tv.hi * nl);
+  }
+  if (isfinite(change.hi)) t.fres = ff_add(t.fres, ff_abs(change));
+  else t.resid += (double)fabsf(change.hi);
+}
+
 // Applies the finished sum of target v and adds its share to the tally. The fused form
 // also writes v's contribution to the next round (half p^1), exactly as the
 // contribution pass would compute it from the new delta.
@@ -428,6 +472,8 @@ __device__ __forceinline__ void pr_finish(const PrArgs& a, uint64_t v, pr_ff_t<M
                                           pr_ff_t<MODE> dang, PrTally& t) {
   if constexpr (MODE == PR_NORM32 || MODE == PR_NORM64)
     pr_apply_norm<MODE>(a, v, sum, p, dang, pr_load_old<MODE, PERSIST>(a, v, p), t);
+  else if constexpr (MODE == PR_W32 || MODE == PR_ADJ32)
+    pr_apply_w32<MODE, PERSIST>(a, v, sum, p, dang, t);
   else
     t.resid += pr_apply<MODE, PERSIST>(a, v, sum, p, dang, &t.rsum, &t.nact);
 }
@@ -440,21 +486,33 @@ __device__ __forceinline__ void pr_tally_flush(LoopState* ls, unsigned p, PrTall
   __shared__ double s_r[32], s_s[32];
   __shared__ unsigned s_n[32];
   constexpr bool kN = pr_fused<MODE>();  // activations (PageRank-delta)
-  constexpr bool kS = MODE != PR_NORM32 && MODE != PR_NORM64;  // rank sum kept
+  // s_s: PageRank-delta's rank sum, the adjoint's t . lambda
+  constexpr bool kS = pr_fused<MODE>() || pr_adj<MODE>();
   if (!kN) t.nact = 0u;
-  if constexpr (MODE == PR_NORM32) {
-    // float-float warp sum of the residual; one conversion per warp
+  if constexpr (pr_ff<MODE>()) {
+    // float-float warp sums; one conversion per warp
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) {
       t.fres = ff_add(t.fres, FF{__shfl_xor_sync(0xFFFFFFFFu, t.fres.hi, o), __shfl_xor_sync(0xFFFFFFFFu, t.fres.lo, o)});
-    t.resid = (double)t.fres.hi + (double)t.fres.lo;
+      if (MODE == PR_ADJ32)
+        t.ftd = ff_add(t.ftd, FF{__shfl_xor_sync(0xFFFFFFFFu, t.ftd.hi, o), __shfl_xor_sync(0xFFFFFFFFu, t.ftd.lo, o)});
+    }
+    if (MODE != PR_NORM32 && __any_sync(0xFFFFFFFFu, t.resid != 0.0 || t.rsum != 0.0)) {  // infinities, NaN
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        t.resid += __shfl_xor_sync(0xFFFFFFFFu, t.resid, o);
+        t.rsum += __shfl_xor_sync(0xFFFFFFFFu, t.rsum, o);
+      }
+    }
+    t.resid += (double)t.fres.hi + (double)t.fres.lo;
+    if (MODE == PR_ADJ32) t.rsum += (double)t.ftd.hi + (double)t.ftd.lo;
   } else {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t.resid += __shfl_xor_sync(0xFFFFFFFFu, t.resid, o);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    if (kS) t.rsum += __shfl_xor_sync(0xFFFFFFFFu, t.rsum, o);
+    if (kS && !pr_ff<MODE>()) t.rsum += __shfl_xor_sync(0xFFFFFFFFu, t.rsum, o);
     if (kN) t.nact += __shfl_xor_sync(0xFFFFFFFFu, t.nact, o);
   }
   const unsigned w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -473,7 +531,7 @@ __device__ __forceinline__ void pr_tally_flush(LoopState* ls, unsigned p, PrTall
       na += s_n[k];
     }
     if (r != 0.0) atomicAdd(&ls->resid[p], r);
-    if (sm != 0.0) atomicAdd(&ls->rank_sum[p], sm);
+    if (kS && sm != 0.0) atomicAdd(pr_adj<MODE>() ? &ls->dangling[p ^ 1u] : &ls->rank_sum[p], sm);
     if (kN && na) atomicAdd(&ls->active[p ^ 1u], na);
   }
   __syncthreads();
@@ -513,10 +571,10 @@ __device__ __forceinline__ void pr_lane_sum(const PrArgs& a, const pr_val_t<MODE
 }
 
 // A compensated FP32 sum as the update takes it: the float pair itself in the
-// FP32-compensated form, s + e in FP64 in the other FP32 forms.
+// FP32-compensated forms, s + e in FP64 in PageRank-delta.
 template <int MODE>
 __device__ __forceinline__ pr_ff_t<MODE> pr_acc32_out(float s, float e) {
-  if constexpr (MODE == PR_NORM32) return FF{s, e};
+  if constexpr (pr_ff<MODE>()) return FF{s, e};
   else return (double)s + (double)e;
 }
 
@@ -688,7 +746,8 @@ __device__ __forceinline__ unsigned pr_control_step(LoopState* ls, int mode) {
     }
   }
   ls->resid[q] = 0.0;
-  ls->dangling[q] = 0.0;
+  // the adjoint's pull filled [q] for the next round; the others' contribution pass fills it
+  ls->dangling[mode == PR_ADJ32 || mode == PR_ADJ64 ? p : q] = 0.0;
   ls->active[p] = 0;
   ls->rank_sum[q] = 0.0;
   ls->cont = more ? 1u : 0u;
