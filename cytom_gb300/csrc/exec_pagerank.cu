@@ -165,7 +165,7 @@ __global__ void csc_src_kernel(const uint64_t* __restrict__ keys, uint64_t E, ui
 // it); tot[k] += the bin sizes (one atomic per bin and block).
 __global__ void csc_cnt_bins_kernel(const uint32_t* seg_lo, const uint32_t* __restrict__ seg_hi, uint64_t n,
                                     uint32_t* __restrict__ cnt, uint64_t* __restrict__ binkey, uint32_t* vid,
-                                    uint32_t* __restrict__ tot) {
+                                    uint32_t* __restrict__ tot, uint32_t warp_hi) {
   __shared__ unsigned s_tot[kPrBins];
   if (threadIdx.x < kPrBins) s_tot[threadIdx.x] = 0;
   __syncthreads();
@@ -173,7 +173,7 @@ __global__ void csc_cnt_bins_kernel(const uint32_t* seg_lo, const uint32_t* __re
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     const uint32_t d = seg_hi[v] - seg_lo[v];
     int k = 0;
-    while (k + 1 < kPrBins && d > pr_bin_hi(k)) ++k;
+    while (k + 1 < kPrBins && d > pr_bin_hi(k, warp_hi)) ++k;
     cnt[v] = d;
     binkey[v] = (uint64_t)k;
     vid[v] = (uint32_t)v;
@@ -364,7 +364,7 @@ static int build_csx_stage(Ctx* c, Csc& q, int by_source, float** w, uint64_t* w
   }
   // segment lengths and bin keys, then the offsets and one stable 3-bit sort of the
   // vertices by bin (vertex order kept inside each bin)
-  csc_cnt_bins_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(seg_lo, seg_hi, n, cnt, k0, seg_lo, tot);
+  csc_cnt_bins_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(seg_lo, seg_hi, n, cnt, k0, seg_lo, tot, pr_warp_bin_hi(E));
   c->launches++;
   rc = exclusive_scan_u32(c, cnt, q.ptr, n, q.ptr + n);
   if (rc) return rc;
@@ -490,7 +490,7 @@ static int merge_csc_stage(Ctx* c, Csc& q) {
   if (mblk) csc_merge_old_kernel<<<mblk, 256, 0, c->stream>>>(q.src, Eo, at, jb, q.src_alt);
   c->launches += 4;
   // bins of the new in-degrees, as build_csx makes them
-  csc_cnt_bins_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(np, np + 1, n, cnt, bk0, vid, tot);
+  csc_cnt_bins_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(np, np + 1, n, cnt, bk0, vid, tot, pr_warp_bin_hi(E));
   c->launches++;
   bool balt = false;
   rc = radix_sort_pairs(c, bk0, bk1, vid, q.bins, n, 3, &balt);
@@ -649,25 +649,68 @@ __device__ __forceinline__ void pull_small_body(const PrArgs& a, const pr_val_t<
   }
 }
 
+// A value of another lane.
+__device__ __forceinline__ FF pr_shfl(FF x, int lane) {
+  return {__shfl_sync(0xFFFFFFFFu, x.hi, lane), __shfl_sync(0xFFFFFFFFu, x.lo, lane)};
+}
+__device__ __forceinline__ double pr_shfl(double x, int lane) { return __shfl_sync(0xFFFFFFFFu, x, lane); }
+
+// The FP32 PageRank's pull is bound by L2 requests, not by its update (22 instructions in
+// float pairs): its groups finish their targets alone, which needs 32 registers instead of
+// 48 and so keeps eight blocks per SM in flight (RMAT-24 26.4 ms, with shared updates 27.0 at
+// eight blocks per SM and 27.4 at five).
+template <int MODE>
+__host__ __device__ constexpr bool pr_group_alone() {
+  return MODE == PR_NORM32;
+}
+
+// Targets of a group bin (VW lanes each). A warp takes S * 32 / VW consecutive targets at a
+// time, lane j the j-th: their ids and offsets are loaded by all lanes at once, the groups
+// sum them in S steps, and each sum goes back to its target's lane, so that the update --
+// 40 to 100 instructions, FP64 ones in the FP64 forms -- runs with 32 / VW * S lanes at work
+// instead of 32 / VW. S is the largest up to VW that leaves every warp of the bin a share.
 template <int MODE, int VW>
 __device__ __forceinline__ void pull_group_body(const PrArgs& a, const pr_val_t<MODE>* cr, unsigned p, pr_ff_t<MODE> dang,
                                                 uint64_t bid, uint64_t nblk, PrTally& t) {
-  constexpr uint64_t GPW = 32 / VW;  // groups per warp
-  const unsigned gl = threadIdx.x & (VW - 1);
-  const uint64_t gid = (bid * blockDim.x + threadIdx.x) / VW;
-  const uint64_t ngroups = (nblk * blockDim.x) / VW;
-  // warp-uniform trip count: every lane stays in the loop for the group shuffles
-  const uint64_t gbase = gid - (gid % GPW);
-  for (uint64_t b = gbase; b < a.bin_count; b += ngroups) {
-    const uint64_t i = b + (gid - gbase);
+  constexpr unsigned GPW = 32 / VW;  // groups per warp
+  const unsigned lane = threadIdx.x & 31, gl = lane & (VW - 1), g = lane / VW;
+  if constexpr (pr_group_alone<MODE>()) {
+    const uint64_t gid = (bid * blockDim.x + threadIdx.x) / VW;
+    const uint64_t ngroups = (nblk * blockDim.x) / VW;
+    for (uint64_t b = gid - g; b < a.bin_count; b += ngroups) {  // the same trips for every lane of the warp
+      const uint64_t i = b + g;
+      uint32_t v = 0, lo = 0, hi = 0;
+      if (i < a.bin_count) {
+        v = a.bins[a.bin_off + i];
+        lo = a.csc_ptr[v];
+        hi = a.csc_ptr[v + 1];
+      }
+      const pr_ff_t<MODE> sum = pr_sum_group<MODE, false, VW>(a, cr, lo, hi, gl);
+      if (gl == 0 && i < a.bin_count) pr_finish<MODE, false>(a, v, sum, p, dang, t);
+    }
+    return;
+  }
+  const uint64_t warp = (bid * blockDim.x + threadIdx.x) >> 5, nwarps = (nblk * blockDim.x) >> 5;
+  unsigned S = VW;
+  while (S > 1 && a.bin_count < nwarps * GPW * S) S >>= 1;
+  const unsigned per = GPW * S;
+  for (uint64_t b = warp * per; b < a.bin_count; b += nwarps * per) {
+    const uint64_t i = b + lane;
+    const bool own = lane < per && i < a.bin_count;
     uint32_t v = 0, lo = 0, hi = 0;
-    if (i < a.bin_count) {
+    if (own) {
       v = a.bins[a.bin_off + i];
       lo = a.csc_ptr[v];
       hi = a.csc_ptr[v + 1];
     }
-    const pr_ff_t<MODE> sum = pr_sum_group<MODE, false, VW>(a, cr, lo, hi, gl);
-    if (gl == 0 && i < a.bin_count) pr_finish<MODE, false>(a, v, sum, p, dang, t);
+    pr_ff_t<MODE> mine{};
+    for (unsigned r = 0; r < S; ++r) {
+      const int src = (int)(r * GPW + g);
+      const uint32_t l = __shfl_sync(0xFFFFFFFFu, lo, src), h = __shfl_sync(0xFFFFFFFFu, hi, src);
+      const pr_ff_t<MODE> x = pr_shfl(pr_sum_group<MODE, false, VW>(a, cr, l, h, gl), (int)((lane & (GPW - 1)) * VW));
+      if (lane / GPW == r) mine = x;
+    }
+    if (own) pr_finish<MODE, false>(a, v, mine, p, dang, t);
   }
 }
 
@@ -737,8 +780,16 @@ __device__ __forceinline__ void pull_vblocks(PrArgs& a, const pr_val_t<MODE>* cr
   }
 }
 
+// Resident blocks the pull is compiled for. Measured with 5 / 6 / 7 / 8: RMAT-22 FP64 11.8 /
+// 11.3 / 11.7 / 11.3 ms, RMAT-20 weighted forward and adjoint 15.0 / 14.0 / 13.4 / 13.4;
+// RMAT-16 PageRank-delta 20.3 with four, 21.1 with six, 21.7 with eight.
 template <int MODE>
-__global__ void __launch_bounds__(PR_T) pr_pull_kernel(PrArgs a, const PrBinLaunch* __restrict__ blp,
+__host__ __device__ constexpr int pr_min_blocks() {
+  return MODE == PR_NORM32 ? 8 : MODE == PR_NORM64 ? 6 : (MODE == PR_W32 || MODE == PR_ADJ32) ? 7 : pr_fused<MODE>() ? 4 : 5;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(PR_T, pr_min_blocks<MODE>()) pr_pull_kernel(PrArgs a, const PrBinLaunch* __restrict__ blp,
                                                        cudaGraphConditionalHandle h, int use_handle) {
   LoopState* ls = a.ls;
   const bool live = ls->cont != 0;
@@ -747,7 +798,11 @@ __global__ void __launch_bounds__(PR_T) pr_pull_kernel(PrArgs a, const PrBinLaun
   PrTally t;
   t.init();
   const uint32_t total = live ? blp->blocks : 0u;
-  const pr_ff_t<MODE> dang = pr_dang_arg<MODE, false>(a, ls, p);
+  // one thread's FP64 conversion of the dangling term, not every thread's
+  __shared__ pr_ff_t<MODE> s_dang;
+  if (threadIdx.x == 0) s_dang = pr_dang_arg<MODE, false>(a, ls, p);
+  __syncthreads();
+  const pr_ff_t<MODE> dang = s_dang;
   const pr_val_t<MODE>* cr = pr_cread<MODE>(a, p);
   pull_vblocks<MODE>(a, cr, p, dang, blp, total, t);
   if (live) pr_tally_flush<MODE>(ls, p, t);

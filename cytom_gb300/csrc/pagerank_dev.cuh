@@ -29,9 +29,19 @@ namespace cytom {
 
 // Targets are binned by in-degree: bin k holds in-degrees in (pr_bin_hi(k-1), pr_bin_hi(k)];
 // its pull uses pr_bin_vw(k) lanes per target (1 = one thread, 0 = one whole block).
+// A warp takes a round trip to L2 per 128 in-edges of a target, so the longest target of the
+// warp bin bounds a round from below (4,096 in-edges: 16 us). Up to 2^21 edges, where the
+// round has less work than that, targets above 512 in-edges (E / 2048 in between) go to a
+// block: the RMAT-16 PageRank-delta stream 20.5 -> 17.8 ms. Above, a block per target costs more
+// than it saves: RMAT-24 FP32 PageRank 26.3 ms with 4,096, 28.4 with 512 or 1,024.
 constexpr int kPrBins = 5;
-__host__ __device__ constexpr uint32_t pr_bin_hi(int k) {
-  return k == 0 ? 4u : k == 1 ? 32u : k == 2 ? 256u : k == 3 ? 4096u : 0xFFFFFFFFu;
+inline uint32_t pr_warp_bin_hi(uint64_t edges) {
+  uint32_t hi = 512u;
+  while (hi < 4096u && (uint64_t)hi * 2048u < edges) hi *= 2;
+  return hi;
+}
+__host__ __device__ constexpr uint32_t pr_bin_hi(int k, uint32_t warp_hi) {
+  return k == 0 ? 4u : k == 1 ? 32u : k == 2 ? 256u : k == 3 ? warp_hi : 0xFFFFFFFFu;
 }
 __host__ __device__ constexpr int pr_bin_vw(int k) { return k == 0 ? 1 : k == 1 ? 4 : k == 2 ? 8 : k == 3 ? 32 : 0; }
 constexpr int PR_T = 256;
@@ -64,10 +74,10 @@ template <int MODE>
 __host__ __device__ constexpr bool pr_fused() {
   return MODE == PR_DELTA_RESIDUAL || MODE == PR_DELTA_PUSH;
 }
-// FP32 forms that carry float-float arithmetic per target (FF below).
+// FP32 forms: float-float arithmetic per target (FF below).
 template <int MODE>
 __host__ __device__ constexpr bool pr_ff() {
-  return MODE == PR_NORM32 || MODE == PR_W32 || MODE == PR_ADJ32;
+  return !pr_is64<MODE>();
 }
 // The adjoint gathers lambda itself, so it has no contribution pass: its pull also adds up
 // t . lambda for the next round.
@@ -113,8 +123,8 @@ struct Acc64 {
 // (|a| >= |b|) and the FMA-exact product. GB300 runs FP64 at a small fraction of its FP32
 // rate, and a warp in which one lane of a group finishes its target pays for all 32, so the
 // FP32-compensated forms keep their per-target arithmetic (update, change, dangling mass) in
-// this form instead of FP64 (RMAT-20, 16.8 M weighted edges: adjoint pull @ADJ@, forward pull
-// @FWD@). The _rn intrinsics keep the compiler from
+// this form instead of FP64 (RMAT-20, 16.8 M weighted edges: adjoint pull 155 -> 108 us, forward
+// pull 137 -> 91). The _rn intrinsics keep the compiler from
 // contracting the transformations' products and sums into FMAs.
 struct FF {
   float hi, lo;
@@ -178,18 +188,20 @@ struct PrArgs {
   LoopState* ls;
   uint64_t n;
   double alpha, delta_param, base;
-  FF alpha_ff, base_ff, inv_n_ff;  // alpha, base and 1/n as float-float (pr_args_ff)
+  // alpha, base, 1/n, 1 - alpha and delta_param as float-float (pr_args_ff)
+  FF alpha_ff, base_ff, inv_n_ff, rest_ff, delta_ff;
 };
 
-// Fills the float-float copies of alpha, base and 1/n (host, after those are set).
+// Fills the float-float copies of the constants (host, after those are set).
 inline void pr_args_ff(PrArgs& a) {
   a.alpha_ff = ff_from_double(a.alpha);
+  a.rest_ff = ff_from_double(1.0 - a.alpha);
+  a.delta_ff = ff_from_double(a.delta_param);
   a.base_ff = ff_from_double(a.base);
   a.inv_n_ff = ff_from_double(a.n ? 1.0 / (double)a.n : 0.0);
 }
 
-// A round's sums and the dangling term: float-float in the FP32-compensated forms, FP64
-// in the others.
+// A round's sums and the dangling term: float-float in the FP32 forms, FP64 in the others.
 template <int MODE>
 using pr_ff_t = typename std::conditional<pr_ff<MODE>(), FF, double>::type;
 
@@ -228,7 +240,7 @@ template <int MODE, bool PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_contrib_range(const PrArgs& a, unsigned p, uint64_t lo, uint64_t hi,
                                                           uint64_t tid, uint64_t nthr) {
   pr_ff_t<MODE> dangling{};
-  if constexpr (MODE == PR_DELTA_RESIDUAL || MODE == PR_DELTA_PUSH) {
+  if constexpr (pr_fused<MODE>()) {
     float* cw = a.contrib + (uint64_t)p * a.n;
     for (uint64_t u = lo + tid; u < hi; u += nthr) {
       const uint32_t d = a.deg[u];
@@ -281,7 +293,7 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_contrib_range(const PrArgs& a, unsig
 // Warp-reduced dangling mass into the loop state (every lane calls it).
 template <int MODE>
 __device__ __forceinline__ void pr_dangling_flush(LoopState* ls, unsigned p, pr_ff_t<MODE> dangling) {
-  if constexpr (pr_ff<MODE>()) {
+  if constexpr (pr_ff<MODE>() && !pr_fused<MODE>()) {
     // float-float warp sum; one conversion per warp
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -289,7 +301,7 @@ __device__ __forceinline__ void pr_dangling_flush(LoopState* ls, unsigned p, pr_
                                      __shfl_xor_sync(0xFFFFFFFFu, dangling.lo, o)});
     if ((threadIdx.x & 31) == 0 && dangling.hi != 0.f)
       atomicAdd(&ls->dangling[p], (double)dangling.hi + (double)dangling.lo);
-  } else if constexpr (MODE >= PR_NORM32) {
+  } else if constexpr (pr_is64<MODE>()) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dangling += __shfl_xor_sync(0xFFFFFFFFu, dangling, o);
     if ((threadIdx.x & 31) == 0 && dangling != 0.0) atomicAdd(&ls->dangling[p], dangling);
@@ -307,8 +319,9 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_dang_arg(const PrArgs& a, const Loop
     return ff_from_double((1.0 - a.alpha) + a.alpha * pr_ld<PERSIST>(&ls->dangling[p]));
   } else if constexpr (MODE == PR_ADJ32) {
     return ff_from_double(pr_ld<PERSIST>(&ls->dangling[p]));
+  } else if constexpr (pr_fused<MODE>()) {
+    return FF{0.f, 0.f};
   } else {
-    if (MODE < PR_NORM32) return 0.0;
     const double d = pr_ld<PERSIST>(&ls->dangling[p]);
     return MODE == PR_NORM64 ? d / (double)a.n : d;
   }
@@ -332,18 +345,18 @@ __device__ __forceinline__ PrOld pr_load_old(const PrArgs& a, uint64_t v, unsign
   return o;
 }
 
-// The update of target v (pr_finish); returns |change| for the FP64 residual.
+// The FP64 weighted forms' update of target v; returns |change|.
 template <int MODE, bool PERSIST>
-__device__ __forceinline__ double pr_apply(const PrArgs& a, uint64_t v, double sum, unsigned p, double dang,
-                                           double* rsum, unsigned* nact) {
-  if (MODE == PR_W64) {
+__device__ __forceinline__ double pr_apply_w64(const PrArgs& a, uint64_t v, double sum, unsigned p, double dang,
+                                               double* rsum) {
+  if constexpr (MODE == PR_W64) {
     const double tv = a.tele ? a.tele[v] : 1.0 / (double)a.n;
     const double nv = tv * ((1.0 - a.alpha) + a.alpha * dang) + a.alpha * sum;
     const double* r = (p == 0) ? a.r64 : a.r64n;
     double* rn = (p == 0) ? a.r64n : a.r64;
     rn[v] = nv;
     return fabs(nv - pr_ld<PERSIST>(r + v));
-  } else if (MODE == PR_ADJ64) {
+  } else {
     // v is a source here: lambda'_v = c_v + alpha ((P^T lambda)_v + a_v (t . lambda))
     const double s = a.wsum[v];
     const double ptv = s > 0.0 ? sum / s : 0.0;
@@ -354,41 +367,17 @@ __device__ __forceinline__ double pr_apply(const PrArgs& a, uint64_t v, double s
     a.pt64[v] = ptv;
     *rsum += (a.tele ? a.tele[v] : 1.0 / (double)a.n) * nl;  // t . lambda of the next round
     return fabs(nl - pr_ld<PERSIST>(l + v));
-  } else {
-    // PageRank-delta: residual round or delta round, rank += change (compensated)
-    const float rank_v = pr_ld<PERSIST>(a.rank + v);
-    const float comp_v = pr_ld<PERSIST>(a.comp + v);
-    float change;
-    if (MODE == PR_DELTA_RESIDUAL) {
-      change = (float)((1.0 - a.alpha) + a.alpha * sum - (double)rank_v - (double)comp_v);
-    } else {
-      change = (sum == 0.0) ? 0.f : (float)(a.alpha * sum);
-    }
-    a.delta[v] = change;
-    // Kahan: rank + comp carries the exact running sum of the changes
-    const float y = change + comp_v;
-    const float t = rank_v + y;
-    a.comp[v] = y - (t - rank_v);
-    a.rank[v] = t;
-    *rsum += (double)change;
-    // v stays active (contributes delta / outdeg next round) while |delta| > delta_param * rank
-    const bool act = change != 0.f && (double)fabsf(change) > a.delta_param * (double)t;
-    *nact += act ? 1u : 0u;
-    const uint32_t dg = a.deg[v];
-    a.contrib[(uint64_t)(p ^ 1u) * a.n + v] = (act && dg) ? change / (float)dg : 0.f;
-    return fabs((double)change);
   }
 }
 
-// A thread's share of a round's totals: FP64 residual (sum of |change|), rank sum and
-// the vertices activated for the next round (PageRank-delta). Flushed once per block
-// (pr_tally_flush).
+// A thread's share of a round's totals: the residual (sum of |change|), a second sum
+// (PageRank-delta: the rank changes; adjoint: t . lambda) and the vertices activated for the
+// next round (PageRank-delta). Flushed once per block (pr_tally_flush).
 struct PrTally {
-  double resid, rsum;
-  FF fres;  // FP32-compensated forms: the residual in float-float
-  FF ftd;   // FP32 adjoint: t . lambda in float-float (FP64 adjoint: rsum)
+  double resid, rsum;  // FP64 forms; the FP32 forms' infinities
+  FF fres, fsum;       // FP32 forms, in float-float
   unsigned nact;
-  __device__ __forceinline__ void init() { resid = rsum = 0.0, fres = ftd = FF{0.f, 0.f}, nact = 0u; }
+  __device__ __forceinline__ void init() { resid = rsum = 0.0, fres = fsum = FF{0.f, 0.f}, nact = 0u; }
 };
 
 // The normalised forms' update of v from its sum and its rank before the round; the
@@ -457,11 +446,37 @@ __device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum
     a.pt[v] = pv;
     change = isfinite(nl - old) ? ff_two_sum(nl, -old) : FF{nl - old, 0.f};
     const FF td = ff_mul(tv, FF{nl, 0.f});
-    if (isfinite(td.hi)) t.ftd = ff_add(t.ftd, td);
+    if (isfinite(td.hi)) t.fsum = ff_add(t.fsum, td);
     else t.rsum += (double)(tv.hi * nl);
   }
   if (isfinite(change.hi)) t.fres = ff_add(t.fres, ff_abs(change));
   else t.resid += (double)fabsf(change.hi);
+}
+
+// PageRank-delta: residual round or delta round, rank += change (compensated). v stays active
+// (contributes change / outdeg to the next round) while |change| > delta_param * rank.
+template <int MODE, bool PERSIST>
+__device__ __forceinline__ void pr_apply_delta(const PrArgs& a, uint64_t v, FF sum, unsigned p, PrTally& t) {
+  const float rank_v = pr_ld<PERSIST>(a.rank + v);
+  const float comp_v = pr_ld<PERSIST>(a.comp + v);
+  const uint32_t dg = a.deg[v];
+  float change;
+  if (MODE == PR_DELTA_RESIDUAL)
+    change = ff_add(ff_add(a.rest_ff, ff_mul(a.alpha_ff, sum)), ff_two_sum(-rank_v, -comp_v)).hi;
+  else
+    change = ff_mul(a.alpha_ff, sum).hi;
+  a.delta[v] = change;
+  // Kahan: rank + comp carries the exact running sum of the changes
+  const float y = change + comp_v;
+  const float r = rank_v + y;
+  a.comp[v] = y - (r - rank_v);
+  a.rank[v] = r;
+  t.fsum = ff_add(t.fsum, FF{change, 0.f});
+  const FF thr = ff_mul(a.delta_ff, FF{r, 0.f});
+  const bool act = change != 0.f && ff_add(FF{fabsf(change), 0.f}, FF{-thr.hi, -thr.lo}).hi > 0.f;
+  t.nact += act ? 1u : 0u;
+  a.contrib[(uint64_t)(p ^ 1u) * a.n + v] = (act && dg) ? change / (float)dg : 0.f;
+  t.fres = ff_add(t.fres, FF{fabsf(change), 0.f});
 }
 
 // Applies the finished sum of target v and adds its share to the tally. The fused form
@@ -474,8 +489,10 @@ __device__ __forceinline__ void pr_finish(const PrArgs& a, uint64_t v, pr_ff_t<M
     pr_apply_norm<MODE>(a, v, sum, p, dang, pr_load_old<MODE, PERSIST>(a, v, p), t);
   else if constexpr (MODE == PR_W32 || MODE == PR_ADJ32)
     pr_apply_w32<MODE, PERSIST>(a, v, sum, p, dang, t);
+  else if constexpr (pr_fused<MODE>())
+    pr_apply_delta<MODE, PERSIST>(a, v, sum, p, t);
   else
-    t.resid += pr_apply<MODE, PERSIST>(a, v, sum, p, dang, &t.rsum, &t.nact);
+    t.resid += pr_apply_w64<MODE, PERSIST>(a, v, sum, p, dang, &t.rsum);
 }
 
 // The block's tally into the loop state: one atomic per quantity and block (every
@@ -494,10 +511,10 @@ __device__ __forceinline__ void pr_tally_flush(LoopState* ls, unsigned p, PrTall
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       t.fres = ff_add(t.fres, FF{__shfl_xor_sync(0xFFFFFFFFu, t.fres.hi, o), __shfl_xor_sync(0xFFFFFFFFu, t.fres.lo, o)});
-      if (MODE == PR_ADJ32)
-        t.ftd = ff_add(t.ftd, FF{__shfl_xor_sync(0xFFFFFFFFu, t.ftd.hi, o), __shfl_xor_sync(0xFFFFFFFFu, t.ftd.lo, o)});
+      if (kS)
+        t.fsum = ff_add(t.fsum, FF{__shfl_xor_sync(0xFFFFFFFFu, t.fsum.hi, o), __shfl_xor_sync(0xFFFFFFFFu, t.fsum.lo, o)});
     }
-    if (MODE != PR_NORM32 && __any_sync(0xFFFFFFFFu, t.resid != 0.0 || t.rsum != 0.0)) {  // infinities, NaN
+    if ((MODE == PR_W32 || MODE == PR_ADJ32) && __any_sync(0xFFFFFFFFu, t.resid != 0.0 || t.rsum != 0.0)) {  // infinities, NaN
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         t.resid += __shfl_xor_sync(0xFFFFFFFFu, t.resid, o);
@@ -505,7 +522,7 @@ __device__ __forceinline__ void pr_tally_flush(LoopState* ls, unsigned p, PrTall
       }
     }
     t.resid += (double)t.fres.hi + (double)t.fres.lo;
-    if (MODE == PR_ADJ32) t.rsum += (double)t.ftd.hi + (double)t.ftd.lo;
+    if (kS) t.rsum += (double)t.fsum.hi + (double)t.fsum.lo;
   } else {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t.resid += __shfl_xor_sync(0xFFFFFFFFu, t.resid, o);
@@ -570,12 +587,11 @@ __device__ __forceinline__ void pr_lane_sum(const PrArgs& a, const pr_val_t<MODE
   }
 }
 
-// A compensated FP32 sum as the update takes it: the float pair itself in the
-// FP32-compensated forms, s + e in FP64 in PageRank-delta.
+// A compensated FP32 sum as the update takes it: the float pair itself.
 template <int MODE>
 __device__ __forceinline__ pr_ff_t<MODE> pr_acc32_out(float s, float e) {
   if constexpr (pr_ff<MODE>()) return FF{s, e};
-  else return (double)s + (double)e;
+  else return (double)s + (double)e;  // never taken
 }
 
 // Sum of target v's in-edge contributions by one thread (in-degree <= 4), in edge order.
@@ -625,7 +641,7 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_sum_group(const PrArgs& a, const pr_
   }
 }
 
-// The same by a whole block (in-degree > 4096: RMAT hubs; up to 1024 threads); thread 0
+// The same by a whole block (in-degrees past the warp bin: RMAT hubs; up to 1024 threads); thread 0
 // returns the sum. Every thread of the block calls it.
 template <int MODE, bool PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_sum_block(const PrArgs& a, const pr_val_t<MODE>* cr, uint32_t v) {
