@@ -12,7 +12,7 @@
 //    take the contributions the previous pull wrote) and the target bins of its pull;
 //  - a block claims a unit of any job with one 64-bit atomic on that job's claim word
 //    [phase : 8][units : 24][next unit : 32], so the phase and its size travel with the
-//    claim;
+//    claim; while it works on a unit it claims the next one of the same job and phase;
 //  - the block that completes the last unit of a phase (a per-phase completion
 //    counter) runs the job's control step — the same device code as the one-job
 //    executors (minprop_dev.cuh, pagerank_dev.cuh) — and publishes the next phase;
@@ -20,7 +20,10 @@
 //    words again (bounded: after kIdleLimit empty polls in a row -- or the limit a test
 //    sets through cytom_set_fault_injection -- it records a timeout and exits, so the
 //    launch always ends).
-// Values written during the launch are read through L2 (the PERSIST load policy).
+// Values written during the launch are read with ordinary loads (the PERSIST load policy 2):
+// the phase that wrote them has ended, and the claim that opened the reading one, with its
+// fence, orders them. Gathered PageRank contributions so hit in L1 (64 jobs: 45.2 -> 43.0 ms
+// a pass against loads through L2).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
@@ -112,7 +115,10 @@ __device__ __forceinline__ uint32_t pr_pull_units(const BJob* J) {
 // of the hub bin), so the longest units start first and the short ones fill the phase's
 // tail.
 __device__ __forceinline__ uint32_t pr_pull_order(const BJob* J, uint32_t unit) { return pr_pull_units(J) - 1u - unit; }
-
+// The units of the hub and warp bins, the first of that order.
+__device__ __forceinline__ uint32_t pr_uneven_units(const BJob* J) {
+  return ceil_div(J->nb[kPrBins - 1], pr_bin_unit(kPrBins - 1)) + ceil_div(J->nb[kPrBins - 2], pr_bin_unit(kPrBins - 2));
+}
 
 // ---- units -----------------------------------------------------------------
 
@@ -129,7 +135,7 @@ __device__ void unit_apply(const BJob* J, bool initial, uint32_t unit) {
   const uint64_t base0 = (uint64_t)unit * BU_APPLY_WORDS;
   for (uint32_t k = 0; k < BU_APPLY_WORDS / BT; ++k) {
     const uint64_t base = base0 + (uint64_t)k * BT;
-    if (base < nwords) apply_step<true>(jd, sd, pw, base, cnt, teps, est);
+    if (base < nwords) apply_step<2>(jd, sd, pw, base, cnt, teps, est);
   }
   apply_flush<BT>(jd->ls, pw, cnt, teps, est);
 }
@@ -139,7 +145,7 @@ __device__ void unit_dense(const BJob* J, uint32_t st) {
   const JobDesc* jd = J->jd;
   const StoreDesc* sd = J->sd;
   const unsigned p = ls_iter(jd->ls) & 1u;
-  if (!stage_active<true>(jd, sd, st, p, J->adaptive)) return;
+  if (!stage_active<2>(jd, sd, st, p, J->adaptive)) return;
   const uint64_t e0 = (uint64_t)st * SG_E;
   // two half-stages of 8 edges per thread: the persistent kernel's register budget is
   // set by its largest unit, and a 16-edge stage would cap it at two blocks per SM
@@ -147,7 +153,7 @@ __device__ void unit_dense(const BJob* J, uint32_t st) {
   for (uint32_t h = 0; h < 2; ++h) {
     const uint64_t st8 = 2ull * st + h, h0 = st8 * (SG_E / 2);
     if (h0 >= sd->E) break;
-    dense_stage<ALGO, true, true, 8>(jd, sd, sd->edges + h0, mp_weighted<ALGO>() ? sd->wts + h0 : nullptr, st8, p,
+    dense_stage<ALGO, 2, true, 8>(jd, sd, sd->edges + h0, mp_weighted<ALGO>() ? sd->wts + h0 : nullptr, st8, p,
                                      J->adaptive);
   }
   if (threadIdx.x == 0) {
@@ -165,7 +171,7 @@ __device__ void unit_sparse(const BJob* J, uint32_t unit) {
   const uint64_t g = (uint64_t)unit * BU_SPARSE_ITEMS + (threadIdx.x >> 5) * 32;
   unsigned long long scanned = 0;
   uint32_t nread = 0;  // items read: the one-job kernels' byte accounting, not kept here
-  if (g < items) scanned = sparse_group<ALGO, true>(jd, sd, g, items, nread);
+  if (g < items) scanned = sparse_group<ALGO, 2>(jd, sd, g, items, nread);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) scanned += __shfl_xor_sync(0xFFFFFFFFu, scanned, o);
   if ((threadIdx.x & 31) == 0 && scanned) atomicAdd(&jd->ls->edges_scanned, scanned);
@@ -181,7 +187,7 @@ __device__ void unit_chunks(const BJob* J, uint32_t unit) {
   if (nq > jd->spq_cap) nq = jd->spq_cap;
   const uint64_t q = (uint64_t)unit * BU_CHUNKS + (threadIdx.x >> 5);
   uint32_t scanned = 0;
-  if (q < nq) scanned = sparse_chunk<ALGO, true>(jd, sd, q, items);
+  if (q < nq) scanned = sparse_chunk<ALGO, 2>(jd, sd, q, items);
   if ((threadIdx.x & 31) == 0 && scanned) atomicAdd(&jd->ls->edges_scanned, (unsigned long long)scanned);
 }
 
@@ -191,7 +197,7 @@ __device__ void unit_pr_contrib(const BJob* J, uint32_t unit) {
   const unsigned p = ls_iter(a.ls) & 1u;
   const uint64_t lo = (uint64_t)unit * BU_PR_VERTS;
   const uint64_t hi = std::min<uint64_t>(lo + BU_PR_VERTS, a.n);
-  const pr_ff_t<MODE> dangling = pr_contrib_range<MODE, true>(a, p, lo, hi, threadIdx.x, BT);
+  const pr_ff_t<MODE> dangling = pr_contrib_range<MODE, 2>(a, p, lo, hi, threadIdx.x, BT);
   pr_dangling_flush<MODE>(a.ls, p, dangling);
 }
 
@@ -210,8 +216,8 @@ __device__ __forceinline__ void pull_groups(const PrArgs& a, const pr_val_t<MODE
       lo = a.csc_ptr[v];
       hi = a.csc_ptr[v + 1];
     }
-    const pr_ff_t<MODE> sum = pr_sum_group<MODE, true, VW>(a, cr, lo, hi, gl);
-    if (gl == 0 && i < cnt) pr_finish<MODE, true>(a, v, sum, p, dang, t);
+    const pr_ff_t<MODE> sum = pr_sum_group<MODE, 2, VW>(a, cr, lo, hi, gl);
+    if (gl == 0 && i < cnt) pr_finish<MODE, 2>(a, v, sum, p, dang, t);
   }
 }
 
@@ -220,7 +226,7 @@ __device__ void unit_pr_pull(const BJob* J, uint32_t unit) {
   const PrArgs& a = J->pr;
   LoopState* ls = a.ls;
   const unsigned p = ls_iter(ls) & 1u;
-  const pr_ff_t<MODE> dang = pr_dang_arg<MODE, true>(a, ls, p);
+  const pr_ff_t<MODE> dang = pr_dang_arg<MODE, 2>(a, ls, p);
   // the bin this unit belongs to
   int k = 0;
   uint64_t off = 0;
@@ -243,8 +249,8 @@ __device__ void unit_pr_pull(const BJob* J, uint32_t unit) {
         const uint64_t i = first + (uint64_t)r * BT + threadIdx.x;
         if (i < cnt) {
           const uint32_t v = a.bins[off + i];
-          const pr_ff_t<MODE> sum = pr_sum_thread<MODE, true>(a, cr, v);
-          pr_finish<MODE, true>(a, v, sum, p, dang, t);
+          const pr_ff_t<MODE> sum = pr_sum_thread<MODE, 2>(a, cr, v);
+          pr_finish<MODE, 2>(a, v, sum, p, dang, t);
         }
       }
       break;
@@ -253,8 +259,8 @@ __device__ void unit_pr_pull(const BJob* J, uint32_t unit) {
     case 32: pull_groups<MODE, 32>(a, cr, off, cnt, first, p, dang, t); break;
     default: {
       const uint32_t v = a.bins[off + first];
-      const pr_ff_t<MODE> sum = pr_sum_block<MODE, true>(a, cr, v);
-      if (threadIdx.x == 0) pr_finish<MODE, true>(a, v, sum, p, dang, t);
+      const pr_ff_t<MODE> sum = pr_sum_block<MODE, 2>(a, cr, v);
+      if (threadIdx.x == 0) pr_finish<MODE, 2>(a, v, sum, p, dang, t);
     }
   }
   pr_tally_flush<MODE>(ls, p, t);
@@ -362,7 +368,7 @@ __device__ __forceinline__ void pr_lane_sum_pair(const PrArgs& a, const pr_pair_
     for (int k = 0; k < B; ++k) {
       const uint32_t ek = e + (uint32_t)k * stride;
       if (ek < hi) {
-        c[k] = __ldcg(cp + id[k]);
+        c[k] = cp[id[k]];
       } else {
         c[k].x = 0;
         c[k].y = 0;
@@ -472,8 +478,8 @@ struct PairFinish {
   pr_ff_t<MODE> dang0, dang1;
   PrTally t0, t1;
   __device__ __forceinline__ void old(uint32_t v, PrOld& o0, PrOld& o1) const {
-    if (on0) o0 = pr_load_old<MODE, true>(a0, v, p0);
-    if (on1) o1 = pr_load_old<MODE, true>(a1, v, p1);
+    if (on0) o0 = pr_load_old<MODE, 2>(a0, v, p0);
+    if (on1) o1 = pr_load_old<MODE, 2>(a1, v, p1);
   }
   __device__ __forceinline__ void operator()(uint32_t v, pr_ff_t<MODE> s0, pr_ff_t<MODE> s1, PrOld o0, PrOld o1) {
     if (on0) pr_apply_norm<MODE>(a0, v, s0, p0, dang0, o0, t0);
@@ -517,7 +523,7 @@ __device__ __forceinline__ void pair_small(const PrArgs& a0, const pr_pair_t<MOD
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         if (lo[2 * h + t] + (uint32_t)k < hi[2 * h + t]) {
-          c[t][k] = __ldcg(cp + id[t][k]);
+          c[t][k] = cp[id[t][k]];
         } else {
           c[t][k].x = 0;
           c[t][k].y = 0;
@@ -586,8 +592,8 @@ __device__ void unit_pr_pull_pair(const BJob* J, uint32_t unit) {
   fin.on1 = pr_on(a1.ls);
   fin.p0 = ls_iter(a0.ls) & 1u;
   fin.p1 = ls_iter(a1.ls) & 1u;
-  fin.dang0 = pr_dang_arg<MODE, true>(a0, a0.ls, fin.p0);
-  fin.dang1 = pr_dang_arg<MODE, true>(a1, a1.ls, fin.p1);
+  fin.dang0 = pr_dang_arg<MODE, 2>(a0, a0.ls, fin.p0);
+  fin.dang1 = pr_dang_arg<MODE, 2>(a1, a1.ls, fin.p1);
   fin.t0.init();
   fin.t1.init();
   int k = 0;
@@ -668,7 +674,7 @@ __device__ void advance(const BJob* J, BSched* S, BCtl* ctl, unsigned phase) {
   if (!pr && (phase == PH_APPLY0 || phase == PH_APPLY) && s_cont) {
     // open the next round (all threads clear the row flags), then pick its gather
     const unsigned p = ls_iter(jd->ls) & 1u;
-    round_open<true>(jd, sd, p, J->adaptive, threadIdx.x, BT);
+    round_open<2>(jd, sd, p, J->adaptive, threadIdx.x, BT);
     __syncthreads();
     if (threadIdx.x == 0) {
       const unsigned mode = *(volatile unsigned*)&jd->ls->mode;
@@ -765,7 +771,7 @@ __device__ void run_unit(const BJob* J, unsigned phase, uint32_t unit, int prmod
 __global__ void __launch_bounds__(BT, 5) batch_kernel(const BJob* __restrict__ jobs, BSched* sched, BCtl* ctl,
                                                         int njobs) {
   __shared__ int s_job, s_state, s_last, s_mode;
-  __shared__ unsigned s_unit, s_total, s_phase;
+  __shared__ unsigned s_unit, s_total, s_phase, s_ahead[2];
   int cursor = (int)(blockIdx.x % (unsigned)njobs);
   unsigned idle = 0;
   unsigned long long done_units = 0;
@@ -838,18 +844,39 @@ __global__ void __launch_bounds__(BT, 5) batch_kernel(const BJob* __restrict__ j
     }
     const int jb = s_job;
     const BJob* J = jobs + jb;
-    run_unit(J, s_phase, s_unit, s_mode);
-    __syncthreads();
+    const unsigned phase = s_phase, total = s_total;
+    const int mode = s_mode;
+    unsigned unit = s_unit;
+    // Units of this job and phase, one after another. The next one is claimed while the
+    // current one runs, so neither its claim nor the completion of the current one is waited
+    // for; while it is held, the phase cannot end. Not past a unit of a pull's hub or warp
+    // bin: those are long and of uneven length, and a block held up by one would hold another.
+    const unsigned uneven = phase == PH_PR_PULL ? pr_uneven_units(J) : 0u;
+    for (int k = 0;; k ^= 1) {
+      unsigned long long ahead = ~0ULL;
+      if (threadIdx.x == 0 && unit >= uneven) ahead = atomicAdd(&sched[jb].claim, 1ULL);
+      run_unit(J, phase, unit, mode);
+      if (threadIdx.x == 0) {
+        s_ahead[k] = (unsigned)ahead < total ? (unsigned)ahead : 0xFFFFFFFFu;
+        ++done_units;
+      }
+      __syncthreads();
+      unit = s_ahead[k];
+      if (unit == 0xFFFFFFFFu) break;
+      if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&sched[jb].done, 1u);
+      }
+    }
     if (threadIdx.x == 0) {
       __threadfence();
       const unsigned d = atomicAdd(&sched[jb].done, 1u);
-      s_last = (d + 1 == s_total) ? 1 : 0;
-      ++done_units;
+      s_last = (d + 1 == total) ? 1 : 0;
     }
     __syncthreads();
     if (s_last) {
       __threadfence();
-      advance(J, sched + jb, ctl, s_phase);
+      advance(J, sched + jb, ctl, phase);
     }
     cursor = jb;
   }
@@ -967,6 +994,11 @@ static int batch_run(Ctx* const* ctxs, const int* job_ids, int count, cytom_run_
       hs[k].claim = (j->params.max_iterations > 0) ? pack_claim(PH_PR_CONTRIB, (unsigned)units)
                                                    : pack_claim(PH_DONE, 0);
     } else {
+      // the heavy items of its sparse rounds go to the job's chunk queue; without one (a job
+      // that cytom_run never prepared) a single warp walked each hub: BFS on RMAT-21 3.9 ms
+      // instead of 1.0
+      rc = ensure_job_queue(c, j);
+      if (rc) return rc;
       b.begin = 1;
       const uint64_t units = (((c->n + 31) >> 5) + BU_APPLY_WORDS - 1) / BU_APPLY_WORDS;
       const uint64_t stages = (c->E + SG_E - 1) / SG_E;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(APPLY_T) apply_minprop_kernel(const JobDesc* _
   unsigned long long teps = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nwords; base += stride)
-    apply_step<false>(jd, sd, pw, base, cnt, teps, est);
+    apply_step<0>(jd, sd, pw, base, cnt, teps, est);
   apply_flush<APPLY_T>(ls, pw, cnt, teps, est);
   if (threadIdx.x == 0) {
     __threadfence();
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(APPLY_T) apply_minprop_kernel(const JobDesc* _
 // lane l takes edges [4l, 4l+4) of it with one 128-bit load. The tile of an edge is found
 // from the chunk's first tile and tile_ptr (edges are tile-major). Returns the edges scanned
 // (lane 0).
-template <int ALGO, bool PERSIST>
+template <int ALGO, int PERSIST>
 __device__ __forceinline__ uint32_t dense_chunk(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                                 uint64_t c, unsigned p, int adaptive) {
   const uint64_t T = sd->T;
@@ -174,13 +174,13 @@ __global__ void __launch_bounds__(GATHER_T) gather_minprop_kernel(const JobDesc*
   LoopState* ls = jd->ls;
   if (!ls->cont || ls->mode != 0) return;
   const unsigned p = ls->iter & 1u;
-  round_open<false>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
+  round_open<0>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
   const uint64_t nchunks = sd->nchunks;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long scanned = 0;
-  for (uint64_t c = warp; c < nchunks; c += nwarps) scanned += dense_chunk<ALGO, false>(jd, sd, c, p, adaptive);
+  for (uint64_t c = warp; c < nchunks; c += nwarps) scanned += dense_chunk<ALGO, 0>(jd, sd, c, p, adaptive);
   // edges-scanned counter
   __shared__ unsigned long long s_sc[GATHER_T / 32];
   if ((threadIdx.x & 31) == 0) s_sc[threadIdx.x >> 5] = scanned;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(SG_T, MINB) gather_stream_kernel(const JobDesc
   LoopState* ls = jd->ls;
   if (!ls->cont || ls->mode != 0) return;
   const unsigned p = ls->iter & 1u;
-  round_open<false>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
+  round_open<0>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
   const uint32_t* __restrict__ edges = sd->edges;
   const uint32_t* __restrict__ wts = sd->wts;
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(SG_T, MINB) gather_stream_kernel(const JobDesc
     return ((s >> lgrp) + G) << lgrp;
   };
   auto next_active = [&](uint64_t s) -> uint64_t {
-    while (s < nst && !stage_active<false, EPT>(jd, sd, s, p, adaptive)) s = advance(s);
+    while (s < nst && !stage_active<0, EPT>(jd, sd, s, p, adaptive)) s = advance(s);
     return s < nst ? s : nst;
   };
   auto issue = [&](int slot, uint64_t s) {
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(SG_T, MINB) gather_stream_kernel(const JobDesc
         const uint64_t rem = E - cur * SE;
         scanned += rem < (uint64_t)SE ? rem : (uint64_t)SE;
       }
-      dense_stage<ALGO, false, false, EPT>(jd, sd, ebuf + slot * SE, wbuf + slot * SE, cur, p, adaptive);
+      dense_stage<ALGO, 0, false, EPT>(jd, sd, ebuf + slot * SE, wbuf + slot * SE, cur, p, adaptive);
     }
     if (__syncthreads_or(!ok)) {  // every thread is done with this slot
       failed = true;
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(TS_T, 1) gather_tiles_kernel(const JobDesc* __
   LoopState* ls = jd->ls;
   if (!ls->cont || ls->mode != 0) return;
   const unsigned p = ls->iter & 1u;
-  round_open<false>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
+  round_open<0>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
   constexpr bool WT = mp_weighted<ALGO>();
   const uint32_t lvpt = sd->lvpt, lT = sd->lT;
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(TS_T, 1) gather_tiles_kernel(const JobDesc* __
 
   auto next_active = [&](uint32_t s) -> uint32_t {
     if (adaptive)
-      while (s < se && ld_plain<false>(rows_cur + (stages[s].tile >> lT)) == 0) ++s;
+      while (s < se && ld_plain<0>(rows_cur + (stages[s].tile >> lT)) == 0) ++s;
     return s;
   };
   auto issue = [&](int slot, uint32_t s) {
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(TS_T, 1) gather_tiles_kernel(const JobDesc* __
       const uint32_t x = st.tile >> lT;
       const uint32_t xb = x << lvpt, yb = y << lvpt;
       const uint32_t off = (uint32_t)(st.e0 & 3ULL), endp = off + st.count;
-      const bool full_row = !adaptive || ld_plain<false>(rows_cur + x) == vpt;
+      const bool full_row = !adaptive || ld_plain<0>(rows_cur + x) == vpt;
       const uint32_t* eb = ebuf + slot * TS_BUF;
       const uint32_t* wb = wbuf + slot * TS_BUF;
       uint32_t qv[8], ww[8], uu[8];
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(TS_T, 1) gather_tiles_kernel(const JobDesc* __
       if (!full_row && vmask) {
         uint32_t fw[8];
 #pragma unroll
-        for (int idx = 0; idx < 8; ++idx) fw[idx] = ((vmask >> idx) & 1u) ? ld_state<false>(fa + (uu[idx] >> 5)) : 0u;
+        for (int idx = 0; idx < 8; ++idx) fw[idx] = ((vmask >> idx) & 1u) ? ld_state<0>(fa + (uu[idx] >> 5)) : 0u;
         amask = 0;
 #pragma unroll
         for (int idx = 0; idx < 8; ++idx) amask |= ((fw[idx] >> (uu[idx] & 31)) & 1u) << idx;
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(TS_T, 1) gather_tiles_kernel(const JobDesc* __
       if (amask) {
         uint32_t cand[8];
 #pragma unroll
-        for (int idx = 0; idx < 8; ++idx) cand[idx] = ((amask >> idx) & 1u) ? ld_src<false>(jd, async, uu[idx]) : kInf;
+        for (int idx = 0; idx < 8; ++idx) cand[idx] = ((amask >> idx) & 1u) ? ld_src<0>(jd, async, uu[idx]) : kInf;
 #pragma unroll
         for (int idx = 0; idx < 8; ++idx)
           if (cand[idx] != kInf) cand[idx] = mp_cand<ALGO>(cand[idx], ww[idx]);
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(256, 4) gather_sparse_kernel(const JobDesc* __
   LoopState* ls = jd->ls;
   if (!ls->cont || ls->mode != 1) return;
   const unsigned p = ls->iter & 1u;
-  round_open<false>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
+  round_open<0>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(256, 4) gather_sparse_kernel(const JobDesc* __
   while (nslice < 8 && groups * nslice * 2 <= nwarps) nslice *= 2;
   const uint32_t slice = (uint32_t)(warp % nslice);
   for (uint64_t g = (warp / nslice) * 32; g < items; g += (nwarps / nslice) * 32)
-    scanned += sparse_group<ALGO, false>(jd, sd, g, items, nread, slice, nslice);
+    scanned += sparse_group<ALGO, 0>(jd, sd, g, items, nread, slice, nslice);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     scanned += __shfl_xor_sync(0xFFFFFFFFu, scanned, o);
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(256, 4) gather_sparse_chunks(const JobDesc* __
   if (nq > jd->spq_cap) nq = jd->spq_cap;
   const uint64_t items = (uint64_t)ls->nact_words[ls->iter & 1u] << sd->lT;
   unsigned long long scanned = 0;
-  for (uint64_t q = warp; q < nq; q += nwarps) scanned += sparse_chunk<ALGO, false>(jd, sd, q, items);
+  for (uint64_t q = warp; q < nq; q += nwarps) scanned += sparse_chunk<ALGO, 0>(jd, sd, q, items);
   if (lane == 0 && scanned) atomicAdd(&ls->edges_scanned, scanned);
 }
 
@@ -1005,18 +1005,18 @@ __global__ void __launch_bounds__(SM_T, 1)
         while (nslice < 8 && groups * nslice * 2 <= nwarps) nslice *= 2;
         const uint32_t slice = warp % nslice;
         for (uint64_t g = (uint64_t)(warp / nslice) * 32; g < items; g += (uint64_t)(nwarps / nslice) * 32)
-          scanned += sparse_group<ALGO, true, SM_ILP, true>(jd, sd, g, items, nread, slice, nslice);
+          scanned += sparse_group<ALGO, 1, SM_ILP, true>(jd, sd, g, items, nread, slice, nslice);
         cluster_barrier();
         uint64_t nq = __ldcg(&ls->spq_count);
         if (nq) {  // the same in every CTA: the queue is complete and CTA 0 resets it past the next barrier
           if (nq > jd->spq_cap) nq = jd->spq_cap;
-          for (uint64_t q = warp; q < nq; q += nwarps) scanned += sparse_chunk<ALGO, true>(jd, sd, q, items);
+          for (uint64_t q = warp; q < nq; q += nwarps) scanned += sparse_chunk<ALGO, 1>(jd, sd, q, items);
           cluster_barrier();
           if (tid == 0) ls->spq_count = 0;
         }
       } else {
         for (uint64_t c = warp; c < sd->nchunks; c += nwarps)
-          scanned += dense_chunk<ALGO, true>(jd, sd, c, p, adaptive);
+          scanned += dense_chunk<ALGO, 1>(jd, sd, c, p, adaptive);
         cluster_barrier();
       }
     }

@@ -630,7 +630,7 @@ __global__ void pr_contrib_kernel(PrArgs a) {
   LoopState* ls = a.ls;
   if (!ls->cont) return;
   const unsigned p = ls->iter & 1u;
-  const pr_ff_t<MODE> dangling = pr_contrib_range<MODE, false>(a, p, 0, a.n, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
+  const pr_ff_t<MODE> dangling = pr_contrib_range<MODE, 0>(a, p, 0, a.n, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                                                         (uint64_t)gridDim.x * blockDim.x);
   pr_dangling_flush<MODE>(ls, p, dangling);
 }
@@ -643,8 +643,8 @@ __device__ __forceinline__ void pull_small_body(const PrArgs& a, const pr_val_t<
     const uint64_t i = base + threadIdx.x;
     if (i < a.bin_count) {
       const uint32_t v = a.bins[a.bin_off + i];
-      const pr_ff_t<MODE> sum = pr_sum_thread<MODE, false>(a, cr, v);
-      pr_finish<MODE, false>(a, v, sum, p, dang, t);
+      const pr_ff_t<MODE> sum = pr_sum_thread<MODE, 0>(a, cr, v);
+      pr_finish<MODE, 0>(a, v, sum, p, dang, t);
     }
   }
 }
@@ -685,8 +685,8 @@ __device__ __forceinline__ void pull_group_body(const PrArgs& a, const pr_val_t<
         lo = a.csc_ptr[v];
         hi = a.csc_ptr[v + 1];
       }
-      const pr_ff_t<MODE> sum = pr_sum_group<MODE, false, VW>(a, cr, lo, hi, gl);
-      if (gl == 0 && i < a.bin_count) pr_finish<MODE, false>(a, v, sum, p, dang, t);
+      const pr_ff_t<MODE> sum = pr_sum_group<MODE, 0, VW>(a, cr, lo, hi, gl);
+      if (gl == 0 && i < a.bin_count) pr_finish<MODE, 0>(a, v, sum, p, dang, t);
     }
     return;
   }
@@ -707,10 +707,10 @@ __device__ __forceinline__ void pull_group_body(const PrArgs& a, const pr_val_t<
     for (unsigned r = 0; r < S; ++r) {
       const int src = (int)(r * GPW + g);
       const uint32_t l = __shfl_sync(0xFFFFFFFFu, lo, src), h = __shfl_sync(0xFFFFFFFFu, hi, src);
-      const pr_ff_t<MODE> x = pr_shfl(pr_sum_group<MODE, false, VW>(a, cr, l, h, gl), (int)((lane & (GPW - 1)) * VW));
+      const pr_ff_t<MODE> x = pr_shfl(pr_sum_group<MODE, 0, VW>(a, cr, l, h, gl), (int)((lane & (GPW - 1)) * VW));
       if (lane / GPW == r) mine = x;
     }
-    if (own) pr_finish<MODE, false>(a, v, mine, p, dang, t);
+    if (own) pr_finish<MODE, 0>(a, v, mine, p, dang, t);
   }
 }
 
@@ -719,8 +719,8 @@ __device__ __forceinline__ void pull_large_body(const PrArgs& a, const pr_val_t<
                                                 uint64_t bid, uint64_t nblk, PrTally& t) {
   for (uint64_t i = bid; i < a.bin_count; i += nblk) {
     const uint32_t v = a.bins[a.bin_off + i];
-    const pr_ff_t<MODE> sum = pr_sum_block<MODE, false>(a, cr, v);
-    if (threadIdx.x == 0) pr_finish<MODE, false>(a, v, sum, p, dang, t);
+    const pr_ff_t<MODE> sum = pr_sum_block<MODE, 0>(a, cr, v);
+    if (threadIdx.x == 0) pr_finish<MODE, 0>(a, v, sum, p, dang, t);
   }
 }
 
@@ -800,7 +800,7 @@ __global__ void __launch_bounds__(PR_T, pr_min_blocks<MODE>()) pr_pull_kernel(Pr
   const uint32_t total = live ? blp->blocks : 0u;
   // one thread's FP64 conversion of the dangling term, not every thread's
   __shared__ pr_ff_t<MODE> s_dang;
-  if (threadIdx.x == 0) s_dang = pr_dang_arg<MODE, false>(a, ls, p);
+  if (threadIdx.x == 0) s_dang = pr_dang_arg<MODE, 0>(a, ls, p);
   __syncthreads();
   const pr_ff_t<MODE> dang = s_dang;
   const pr_val_t<MODE>* cr = pr_cread<MODE>(a, p);

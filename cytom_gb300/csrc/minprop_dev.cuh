@@ -11,10 +11,12 @@
 //   control — the convergence test and the swap of the active bitmaps
 //             (continuous-algorithm-executor.h:193-218).
 //
-// Load policy: the one-job kernels read state written by earlier launches through the
-// read-only path (PERSIST = false). The persistent kernel writes that state in the same
-// launch on other SMs, so it reads every mutable word through L2 (PERSIST = true);
-// the L1 of an SM is not coherent with stores of other SMs within a launch.
+// Load policy (PERSIST): the one-job kernels read state written by earlier launches through
+// the read-only path (0). The cluster kernel of the small rounds writes that state in the same
+// launch on other SMs and reads every mutable word through L2 (1). The batched executor also
+// writes it in the same launch, but a block reads it only in a phase that it entered by a
+// claim and a fence after the phase that wrote it had ended, so ordinary loads see it and may
+// hit in L1 (2); words that change within a phase (next) are read through L2 by all.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,16 +33,17 @@ constexpr int SG_E = 4096;    // edges per dense stage
 static_assert(SG_E == SG_T * 16, "16 edges per thread per stage");
 
 // Loads of data that a launch may have written (current values, frontier, changed bits,
-// row flags): read-only cache path across launches, L2 within a persistent launch.
-template <bool PERSIST, class T>
+// row flags).
+template <int PERSIST, class T>
 __device__ __forceinline__ T ld_state(const T* p) {
-  if constexpr (PERSIST) return __ldcg(p);
+  if constexpr (PERSIST == 1) return __ldcg(p);
+  else if constexpr (PERSIST == 2) return *p;
   else return __ldg(p);
 }
 // The same for words that the one-job kernels also read with plain loads.
-template <bool PERSIST, class T>
+template <int PERSIST, class T>
 __device__ __forceinline__ T ld_plain(const T* p) {
-  if constexpr (PERSIST) return __ldcg(p);
+  if constexpr (PERSIST == 1) return __ldcg(p);
   else return *p;
 }
 
@@ -67,7 +70,7 @@ __device__ __forceinline__ uint32_t mp_cand(uint32_t c, uint32_t w) {
 // would do: next only decreases during a round and never exceeds current. Reading the
 // one-job kernels' pre-checks through L1 instead measured 2-3 % slower on the RMAT-22
 // stream's dense SSSP rounds.)
-template <bool PERSIST>
+template <int PERSIST>
 __device__ __forceinline__ uint32_t ld_next(const uint32_t* p) {
   return __ldcg(p);
 }
@@ -76,7 +79,7 @@ __device__ __forceinline__ uint32_t ld_next(const uint32_t* p) {
 // cc-async.cc: ASYNC = true) pull from next[src], which other blocks lower during the
 // round (algorithm-executor.h:303-312); read through L2, a value is either the one at
 // the round's start or a lower one, and both are valid bounds.
-template <bool PERSIST>
+template <int PERSIST>
 __device__ __forceinline__ uint32_t ld_src(const JobDesc* __restrict__ jd, bool async, uint64_t u) {
   if (async) return __ldcg(jd->next + u);
   return ld_state<PERSIST>(jd->cur + u);
@@ -89,7 +92,7 @@ __device__ __forceinline__ unsigned long long row_edges(const StoreDesc* sd, uin
 // Opening of gather round p: clears the next parity's row flags (threads tid, tid+nthr,
 // ...) and, on thread 0, the next parity's counters; adds the round's processed-edge
 // count (edges of tile rows with an active source, algorithm-executor.h:424-426).
-template <bool PERSIST>
+template <int PERSIST>
 __device__ __forceinline__ void round_open(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                            unsigned p, int adaptive, uint64_t tid, uint64_t nthr) {
   LoopState* ls = jd->ls;
@@ -187,7 +190,7 @@ __device__ __forceinline__ unsigned pick_mode(const JobDesc* __restrict__ jd, co
 // test is skipped). A warp covers 32 consecutive words; when they share one row
 // (vpt >= 1024) it adds its row count with a single atomic. The non-zero frontier
 // words are listed (warp-ballot compaction) for sparse rounds.
-template <bool PERSIST>
+template <int PERSIST>
 __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                            unsigned pw, uint64_t base, unsigned& cnt, unsigned long long& teps,
                                            unsigned& est) {
@@ -365,7 +368,7 @@ __device__ __forceinline__ void minprop_begin_state(LoopState* ls, unsigned max_
 // with an active source look up their target tile. Target updates are fire-and-forget
 // red.min / red.or: a candidate below the value read is below current[v] too
 // (next <= current), so next[v] ends the round below current[v] and v changed.
-template <int ALGO, bool PERSIST, bool FROM_GLOBAL, int EPT = 16>
+template <int ALGO, int PERSIST, bool FROM_GLOBAL, int EPT = 16>
 __device__ __forceinline__ void dense_stage(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                             const uint32_t* eb, const uint32_t* wb, uint64_t st, unsigned p,
                                             int adaptive) {
@@ -528,7 +531,7 @@ __device__ __forceinline__ void dense_stage(const JobDesc* __restrict__ jd, cons
 }
 
 // Whether stage st holds an edge of an active tile row (adaptive scheduling).
-template <bool PERSIST, int EPT = 16>
+template <int PERSIST, int EPT = 16>
 __device__ __forceinline__ bool stage_active(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                              uint64_t st, unsigned p, int adaptive) {
   if (!adaptive) return true;
@@ -572,7 +575,7 @@ struct SpItem {
 };
 
 // Item (word w, tile column y): its frontier bits, directory range and tile base.
-template <bool PERSIST>
+template <int PERSIST>
 __device__ __forceinline__ SpItem sp_item_at(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                              uint32_t w, uint32_t y) {
   const uint32_t lT = sd->lT, lnbw = sd->lvpt - 5, nbw = sd->nbw;
@@ -589,7 +592,7 @@ __device__ __forceinline__ SpItem sp_item_at(const JobDesc* __restrict__ jd, con
   return r;
 }
 
-template <bool PERSIST>
+template <int PERSIST>
 __device__ __forceinline__ SpItem sp_item(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                           uint64_t it) {
   const uint32_t w = ld_plain<PERSIST>(jd->aw + (it >> sd->lT));
@@ -600,7 +603,7 @@ __device__ __forceinline__ SpItem sp_item(const JobDesc* __restrict__ jd, const 
 // loads of all ILP edges are issued before any of them is used.
 // LAT: a target's value is loaded beside the source's, for every edge with an active source
 // (one dependent step less; otherwise only for edges that offer a value).
-template <int ALGO, bool PERSIST, int ILP, bool LAT = false>
+template <int ALGO, int PERSIST, int ILP, bool LAT = false>
 __device__ __forceinline__ void sp_batch(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                          const uint32_t (&xs)[ILP], const uint32_t (&ys)[ILP],
                                          const uint32_t (&bits)[ILP], const unsigned long long (&pos)[ILP],
@@ -712,7 +715,7 @@ __device__ __forceinline__ void sp_narrow_wide(const StoreDesc* __restrict__ sd,
 // alone queues the heavy ones, and the light edges are dealt out in steps of 32 * ILP
 // (slice k takes steps k, k + nslice, ...); if the queue overflowed, slice 0 walks every
 // light edge itself (the others' share is then walked twice, which changes nothing).
-template <int ALGO, bool PERSIST, int ILP = SP_ILP, bool WIDE = false>
+template <int ALGO, int PERSIST, int ILP = SP_ILP, bool WIDE = false>
 __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                                  uint64_t g, uint64_t items, uint32_t& nread,
                                                  uint32_t slice = 0, uint32_t nslice = 1) {
@@ -801,7 +804,7 @@ __device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd,
 // Queue entry q (a chunk of a heavy item) for the calling warp; returns the edges walked
 // (lane 0). Sources are sorted inside an item, so a chunk whose first and last edges
 // span no source of the item's frontier word is skipped after two loads.
-template <int ALGO, bool PERSIST>
+template <int ALGO, int PERSIST>
 __device__ __forceinline__ uint32_t sparse_chunk(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                                  uint64_t q, uint64_t items) {
   const unsigned lane = threadIdx.x & 31;

@@ -14,8 +14,8 @@
 // (residual) round needs a contribution pass. The PAGERANK forms keep the pass: at RMAT
 // scale 26 their pull's scattered per-target writes cost more than the pass's streamed ones.
 //
-// Load policy as in minprop_dev.cuh: PERSIST = the persistent kernel, which reads every
-// value written in the same launch (ranks, contributions) through L2.
+// Load policy as in minprop_dev.cuh: the batched executor (PERSIST = 2) reads values written
+// in the same launch (ranks, contributions) with ordinary loads, after a claim and a fence.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -205,9 +205,9 @@ inline void pr_args_ff(PrArgs& a) {
 template <int MODE>
 using pr_ff_t = typename std::conditional<pr_ff<MODE>(), FF, double>::type;
 
-template <bool PERSIST, class T>
+template <int PERSIST, class T>
 __device__ __forceinline__ T pr_ld(const T* p) {
-  if constexpr (PERSIST) return __ldcg(p);
+  if constexpr (PERSIST == 1) return __ldcg(p);
   else return *p;
 }
 
@@ -224,7 +224,7 @@ __device__ __forceinline__ const pr_val_t<MODE>* pr_cread(const PrArgs& a, unsig
 
 // Contribution of in-edge e with source s: cr[s], times the edge's raw weight in the
 // weighted modes (an FP32 product in the FP32 modes).
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ pr_val_t<MODE> pr_cval(const PrArgs& a, const pr_val_t<MODE>* cr, uint32_t e, uint32_t s) {
   const pr_val_t<MODE> c = pr_ld<PERSIST>(cr + s);
   if constexpr (pr_weighted<MODE>()) return c * (pr_val_t<MODE>)a.csc_w[e];
@@ -236,7 +236,7 @@ __device__ __forceinline__ pr_val_t<MODE> pr_cval(const PrArgs& a, const pr_val_
 // its later rounds take the previous pull's contributions) and every round of the
 // other forms.
 // Returns the thread's share of the dangling mass (PAGERANK).
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_contrib_range(const PrArgs& a, unsigned p, uint64_t lo, uint64_t hi,
                                                           uint64_t tid, uint64_t nthr) {
   pr_ff_t<MODE> dangling{};
@@ -311,7 +311,7 @@ __device__ __forceinline__ void pr_dangling_flush(LoopState* ls, unsigned p, pr_
 // The round's dangling term as pr_finish takes it: D / n (normalised PageRank), D
 // (weighted FP64: scaled by t_v in pr_finish), (1 - alpha) + alpha D (weighted FP32),
 // t . lambda (adjoint), none (PageRank-delta).
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_dang_arg(const PrArgs& a, const LoopState* ls, unsigned p) {
   if constexpr (MODE == PR_NORM32) {
     return ff_mul(ff_from_double(pr_ld<PERSIST>(&ls->dangling[p])), a.inv_n_ff);
@@ -333,7 +333,7 @@ struct PrOld {
   double d;
   float hi, lo;
 };
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ PrOld pr_load_old(const PrArgs& a, uint64_t v, unsigned p) {
   PrOld o{};
   if constexpr (MODE == PR_NORM32) {
@@ -346,7 +346,7 @@ __device__ __forceinline__ PrOld pr_load_old(const PrArgs& a, uint64_t v, unsign
 }
 
 // The FP64 weighted forms' update of target v; returns |change|.
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ double pr_apply_w64(const PrArgs& a, uint64_t v, double sum, unsigned p, double dang,
                                                double* rsum) {
   if constexpr (MODE == PR_W64) {
@@ -407,7 +407,7 @@ __device__ __forceinline__ void pr_apply_norm(const PrArgs& a, uint64_t v, pr_ff
 // float pair. PR_ADJ32 (v is a source): lambda'_v = c_v + alpha ((P^T lambda)_v + a_v (t . lambda)),
 // kept as a float; its share of the next round's t . lambda joins the tally. Float pairs
 // turn an infinity into NaN, so a result that is not finite is taken in FP64 instead.
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum, unsigned p, FF dang, PrTally& t) {
   FF tv = a.inv_n_ff;
   if (a.tele2) {
@@ -455,7 +455,7 @@ __device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum
 
 // PageRank-delta: residual round or delta round, rank += change (compensated). v stays active
 // (contributes change / outdeg to the next round) while |change| > delta_param * rank.
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ void pr_apply_delta(const PrArgs& a, uint64_t v, FF sum, unsigned p, PrTally& t) {
   const float rank_v = pr_ld<PERSIST>(a.rank + v);
   const float comp_v = pr_ld<PERSIST>(a.comp + v);
@@ -482,7 +482,7 @@ __device__ __forceinline__ void pr_apply_delta(const PrArgs& a, uint64_t v, FF s
 // Applies the finished sum of target v and adds its share to the tally. The fused form
 // also writes v's contribution to the next round (half p^1), exactly as the
 // contribution pass would compute it from the new delta.
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ void pr_finish(const PrArgs& a, uint64_t v, pr_ff_t<MODE> sum, unsigned p,
                                           pr_ff_t<MODE> dang, PrTally& t) {
   if constexpr (MODE == PR_NORM32 || MODE == PR_NORM64)
@@ -557,7 +557,7 @@ __device__ __forceinline__ void pr_tally_flush(LoopState* ls, unsigned p, PrTall
 // One lane's ordered sum of the in-edges e0, e0 + stride, ... below hi into acc: the
 // source ids of B edges, then their B contributions in flight, the next B ids loaded
 // while those contributions arrive (one dependent L2 round trip per B edges).
-template <int MODE, bool PERSIST, int B, class Acc>
+template <int MODE, int PERSIST, int B, class Acc>
 __device__ __forceinline__ void pr_lane_sum(const PrArgs& a, const pr_val_t<MODE>* cr, uint32_t e0, uint32_t hi,
                                             uint32_t stride, Acc& acc) {
   // 32-bit edge indices: the CSC holds fewer than 2^32 - 2^20 edges (build_csx), so
@@ -595,7 +595,7 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_acc32_out(float s, float e) {
 }
 
 // Sum of target v's in-edge contributions by one thread (in-degree <= 4), in edge order.
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_sum_thread(const PrArgs& a, const pr_val_t<MODE>* cr, uint32_t v) {
   const uint32_t lo = a.csc_ptr[v], hi = a.csc_ptr[v + 1];
   if constexpr (pr_is64<MODE>()) {
@@ -615,7 +615,7 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_sum_thread(const PrArgs& a, const pr
 // warp; every lane of the warp calls it, an idle group with lo = hi): lane gl of the
 // group sums edges lo+gl, lo+gl+VW, ... in order, then the group merges its lanes by an
 // xor tree. Every lane of the group returns the sum.
-template <int MODE, bool PERSIST, int VW>
+template <int MODE, int PERSIST, int VW>
 __device__ __forceinline__ pr_ff_t<MODE> pr_sum_group(const PrArgs& a, const pr_val_t<MODE>* cr, uint32_t lo, uint32_t hi,
                                                unsigned gl) {
   constexpr int B = 4;
@@ -643,7 +643,7 @@ __device__ __forceinline__ pr_ff_t<MODE> pr_sum_group(const PrArgs& a, const pr_
 
 // The same by a whole block (in-degrees past the warp bin: RMAT hubs; up to 1024 threads); thread 0
 // returns the sum. Every thread of the block calls it.
-template <int MODE, bool PERSIST>
+template <int MODE, int PERSIST>
 __device__ __forceinline__ pr_ff_t<MODE> pr_sum_block(const PrArgs& a, const pr_val_t<MODE>* cr, uint32_t v) {
   __shared__ float s_s[32], s_e[32];
   __shared__ double s_d[32];
