@@ -85,36 +85,45 @@ static void rmat_threshold(double t, unsigned long long* h, int* all) {
   *h = lo;
 }
 
-__device__ __forceinline__ bool below(uint64_t v, const RmatThr& t, int k) {
-  return t.all[k] ? true : (v < t.h[k]);
+// hash64 with its shift-and-add steps as multiplications (a + (a << 12) = 4097 a, a + (a << 3)
+// = 9 a): one wide multiply-add and one 32-bit one each, on the pipe that the rest of the
+// hash leaves idle.
+__device__ __forceinline__ uint64_t hash64_mad(uint64_t a) {
+  a = a * 4097ULL + 0x7ed55d166bef7a1dULL;
+  a = (a ^ 0xc761c23c510fa2ddULL) ^ (a >> 9);
+  a = (a + 0x165667b183a9c0e1ULL) + (a << 59);
+  a = (a + 0xd3a2646cab3487e3ULL) ^ (a << 49);
+  a = a * 9ULL + 0xfd7046c5ef9ab54cULL;
+  a = (a ^ 0xb55a4f090dd4a67bULL) ^ (a >> 32);
+  return a;
 }
 
+// One edge per thread and step; `scale` hashes per edge: bound by integer instructions. The
+// thresholds ascend (rmat_generate sees to that), so the quadrant of hash h is the number of
+// thresholds at or below it: the source bit is h >= h1, the target bit the parity of the three
+// comparisons (12.5 M edges of scale 22 with weights: 645 -> 448 us). ALL: some threshold lies above every hash (RmatThr::all).
+template <bool ALL>
 __global__ void rmat_kernel(RmatThr thr, uint32_t scale, uint64_t hseed, uint64_t first,
                             uint64_t count, uint32_t* __restrict__ src, uint32_t* __restrict__ tgt,
                             uint32_t* __restrict__ w, uint64_t wseed_h, uint32_t wmin,
                             uint64_t wspan) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t t0 = thr.h[0], t1 = thr.h[1], t2 = thr.h[2];
+  const uint32_t m0 = ALL && thr.all[0] ? 0u : 1u, m1 = ALL && thr.all[1] ? 0u : 1u, m2 = ALL && thr.all[2] ? 0u : 1u;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += stride) {
     uint64_t index = first + k;
-    uint64_t rs = hash64(2ULL * index * hseed);
+    uint64_t r = hash64(2ULL * index * hseed);
     uint64_t st = hash64((2ULL * index + 1ULL) * hseed);
     // bit j (value 2^j) uses hash(rs + (scale-1-j)*st): the most significant bit
     // uses hash(rs), as rMatIterative walks back from the finest level.
     uint32_t es = 0, et = 0;
-    uint64_t r = rs;
-    for (int j = (int)scale - 1; j >= 0; --j) {
-      uint64_t h = hash64(r);
+#pragma unroll 2
+    for (uint32_t j = 0; j < scale; ++j) {
+      const uint64_t h = hash64_mad(r);
       r += st;
-      uint32_t bit = 1u << j;
-      if (below(h, thr, 0)) {
-      } else if (below(h, thr, 1)) {
-        et |= bit;
-      } else if (below(h, thr, 2)) {
-        es |= bit;
-      } else {
-        es |= bit;
-        et |= bit;
-      }
+      const uint32_t c0 = h >= t0 ? m0 : 0u, c1 = h >= t1 ? m1 : 0u, c2 = h >= t2 ? m2 : 0u;
+      es = es * 2u + c1;
+      et = et * 2u + (c0 ^ c1 ^ c2);
     }
     src[k] = es;
     tgt[k] = et;
@@ -141,10 +150,17 @@ int rmat_generate(Ctx* c, const cytom_rmat_params* p, uint64_t first, uint64_t c
   rmat_threshold(a_, &thr.h[0], &thr.all[0]);
   rmat_threshold(ab_, &thr.h[1], &thr.all[1]);
   rmat_threshold(abc_, &thr.h[2], &thr.all[2]);
+  // the walk takes the first threshold above the hash, so a later one below it never counts
+  for (int k = 1; k < 3; ++k) {
+    if (thr.all[k - 1]) thr.all[k] = 1;
+    else if (!thr.all[k]) thr.h[k] = std::max(thr.h[k], thr.h[k - 1]);
+  }
+  const bool all = thr.all[0] || thr.all[1] || thr.all[2];
   uint64_t hseed = hash64(p->seed);
   uint64_t wspan = (uint64_t)p->wmax - (uint64_t)p->wmin + 1ULL;
   int slot = prof_begin(c, KC_RMAT);
-  rmat_kernel<<<grid_for(c, count, 256, 16), 256, 0, c->stream>>>(
+  auto fn = all ? rmat_kernel<true> : rmat_kernel<false>;
+  fn<<<grid_for(c, count, 256, 16), 256, 0, c->stream>>>(
       thr, p->scale, hseed, first, count, src, tgt, (p->wmax > 0) ? w : nullptr,
       hash64(p->weight_seed), p->wmin, wspan);
   c->launches++;
@@ -192,15 +208,6 @@ int gridgraph_decode(Ctx* c, const void* dbytes, uint64_t m, uint32_t* src, uint
 // --------------------------------------------------------------------------
 // Insert
 // --------------------------------------------------------------------------
-__global__ void validate_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ tgt,
-                                uint64_t count, uint64_t n, unsigned int* bad) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  unsigned int nb = 0;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride)
-    nb += (src[i] >= n || tgt[i] >= n) ? 1u : 0u;
-  if (nb) atomicAdd(bad, nb);
-}
-
 // Composite key: [x : lT][y : lT][src_local : lvpt][tgt_local : lvpt].
 __device__ __forceinline__ uint64_t make_key(uint32_t s, uint32_t t, uint32_t lvpt, uint32_t lT) {
   uint64_t m = (1ULL << lvpt) - 1ULL;
@@ -209,32 +216,44 @@ __device__ __forceinline__ uint64_t make_key(uint32_t s, uint32_t t, uint32_t lv
   return (tile << (2 * lvpt)) | (((uint64_t)s & m) << lvpt) | ((uint64_t)t & m);
 }
 
-// Appends one batch to the append region and counts degrees. Degree increments
-// are warp-aggregated: lanes holding the same vertex elect one leader that adds
-// the group's size (RMAT hubs repeat often within a warp).
-// Appends the batch and counts its degrees -- unless validate_kernel, earlier on the same
-// stream, found an endpoint out of range: then the whole batch is rejected and nothing
-// is written, so the host reads the verdict once, after both kernels.
+// Appends one batch to the append region and counts its degrees, checking every endpoint: an
+// edge with an endpoint out of range is left out and counted in *bad. The host then rejects
+// the whole batch (append_undo_kernel takes its degrees back; the keys lie past the region's
+// end). One pass over the batch instead of a checking pass before; the degree atomics are
+// one per endpoint: aggregating a warp's equal vertices first (two __match_any_sync an edge)
+// took longer than the atomics it saved. Bound by the atomics (16.8 M edges, ids without
+// order: 320 -> 262 us; 12.5 M RMAT edges, whose hubs share sectors, 417 -> 385; 20,011
+// edges 14.2 -> 8.7).
 __global__ void append_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ tgt,
-                              const uint32_t* __restrict__ w, uint64_t count,
+                              const uint32_t* __restrict__ w, uint64_t count, uint64_t n,
                               uint64_t* __restrict__ keys, uint32_t* __restrict__ kw,
                               uint32_t* __restrict__ out_deg, uint32_t* __restrict__ in_deg,
-                              uint32_t lvpt, uint32_t lT, const unsigned int* __restrict__ bad) {
-  if (*bad) return;
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const unsigned lane = threadIdx.x & 31;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < count; base += stride) {
-    uint64_t i = base + threadIdx.x;
-    bool valid = i < count;
-    unsigned vmask = __ballot_sync(0xFFFFFFFFu, valid);
-    if (!valid) continue;
-    uint32_t s = src[i], t = tgt[i];
+                              uint32_t lvpt, uint32_t lT, unsigned int* __restrict__ bad) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  unsigned nb = 0;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
+    const uint32_t s = src[i], t = tgt[i];
+    if (s >= n || t >= n) {
+      ++nb;
+      continue;
+    }
     keys[i] = make_key(s, t, lvpt, lT);
     if (w) kw[i] = w[i];
-    unsigned ps = __match_any_sync(vmask, s);
-    if ((__ffs(ps) - 1) == (int)lane) atomicAdd(&out_deg[s], (uint32_t)__popc(ps));
-    unsigned pt = __match_any_sync(vmask, t);
-    if ((__ffs(pt) - 1) == (int)lane) atomicAdd(&in_deg[t], (uint32_t)__popc(pt));
+    atomicAdd(&out_deg[s], 1u);
+    atomicAdd(&in_deg[t], 1u);
+  }
+  if (nb) atomicAdd(bad, nb);
+}
+
+// Takes back the degrees of a rejected batch.
+__global__ void append_undo_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ tgt, uint64_t count,
+                                   uint64_t n, uint32_t* __restrict__ out_deg, uint32_t* __restrict__ in_deg) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
+    const uint32_t s = src[i], t = tgt[i];
+    if (s >= n || t >= n) continue;
+    atomicSub(&out_deg[s], 1u);
+    atomicSub(&in_deg[t], 1u);
   }
 }
 
@@ -310,25 +329,26 @@ int insert_device(Ctx* c, const uint32_t* src, const uint32_t* tgt, const uint32
   if (e != cudaSuccess) return cuda_err(c, e, "memset");
   int rc = ensure_app_capacity(c, c->A + count);
   if (rc) return rc;
-  int slot = prof_begin(c, KC_INSERT);
-  validate_kernel<<<grid_for(c, count, 256), 256, 0, c->stream>>>(src, tgt, count, c->n, c->d_flag);
-  c->launches++;
-  prof_end(c, slot, (double)count * 8.0);
   const uint32_t* wuse = (c->wtype != CYTOM_UNWEIGHTED) ? w : nullptr;
-  slot = prof_begin(c, KC_INSERT);
+  int slot = prof_begin(c, KC_INSERT);
   append_kernel<<<grid_for(c, count, 256), 256, 0, c->stream>>>(
-      src, tgt, wuse, count, c->app_keys + c->A, wuse ? c->app_w + c->A : nullptr, c->out_deg,
+      src, tgt, wuse, count, c->n, c->app_keys + c->A, wuse ? c->app_w + c->A : nullptr, c->out_deg,
       c->in_deg, c->lvpt, c->lT, c->d_flag);
   c->launches++;
   prof_end(c, slot, (double)count * (wuse ? 28.0 : 24.0));
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "append_kernel");
-  // one wait: the batch's copies (host path), validation and append
+  // one wait: the batch's copies (host path) and the append
   e = cudaMemcpyAsync(c->h_pinned, c->d_flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "insert");
-  if (*(unsigned int*)c->h_pinned)
+  if (*(unsigned int*)c->h_pinned) {
+    append_undo_kernel<<<grid_for(c, count, 256), 256, 0, c->stream>>>(src, tgt, count, c->n, c->out_deg, c->in_deg);
+    c->launches++;
+    e = cudaStreamSynchronize(c->stream);  // the caller's buffers are borrowed for this call only
+    if (e != cudaSuccess) return cuda_err(c, e, "insert");
     return set_err(c, CYTOM_ERR_RANGE, "edge endpoint >= vertex count; batch rejected");
+  }
   // the jobs are seeded by these edges when the compaction installs them
   c->A += count;
   if (c->cfg.use_dynamic_compaction) return dynamic_compaction(c, c->A - count, count);
@@ -742,11 +762,12 @@ __global__ void new_tile_ptr_kernel(const unsigned long long* __restrict__ tile_
 // otherwise old store element o - (number of q below o). One warp produces 32
 // consecutive outputs per step, 1024 per span. merge_spans_kernel gives every span its
 // first new element (sb) and the tile of its first output (ts) by binary searches that
-// all run at once. When a span holds at most 64 new elements (the usual case: new edges
-// are sparse in the store) they sit in two registers per lane and each step finds its
-// candidates by shuffles, so the sources of MG steps are known without memory round
-// trips and their loads issue together; a span with more new elements loads its
-// candidates step by step. Stores are coalesced 128-byte warp writes.
+// all run at once. A warp marks its span's new elements in a 1024-bit map, one word per
+// step: lane k holds step k's word and, by a warp scan, the new elements before it, so the
+// sources of every step are known without further memory round trips and the loads of MG
+// steps issue together, however many elements are new. Stores are coalesced 128-byte warp
+// writes. (Spans with more than 64 new elements used to load their candidates step by step:
+// 12.5 M new edges into 37.5 M, look-up included, 902 -> 703 us; 1 M into 42 M 254 -> 244.)
 //
 // The store is streamed with evict-first loads and stores, leaving L2 to the jobs that
 // run on the installed snapshot meanwhile (the pipelined stream).
@@ -829,6 +850,7 @@ __global__ void merge_gather_kernel(const uint32_t* __restrict__ edges, const ui
                                     const unsigned long long* __restrict__ tp, uint32_t* __restrict__ chunk_tile,
                                     uint32_t* __restrict__ dir, uint32_t nbw, uint32_t* __restrict__ oe,
                                     uint32_t* __restrict__ ow) {
+  __shared__ uint32_t s_map[256 / 32][MERGE_STEPS];
   const uint64_t K = *Kdev;
   const uint64_t total = E + K;
   const unsigned lane = threadIdx.x & 31;
@@ -864,89 +886,68 @@ __global__ void merge_gather_kernel(const uint32_t* __restrict__ edges, const ui
       else plast = edges[wbase - 1 - b0];
     }
     plast = __shfl_sync(0xFFFFFFFFu, plast, 0);
-    if (cnt <= 64) {
-      const uint32_t qa = (lane < cnt) ? (uint32_t)(q[b0 + lane] - wbase) : 0xFFFFFFFFu;
-      const uint32_t qb = (32 + lane < cnt) ? (uint32_t)(q[b0 + 32 + lane] - wbase) : 0xFFFFFFFFu;
-      uint32_t r = 0;  // new elements consumed so far in this span
-      for (int g = 0; g < MERGE_STEPS; g += MG) {
-        if ((uint32_t)g * 32 >= nout) break;
-        uint32_t src[MG];
-        unsigned isnew = 0;
-#pragma unroll
-        for (int k = 0; k < MG; ++k) {
-          const uint32_t o_start = (uint32_t)(g + k) * 32;
-          const uint32_t idx = r + lane;
-          const uint32_t ca = __shfl_sync(0xFFFFFFFFu, qa, idx & 31);
-          const uint32_t cb = __shfl_sync(0xFFFFFFFFu, qb, idx & 31);
-          const uint32_t rel = (idx < 32 ? ca : (idx < 64 ? cb : 0xFFFFFFFFu)) - o_start;
-          const unsigned mask = __reduce_or_sync(0xFFFFFFFFu, rel < 32u ? (1u << rel) : 0u);
-          const uint32_t y = r + __popc(mask & lt);
-          if ((mask >> lane) & 1u) {
-            isnew |= 1u << k;
-            src[k] = y;
-          } else {
-            src[k] = o_start + lane - y;
-          }
-          r += __popc(mask);
-        }
-        uint32_t ev[MG], wv[MG];
-#pragma unroll
-        for (int k = 0; k < MG; ++k) {
-          const uint32_t o = (uint32_t)(g + k) * 32 + lane;
-          ev[k] = 0;
-          wv[k] = 0;
-          if (o < nout) {
-            if ((isnew >> k) & 1u) {
-              ev[k] = nb[src[k]];
-              if (owb) wv[k] = nwb[src[k]];
-            } else {
-              ev[k] = __ldcs(eb + src[k]);
-              if (owb) wv[k] = __ldcs(wb + src[k]);
-            }
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < MG; ++k) {
-          const uint32_t o = (uint32_t)(g + k) * 32 + lane;
-          if (o < nout) {
-            __stcs(oeb + o, ev[k]);
-            if (owb) __stcs(owb + o, wv[k]);
-          }
-          uint32_t pv = __shfl_up_sync(0xFFFFFFFFu, ev[k], 1);
-          if (lane == 0) pv = plast;
-          merge_index_step(o, nout, ev[k], pv, t, toff, tend, wbase, tp, ctb, dir, nbw);
-          plast = __shfl_sync(0xFFFFFFFFu, ev[k], 31);
-        }
-      }
-      continue;
+    uint32_t* bm = s_map[threadIdx.x >> 5];
+    bm[lane] = 0;
+    __syncwarp();
+#pragma unroll 4
+    for (uint32_t i = lane; i < cnt; i += 32) {
+      const uint32_t o = (uint32_t)(q[b0 + i] - wbase);
+      atomicOr(&bm[o >> 5], 1u << (o & 31));
     }
-    uint32_t r = 0;
-    for (int st = 0; st < MERGE_STEPS; ++st) {
-      const uint32_t o_start = (uint32_t)st * 32;
-      if (o_start >= nout) break;
-      const uint32_t cand = (r + lane < cnt) ? (uint32_t)(q[b0 + r + lane] - wbase) : 0xFFFFFFFFu;
-      const uint32_t rel = cand - o_start;
-      const unsigned mask = __reduce_or_sync(0xFFFFFFFFu, rel < 32u ? (1u << rel) : 0u);
-      const uint32_t o = o_start + lane;
-      uint32_t ev = 0, wv = 0;
-      if (o < nout) {
-        const uint32_t y = r + __popc(mask & lt);
+    __syncwarp();
+    const uint32_t word = bm[lane];
+    uint32_t before = __popc(word);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, before, o);
+      if (lane >= (unsigned)o) before += x;
+    }
+    before -= __popc(word);  // new elements of the span before step `lane`
+    for (int g = 0; g < MERGE_STEPS; g += MG) {
+      if ((uint32_t)g * 32 >= nout) break;
+      uint32_t src[MG];
+      unsigned isnew = 0;
+#pragma unroll
+      for (int k = 0; k < MG; ++k) {
+        const unsigned mask = __shfl_sync(0xFFFFFFFFu, word, g + k);
+        const uint32_t y = __shfl_sync(0xFFFFFFFFu, before, g + k) + __popc(mask & lt);
         if ((mask >> lane) & 1u) {
-          ev = nb[y];
-          if (owb) wv = nwb[y];
+          isnew |= 1u << k;
+          src[k] = y;
         } else {
-          ev = __ldcs(eb + (o - y));
-          if (owb) wv = __ldcs(wb + (o - y));
+          src[k] = (uint32_t)(g + k) * 32 + lane - y;
         }
-        __stcs(oeb + o, ev);
-        if (owb) __stcs(owb + o, wv);
       }
-      uint32_t pv = __shfl_up_sync(0xFFFFFFFFu, ev, 1);
-      if (lane == 0) pv = plast;
-      merge_index_step(o, nout, ev, pv, t, toff, tend, wbase, tp, ctb, dir, nbw);
-      plast = __shfl_sync(0xFFFFFFFFu, ev, 31);
-      r += __popc(mask);
+      uint32_t ev[MG], wv[MG];
+#pragma unroll
+      for (int k = 0; k < MG; ++k) {
+        const uint32_t o = (uint32_t)(g + k) * 32 + lane;
+        ev[k] = 0;
+        wv[k] = 0;
+        if (o < nout) {
+          if ((isnew >> k) & 1u) {
+            ev[k] = nb[src[k]];
+            if (owb) wv[k] = nwb[src[k]];
+          } else {
+            ev[k] = __ldcs(eb + src[k]);
+            if (owb) wv[k] = __ldcs(wb + src[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < MG; ++k) {
+        const uint32_t o = (uint32_t)(g + k) * 32 + lane;
+        if (o < nout) {
+          __stcs(oeb + o, ev[k]);
+          if (owb) __stcs(owb + o, wv[k]);
+        }
+        uint32_t pv = __shfl_up_sync(0xFFFFFFFFu, ev[k], 1);
+        if (lane == 0) pv = plast;
+        merge_index_step(o, nout, ev[k], pv, t, toff, tend, wbase, tp, ctb, dir, nbw);
+        plast = __shfl_sync(0xFFFFFFFFu, ev[k], 31);
+      }
     }
+    __syncwarp();  // the map is cleared for the next span
   }
 }
 

@@ -1,0 +1,72 @@
+"""Ingest kernels at their edges: RMAT thresholds that do not ascend or lie above every hash;
+a rejected batch (the only bad endpoint first, last, on either side) leaves keys, counts and
+degrees as they were; merges whose 1,024-output spans hold no, one, 64, 65 or only new edges.
+Against the oracle, bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("abc", [(1.0, 0.0, 0.0), (0.0, 1.0, 0.0), (0.0, 0.0, 1.0), (0.5, -0.2, 0.4), (0.6, 0.3, -0.5),
+                                 (2.0, -1.5, 0.1), (0.0, 0.0, 0.0)])
+def test_rmat_thresholds(cg, orc, abc):
+    a, b, c = abc
+    with cg.Engine(1 << 12, 1024) as eng:
+        gs, gt, _ = eng.generate_rmat(5, 20000, 11, seed=9, a=a, b=b, c=c)
+    s, t = orc.rmat(11, 5, 20000, 9, a=a, b=b, c=c)
+    assert np.array_equal(gs, s) and np.array_equal(gt, t)
+
+
+@pytest.mark.parametrize("where", ["first_src", "last_src", "first_tgt", "last_tgt"])
+@pytest.mark.parametrize("count", [1, 255, 5000])
+def test_rejected_batch_leaves_no_trace(cg, orc, where, count):
+    n, vpt = 1 << 12, 1024
+    rng = np.random.default_rng(count)
+    s, t = (rng.integers(0, n, 3000, dtype=np.uint32) for _ in range(2))
+    bs, bt = (rng.integers(0, n, count, dtype=np.uint32) for _ in range(2))
+    bad = bs if where.endswith("src") else bt
+    bad[0 if where.startswith("first") else -1] = n
+    st = orc.Store(n, vpt)
+    st.insert(s, t)
+    with cg.Engine(n, vpt) as eng:
+        eng.insert_edges(s, t)
+        with pytest.raises(cg.CytomError) as ei:
+            eng.insert_edges(bs, bt)
+        assert ei.value.code == -3
+        assert eng.count_edges() == (0, 3000)
+        assert all(np.array_equal(x, y) for x, y in zip(eng.degrees(), st.degrees()))
+        st.insert(s[::-1].copy(), t)
+        st.compact()
+        eng.insert_edges(s[::-1].copy(), t)
+        eng.do_global_compaction()
+        got, want = eng.dump_tiles(), st.dump()
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        assert all(np.array_equal(x, y) for x, y in zip(eng.degrees(), st.degrees()))
+
+
+@pytest.mark.parametrize("old,new", [(0, 1), (0, 1024), (0, 5000), (1023, 1), (1024, 1), (1025, 2), (40000, 64),
+                                     (40000, 65), (40000, 20000), (100, 40000)])
+def test_merge_spans(cg, orc, old, new):
+    n, vpt = 1 << 11, 512
+    rng = np.random.default_rng(old + new)
+    pick = rng.permutation(n * n)[: old + new].astype(np.int64)  # distinct pairs
+    if (old, new) in ((40000, 64), (40000, 65)):
+        pick[old:] = np.sort(pick[:old])[20000] + 1 + np.arange(new)  # the new edges next to one another
+    s, t = (pick // n).astype(np.uint32), (pick % n).astype(np.uint32)
+    w = orc.edge_weights(s, t, 3, 1, 1000)
+    st = orc.Store(n, vpt, True)
+    with cg.Engine(n, vpt, weight_type=cg.WEIGHT_U32) as eng:
+        bfs = cg.BFS(eng, start_vertex=int(s[0]), max_iterations=1000)
+        for lo, hi in ((0, old), (old, old + new)):
+            if lo == hi:
+                continue
+            st.insert(s[lo:hi], t[lo:hi], w[lo:hi])
+            st.compact()
+            eng.insert_edges(s[lo:hi], t[lo:hi], w[lo:hi])
+            eng.do_global_compaction()
+            got, want = eng.dump_tiles(weights=True), st.dump()
+            for x, y in zip(got, want):
+                assert np.array_equal(x, y)
+            bfs.execute_algorithm()  # the directory and chunk table written by the merge
+            assert np.array_equal(bfs.result(), st.run_minprop(orc.BFS, start=int(s[0]), max_iter=1000)[0])
