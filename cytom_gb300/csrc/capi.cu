@@ -241,6 +241,20 @@ static bool autotune_due(Ctx* c) {
   return env && !c->profiling && c->tune_E == 0 && c->E >= (1ULL << 20);
 }
 
+// The tuned sparse-round threshold of a program class on the current store. A dense round's
+// time grows with the edges and a sparse one's with its frontier, so on a store that has
+// grown since it was tuned the tuner's table is read again with the dense times grown
+// alike (a store tuned at 1 M edges, where no sparse round of the table wins, would keep to
+// dense rounds at 65 M: first pass of the RMAT-22 stream 110 ms, with this rule 86).
+static uint32_t sparse_div_now(const Ctx* c, int cls) {
+  uint32_t div = c->tune_div[cls];
+  if (!div || c->E <= c->tune_E) return div;
+  const double grown = (double)c->E / (double)c->tune_E;
+  for (int k = 0; k < 6 && c->tune_sparse_us[cls][k] < c->tune_dense_us[cls][k] * grown; ++k)
+    div = std::min(div, kDivCandidates[k]);
+  return div;
+}
+
 // Everything a run needs before its loop: pending edges merged, the source directory,
 // the job's sparse queue, the one-time shape tuning, and the initial state of a fresh job.
 static int job_prepare(Ctx* c, Job* j) {
@@ -252,8 +266,8 @@ static int job_prepare(Ctx* c, Job* j) {
     if (!rc && autotune_due(c)) rc = minprop_autotune(c);
     if (!rc && tiles_in_use(c, j->algo)) rc = build_tile_stages(c);
     if (rc) return rc;
-    // the tuned sparse-round threshold of the job's class, read by its control step
-    const uint32_t div = c->tune_div[(j->algo == CYTOM_ALGO_SSSP || j->algo == CYTOM_ALGO_SSWP) ? 1 : 0];
+    // the sparse-round threshold of the job's class, read by its control step
+    const uint32_t div = sparse_div_now(c, (j->algo == CYTOM_ALGO_SSSP || j->algo == CYTOM_ALGO_SSWP) ? 1 : 0);
     if (div != j->h.sparse_div) {
       j->h.sparse_div = div;
       cudaError_t e = cudaMemcpyAsync(j->d, &j->h, sizeof(JobDesc), cudaMemcpyHostToDevice, c->stream);
@@ -1035,8 +1049,7 @@ static void fill_tune_report(const Ctx* c, cytom_tune_report* out) {
       out->sparse_round_us[k][i] = c->tune_sparse_us[k][i];
     }
   }
-  const int32_t divs[6] = {128, 64, 32, 16, 8, 4};
-  for (int i = 0; i < 6; ++i) out->div_candidates[i] = divs[i];
+  for (int i = 0; i < 6; ++i) out->div_candidates[i] = (int32_t)kDivCandidates[i];
 }
 
 int cytom_autotune(cytom_ctx* ctx, cytom_tune_report* out) {

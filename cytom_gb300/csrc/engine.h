@@ -26,6 +26,8 @@ namespace cytom {
 
 constexpr int kChunk = 128;  // edges per warp chunk (32 lanes x uint4)
 constexpr uint32_t kInf = 0xFFFFFFFFu;
+// frontier densities 1/div that the sparse-round threshold is tuned on, in growing density
+constexpr uint32_t kDivCandidates[6] = {128, 64, 32, 16, 8, 4};
 
 // One stage of the column-ordered dense round: `count` (<= 4096) consecutive edges of one
 // tile, starting at edge e0 of the store.

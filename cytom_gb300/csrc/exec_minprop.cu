@@ -1801,8 +1801,6 @@ __global__ void tune_mode_kernel(LoopState* ls, unsigned mode) {
   ls->spq_count = 0;
 }
 
-static const uint32_t kDivCandidates[6] = {128, 64, 32, 16, 8, 4};
-
 static bool sparse_div_from_env() {
   static int v = -1;
   if (v < 0) v = getenv("CYTOM_SPARSE_DIV") ? 1 : 0;
