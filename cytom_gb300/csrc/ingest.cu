@@ -773,10 +773,18 @@ __global__ void new_tile_ptr_kernel(const unsigned long long* __restrict__ tile_
 // run on the installed snapshot meanwhile (the pipelined stream).
 // The same pass writes the chunk table of the new store and, when the context keeps a
 // source directory, its per-edge entries (the work of dir_edges_kernel): each output
-// knows its tile (walked from the span's first tile) and the edge before it.
+// knows its tile (searched from the span's first tile on) and the edge before it. A step
+// inside one tile keeps the tile in uniform registers. Where sources lie thinly an edge
+// starts up to vpt / 32 directory entries: a warp writes long runs together, and tiles of few
+// edges are left to dir_tiles_kernel, or a handful of warps at the corners of the graph hold
+// up the whole merge (SMs active 22 % of its time at 13 M edges of an RMAT-22 stream).
+// The instructions of a step bound it (104 before, 38 without and 60 with a directory), then
+// DRAM: the 64 merges of that stream 14.2 -> 9.3 ms, four merges of 12.5 M new edges
+// 853 -> 597 us; without a directory 37.5 M outputs take 115 us (5.2 TB/s).
 constexpr int MERGE_STEPS = 32;  // 1024 outputs per warp span
 constexpr uint64_t MERGE_SPAN = 32ULL * MERGE_STEPS;
 constexpr int MG = 8;            // steps whose loads are issued together
+constexpr int MG_MINB = 4;       // 5 blocks per SM: 9.9 ms for the stream's merges, 6: 13.3
 
 __global__ void merge_spans_kernel(const unsigned long long* __restrict__ q, const uint32_t* __restrict__ Kdev,
                                    uint64_t E, const unsigned long long* __restrict__ tp, uint64_t ntiles,
@@ -808,55 +816,83 @@ __global__ void merge_spans_kernel(const unsigned long long* __restrict__ q, con
   }
 }
 
-// Per output (offsets relative to the span start): its tile, walked forward from the
+// Directory entries that start at one edge per lane: blocks b0..b1 (none if b0 > b1) of the
+// directory slice at `dt` hold `off`. Called by whole warps: a lane writes a short run by
+// itself, a long one is written by the warp together.
+constexpr int DIR_RUN = 32;
+// Tiles of fewer edges are written by dir_tiles_kernel, a warp each, in place of the kernels
+// that go over the edges.
+constexpr uint32_t DIR_SMALL = 256;  // 1: the stream's merges 12.6 ms; 1024: its dir_tiles 1.8 ms, not 0.8
+
+__device__ __forceinline__ void dir_runs(uint32_t* __restrict__ dir, uint64_t dt, int b0, int b1, uint32_t off) {
+  unsigned lng = __ballot_sync(0xFFFFFFFFu, b1 - b0 >= DIR_RUN);
+  if (b1 - b0 < DIR_RUN)
+    for (int bb = b0; bb <= b1; ++bb) dir[dt + bb] = off;
+  while (lng) {
+    const int j = __ffs(lng) - 1;
+    lng &= lng - 1;
+    const uint64_t d = __shfl_sync(0xFFFFFFFFu, dt, j);
+    const int e = __shfl_sync(0xFFFFFFFFu, b1, j);
+    const uint32_t v = __shfl_sync(0xFFFFFFFFu, off, j);
+    for (int bb = __shfl_sync(0xFFFFFFFFu, b0, j) + (int)(threadIdx.x & 31); bb <= e; bb += 32) dir[d + bb] = v;
+  }
+}
+
+// Per output (offsets relative to the span start): its tile, found forward from the
 // warp's tile state (tile t; toff turns a span offset into an offset within the tile;
-// tend = the span offset where the tile ends), the chunk-table entry at every 128th
-// output, and the directory entries of the 32-source blocks that start at this edge.
-// The tile state of lane 31 carries over to the next step.
+// tend = the span offset where the tile ends; tlast = the tile of the next span's first
+// output), the chunk-table entry at every 128th output, and the directory entries of the
+// 32-source blocks that start at this edge. The tile state of lane 31 carries over to the
+// next step.
 __device__ __forceinline__ void merge_index_step(uint32_t o, uint32_t nout, uint32_t ev, uint32_t pv, uint32_t& t,
-                                                 uint32_t& toff, uint32_t& tend, uint64_t wbase,
+                                                 uint32_t& toff, uint32_t& tend, uint32_t tlast, uint64_t wbase,
                                                  const unsigned long long* __restrict__ tp,
                                                  uint32_t* __restrict__ ctb, uint32_t* __restrict__ dir,
                                                  uint32_t nbw) {
   uint32_t lt = t, loff = toff, lend = tend;
+  int b0 = 0, b1 = -1;
+  uint32_t off = 0;
   if (o < nout) {
-    while (o >= lend) {
-      ++lt;
-      loff = 0u - lend;
+    if (o >= lend) {  // the last tile of (lt, tlast] that starts at or before this output
+      uint32_t lo = lt + 1, hi = tlast;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (tp[mid] <= wbase + o) lo = mid;
+        else hi = mid - 1;
+      }
+      lt = lo;
+      loff = (uint32_t)(wbase - tp[lt]);
       const unsigned long long nx = tp[lt + 1] - wbase;
       lend = nx > 0xFFFFFFFFULL ? 0xFFFFFFFFu : (uint32_t)nx;
     }
     if ((o & (kChunk - 1)) == 0) ctb[o / kChunk] = lt;
-    if (dir) {
-      const uint32_t off = o + loff;
-      const int bk = (int)(ev >> 21);
-      const int bprev = off == 0 ? -1 : (int)(pv >> 21);
-      if (bk != bprev) {
-        uint32_t* dt = dir + (uint64_t)lt * (nbw + 1);
-        for (int bb = bprev + 1; bb <= bk; ++bb) dt[bb] = off;
-      }
+    if (dir && (lend == 0xFFFFFFFFu || lend + loff >= DIR_SMALL)) {
+      off = o + loff;
+      b1 = (int)(ev >> 21);
+      b0 = off == 0 ? 0 : (int)(pv >> 21) + 1;
     }
   }
+  if (dir) dir_runs(dir, (uint64_t)lt * (nbw + 1), b0, b1, off);
   t = __shfl_sync(0xFFFFFFFFu, lt, 31);
   toff = __shfl_sync(0xFFFFFFFFu, loff, 31);
   tend = __shfl_sync(0xFFFFFFFFu, lend, 31);
 }
 
-__global__ void merge_gather_kernel(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ wts,
-                                    uint64_t E, const unsigned long long* __restrict__ q,
-                                    const uint32_t* __restrict__ nloc, const uint32_t* __restrict__ nw,
-                                    const uint32_t* __restrict__ Kdev, const uint32_t* __restrict__ sb,
-                                    const uint32_t* __restrict__ ts, uint64_t nsp,
-                                    const unsigned long long* __restrict__ tp, uint32_t* __restrict__ chunk_tile,
-                                    uint32_t* __restrict__ dir, uint32_t nbw, uint32_t* __restrict__ oe,
-                                    uint32_t* __restrict__ ow) {
-  __shared__ uint32_t s_map[256 / 32][MERGE_STEPS];
+template <bool W, bool DIR>
+__global__ void __launch_bounds__(256, MG_MINB) merge_gather_kernel(
+    const uint32_t* __restrict__ edges, const uint32_t* __restrict__ wts, uint64_t E,
+    const unsigned long long* __restrict__ q, const uint32_t* __restrict__ nloc, const uint32_t* __restrict__ nw,
+    const uint32_t* __restrict__ Kdev, const uint32_t* __restrict__ sb, const uint32_t* __restrict__ ts, uint64_t nsp,
+    const unsigned long long* __restrict__ tp, uint32_t* __restrict__ chunk_tile, uint32_t* __restrict__ dir,
+    uint32_t nbw, uint32_t* __restrict__ oe, uint32_t* __restrict__ ow) {
+  __shared__ uint2 s_map[256 / 32][MERGE_STEPS];  // per step: map word, new elements before it
   const uint64_t K = *Kdev;
   const uint64_t total = E + K;
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lt = (1u << lane) - 1u;
+  uint2* bm = s_map[threadIdx.x >> 5];
   for (uint64_t sp = warp; sp < nsp; sp += nwarps) {
     const uint64_t wbase = sp * MERGE_SPAN;
     if (wbase >= total) break;
@@ -866,13 +902,14 @@ __global__ void merge_gather_kernel(const uint32_t* __restrict__ edges, const ui
     // span-relative views: output x preceded by y new elements of the span comes from
     // eb[x - y] (old) or nb[y] (new)
     const uint32_t* eb = edges + (wbase - b0);
-    const uint32_t* wb = wts ? wts + (wbase - b0) : nullptr;
+    const uint32_t* wb = W ? wts + (wbase - b0) : nullptr;
     const uint32_t* nb = nloc + b0;
-    const uint32_t* nwb = nw ? nw + b0 : nullptr;
+    const uint32_t* nwb = W ? nw + b0 : nullptr;
     uint32_t* oeb = oe + wbase;
-    uint32_t* owb = ow ? ow + wbase : nullptr;
+    uint32_t* owb = W ? ow + wbase : nullptr;
     uint32_t* ctb = chunk_tile + wbase / kChunk;
     uint32_t t = ts[sp];
+    const uint32_t tlast = ts[sp + 1];
     uint32_t toff = (uint32_t)(wbase - tp[t]);
     uint32_t tend;
     {
@@ -881,57 +918,42 @@ __global__ void merge_gather_kernel(const uint32_t* __restrict__ edges, const ui
     }
     // the edge before the span (the first output's predecessor)
     uint32_t plast = 0;
-    if (lane == 0 && wbase > 0) {
+    if (DIR && lane == 0 && wbase > 0) {
       if (b0 > 0 && q[b0 - 1] == wbase - 1) plast = nloc[b0 - 1];
       else plast = edges[wbase - 1 - b0];
     }
-    plast = __shfl_sync(0xFFFFFFFFu, plast, 0);
-    uint32_t* bm = s_map[threadIdx.x >> 5];
-    bm[lane] = 0;
+    bm[lane].x = 0;
     __syncwarp();
 #pragma unroll 4
     for (uint32_t i = lane; i < cnt; i += 32) {
       const uint32_t o = (uint32_t)(q[b0 + i] - wbase);
-      atomicOr(&bm[o >> 5], 1u << (o & 31));
+      atomicOr(&bm[o >> 5].x, 1u << (o & 31));
     }
     __syncwarp();
-    const uint32_t word = bm[lane];
+    const uint32_t word = bm[lane].x;
     uint32_t before = __popc(word);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, before, o);
       if (lane >= (unsigned)o) before += x;
     }
-    before -= __popc(word);  // new elements of the span before step `lane`
+    bm[lane].y = before - __popc(word);
+    __syncwarp();
     for (int g = 0; g < MERGE_STEPS; g += MG) {
       if ((uint32_t)g * 32 >= nout) break;
-      uint32_t src[MG];
-      unsigned isnew = 0;
-#pragma unroll
-      for (int k = 0; k < MG; ++k) {
-        const unsigned mask = __shfl_sync(0xFFFFFFFFu, word, g + k);
-        const uint32_t y = __shfl_sync(0xFFFFFFFFu, before, g + k) + __popc(mask & lt);
-        if ((mask >> lane) & 1u) {
-          isnew |= 1u << k;
-          src[k] = y;
-        } else {
-          src[k] = (uint32_t)(g + k) * 32 + lane - y;
-        }
-      }
       uint32_t ev[MG], wv[MG];
 #pragma unroll
       for (int k = 0; k < MG; ++k) {
         const uint32_t o = (uint32_t)(g + k) * 32 + lane;
+        const uint2 m = bm[g + k];
+        const uint32_t y = m.y + __popc(m.x & lt);
+        const bool fresh = (m.x >> lane) & 1u;
+        const uint32_t i = fresh ? y : o - y;
         ev[k] = 0;
         wv[k] = 0;
         if (o < nout) {
-          if ((isnew >> k) & 1u) {
-            ev[k] = nb[src[k]];
-            if (owb) wv[k] = nwb[src[k]];
-          } else {
-            ev[k] = __ldcs(eb + src[k]);
-            if (owb) wv[k] = __ldcs(wb + src[k]);
-          }
+          ev[k] = __ldcs((fresh ? nb : eb) + i);
+          if (W) wv[k] = __ldcs((fresh ? nwb : wb) + i);
         }
       }
 #pragma unroll
@@ -939,12 +961,25 @@ __global__ void merge_gather_kernel(const uint32_t* __restrict__ edges, const ui
         const uint32_t o = (uint32_t)(g + k) * 32 + lane;
         if (o < nout) {
           __stcs(oeb + o, ev[k]);
-          if (owb) __stcs(owb + o, wv[k]);
+          if (W) __stcs(owb + o, wv[k]);
         }
-        uint32_t pv = __shfl_up_sync(0xFFFFFFFFu, ev[k], 1);
-        if (lane == 0) pv = plast;
-        merge_index_step(o, nout, ev[k], pv, t, toff, tend, wbase, tp, ctb, dir, nbw);
-        plast = __shfl_sync(0xFFFFFFFFu, ev[k], 31);
+        // the predecessor: lane 31's edge comes round to lane 0 for the next step
+        const uint32_t rot = DIR ? __shfl_sync(0xFFFFFFFFu, ev[k], (lane + 31) & 31) : 0u;
+        const uint32_t pv = lane ? rot : plast;
+        plast = rot;
+        if ((uint32_t)(g + k) * 32 + 31 < min(tend, nout)) {  // the whole step inside one tile
+          if ((g + k) % (kChunk / 32) == 0 && lane == 0) ctb[(g + k) / (kChunk / 32)] = t;
+          if (DIR && (tend == 0xFFFFFFFFu || tend + toff >= DIR_SMALL)) {
+            const uint32_t off = o + toff;
+            const int b1 = (int)(ev[k] >> 21);
+            const int bs = off == 0 ? 0 : (int)(pv >> 21) + 1;
+            uint32_t* dt = dir + (uint64_t)t * (nbw + 1);
+            if (bs <= b1) dt[bs] = off;
+            if (__any_sync(0xFFFFFFFFu, bs < b1)) dir_runs(dt, 0, bs + 1, b1, off);
+          }
+        } else {
+          merge_index_step(o, nout, ev[k], pv, t, toff, tend, tlast, wbase, tp, ctb, DIR ? dir : nullptr, nbw);
+        }
       }
     }
     __syncwarp();  // the map is cleared for the next span
@@ -1114,10 +1149,11 @@ int compact(Ctx* c) {
   }
   merge_spans_kernel<<<grid_for(c, nsp + 1, 256), 256, 0, c->stream>>>(q, Kdev, c->E, c->tile_ptr_alt, c->ntiles,
                                                                        nsp, sb, ts, c->chunk_tile_alt);
-  merge_gather_kernel<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>((nsp + 7) / 8, (uint64_t)c->num_sms * 8)),
-                        256, 0, c->stream>>>(c->edges, c->wts, c->E, q, nloc, nw, Kdev, sb, ts, nsp, c->tile_ptr_alt,
-                                             c->chunk_tile_alt, mdir, (uint32_t)(c->vpt / 32), c->edges_alt,
-                                             wt ? c->wts_alt : nullptr);
+  auto* mg = wt ? (mdir ? merge_gather_kernel<true, true> : merge_gather_kernel<true, false>)
+                : (mdir ? merge_gather_kernel<false, true> : merge_gather_kernel<false, false>);
+  mg<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>((nsp + 7) / 8, (uint64_t)c->num_sms * 8)), 256, 0,
+       c->stream>>>(c->edges, c->wts, c->E, q, nloc, nw, Kdev, sb, ts, nsp, c->tile_ptr_alt, c->chunk_tile_alt, mdir,
+                    (uint32_t)(c->vpt / 32), c->edges_alt, wt ? c->wts_alt : nullptr);
   c->launches += 2;
   e = cudaMemcpyAsync(c->h_pinned, Kdev, 4, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1221,35 +1257,38 @@ __global__ void dir_edges_kernel(const StoreDesc* __restrict__ sd, uint32_t* __r
     unsigned long long tlo = sd->tile_ptr[t], thi = sd->tile_ptr[t + 1];
     const uint64_t cend = cbase + kChunk < E ? cbase + kChunk : E;
     if (tlo <= cbase && cend <= thi) {
-      uint32_t* dt = dir + (uint64_t)t * (nbw + 1);
+      if (thi - tlo < DIR_SMALL) continue;
+      const uint64_t dt = (uint64_t)t * (nbw + 1);
       const uint32_t r0 = (uint32_t)(e0 - tlo);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        if (e0 + k >= E) break;
-        const int b = (int)(ev[k + 1] >> 21);
-        const int bprev = (r0 + k == 0) ? -1 : (int)(ev[k] >> 21);
-        for (int bb = bprev + 1; bb <= b; ++bb) dt[bb] = r0 + k;
+        const bool in = e0 + k < E;
+        dir_runs(dir, dt, r0 + k == 0 ? 0 : (int)(ev[k] >> 21) + 1, in ? (int)(ev[k + 1] >> 21) : -1, r0 + k);
       }
       continue;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint64_t e = e0 + k;
-      if (e >= E) break;
-      while (thi <= e) {
-        ++t;
-        tlo = thi;
-        thi = sd->tile_ptr[t + 1];
+      int b0 = 0, b1 = -1;
+      if (e < E) {
+        while (thi <= e) {
+          ++t;
+          tlo = thi;
+          thi = sd->tile_ptr[t + 1];
+        }
+        if (thi - tlo >= DIR_SMALL) {
+          b1 = (int)(ev[k + 1] >> 21);
+          b0 = e == tlo ? 0 : (int)(ev[k] >> 21) + 1;
+        }
       }
-      const int b = (int)((ev[k + 1] >> 16) >> 5);
-      const int bprev = (e == tlo) ? -1 : (int)((ev[k] >> 16) >> 5);
-      if (b == bprev) continue;
-      uint32_t* dt = dir + (uint64_t)t * (nbw + 1);
-      for (int bb = bprev + 1; bb <= b; ++bb) dt[bb] = (uint32_t)(e - tlo);
+      dir_runs(dir, (uint64_t)t * (nbw + 1), b0, b1, (uint32_t)(e - tlo));
     }
   }
 }
 
+// The end of every tile's directory, and all of it for tiles of fewer than DIR_SMALL edges,
+// where an edge may start many blocks. One warp per tile.
 __global__ void dir_tiles_kernel(const StoreDesc* __restrict__ sd, uint32_t* __restrict__ dir, uint32_t nbw) {
   const uint64_t ntiles = sd->ntiles;
   const unsigned lane = threadIdx.x & 31;
@@ -1257,9 +1296,20 @@ __global__ void dir_tiles_kernel(const StoreDesc* __restrict__ sd, uint32_t* __r
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t t = warp; t < ntiles; t += nwarps) {
     const uint64_t lo = sd->tile_ptr[t], hi = sd->tile_ptr[t + 1];
-    const int blast = (hi > lo) ? (int)((sd->edges[hi - 1] >> 16) >> 5) : -1;
-    uint32_t* dt = dir + t * (nbw + 1);
-    for (int bb = blast + 1 + (int)lane; bb <= (int)nbw; bb += 32) dt[bb] = (uint32_t)(hi - lo);
+    const uint32_t m = (uint32_t)(hi - lo);
+    const uint64_t dt = t * (nbw + 1);
+    const int blast = m ? (int)(sd->edges[hi - 1] >> 21) : -1;
+    if (hi - lo < DIR_SMALL) {
+      int prev = -1;
+      for (uint32_t i = 0; i < m; i += 32) {
+        const int b = i + lane < m ? (int)(sd->edges[lo + i + lane] >> 21) : -1;
+        int bp = __shfl_up_sync(0xFFFFFFFFu, b, 1);
+        if (lane == 0) bp = prev;
+        prev = __shfl_sync(0xFFFFFFFFu, b, 31);
+        dir_runs(dir, dt, bp + 1, b, i + lane);
+      }
+    }
+    for (int bb = blast + 1 + (int)lane; bb <= (int)nbw; bb += 32) dir[dt + bb] = m;
   }
 }
 

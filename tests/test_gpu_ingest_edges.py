@@ -70,3 +70,38 @@ def test_merge_spans(cg, orc, old, new):
                 assert np.array_equal(x, y)
             bfs.execute_algorithm()  # the directory and chunk table written by the merge
             assert np.array_equal(bfs.result(), st.run_minprop(orc.BFS, start=int(s[0]), max_iter=1000)[0])
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("size", [1, 31, 255, 256, 257, 1500])
+def test_merge_directory_of_uneven_tiles(cg, orc, size, weighted):
+    """Tiles of `size` edges next to empty ones and to a full one, with source blocks close
+    together and far apart: the directory that merges write and the one built at once lead
+    sparse rounds to the same values."""
+    n, vpt = 1 << 15, 4096
+    rng = np.random.default_rng(size)
+    parts = []
+    for x, y in ((0, 0), (0, 7), (3, 2), (3, 3), (7, 0), (7, 7)):
+        m = 20000 if (x, y) == (3, 3) else size
+        src = rng.integers(0, vpt, m) if y else rng.choice(np.array([0, 31, 32, vpt - 1]), m)
+        parts.append(np.stack([x * vpt + src, y * vpt + rng.integers(0, vpt, m)]))
+    s, t = (a.astype(np.uint32) for a in np.concatenate(parts, 1))
+    order = rng.permutation(len(s))
+    s, t = s[order], t[order]
+    w = orc.edge_weights(s, t, 5, 1, 1000) if weighted else None
+    start = int(s[0])
+    algo, cls = (orc.SSSP, cg.SSSP) if weighted else (orc.BFS, cg.BFS)
+    with cg.Engine(n, vpt, weight_type=cg.WEIGHT_U32 if weighted else 0) as eng:
+        job = cls(eng, start_vertex=start, max_iterations=1000)
+        st = orc.Store(n, vpt, weighted)
+        cuts = [0, len(s) // 3, len(s) - 1, len(s)]
+        for lo, hi in zip(cuts, cuts[1:]):
+            if lo == hi:
+                continue
+            part = [a[lo:hi] for a in ((s, t, w) if weighted else (s, t))]
+            st.insert(*part)
+            st.compact()
+            eng.insert_edges(*part)
+            eng.do_global_compaction()
+            job.execute_algorithm()
+            assert np.array_equal(job.result(), st.run_minprop(algo, start=start, max_iter=1000)[0])
