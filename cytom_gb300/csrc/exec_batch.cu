@@ -48,7 +48,7 @@ enum BatchPhase : unsigned {
   PH_NONE = 0,
   PH_APPLY0 = 1,     // seeding apply of a BFS / CC / SSSP run
   PH_DENSE = 2,      // dense gather: one 4096-edge stage per unit
-  PH_SPARSE = 3,     // sparse gather: 256 items per unit
+  PH_SPARSE = 3,     // sparse gather: a run of the frontier list per unit
   PH_CHUNKS = 4,     // sparse chunk pass: 8 queued chunks per unit
   PH_APPLY = 5,      // apply: 1024 frontier words per unit
   PH_PR_CONTRIB = 6, // PageRank contributions: 4096 sources per unit
@@ -56,7 +56,10 @@ enum BatchPhase : unsigned {
   PH_DONE = 8
 };
 constexpr uint32_t BU_APPLY_WORDS = 1024;
-constexpr uint32_t BU_SPARSE_ITEMS = 256;
+// entries of the frontier list a warp of a sparse unit takes: 128 items before the column masks
+__device__ __forceinline__ uint32_t sparse_words_per_warp(uint32_t lT) {
+  return lT <= 2 ? 32u : max(128u >> lT, 1u);
+}
 constexpr uint32_t BU_CHUNKS = BT / 32;
 constexpr uint32_t BU_PR_VERTS = 4096;
 // targets per pull unit of each bin: 4 per thread (one thread per target), 4 per group of
@@ -167,11 +170,11 @@ __device__ void unit_sparse(const BJob* J, uint32_t unit) {
   const JobDesc* jd = J->jd;
   const StoreDesc* sd = J->sd;
   const unsigned p = ls_iter(jd->ls) & 1u;
-  const uint64_t items = (uint64_t)__ldcg(&jd->ls->nact_words[p]) << sd->lT;
-  const uint64_t g = (uint64_t)unit * BU_SPARSE_ITEMS + (threadIdx.x >> 5) * 32;
+  const uint32_t nact = __ldcg(&jd->ls->nact_words[p]);
+  const uint32_t per = sparse_words_per_warp(sd->lT), e = (unit * (BT / 32) + (threadIdx.x >> 5)) * per;
   unsigned long long scanned = 0;
   uint32_t nread = 0;  // items read: the one-job kernels' byte accounting, not kept here
-  if (g < items) scanned = sparse_group<ALGO, 2>(jd, sd, g, items, nread);
+  if (e < nact) scanned = sparse_words<ALGO, 2>(jd, sd, e, 1, min(per, nact - e), nread);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) scanned += __shfl_xor_sync(0xFFFFFFFFu, scanned, o);
   if ((threadIdx.x & 31) == 0 && scanned) atomicAdd(&jd->ls->edges_scanned, scanned);
@@ -683,7 +686,7 @@ __device__ void advance(const BJob* J, BSched* S, BCtl* ctl, unsigned phase) {
         s_total = ceil_div(sd->E, SG_E);
       } else {
         s_next = PH_SPARSE;
-        s_total = ceil_div((uint64_t)__ldcg(&jd->ls->nact_words[p]) << sd->lT, BU_SPARSE_ITEMS);
+        s_total = ceil_div(__ldcg(&jd->ls->nact_words[p]), BT / 32 * sparse_words_per_warp(sd->lT));
       }
     }
     __syncthreads();

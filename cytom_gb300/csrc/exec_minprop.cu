@@ -777,29 +777,27 @@ int build_tile_stages(Ctx* c) {
   return upload_store_desc(c);
 }
 
-// Sparse gather (sparse_group over every group of 32 items) and its chunk pass
+// Sparse gather (sparse_block over the frontier list) and its chunk pass
 // (sparse_chunk over the queue the first pass filled).
 template <int ALGO>
 __global__ void __launch_bounds__(256, 4) gather_sparse_kernel(const JobDesc* __restrict__ jd,
                                                              const StoreDesc* __restrict__ sd, int adaptive) {
+  __shared__ SparseList<256> s_list;
   LoopState* ls = jd->ls;
   if (!ls->cont || ls->mode != 1) return;
   const unsigned p = ls->iter & 1u;
   round_open<0>(jd, sd, p, adaptive, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                     (uint64_t)gridDim.x * blockDim.x);
   const unsigned lane = threadIdx.x & 31;
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint64_t items = (uint64_t)ls->nact_words[p] << sd->lT;
+  const uint32_t nact = ls->nact_words[p];
   unsigned long long scanned = 0;
   uint32_t nread = 0;
-  // few groups: up to 8 warps share each group's light edges
-  const uint64_t groups = (items + 31) / 32;
-  uint32_t nslice = 1;
-  while (nslice < 8 && groups * nslice * 2 <= nwarps) nslice *= 2;
-  const uint32_t slice = (uint32_t)(warp % nslice);
-  for (uint64_t g = (warp / nslice) * 32; g < items; g += (nwarps / nslice) * 32)
-    scanned += sparse_group<ALGO, 0>(jd, sd, g, items, nread, slice, nslice);
+  // entry e belongs to block e % shares: hubs' words lie side by side in the list
+  const uint32_t shares = max(min(nact, gridDim.x), (nact + 255) / 256);
+  for (uint32_t u = blockIdx.x; u < shares; u += gridDim.x) {
+    scanned += sparse_block<ALGO, 0, 256>(jd, sd, s_list, u, shares, (nact - u + shares - 1) / shares, nread);
+    __syncthreads();  // the list is filled anew
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     scanned += __shfl_xor_sync(0xFFFFFFFFu, scanned, o);
@@ -1000,12 +998,12 @@ __global__ void __launch_bounds__(SM_T, 1)
       }
       if (listed && (E > SMALL_E || (uint64_t)est0 * 8 <= E)) {
         const uint64_t items = (uint64_t)nact << sd->lT;
-        const uint32_t groups = (uint32_t)((items + 31) / 32);
-        uint32_t nslice = 1;
-        while (nslice < 8 && groups * nslice * 2 <= nwarps) nslice *= 2;
+        uint32_t units, nslice;
+        sparse_split(nact, nwarps, units, nslice);
         const uint32_t slice = warp % nslice;
-        for (uint64_t g = (uint64_t)(warp / nslice) * 32; g < items; g += (uint64_t)(nwarps / nslice) * 32)
-          scanned += sparse_group<ALGO, 1, SM_ILP, true>(jd, sd, g, items, nread, slice, nslice);
+        for (uint32_t u = warp / nslice; u < units; u += nwarps / nslice)
+          scanned += sparse_words<ALGO, 1, SM_ILP, true>(jd, sd, u, units, (nact - u + units - 1) / units, nread,
+                                                         slice, nslice);
         cluster_barrier();
         uint64_t nq = __ldcg(&ls->spq_count);
         if (nq) {  // the same in every CTA: the queue is complete and CTA 0 resets it past the next barrier

@@ -822,7 +822,7 @@ __global__ void merge_spans_kernel(const unsigned long long* __restrict__ q, con
 constexpr int DIR_RUN = 32;
 // Tiles of fewer edges are written by dir_tiles_kernel, a warp each, in place of the kernels
 // that go over the edges.
-constexpr uint32_t DIR_SMALL = 256;  // 1: the stream's merges 12.6 ms; 1024: its dir_tiles 1.8 ms, not 0.8
+constexpr uint32_t DIR_SMALL = 256;  // 1: the stream's merges 11.6 ms, not 9.3; 1024: its dir_tiles 1.8, not 0.8
 
 __device__ __forceinline__ void dir_runs(uint32_t* __restrict__ dir, uint64_t dt, int b0, int b1, uint32_t off) {
   unsigned lng = __ballot_sync(0xFFFFFFFFu, b1 - b0 >= DIR_RUN);

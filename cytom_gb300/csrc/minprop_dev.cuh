@@ -513,62 +513,71 @@ __device__ __forceinline__ bool stage_active(const JobDesc* __restrict__ jd, con
 // Sparse gather: the round restricted to the edges of the listed non-zero frontier
 // words. Work item = (frontier word, tile column y); the source directory gives the
 // item's edge range inside tile (x, y), x being the word's tile row. A warp takes 32
-// consecutive items (consecutive y of one word) and walks the light items' edges with
+// items that its words' column masks leave and walks the light items' edges with
 // all 32 lanes. Items longer than SP_HEAVY edges, and, when the 32 items of a warp hold
-// more than SP_WARP_MAX edges in total, every item longer than SP_LIGHT, are cut into
-// SP_CHUNK-edge chunks queued for the chunk pass, so no warp is left with more than
-// about SP_WARP_MAX edges of light items or one chunk per queue entry (RMAT hub blocks).
-constexpr uint32_t SP_HEAVY = 256;
+// more than SP_WARP_MAX (SP_BLOCK_MAX where a block shares a list) edges in total, every
+// item longer than SP_LIGHT, are cut into SP_CHUNK-edge chunks queued for the chunk pass, so
+// no warp is left with more than about that many edges of light items or one chunk per queue
+// entry (RMAT hub blocks).
+//
+// What bounds such a round is the serial chain of its busiest warp, each link an L2 access,
+// and was the work done for items that hold nothing: in an RMAT-22 stream 1 to 12 % of (word,
+// column) pairs are live, and walking them all took 39 M warp instructions and 100 us where
+// 163,000 live items hold 3.3 M edges; numbered through they take 6 M and 44 us, and the
+// stream 70.5 -> 60.0 ms. (Live items dealt out by whole words, a warp each: 80 us, a hub's
+// 64 items in one warp.) SP_BLOCK_MAX 1024: 61.9 ms, 256: 60.3.
+constexpr uint32_t SP_HEAVY = 2048;
 constexpr uint32_t SP_CHUNK = 256;
 constexpr uint32_t SP_LIGHT = 32;
 constexpr uint32_t SP_WARP_MAX = 2048;
+constexpr uint32_t SP_BLOCK_MAX = 512;
 // Every light item is first narrowed to the edges of its word's active sources
 // (sp_narrow). Streaming RMAT-22 by the shortest item narrowed: none 307.6 GTEPS, 64
-// edges 313.8, 16 edges 326.7, 4 edges 326-329, every item 335.7; narrowing heavy items
-// as well (up to 1,024 / 8,192 / all edges) gained nothing over the chunk pass's own
-// skip of inactive chunks.
+// edges 313.8, 16 edges 326.7, 4 edges 326-329, every item 335.7. Items up to SP_HEAVY are
+// narrowed before they may be queued: 256 edges 61.7 ms for the stream, 512 60.6, 1,024 60.3,
+// 2,048 and 8,192 60.0.
 constexpr uint32_t SP_NARROW = 0;
-constexpr int SP_ILP = 8;
+constexpr int SP_ILP = 8;   // edges per lane and step of a chunk
+constexpr int SP_WILP = 4;  // of a batch of light items (8 and 6: within noise or slower)
+constexpr int SP_TAIL = 2;  // steps of a batch's last edges
 
 struct SpItem {
   uint32_t x, y, bits, lo, hi, b;  // b: the word's 32-source block in its tile row
   unsigned long long base;
 };
 
-// Item (word w, tile column y): its frontier bits, directory range and tile base.
-template <int PERSIST>
-__device__ __forceinline__ SpItem sp_item_at(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                             uint32_t w, uint32_t y) {
+// Item (word w, tile column y): its directory range and tile base.
+__device__ __forceinline__ void sp_item_at(const StoreDesc* __restrict__ sd, uint32_t w, uint32_t y, SpItem& r) {
   const uint32_t lT = sd->lT, lnbw = sd->lvpt - 5, nbw = sd->nbw;
-  SpItem r;
   r.y = y;
   r.x = w >> lnbw;
   const uint32_t b = w & (nbw - 1);
   r.b = b;
-  r.bits = ld_state<PERSIST>(jd->fa + w);
   const uint64_t dbase = (((uint64_t)r.x << lT) + r.y) * (nbw + 1) + b;
   r.lo = sd->dir[dbase];
   r.hi = sd->dir[dbase + 1];
   r.base = sd->tile_ptr[((uint64_t)r.x << lT) | r.y];
-  return r;
 }
 
 template <int PERSIST>
 __device__ __forceinline__ SpItem sp_item(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                           uint64_t it) {
   const uint32_t w = ld_plain<PERSIST>(jd->aw + (it >> sd->lT));
-  return sp_item_at<PERSIST>(jd, sd, w, (uint32_t)(it & (sd->T - 1)));
+  SpItem r;
+  r.bits = ld_state<PERSIST>(jd->fa + w);
+  sp_item_at(sd, w, (uint32_t)(it & (sd->T - 1)), r);
+  return r;
 }
 
-// Relaxes ILP edges per lane whose sources are in their item's frontier word; the
+// Relaxes ILP edges per lane whose sources are in their item's frontier word (xy: the item's
+// tile, row << 16 | column; a directory exists for up to 2^14 tiles a side only); the
 // loads of all ILP edges are issued before any of them is used.
 // LAT: a target's value is loaded beside the source's, for every edge with an active source
 // (one dependent step less; otherwise only for edges that offer a value).
 template <int ALGO, int PERSIST, int ILP, bool LAT = false>
 __device__ __forceinline__ void sp_batch(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                         const uint32_t (&xs)[ILP], const uint32_t (&ys)[ILP],
-                                         const uint32_t (&bits)[ILP], const unsigned long long (&pos)[ILP],
-                                         uint32_t valid) {
+                                         const uint32_t (&xy)[ILP], const uint32_t (&bits)[ILP],
+                                         const unsigned long long (&pos)[ILP], uint32_t valid) {
   const uint32_t lvpt = sd->lvpt;
   const bool async = jd->async != 0;
   uint32_t pk[ILP], wv[ILP], cand[ILP], nv[ILP];
@@ -580,20 +589,20 @@ __device__ __forceinline__ void sp_batch(const JobDesc* __restrict__ jd, const S
   for (int k = 0; k < ILP; ++k) {
     const uint32_t sl = pk[k] >> 16;
     const bool act = ((valid >> k) & 1u) && ((bits[k] >> (sl & 31)) & 1u);
-    cand[k] = act ? ld_src<PERSIST>(jd, async, (xs[k] << lvpt) | sl) : kInf;
+    cand[k] = act ? ld_src<PERSIST>(jd, async, ((xy[k] >> 16) << lvpt) | sl) : kInf;
     wv[k] = (mp_weighted<ALGO>() && act) ? sd->wts[pos[k]] : 0u;
-    if (LAT) nv[k] = act ? ld_next<PERSIST>(jd->next + ((ys[k] << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
+    if (LAT) nv[k] = act ? ld_next<PERSIST>(jd->next + (((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
   }
 #pragma unroll
   for (int k = 0; k < ILP; ++k)
     if (cand[k] != kInf) cand[k] = mp_cand<ALGO>(cand[k], wv[k]);
 #pragma unroll
   for (int k = 0; k < ILP && !LAT; ++k)
-    nv[k] = (cand[k] != kInf) ? ld_next<PERSIST>(jd->next + ((ys[k] << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
+    nv[k] = (cand[k] != kInf) ? ld_next<PERSIST>(jd->next + (((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
 #pragma unroll
   for (int k = 0; k < ILP; ++k) {
     if (cand[k] != kInf && cand[k] < nv[k]) {
-      const uint32_t v = (ys[k] << lvpt) | (pk[k] & 0xFFFFu);
+      const uint32_t v = ((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu);
       atomicMin(jd->next + v, cand[k]);
       atomicOr(jd->ch + (v >> 5), 1u << (v & 31));
     }
@@ -670,101 +679,256 @@ __device__ __forceinline__ void sp_narrow_wide(const StoreDesc* __restrict__ sd,
   m.hi = top ? m.hi : c0;
 }
 
-// One group of 32 items [g, g + 32) for the calling warp; returns the light edges walked
-// and adds the items whose directory entries it read to `nread` (slice 0 only).
-// With nslice > 1 several warps share the group: each reads the group's items, slice 0
-// alone queues the heavy ones, and the light edges are dealt out in steps of 32 * ILP
-// (slice k takes steps k, k + nslice, ...); if the queue overflowed, slice 0 walks every
-// light edge itself (the others' share is then walked twice, which changes nothing).
-template <int ALGO, int PERSIST, int ILP = SP_ILP, bool WIDE = false>
-__device__ __forceinline__ uint32_t sparse_group(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                                 uint64_t g, uint64_t items, uint32_t& nread,
-                                                 uint32_t slice = 0, uint32_t nslice = 1) {
-  LoopState* ls = jd->ls;
-  const unsigned lane = threadIdx.x & 31;
-  const uint64_t qcap = jd->spq_cap;
-  const uint64_t it = g + lane;
-  SpItem m{};
-  uint32_t len = 0;
-  if (it < items) {
-    // an item whose column no active source of its word reaches holds none of their
-    // edges: it is left empty without reading the directory
-    const uint64_t li = it >> sd->lT;
-    const uint32_t y = (uint32_t)(it & (sd->T - 1));
-    const uint32_t w = ld_plain<PERSIST>(jd->aw + li);
-    const unsigned long long cols = ld_plain<PERSIST>(jd->awm + li);
-    if ((cols >> (y >> sd->cshift)) & 1ULL) {
-      nread += slice == 0 ? 1u : 0u;
-      m = sp_item_at<PERSIST>(jd, sd, w, y);
-      len = m.hi > m.lo ? m.hi - m.lo : 0u;
-      if (len > SP_NARROW && len <= SP_HEAVY) {
-        if (WIDE) sp_narrow_wide(sd, m);
-        else sp_narrow(sd, m);
-        len = m.hi > m.lo ? m.hi - m.lo : 0u;
-      }
+// Position of the r-th set bit of m (r < its set bits).
+__device__ __forceinline__ uint32_t nth_bit(unsigned long long m, uint32_t r) {
+  uint32_t lo = (uint32_t)m, pos = 0;
+  const uint32_t c0 = (uint32_t)__popc(lo);
+  if (r >= c0) {
+    r -= c0;
+    lo = (uint32_t)(m >> 32);
+    pos = 32;
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const uint32_t c = (uint32_t)__popc(lo & ((1u << s) - 1u));
+    if (r >= c) {
+      r -= c;
+      lo >>= s;
+      pos += s;
     }
   }
+  return pos;
+}
+
+// Lane whose run holds element f: the least j with incl[j] > f (incl: the lanes' inclusive
+// prefix sums).
+__device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t f) {
+  uint32_t j = 0;
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1) {
+    const uint32_t probe = __shfl_sync(0xFFFFFFFFu, incl, j + step - 1);
+    if (probe <= f) j += step;
+  }
+  return j;
+}
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if ((threadIdx.x & 31) >= (unsigned)o) v += y;
+  }
+  return v;
+}
+
+// Light edges [f0, f0 + 32 ILP) of a batch of items, one item per lane: the batch's edges are
+// numbered 0..total-1 by `incl`, the prefix sums of the items' lengths `mine`.
+template <int ALGO, int PERSIST, int ILP, bool LAT>
+__device__ __forceinline__ void sp_light(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                         const SpItem& m, uint32_t incl, uint32_t mine, uint32_t f0, uint32_t total) {
+  const uint32_t mxy = (m.x << 16) | m.y;
+  const unsigned long long first = m.base + m.lo - (incl - mine);  // of edge number 0
+  uint32_t xy[ILP], bits[ILP];
+  unsigned long long pos[ILP];
+  uint32_t valid = 0;
+#pragma unroll
+  for (int k = 0; k < ILP; ++k) {
+    const uint32_t f = f0 + (threadIdx.x & 31) + 32u * k;
+    const uint32_t j = lane_of(incl, f);
+    xy[k] = __shfl_sync(0xFFFFFFFFu, mxy, j);
+    bits[k] = __shfl_sync(0xFFFFFFFFu, m.bits, j);
+    pos[k] = __shfl_sync(0xFFFFFFFFu, first, j) + f;
+    valid |= (f < total) ? (1u << k) : 0u;
+  }
+  sp_batch<ALGO, PERSIST, ILP, LAT>(jd, sd, xy, bits, pos, valid);
+}
+
+// Loads item (word w with frontier bits m.bits, tile column y) into m, narrowed if it is light.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t sp_load(const StoreDesc* __restrict__ sd, uint32_t w, uint32_t y, SpItem& m) {
+  sp_item_at(sd, w, y, m);
+  uint32_t len = m.hi > m.lo ? m.hi - m.lo : 0u;
+  if (len > SP_NARROW && len <= SP_HEAVY) {
+    if (WIDE) sp_narrow_wide(sd, m);
+    else sp_narrow(sd, m);
+    len = m.hi > m.lo ? m.hi - m.lo : 0u;
+  }
+  return len;
+}
+
+// Walks a batch of up to 32 items, lane k's being m of len edges (0: none) with the number it;
+// returns the light edges walked. Items of more than SP_HEAVY edges and, when the batch holds
+// more than WMAX, those of more than SP_LIGHT, are queued for the chunk pass. nes warps share
+// the batch: they deal out its light edges in steps of 32 * ILP; the first of them (es 0) alone
+// queues the heavy items, and if the queue overflowed it walks every light edge of the batch
+// itself (the others' share is then walked twice, which changes nothing).
+template <int ALGO, int PERSIST, int ILP, uint32_t WMAX, bool WIDE>
+__device__ __forceinline__ uint32_t sp_walk(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                            const SpItem& m, uint32_t len, uint32_t it, uint32_t es, uint32_t nes) {
   uint32_t tot = len;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xFFFFFFFFu, tot, o);
-  const bool heavy = len > SP_HEAVY || (tot > SP_WARP_MAX && len > SP_LIGHT);
-  bool queued = heavy && slice != 0;  // slice 0 queues; the others leave those items to it
+  const bool heavy = len > SP_HEAVY || (tot > WMAX && len > SP_LIGHT);
+  bool queued = heavy && es != 0;  // the first warp queues; the others leave those items to it
   bool overflow = false;
-  if (heavy && slice == 0) {
+  if (heavy && es == 0) {
     const uint32_t nch = (len + SP_CHUNK - 1) / SP_CHUNK;
-    const unsigned slot = atomicAdd(&ls->spq_count, nch);
-    if ((uint64_t)slot + nch <= qcap) {
-      for (uint32_t k = 0; k < nch; ++k) jd->spq[slot + k] = make_uint2((uint32_t)it, k);
+    const unsigned slot = atomicAdd(&jd->ls->spq_count, nch);
+    if ((uint64_t)slot + nch <= jd->spq_cap) {
+      for (uint32_t k = 0; k < nch; ++k) jd->spq[slot + k] = make_uint2(it, k);
       queued = true;
     } else {
       overflow = true;
     }
   }
-  const bool walk_all = nslice > 1 && slice == 0 && __any_sync(0xFFFFFFFFu, overflow);
-  // light items: the group's edges are numbered 0..total-1 (warp prefix sum over the
-  // items' lengths); lanes take ILP of them per step and find their item by a
-  // binary search over the prefix sums held in the lanes
+  const bool walk_all = nes > 1 && es == 0 && __any_sync(0xFFFFFFFFu, overflow);
   const uint32_t mine = (len > 0 && !queued) ? len : 0u;
-  uint32_t incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y2 = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-    if (lane >= (unsigned)o) incl += y2;
-  }
+  const uint32_t incl = warp_incl_scan(mine);
   const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  const uint32_t step0 = walk_all ? 0u : slice, nstep = walk_all ? 1u : nslice;
+  const uint32_t step0 = walk_all ? 0u : es, nstep = walk_all ? 1u : nes;
   for (uint32_t f0 = step0 * 32 * ILP; f0 < total; f0 += nstep * 32 * ILP) {
-    uint32_t xs[ILP], ys[ILP], bits[ILP];
-    unsigned long long pos[ILP];
-    uint32_t valid = 0;
-#pragma unroll
-    for (int k = 0; k < ILP; ++k) {
-      const uint32_t f = f0 + lane + 32u * k;
-      // item j holding flattened edge f: the least j with incl[j] > f
-      uint32_t j = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const uint32_t probe = __shfl_sync(0xFFFFFFFFu, incl, j + step - 1);
-        if (probe <= f) j += step;
-      }
-      const uint32_t incl_j = __shfl_sync(0xFFFFFFFFu, incl, j);
-      const uint32_t mine_j = __shfl_sync(0xFFFFFFFFu, mine, j);
-      xs[k] = __shfl_sync(0xFFFFFFFFu, m.x, j);
-      ys[k] = __shfl_sync(0xFFFFFFFFu, m.y, j);
-      bits[k] = __shfl_sync(0xFFFFFFFFu, m.bits, j);
-      const uint32_t lo_j = __shfl_sync(0xFFFFFFFFu, m.lo, j);
-      const unsigned long long base_j = __shfl_sync(0xFFFFFFFFu, m.base, j);
-      pos[k] = base_j + lo_j + (f - (incl_j - mine_j));
-      valid |= (f < total) ? (1u << k) : 0u;
-    }
-    sp_batch<ALGO, PERSIST, ILP, WIDE>(jd, sd, xs, ys, bits, pos, valid);
+    if (total - f0 <= 32 * SP_TAIL) sp_light<ALGO, PERSIST, SP_TAIL, WIDE>(jd, sd, m, incl, mine, f0, total);
+    else sp_light<ALGO, PERSIST, ILP, WIDE>(jd, sd, m, incl, mine, f0, total);
   }
-  return slice == 0 ? mine : 0u;
+  return es == 0 ? mine : 0u;
+}
+
+// Column mask of list entry e, as a number of items: bits of columns, times the columns of a bit.
+template <int PERSIST>
+__device__ __forceinline__ unsigned long long sp_columns(const JobDesc* __restrict__ jd,
+                                                         const StoreDesc* __restrict__ sd, uint32_t e) {
+  const unsigned long long cols = ld_plain<PERSIST>(jd->awm + e);
+  return sd->lT < 6 ? cols & ((1ULL << (1u << sd->lT)) - 1ULL) : cols;
+}
+// Column of item r of an entry.
+__device__ __forceinline__ uint32_t sp_column(unsigned long long cols, uint32_t r, uint32_t cshift) {
+  return (nth_bit(cols, r >> cshift) << cshift) | (r & ((1u << cshift) - 1u));
+}
+
+// The frontier list of a round is walked by items (word, tile column), and an item is taken up
+// only where the word's column mask says that an active source may have edges there: in late
+// rounds of a stream a word reaches 1 to 8 of 64 columns, hubs' words all. The live items
+// of a share of the list are numbered through and warps take them 32 at a time, one per lane.
+//
+// sparse_words: up to 32 entries e0 + k estep, k < ne, for the calling warp, or for nslice warps
+// that share them: these deal out the batches of 32 items, and the light edges of a batch
+// where there are fewer batches than warps. Returns the light edges walked and adds the
+// items whose directory entries it read to `nread`.
+template <int ALGO, int PERSIST, int ILP = SP_WILP, bool WIDE = false>
+__device__ __forceinline__ uint32_t sparse_words(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                                 uint32_t e0, uint32_t estep, uint32_t ne, uint32_t& nread,
+                                                 uint32_t slice = 0, uint32_t nslice = 1) {
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t cshift = sd->cshift;
+  uint32_t w = 0, wbits = 0, ni = 0;
+  unsigned long long cols = 0;
+  if (lane < ne) {
+    const uint32_t e = e0 + lane * estep;
+    w = ld_plain<PERSIST>(jd->aw + e);
+    cols = sp_columns<PERSIST>(jd, sd, e);
+    wbits = ld_state<PERSIST>(jd->fa + w);
+    ni = (uint32_t)__popcll(cols) << cshift;
+  }
+  const uint32_t iincl = warp_incl_scan(ni);
+  const uint32_t nitems = __shfl_sync(0xFFFFFFFFu, iincl, 31);
+  uint32_t nb = 1;  // batches that run side by side, each with nslice / nb slices
+  while (nb < nslice && nb * 32 < nitems) nb *= 2;
+  const uint32_t es = slice / nb, nes = nslice / nb;
+  uint32_t walked = 0;
+  for (uint32_t i0 = (slice % nb) * 32; i0 < nitems; i0 += nb * 32) {
+    const uint32_t f = i0 + lane;
+    const uint32_t j = lane_of(iincl, f);
+    const uint32_t r = f - __shfl_sync(0xFFFFFFFFu, iincl - ni, j);
+    const unsigned long long cj = __shfl_sync(0xFFFFFFFFu, cols, j);
+    const uint32_t wj = __shfl_sync(0xFFFFFFFFu, w, j);
+    SpItem m{};
+    m.bits = __shfl_sync(0xFFFFFFFFu, wbits, j);
+    uint32_t len = 0;
+    if (f < nitems) {
+      nread += es == 0 ? 1u : 0u;
+      len = sp_load<WIDE>(sd, wj, sp_column(cj, r, cshift), m);
+    }
+    walked += sp_walk<ALGO, PERSIST, ILP, SP_WARP_MAX, WIDE>(jd, sd, m, len, ((e0 + j * estep) << sd->lT) | m.y, es,
+                                                             nes);
+  }
+  return walked;
+}
+
+// Split of a list of nact entries over nwarps warps for sparse_words: `units` shares of at most
+// 32 entries (entry e belongs to unit e % units, so that the hubs' words, which lie side by
+// side, go to different warps); with few entries nslice warps on each.
+__device__ __forceinline__ void sparse_split(uint32_t nact, uint32_t nwarps, uint32_t& units, uint32_t& nslice) {
+  units = min(nact, max(nwarps, (nact + 31) / 32));
+  nslice = 1;
+  while (nslice < 8 && units * nslice * 2 <= nwarps) nslice *= 2;
+}
+
+// sparse_block: the same for up to NT entries and the calling block of NT threads, which share
+// them all, so that a hub's 64 items don't keep one warp busy when the others are done.
+template <int NT>
+struct SparseList {
+  unsigned long long cols[NT];
+  uint32_t w[NT], bits[NT], incl[NT];  // incl: live items up to and with this entry
+  uint32_t wsum[NT / 32];
+};
+
+template <int ALGO, int PERSIST, int NT, int ILP = SP_WILP>
+__device__ __forceinline__ uint32_t sparse_block(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
+                                                 SparseList<NT>& sl, uint32_t e0, uint32_t estep, uint32_t ne,
+                                                 uint32_t& nread) {
+  constexpr uint32_t NW = NT / 32;
+  const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t cshift = sd->cshift;
+  uint32_t ni = 0;
+  if (tid < ne) {
+    const uint32_t e = e0 + tid * estep;
+    const uint32_t w = ld_plain<PERSIST>(jd->aw + e);
+    const unsigned long long cols = sp_columns<PERSIST>(jd, sd, e);
+    ni = (uint32_t)__popcll(cols) << cshift;
+    sl.w[tid] = w;
+    sl.cols[tid] = cols;
+    sl.bits[tid] = ld_state<PERSIST>(jd->fa + w);
+  }
+  uint32_t iincl = warp_incl_scan(ni);
+  if (lane == 31) sl.wsum[warp] = iincl;
+  __syncthreads();
+  uint32_t nitems = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < NW; ++k) {
+    const uint32_t x = sl.wsum[k];
+    iincl += k < warp ? x : 0u;
+    nitems += x;
+  }
+  sl.incl[tid] = iincl;
+  __syncthreads();
+  uint32_t nb = 1;  // batches that run side by side, each by NW / nb warps
+  while (nb < NW && nb * 32 < nitems) nb *= 2;
+  const uint32_t es = warp / nb, nes = NW / nb;
+  uint32_t walked = 0;
+  for (uint32_t i0 = (warp % nb) * 32; i0 < nitems; i0 += nb * 32) {
+    const uint32_t f = i0 + lane;
+    SpItem m{};
+    uint32_t len = 0, ent = 0;
+    if (f < nitems) {
+      nread += es == 0 ? 1u : 0u;
+#pragma unroll
+      for (uint32_t step = NT / 2; step > 0; step >>= 1)
+        if (sl.incl[ent + step - 1] <= f) ent += step;
+      const unsigned long long cols = sl.cols[ent];
+      const uint32_t r = f - (sl.incl[ent] - ((uint32_t)__popcll(cols) << cshift));
+      m.bits = sl.bits[ent];
+      len = sp_load<false>(sd, sl.w[ent], sp_column(cols, r, cshift), m);
+    }
+    walked += sp_walk<ALGO, PERSIST, ILP, SP_BLOCK_MAX, false>(jd, sd, m, len,
+                                                               ((e0 + ent * estep) << sd->lT) | m.y, es, nes);
+  }
+  return walked;
 }
 
 // Queue entry q (a chunk of a heavy item) for the calling warp; returns the edges walked
 // (lane 0). Sources are sorted inside an item, so a chunk whose first and last edges
-// span no source of the item's frontier word is skipped after two loads.
+// span no source of the item's frontier word is skipped after two loads. (A skipped chunk of
+// an item that its neighbours made heavy still counts as walked, so that the count does not
+// hang on the order of the frontier list.)
 template <int ALGO, int PERSIST>
 __device__ __forceinline__ uint32_t sparse_chunk(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                                  uint64_t q, uint64_t items) {
@@ -772,11 +936,9 @@ __device__ __forceinline__ uint32_t sparse_chunk(const JobDesc* __restrict__ jd,
   const uint2 c = ld_plain<PERSIST>(jd->spq + q);
   if (c.x >= items) return 0;  // never indexes outside this round's items
   SpItem m = sp_item<PERSIST>(jd, sd, c.x);
-  {
-    // the item as sparse_group cut it into chunks: narrowed by the same rule
-    const uint32_t len = m.hi > m.lo ? m.hi - m.lo : 0u;
-    if (len > SP_NARROW && len <= SP_HEAVY) sp_narrow(sd, m);
-  }
+  const bool own = m.hi > m.lo && m.hi - m.lo > SP_HEAVY;  // queued for its own length
+  // the item as sp_walk cut it into chunks: narrowed by the same rule
+  if (!own && m.hi > m.lo) sp_narrow(sd, m);
   const uint32_t e0 = m.lo + c.y * SP_CHUNK;
   const uint32_t e1 = min(m.hi, e0 + SP_CHUNK);
   if (e0 >= e1) return 0;
@@ -786,12 +948,11 @@ __device__ __forceinline__ uint32_t sparse_chunk(const JobDesc* __restrict__ jd,
   const uint32_t s_first = (__shfl_sync(0xFFFFFFFFu, bound, 0) >> 16) & 31u;
   const uint32_t s_last = (__shfl_sync(0xFFFFFFFFu, bound, 1) >> 16) & 31u;
   const uint32_t span = (s_last >= 31u ? 0xFFFFFFFFu : ((2u << s_last) - 1u)) & ~((1u << s_first) - 1u);
-  if ((m.bits & span) == 0) return 0;
-  uint32_t xs[SP_ILP], ys[SP_ILP], bits[SP_ILP];
+  if ((m.bits & span) == 0) return own || lane != 0 ? 0u : e1 - e0;
+  uint32_t xy[SP_ILP], bits[SP_ILP];
 #pragma unroll
   for (int k = 0; k < SP_ILP; ++k) {
-    xs[k] = m.x;
-    ys[k] = m.y;
+    xy[k] = (m.x << 16) | m.y;
     bits[k] = m.bits;
   }
   for (uint32_t e = e0 + lane; e < e1; e += 32 * SP_ILP) {
@@ -803,7 +964,7 @@ __device__ __forceinline__ uint32_t sparse_chunk(const JobDesc* __restrict__ jd,
       pos[k] = m.base + ek;
       valid |= (ek < e1) ? (1u << k) : 0u;
     }
-    sp_batch<ALGO, PERSIST, SP_ILP>(jd, sd, xs, ys, bits, pos, valid);
+    sp_batch<ALGO, PERSIST, SP_ILP>(jd, sd, xy, bits, pos, valid);
   }
   return lane == 0 ? e1 - e0 : 0u;
 }
