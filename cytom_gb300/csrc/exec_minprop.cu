@@ -1191,15 +1191,18 @@ struct SeedJobs {
   int count;
 };
 
-template <int ALGO>
-__device__ __forceinline__ void seed_one(const JobDesc* __restrict__ jd, uint32_t u, uint32_t v, uint32_t w) {
-  const uint32_t uv = jd->cur[u];
-  if (uv == kInf) return;
-  const uint32_t cand = mp_cand<ALGO>(uv, w);
-  if (cand == kInf) return;
-  if (cand < __ldcg(jd->next + v)) {
-    uint32_t old = atomicMin(jd->next + v, cand);
-    if (cand < old) atomicOr(jd->ch + (v >> 5), 1u << (v & 31));
+// A key's chain is its load, the jobs' source values, their targets' values and the updates;
+// SEED_JOBS jobs go through it side by side (job after job a batch of 2^20 edges under three
+// jobs took 30 us, 25 now).
+constexpr int SEED_JOBS = 4;
+
+__device__ __forceinline__ uint32_t seed_cand(int algo, uint32_t uv, uint32_t w) {
+  if (uv == kInf) return kInf;
+  switch (algo) {
+    case CYTOM_ALGO_BFS: return mp_cand<0>(uv, w);
+    case CYTOM_ALGO_CC: return mp_cand<1>(uv, w);
+    case CYTOM_ALGO_SSWP: return mp_cand<3>(uv, w);
+    default: return mp_cand<2>(uv, w);
   }
 }
 
@@ -1210,16 +1213,25 @@ __global__ void seed_keys_multi_kernel(SeedJobs sj, const uint64_t* __restrict__
   const uint64_t tmask = (1ULL << lT) - 1ULL;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
     const uint64_t key = K[i];
+    const uint32_t w = W ? W[i] : 1u;
     const uint64_t tile = key >> (2 * lvpt);
     const uint32_t u = (uint32_t)(((tile >> lT) << lvpt) | ((key >> lvpt) & m));
     const uint32_t v = (uint32_t)(((tile & tmask) << lvpt) | (key & m));
-    const uint32_t w = W ? W[i] : 1u;
-    for (int k = 0; k < sj.count; ++k) {
-      switch (sj.algo[k]) {
-        case CYTOM_ALGO_BFS: seed_one<0>(sj.jd[k], u, v, w); break;
-        case CYTOM_ALGO_CC: seed_one<1>(sj.jd[k], u, v, w); break;
-        case CYTOM_ALGO_SSWP: seed_one<3>(sj.jd[k], u, v, w); break;
-        default: seed_one<2>(sj.jd[k], u, v, w); break;
+    for (int k0 = 0; k0 < sj.count; k0 += SEED_JOBS) {
+      uint32_t cand[SEED_JOBS], nv[SEED_JOBS];
+#pragma unroll
+      for (int k = 0; k < SEED_JOBS; ++k) cand[k] = k0 + k < sj.count ? sj.jd[k0 + k]->cur[u] : kInf;
+#pragma unroll
+      for (int k = 0; k < SEED_JOBS; ++k) {
+        cand[k] = k0 + k < sj.count ? seed_cand(sj.algo[k0 + k], cand[k], w) : kInf;
+        nv[k] = cand[k] != kInf ? __ldcg(sj.jd[k0 + k]->next + v) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < SEED_JOBS; ++k) {
+        if (cand[k] != kInf && cand[k] < nv[k]) {
+          const JobDesc* jd = sj.jd[k0 + k];
+          if (cand[k] < atomicMin(jd->next + v, cand[k])) atomicOr(jd->ch + (v >> 5), 1u << (v & 31));
+        }
       }
     }
   }

@@ -1092,7 +1092,8 @@ int ensure_app_capacity(Ctx* c, uint64_t need) {
   return CYTOM_OK;
 }
 
-__global__ void dir_tiles_kernel(const StoreDesc* __restrict__ sd, uint32_t* __restrict__ dir, uint32_t nbw);
+__global__ void dir_tiles_kernel(const unsigned long long* __restrict__ tile_ptr, const uint32_t* __restrict__ edges,
+                                 uint64_t ntiles, uint32_t* __restrict__ dir, uint32_t nbw);
 
 int compact(Ctx* c) {
   if (c->A == 0) return CYTOM_OK;
@@ -1155,6 +1156,15 @@ int compact(Ctx* c) {
        c->stream>>>(c->edges, c->wts, c->E, q, nloc, nw, Kdev, sb, ts, nsp, c->tile_ptr_alt, c->chunk_tile_alt, mdir,
                     (uint32_t)(c->vpt / 32), c->edges_alt, wt ? c->wts_alt : nullptr);
   c->launches += 2;
+  if (wt) {
+    fixup_weights_kernel<<<grid_for(c, A, 256), 256, 0, c->stream>>>(lb, wsel, A, q, Kdev, c->wts_alt);
+    c->launches++;
+  }
+  if (mdir) {  // the merge wrote every directory entry up to each tile's last source block
+    dir_tiles_kernel<<<grid_for(c, c->ntiles * 32, 256), 256, 0, c->stream>>>(c->tile_ptr_alt, c->edges_alt, c->ntiles,
+                                                                              mdir, (uint32_t)(c->vpt / 32));
+    c->launches++;
+  }
   e = cudaMemcpyAsync(c->h_pinned, Kdev, 4, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
@@ -1168,9 +1178,9 @@ int compact(Ctx* c) {
     cudaFreeAsync(tmp, c->stream);
     return rc;
   }
-  // Installing the merged snapshot: runs on the previous one must have finished. The jobs
-  // are then seeded by the merged edges (edgeChanged(INSERT)) and lowered weights of
-  // stored edges are applied to the merged copy.
+  // Installing the merged snapshot: runs on the previous one must have finished (everything
+  // above wrote to the new snapshot alone). The jobs are then seeded by the merged edges
+  // (edgeChanged(INSERT)).
   join_runs(c);
   {
     std::vector<Job*> mp;
@@ -1189,10 +1199,6 @@ int compact(Ctx* c) {
       return rc;
     }
   }
-  if (wt) {
-    fixup_weights_kernel<<<grid_for(c, A, 256), 256, 0, c->stream>>>(lb, wsel, A, q, Kdev, c->wts_alt);
-    c->launches++;
-  }
   cudaFreeAsync(tmp, c->stream);
   if (c->dyn_pending) cudaMemsetAsync(c->dyn_pending, 0, c->ntiles * 4, c->stream);  // nothing appended now
   std::swap(c->edges, c->edges_alt);
@@ -1205,13 +1211,8 @@ int compact(Ctx* c) {
   c->version++;
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "merge");
-  if (mdir) c->dir_version = c->version;  // completed below, before any later launch reads it
-  int urc = upload_store_desc(c);
-  if (urc || !mdir) return urc;
-  // the merge wrote every directory entry up to each tile's last source block
-  dir_tiles_kernel<<<grid_for(c, c->ntiles * 32, 256), 256, 0, c->stream>>>(c->dsd, c->dir, (uint32_t)(c->vpt / 32));
-  c->launches++;
-  return cuda_err(c, cudaGetLastError(), "directory");
+  if (mdir) c->dir_version = c->version;
+  return upload_store_desc(c);
 }
 
 // Compact-vs-sparse flag per tile: distinct sources >= vpt / 2 (tile-manager.h:261-263).
@@ -1289,20 +1290,20 @@ __global__ void dir_edges_kernel(const StoreDesc* __restrict__ sd, uint32_t* __r
 
 // The end of every tile's directory, and all of it for tiles of fewer than DIR_SMALL edges,
 // where an edge may start many blocks. One warp per tile.
-__global__ void dir_tiles_kernel(const StoreDesc* __restrict__ sd, uint32_t* __restrict__ dir, uint32_t nbw) {
-  const uint64_t ntiles = sd->ntiles;
+__global__ void dir_tiles_kernel(const unsigned long long* __restrict__ tile_ptr, const uint32_t* __restrict__ edges,
+                                 uint64_t ntiles, uint32_t* __restrict__ dir, uint32_t nbw) {
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t t = warp; t < ntiles; t += nwarps) {
-    const uint64_t lo = sd->tile_ptr[t], hi = sd->tile_ptr[t + 1];
+    const uint64_t lo = tile_ptr[t], hi = tile_ptr[t + 1];
     const uint32_t m = (uint32_t)(hi - lo);
     const uint64_t dt = t * (nbw + 1);
-    const int blast = m ? (int)(sd->edges[hi - 1] >> 21) : -1;
+    const int blast = m ? (int)(edges[hi - 1] >> 21) : -1;
     if (hi - lo < DIR_SMALL) {
       int prev = -1;
       for (uint32_t i = 0; i < m; i += 32) {
-        const int b = i + lane < m ? (int)(sd->edges[lo + i + lane] >> 21) : -1;
+        const int b = i + lane < m ? (int)(edges[lo + i + lane] >> 21) : -1;
         int bp = __shfl_up_sync(0xFFFFFFFFu, b, 1);
         if (lane == 0) bp = prev;
         prev = __shfl_sync(0xFFFFFFFFu, b, 31);
@@ -1369,7 +1370,8 @@ int build_directory(Ctx* c) {
       c->launches++;
     }
   }
-  dir_tiles_kernel<<<grid_for(c, c->ntiles * 32, 256), 256, 0, c->stream>>>(c->dsd, c->dir, (uint32_t)nbw);
+  dir_tiles_kernel<<<grid_for(c, c->ntiles * 32, 256), 256, 0, c->stream>>>(c->tile_ptr, c->edges, c->ntiles, c->dir,
+                                                                            (uint32_t)nbw);
   c->launches++;
   prof_end(c, slot, (double)c->E * 8.0 + (double)entries * 4.0);
   cudaError_t e = cudaGetLastError();
