@@ -151,6 +151,7 @@ struct Job {
   cudaGraphExec_t loop_exec = nullptr;
   bool graph_failed = false;
   bool last_run_graph = false;  // the last run went through the graph (launch accounting)
+  unsigned last_rounds = 0;  // of the last run: the longest of several is launched first
   uint64_t graph_epoch = 0;     // tune epoch the captured graph was built with
   void* ext = nullptr;          // per-algorithm state (PageRank family)
 };
