@@ -620,26 +620,19 @@ int radix_sort_pairs(Ctx* c, uint64_t* keys, uint64_t* keys_alt, uint32_t* vals,
 // --------------------------------------------------------------------------
 // Compaction
 // --------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t lower_bound_u32(const uint32_t* a, uint64_t lo, uint64_t hi,
-                                                    uint32_t v) {
-  while (lo < hi) {
-    uint64_t mid = lo + ((hi - lo) >> 1);
-    if (a[mid] < v) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
 // For each sorted appended key: first of its run? present in the compacted tile?
 // keep[i] = 1 for a new distinct edge; lb[i] = its insertion index in the old store;
 // wsel[i] = the least weight of its run. A weight that undercuts the stored copy of
-// an existing edge lowers that copy in place.
+// an existing edge lowers that copy in place. Bound by the search's instructions: offsets in
+// the tile are 32-bit, and a snapshot with a source directory is searched from there (12.5 M
+// keys against 12.5 to 37.5 M stored edges 253 us, 232 by the offsets, 154 by both).
 constexpr unsigned long long kNoFix = ~0ULL, kFixFlag = 1ULL << 62;
 
 __global__ void dedupe_lookup_kernel(const uint64_t* __restrict__ K, const uint32_t* __restrict__ W,
                                      uint64_t A, const uint32_t* __restrict__ edges,
                                      const uint32_t* __restrict__ wts,
                                      const unsigned long long* __restrict__ tile_ptr,
+                                     const uint32_t* __restrict__ dir, uint32_t nbw,
                                      uint32_t lvpt, uint32_t* __restrict__ keep,
                                      unsigned long long* __restrict__ lb,
                                      uint32_t* __restrict__ wsel) {
@@ -668,8 +661,26 @@ __global__ void dedupe_lookup_kernel(const uint64_t* __restrict__ K, const uint3
       lb[i] = kNoFix;
       continue;
     }
-    uint64_t pos = lower_bound_u32(edges, lo, hi, local);
-    bool found = pos < hi && edges[pos] == local;
+    const uint32_t* te = edges + lo;
+    const bool full = hi - lo > 0xFFFFFFFFULL;  // all 2^32 pairs of the tile
+    uint32_t at = 0, left = full ? 0xFFFFFFFFu : (uint32_t)(hi - lo);
+    if (dir && !full) {  // the edges of the source's block alone
+      const uint32_t* d = dir + tile * (nbw + 1) + (local >> 21);
+      at = d[0];
+      left = d[1] - at;
+    }
+    const uint32_t end = at + left;
+    while (left) {
+      const uint32_t half = left >> 1;
+      if (te[at + half] < local) {
+        at += half + 1;
+        left -= half + 1;
+      } else {
+        left = half;
+      }
+    }
+    const uint64_t pos = lo + at;
+    const bool found = (at < end || full) && te[at] == local;
     if (found) {
       // a lower weight for a stored edge is applied to the merged copy (fixup_weights_kernel):
       // the store itself may still be read by runs of the previous batch
@@ -1126,7 +1137,9 @@ int compact(Ctx* c) {
   uint32_t* ts = sb + (nsp + 1);
   int slot = prof_begin(c, KC_MERGE);
   dedupe_lookup_kernel<<<grid_for(c, A, 256), 256, 0, c->stream>>>(
-      K, W, A, c->edges, c->wts, c->tile_ptr, c->lvpt, keep, lb, wsel);
+      K, W, A, c->edges, c->wts, c->tile_ptr,
+      c->dir && !c->dir_disabled && c->dir_version == c->version ? c->dir : nullptr, (uint32_t)(c->vpt / 32), c->lvpt,
+      keep, lb, wsel);
   c->launches++;
   rc = exclusive_scan_u32(c, keep, P, A, Kdev);
   if (rc) return rc;
