@@ -729,14 +729,17 @@ __device__ __forceinline__ void pull_large_body(const PrArgs& a, const pr_val_t<
 // (max_iter + 2; beyond it the run stops with err = 2).
 __device__ __forceinline__ void pr_loop_control(LoopState* ls, int mode, cudaGraphConditionalHandle h,
                                                 int use_handle) {
+  const bool live = __ldcg(&ls->cont) != 0u;
   unsigned cont = pr_control_step(ls, mode);
   if (use_handle) {
-    const unsigned started = ls->sel_rounds + 1;
-    ls->sel_rounds = started;
-    if ((unsigned long long)started > (unsigned long long)ls->max_iter + 2ULL) {
-      ls->err = 2u;
-      ls->cont = 0u;
-      cont = 0u;
+    if (live) {
+      const unsigned started = ls->sel_rounds + 1;
+      ls->sel_rounds = started;
+      if ((unsigned long long)started > (unsigned long long)ls->max_iter + 2ULL) {
+        ls->err = 2u;
+        ls->cont = 0u;
+        cont = 0u;
+      }
     }
     cudaGraphSetConditional(h, cont);
   }
@@ -757,8 +760,6 @@ __device__ __forceinline__ void pr_round_end(LoopState* ls, int mode, cudaGraphC
   }
 }
 
-// Every block takes part in the round end of the fused forms, whether or not the run
-// still continues (a captured loop's condition is only set here).
 // The virtual blocks of the bin layout from blockIdx.x on, gridDim.x apart.
 template <int MODE>
 __device__ __forceinline__ void pull_vblocks(PrArgs& a, const pr_val_t<MODE>* cr, unsigned p, pr_ff_t<MODE> dang,
@@ -793,11 +794,14 @@ __global__ void __launch_bounds__(PR_T, pr_min_blocks<MODE>()) pr_pull_kernel(Pr
                                                        cudaGraphConditionalHandle h, int use_handle) {
   LoopState* ls = a.ls;
   const bool live = ls->cont != 0;
-  if (!live && !pr_fused<MODE>()) return;
+  if (!live) {  // a round of the loop's body past the last one
+    if (pr_fused<MODE>() && use_handle && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
+    return;
+  }
   const unsigned p = ls->iter & 1u;
   PrTally t;
   t.init();
-  const uint32_t total = live ? blp->blocks : 0u;
+  const uint32_t total = blp->blocks;
   // one thread's FP64 conversion of the dangling term, not every thread's
   __shared__ pr_ff_t<MODE> s_dang;
   if (threadIdx.x == 0) s_dang = pr_dang_arg<MODE, 0>(a, ls, p);
@@ -805,7 +809,7 @@ __global__ void __launch_bounds__(PR_T, pr_min_blocks<MODE>()) pr_pull_kernel(Pr
   const pr_ff_t<MODE> dang = s_dang;
   const pr_val_t<MODE>* cr = pr_cread<MODE>(a, p);
   pull_vblocks<MODE>(a, cr, p, dang, blp, total, t);
-  if (live) pr_tally_flush<MODE>(ls, p, t);
+  pr_tally_flush<MODE>(ls, p, t);
   if constexpr (pr_fused<MODE>()) pr_round_end(ls, MODE, h, use_handle);
 }
 
@@ -1063,6 +1067,12 @@ static cudaError_t pr_add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cud
 // The round loop as one CUDA graph; a run is one graph launch. Fused form: while(cont)
 // { pull, whose last block sets the condition }; the others: while(cont) { contributions
 // -> pull -> control, which sets the condition }.
+// The body holds several rounds: a pass of the while node adds some 4 us to its kernels, a round
+// past the last one kernels that exit at once. RMAT-16 PageRank-delta stream with 1 / 4 / 8 / 16
+// rounds 18.1 / 16.0 / 15.6 / 15.5 ms; RMAT-20 adjoint with 1 / 2 / 4 / 8 13.6 / 13.3 / 13.4 /
+// 13.1, RMAT-22 FP64 11.9 / 11.8 / 12.0 / 11.7. (The five kernels of a BFS / CC / SSSP round
+// gain nothing by it.)
+constexpr int kPrBody = 8, kPrBodyFused = 8;
 template <int MODE>
 static int build_round_graph(Ctx* c, const PrArgs& base, const Csc& q, cudaGraphExec_t* out) {
   constexpr bool F = pr_fused<MODE>();
@@ -1091,19 +1101,22 @@ static int build_round_graph(Ctx* c, const PrArgs& base, const Csc& q, cudaGraph
     LoopState* ls = base.ls;
     int mode = MODE, one = 1;
     void* a_p[] = {(void*)&a, (void*)&blp, (void*)&h, (void*)&one};
-    if (F) {
-      cudaGraphNode_t n_p;
-      e = pr_add_kernel(body, &n_p, nullptr, 0, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p);
-    } else {
-      cudaGraphNode_t n_c, n_p, n_ctl;
-      int zero = 0;
-      void* a_p0[] = {(void*)&a, (void*)&blp, (void*)&h, (void*)&zero};
-      const bool con = pr_opens_with_contrib<MODE>();
+    cudaGraphNode_t n_c, n_p, n_ctl;
+    int zero = 0;
+    void* a_p0[] = {(void*)&a, (void*)&blp, (void*)&h, (void*)&zero};
+    void* a_ctl[] = {(void*)&ls, (void*)&mode, (void*)&h, (void*)&one};
+    const bool con = pr_opens_with_contrib<MODE>();
+    for (int k = 0; k < (F ? kPrBodyFused : kPrBody) && e == cudaSuccess; ++k) {
+      if (F) {
+        const cudaGraphNode_t before = k ? n_p : nullptr;
+        e = pr_add_kernel(body, &n_p, k ? &before : nullptr, k ? 1 : 0, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p);
+        continue;
+      }
+      const cudaGraphNode_t* dep = k ? &n_ctl : nullptr;
       if (con)
-        e = pr_add_kernel(body, &n_c, nullptr, 0, (void*)pr_contrib_kernel<MODE>, dim3(grid_n(c, c->n)), dim3(256), a_c);
+        e = pr_add_kernel(body, &n_c, dep, k ? 1 : 0, (void*)pr_contrib_kernel<MODE>, dim3(grid_n(c, c->n)), dim3(256), a_c);
       if (e == cudaSuccess)
-        e = pr_add_kernel(body, &n_p, con ? &n_c : nullptr, con ? 1 : 0, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p0);
-      void* a_ctl[] = {(void*)&ls, (void*)&mode, (void*)&h, (void*)&one};
+        e = pr_add_kernel(body, &n_p, con ? &n_c : dep, con || k ? 1 : 0, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p0);
       if (e == cudaSuccess)
         e = pr_add_kernel(body, &n_ctl, &n_p, 1, (void*)pr_control_kernel, dim3(1), dim3(1), a_ctl);
     }

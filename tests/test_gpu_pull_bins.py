@@ -84,3 +84,29 @@ def test_pull_bins(cg, orc, per_degree, reverse):
                 gw, gt, _ = p.adjoint(c)
                 assert np.abs(gw - gw_ref).max() <= 1e-4 * np.abs(gw_ref).max()
                 assert np.abs(gt - gt_ref).max() <= 1e-4 * np.abs(gt_ref).max()
+
+
+@pytest.mark.parametrize("rounds", [1, 2, 7, 8, 9, 17])
+def test_round_counts_of_captured_loop(cg, rounds):
+    """Runs that end within, at and past the rounds of the captured loop's body, again on the
+    same captured loop, against the loop driven by the host: the same rounds and edge counts;
+    values but for the order of the dangling mass's FP64 atomics (one FP32 ulp, 1e-12)."""
+    s, t = edges(3, False)
+    with cg.Engine(N, VPT) as eng:
+        eng.insert_edges(s, t)
+        forms = [(lambda: cg.PageRank(eng, max_iterations=rounds, tolerance=0.0, kahan=True), "result", 1.2e-7),
+                 (lambda: cg.PageRank(eng, max_iterations=rounds, tolerance=0.0, kahan=False), "result64", 1e-12),
+                 (lambda: cg.PageRankDelta(eng, delta=0.0, max_iterations=rounds, tolerance=0.0), "result", 1.2e-7)]
+        for make, result, tol in forms:
+            got = []
+            for host in (False, True):
+                p = make()
+                eng.set_profiling(host)
+                for again in range(2):
+                    st = p.execute_algorithm()
+                    got.append((np.asarray(getattr(p, result)(), np.float64), st["iterations"], st["count_edges"]))
+                eng.set_profiling(False)
+            for a, b in zip(got[:2], got[2:]):
+                assert a[1:] == b[1:] and a[1] <= rounds
+                assert (np.abs(a[0] - b[0]) <= tol * np.abs(b[0])).all()
+            assert got[0][1] == rounds
