@@ -222,13 +222,27 @@ __device__ __forceinline__ uint64_t make_key(uint32_t s, uint32_t t, uint32_t lv
 // end). One pass over the batch instead of a checking pass before; the degree atomics are
 // one per endpoint: aggregating a warp's equal vertices first (two __match_any_sync an edge)
 // took longer than the atomics it saved. Bound by the atomics (16.8 M edges, ids without
-// order: 320 -> 262 us; 12.5 M RMAT edges, whose hubs share sectors, 417 -> 385; 20,011
-// edges 14.2 -> 8.7).
+// order: 320 -> 262 us; 20,011 edges 14.2 -> 8.7).
+//
+// HUBS: a block counts the first APPEND_HUBS vertices in shared memory and adds them up at its
+// end. Atomics on one sector go one after another, and in graphs numbered by degree or by a
+// generator the first take several per cent of the endpoints (12.5 M RMAT-22 edges 366 us
+// without, 326 with one such vertex, 253 with 64 or 512, 255 with 2,048, 236 with 4,096, which
+// leaves fewer blocks per SM).
+constexpr uint32_t APPEND_HUBS = 2048;
+constexpr uint64_t kAppendHubsMin = 1ULL << 17;  // edges; below, a block's share is too small to pay the adding up
+
+template <bool HUBS>
 __global__ void append_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ tgt,
                               const uint32_t* __restrict__ w, uint64_t count, uint64_t n,
                               uint64_t* __restrict__ keys, uint32_t* __restrict__ kw,
                               uint32_t* __restrict__ out_deg, uint32_t* __restrict__ in_deg,
                               uint32_t lvpt, uint32_t lT, unsigned int* __restrict__ bad) {
+  __shared__ uint32_t s_out[HUBS ? APPEND_HUBS : 1], s_in[HUBS ? APPEND_HUBS : 1];
+  if (HUBS) {
+    for (uint32_t i = threadIdx.x; i < APPEND_HUBS; i += blockDim.x) s_out[i] = s_in[i] = 0;
+    __syncthreads();
+  }
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   unsigned nb = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
@@ -239,10 +253,19 @@ __global__ void append_kernel(const uint32_t* __restrict__ src, const uint32_t* 
     }
     keys[i] = make_key(s, t, lvpt, lT);
     if (w) kw[i] = w[i];
-    atomicAdd(&out_deg[s], 1u);
-    atomicAdd(&in_deg[t], 1u);
+    if (HUBS && s < APPEND_HUBS) atomicAdd(&s_out[s], 1u);
+    else atomicAdd(&out_deg[s], 1u);
+    if (HUBS && t < APPEND_HUBS) atomicAdd(&s_in[t], 1u);
+    else atomicAdd(&in_deg[t], 1u);
   }
   if (nb) atomicAdd(bad, nb);
+  if (HUBS) {
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < APPEND_HUBS && i < n; i += blockDim.x) {
+      if (s_out[i]) atomicAdd(&out_deg[i], s_out[i]);
+      if (s_in[i]) atomicAdd(&in_deg[i], s_in[i]);
+    }
+  }
 }
 
 // Takes back the degrees of a rejected batch.
@@ -331,7 +354,8 @@ int insert_device(Ctx* c, const uint32_t* src, const uint32_t* tgt, const uint32
   if (rc) return rc;
   const uint32_t* wuse = (c->wtype != CYTOM_UNWEIGHTED) ? w : nullptr;
   int slot = prof_begin(c, KC_INSERT);
-  append_kernel<<<grid_for(c, count, 256), 256, 0, c->stream>>>(
+  auto* append = count >= kAppendHubsMin ? append_kernel<true> : append_kernel<false>;
+  append<<<grid_for(c, count, 256), 256, 0, c->stream>>>(
       src, tgt, wuse, count, c->n, c->app_keys + c->A, wuse ? c->app_w + c->A : nullptr, c->out_deg,
       c->in_deg, c->lvpt, c->lT, c->d_flag);
   c->launches++;

@@ -105,3 +105,24 @@ def test_merge_directory_of_uneven_tiles(cg, orc, size, weighted):
             eng.do_global_compaction()
             job.execute_algorithm()
             assert np.array_equal(job.result(), st.run_minprop(algo, start=start, max_iter=1000)[0])
+
+
+@pytest.mark.parametrize("n", [1 << 10, 1 << 11, 1 << 13])
+@pytest.mark.parametrize("count,bad", [((1 << 17) - 1, False), (1 << 17, False), ((1 << 17) + 1, True), (300001, False)])
+def test_degrees_of_large_batches(cg, n, count, bad):
+    """Degrees of batches around the size from which blocks count the first vertices by
+    themselves, with fewer vertices than such counters, as many and more; a rejected batch
+    takes its degrees back."""
+    rng = np.random.default_rng(count + n)
+    s = np.minimum(rng.geometric(0.002, count) - 1, n - 1).astype(np.uint32)
+    t = rng.integers(0, n, count, dtype=np.uint32)
+    with cg.Engine(n, 512) as eng:
+        if bad:
+            b = t.copy()
+            b[count // 2] = n
+            with pytest.raises(cg.CytomError):
+                eng.insert_edges(s, b)
+            assert not any(x.any() for x in eng.degrees())
+        eng.insert_edges(s, t)
+        out_deg, in_deg = eng.degrees()
+        assert np.array_equal(out_deg, np.bincount(s, minlength=n)) and np.array_equal(in_deg, np.bincount(t, minlength=n))
