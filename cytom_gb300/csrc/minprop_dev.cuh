@@ -111,20 +111,17 @@ __device__ __forceinline__ void round_open(const JobDesc* __restrict__ jd, const
 // Tile columns in which the active sources of frontier word i (bits w) may have edges:
 // the OR of their column masks, read for words with at most four active sources (the
 // sparse rounds' words hold about one); all columns for denser words or without masks.
-constexpr int CM_MAX = 4;
 __device__ __forceinline__ unsigned long long word_columns(const StoreDesc* __restrict__ sd, uint64_t i,
                                                            uint32_t w) {
   const unsigned long long* cm = sd->cmask;
-  if (!cm || __popc(w) > CM_MAX) return ~0ULL;
+  if (!cm || __popc(w) > 4) return ~0ULL;
   unsigned long long m = 0;
   const unsigned long long* row = cm + (i << 5);
-  while (w) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (w) {
-        m |= row[__ffs(w) - 1];
-        w &= w - 1;
-      }
+  for (int k = 0; k < 4; ++k) {
+    if (w) {
+      m |= row[__ffs(w) - 1];
+      w &= w - 1;
     }
   }
   return m;
@@ -208,66 +205,60 @@ __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const
   const uint32_t* __restrict__ next = jd->next;
   const unsigned lane = threadIdx.x & 31;
   const uint64_t i = base + threadIdx.x;
-  // the step's time is its chain of L2 accesses: the changed word; then the list slot, the
-  // row count, the column masks and the new values, all in flight at once; then what hangs on
-  // the slot and the row (a sparse round's apply on 4 M vertices 11.3 us in turn, 8.4 so)
   uint32_t w = 0;
   if (i < nwords) {
     w = ld_plain<PERSIST>(ch + i);
     fa[i] = w;
-    if (w) ch[i] = 0;
-  }
-  const unsigned nz = __ballot_sync(0xFFFFFFFFu, w != 0);
-  if (!nz) return;
-  const unsigned pc = __popc(w);
-  cnt += pc;
-  unsigned slot0 = 0, row_was = 1;
-  const uint64_t row = ((base + (threadIdx.x & ~31u)) << 5) >> lvpt;  // the warp's, where a row holds whole warps
-  {
-    const unsigned tot = __reduce_add_sync(0xFFFFFFFFu, pc);
-    if (lane == 0) {
-      slot0 = atomicAdd(&ls->nact_words[pw], (unsigned)__popc(nz));
-      if (lvpt >= 10) row_was = atomicAdd(&rows_w[row], tot);
-    }
-  }
-  unsigned long long cols = 0;
-  if (w) {
-    cols = word_columns(sd, i, w);
-    if (!PERSIST && pc > 2 && ((i + 1) << 5) <= n) {
-      // many changed vertices: the whole word's 32 values in one round trip. A vertex
-      // without its changed bit holds next == current (every lowering of next sets
-      // the bit), so copying it is a no-op. (Not in the persistent kernel, whose
-      // register budget would spill the eight vectors.)
-      const uint4* src = reinterpret_cast<const uint4*>(next + (i << 5));
-      uint4* dst = reinterpret_cast<uint4*>(cur + (i << 5));
-      uint4 q[8];
+    if (w) {
+      ch[i] = 0;
+      if (!PERSIST && __popc(w) > 2 && ((i + 1) << 5) <= n) {
+        // many changed vertices: the whole word's 32 values in one round trip. A vertex
+        // without its changed bit holds next == current (every lowering of next sets
+        // the bit), so copying it is a no-op. (Not in the persistent kernel, whose
+        // register budget would spill the eight vectors.)
+        const uint4* src = reinterpret_cast<const uint4*>(next + (i << 5));
+        uint4* dst = reinterpret_cast<uint4*>(cur + (i << 5));
+        uint4 q[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) q[k] = ld_plain<PERSIST>(src + k);
+        for (int k = 0; k < 8; ++k) q[k] = ld_plain<PERSIST>(src + k);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) dst[k] = q[k];
-    } else {
-      uint32_t bits = w;
-      while (bits) {
-        const uint64_t v0 = (i << 5) + (__ffs(bits) - 1);
-        bits &= bits - 1;
-        const uint64_t v1 = bits ? (i << 5) + (__ffs(bits) - 1) : v0;
-        bits &= bits - 1;
-        const uint32_t x0 = ld_plain<PERSIST>(next + v0), x1 = ld_plain<PERSIST>(next + v1);
-        cur[v0] = x0;
-        cur[v1] = x1;
+        for (int k = 0; k < 8; ++k) dst[k] = q[k];
+      } else {
+        uint32_t bits = w;
+        while (bits) {
+          const int b = __ffs(bits) - 1;
+          bits &= bits - 1;
+          const uint64_t v = (i << 5) + b;
+          cur[v] = ld_plain<PERSIST>(next + v);
+        }
       }
     }
   }
-  slot0 = __shfl_sync(0xFFFFFFFFu, slot0, 0);
-  if (w) {
-    const unsigned slot = slot0 + __popc(nz & ((1u << lane) - 1u));
-    jd->aw[slot] = (uint32_t)i;
-    jd->awm[slot] = cols;
-    // past this many words the round is not a small one whatever the estimate
-    if (!PERSIST && slot < (SMALL_ITEMS >> sd->lT) + 1u) est = min(est + word_edges(sd, i, w), EST_MAX);
+  const unsigned pc = __popc(w);
+  cnt += pc;
+  {
+    const unsigned nz = __ballot_sync(0xFFFFFFFFu, w != 0);
+    if (nz) {
+      unsigned slot0 = 0;
+      if (lane == 0) slot0 = atomicAdd(&ls->nact_words[pw], (unsigned)__popc(nz));
+      slot0 = __shfl_sync(0xFFFFFFFFu, slot0, 0);
+      if (w) {
+        const unsigned slot = slot0 + __popc(nz & ((1u << lane) - 1u));
+        jd->aw[slot] = (uint32_t)i;
+        jd->awm[slot] = word_columns(sd, i, w);
+        // past this many words the round is not a small one whatever the estimate
+        if (!PERSIST && slot < (SMALL_ITEMS >> sd->lT) + 1u) est = min(est + word_edges(sd, i, w), EST_MAX);
+      }
+    }
   }
   if (lvpt >= 10) {
-    if (row_was == 0) teps += row_edges(sd, row);  // lane 0
+    unsigned tot = pc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xFFFFFFFFu, tot, o);
+    if (lane == 0 && tot) {
+      const uint64_t x = ((base + (threadIdx.x & ~31u)) << 5) >> lvpt;
+      if (atomicAdd(&rows_w[x], tot) == 0) teps += row_edges(sd, x);
+    }
   } else if (w) {
     uint32_t bits = w;
     while (bits) {
