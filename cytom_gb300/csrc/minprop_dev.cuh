@@ -573,7 +573,7 @@ __device__ __forceinline__ SpItem sp_item(const JobDesc* __restrict__ jd, const 
 // tile, row << 16 | column; a directory exists for up to 2^14 tiles a side only); the
 // loads of all ILP edges are issued before any of them is used.
 // LAT: a target's value is loaded beside the source's, for every edge with an active source
-// (one dependent step less, 55.2 -> 54.2 ms for an RMAT-22 stream; otherwise only for edges
+// (one dependent step less, 53.9 -> 52.7 ms for an RMAT-22 stream; otherwise only for edges
 // that offer a value).
 template <int ALGO, int PERSIST, int ILP, bool LAT = false>
 __device__ __forceinline__ void sp_batch(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
