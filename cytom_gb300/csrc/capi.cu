@@ -130,6 +130,7 @@ int upload_store_desc(Ctx* c) {
   h.cmask = h.dir_ok ? c->cmask : nullptr;
   h.cshift = c->lT > 6 ? c->lT - 6 : 0u;
   h.traversal = (uint32_t)c->cfg.traversal;
+  h.small_ok = c->small_max ? 1u : 0u;
   h.xst = c->xs_stage;
   h.xcum = c->xs_cum;
   h.xcolcum = c->xs_colcum;
@@ -263,6 +264,7 @@ static int job_prepare(Ctx* c, Job* j) {
   if (is_minprop(j->algo)) {
     rc = build_directory(c);
     if (!rc) rc = ensure_job_queue(c, j);
+    if (!rc) rc = ensure_small(c, j);
     if (!rc && autotune_due(c)) rc = minprop_autotune(c);
     if (!rc && tiles_in_use(c, j->algo)) rc = build_tile_stages(c);
     if (rc) return rc;
@@ -290,8 +292,8 @@ static int job_finish(Ctx* c, Job* j, const LoopState& ls, cudaEvent_t ev_a, cud
                       cytom_run_stats* st) {
   if (ls.err) return set_err(c, CYTOM_ERR_TIMEOUT, "a bounded device wait gave up");
   j->last_rounds = ls.iter;
-  // passes of the captured loop (the seeding apply counts one): small rounds, two gathers, chunk pass, apply
-  if (j->last_run_graph && ls.sel_rounds) c->launches += 5ULL * (ls.sel_rounds - 1);
+  // passes of the captured loop (the seeding apply counts one): two gathers, chunk pass, apply, and small rounds
+  if (j->last_run_graph && ls.sel_rounds) c->launches += (c->small_max ? 5ULL : 4ULL) * (ls.sel_rounds - 1);
   if (st) {
     memset(st, 0, sizeof(*st));
     st->iterations = ls.iter;
@@ -499,6 +501,7 @@ int cytom_create(const cytom_config* cfg, cytom_ctx** out) {
     delete c;
     return CYTOM_ERR_CUDA;
   }
+  if (const char* ev = getenv("CYTOM_SMALL_ROUNDS")) c->small_max = atoi(ev) >= 16 ? 16u : atoi(ev) >= 8 ? 8u : 0u;
   cudaGetDevice(&c->device);
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
   if (cfg->stream) {

@@ -58,7 +58,7 @@ struct StoreDesc {
   uint32_t nbw;                // 32-source blocks per tile row (vpt / 32)
   int dir_ok;                  // directory current (sparse rounds allowed)
   uint32_t sparse_div;         // sparse round while non-zero frontier words * sparse_div <= all words
-  uint32_t pad_sd;
+  uint32_t small_ok;           // small rounds may run in one cluster (Ctx::small_max)
   // column-ordered stages of the dense round (gather_tiles_kernel): stages of every tile in
   // column-major tile order (column y, then row x); xcum[i] = partition weight before
   // stage i in that order (edges + a fixed cost per stage; xcum[*xnst] = the total);
@@ -222,6 +222,10 @@ struct Ctx {
   std::vector<cudaEvent_t> ev_pool;
   cytom_kernel_stats kstats{};
   cudaEvent_t run_a = nullptr, run_b = nullptr;
+  // small rounds: the most CTAs of their cluster (16, or CYTOM_SMALL_ROUNDS: 8, or 0 for none)
+  // and the size found to fit per program (0: not asked yet)
+  unsigned small_max = 16;
+  unsigned small_cl[4] = {};
   // batched executor: device tables kept by the first context of a batch
   void* batch = nullptr;
   uint64_t batch_units = 0;
@@ -344,6 +348,7 @@ void settle_runs(Ctx* c);
 int job_run(Ctx* c, Job* j, cytom_run_stats* st);
 int job_result(Ctx* c, Job* j, void* out, int where);
 int ensure_job_queue(Ctx* c, Job* j);
+int ensure_small(Ctx* c, Job* j);
 int minprop_autotune(Ctx* c);
 void sg_shapes(int* ept, int* nst, int* minb, int* count);
 void batch_free(Ctx* c);

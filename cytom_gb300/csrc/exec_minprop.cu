@@ -1430,27 +1430,47 @@ static void* small_fn(int algo) {
                                    : (void*)small_rounds_kernel<2>;
 }
 
-// CTAs of the cluster: SM_CL where the device can hold one such cluster of `fn`, else 8.
-static unsigned small_cluster(void* fn) {
-  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = SM_CL;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(SM_CL);
-  cfg.blockDim = dim3(SM_T);
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) return SM_CL;
-  cudaGetLastError();
-  return 8;
+static int small_index(int algo) {
+  return algo == CYTOM_ALGO_BFS ? 0 : algo == CYTOM_ALGO_CC ? 1 : algo == CYTOM_ALGO_SSWP ? 3 : 2;
+}
+
+// CTAs of a cluster of `fn`, at most `most`: 16 where the device can hold one such cluster,
+// else 8; 0 where it holds neither.
+static unsigned small_cluster(void* fn, unsigned most) {
+  for (unsigned cl = most; cl >= 8; cl /= 2) {
+    if (cl > 8) cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cl);
+    cfg.blockDim = dim3(SM_T);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) return cl;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
+// The cluster size of the job's program, asked once per context (an occupancy query per run cost
+// the shortest runs some 5 us of host time). Where no cluster fits, the context runs every
+// round grid-wide.
+int ensure_small(Ctx* c, Job* j) {
+  unsigned& cl = c->small_cl[small_index(j->algo)];
+  if (!c->small_max || cl) return CYTOM_OK;
+  cl = small_cluster(small_fn(j->algo), c->small_max);
+  if (cl) return CYTOM_OK;
+  c->small_max = 0;
+  c->tune_epoch++;  // captured loops are built again, without the cluster's node
+  return upload_store_desc(c);
 }
 
 static cudaError_t launch_small(Ctx* c, Job* j, int adaptive, unsigned max_rounds, int initial, unsigned max_iter) {
   void* fn = small_fn(j->algo);
-  const unsigned cl = small_cluster(fn);
+  const unsigned cl = c->small_cl[small_index(j->algo)];
   const JobDesc* jd = j->d;
   const StoreDesc* sd = c->dsd;
   cudaGraphConditionalHandle h{};
@@ -1531,7 +1551,7 @@ static cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGr
 
 // A run on a graph of at most SMALL_E edges is one launch of the cluster, begin and seeding
 // apply included: pick_mode keeps every round of it small.
-static bool whole_run_small(const Ctx* c) { return c->E <= SMALL_E && (c->n + 31) / 32 <= SMALL_WORDS; }
+static bool whole_run_small(const Ctx* c) { return c->small_max && c->E <= SMALL_E && (c->n + 31) / 32 <= SMALL_WORDS; }
 
 // Graph: begin -> seeding apply + control -> while(cont) { small rounds -> dense gather ->
 // sparse gather -> chunk pass -> apply + control }. The kind of round is picked on the device
@@ -1569,9 +1589,9 @@ static int build_minprop_graph(Ctx* c, Job* j) {
     unsigned max_rounds = SM_ROUNDS;
     void* a_s[] = {(void*)&jd,   (void*)&sd,       (void*)&adaptive, (void*)&max_rounds,
                    (void*)&zero, (void*)&max_iter, (void*)&h,        (void*)&one};
-    const unsigned cl = small_cluster(small_fn(j->algo));
-    e = add_kernel(body, &b_small, nullptr, 0, small_fn(j->algo), dim3(cl), dim3(SM_T), a_s);
-    if (e == cudaSuccess) {
+    const unsigned cl = c->small_max ? c->small_cl[small_index(j->algo)] : 0u;
+    if (cl) e = add_kernel(body, &b_small, nullptr, 0, small_fn(j->algo), dim3(cl), dim3(SM_T), a_s);
+    if (cl && e == cudaSuccess) {
       cudaLaunchAttributeValue av{};
       av.clusterDim.x = cl;
       av.clusterDim.y = av.clusterDim.z = 1;
@@ -1579,7 +1599,7 @@ static int build_minprop_graph(Ctx* c, Job* j) {
     }
     void* a_g[] = {(void*)&jd, (void*)&sd, (void*)&adaptive};
     GatherLaunch gl = gather_launch(c, j->algo);
-    if (e == cudaSuccess) e = add_kernel(body, &d_gather, &b_small, 1, gl.fn, gl.grid, gl.block, a_g, gl.smem);
+    if (e == cudaSuccess) e = add_kernel(body, &d_gather, &b_small, cl ? 1 : 0, gl.fn, gl.grid, gl.block, a_g, gl.smem);
     if (e == cudaSuccess)
       e = add_kernel(body, &s_sparse, &d_gather, 1, sparse_fn(j->algo), dim3(g_sparse), dim3(256), a_g);
     void* a_q[] = {(void*)&jd, (void*)&sd};
@@ -1716,7 +1736,7 @@ int minprop_run(Ctx* c, Job* j) {
     }
     // launch a few rounds before checking: kernels are no-ops once the run ended
     for (int k = 0; k < 4 && round < max_iter; ++k, ++round) {
-      e = launch_small(c, j, adaptive, SM_ROUNDS, 0, max_iter);
+      if (c->small_max) e = launch_small(c, j, adaptive, SM_ROUNDS, 0, max_iter);
       if (e != cudaSuccess) return cuda_err(c, e, "small rounds");
       int rc = launch_gather(c, j, adaptive);
       if (rc) return rc;

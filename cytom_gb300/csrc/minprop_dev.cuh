@@ -175,7 +175,7 @@ __device__ __forceinline__ unsigned pick_mode(const JobDesc* __restrict__ jd, co
                                               unsigned nact, unsigned est, int allow_small) {
   const uint64_t nwords = (sd->n + 31) >> 5;
   const bool listed = sd->dir_ok && sd->adaptive;
-  if (allow_small && nwords <= SMALL_WORDS &&
+  if (allow_small && sd->small_ok && nwords <= SMALL_WORDS &&
       (sd->E <= SMALL_E || (listed && ((uint64_t)nact << sd->lT) <= SMALL_ITEMS && est <= SMALL_EDGES)))
     return 2u;
   const uint32_t div = jd->sparse_div ? jd->sparse_div : sd->sparse_div;
