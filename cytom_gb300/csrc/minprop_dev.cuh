@@ -139,6 +139,13 @@ constexpr uint32_t SMALL_EDGES = 1u << 16;
 constexpr uint32_t SMALL_WORDS = 1u << 19;
 constexpr uint32_t EST_MAX = 1u << 20;  // est saturates per block here
 
+// Listed frontier words whose out-edges the estimate needs: with more the round is not a small
+// one whatever they hold. (On a graph of at most SMALL_E edges the estimate also chooses a small
+// round's gather.)
+__device__ __forceinline__ uint32_t est_words(const StoreDesc* __restrict__ sd) {
+  return sd->E <= SMALL_E ? 0xFFFFFFFFu : (SMALL_ITEMS >> sd->lT) + 1u;
+}
+
 // Out-edges of the active vertices of frontier word i (bits w), their degrees in flight
 // together; words past the vertex count (fewer than 32 vertices) one by one.
 __device__ __forceinline__ unsigned word_edges(const StoreDesc* __restrict__ sd, uint64_t i, uint32_t w) {
@@ -246,8 +253,7 @@ __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const
         const unsigned slot = slot0 + __popc(nz & ((1u << lane) - 1u));
         jd->aw[slot] = (uint32_t)i;
         jd->awm[slot] = word_columns(sd, i, w);
-        // past this many words the round is not a small one whatever the estimate
-        if (!PERSIST && slot < (SMALL_ITEMS >> sd->lT) + 1u) est = min(est + word_edges(sd, i, w), EST_MAX);
+        if (!PERSIST && slot < est_words(sd)) est = min(est + word_edges(sd, i, w), EST_MAX);
       }
     }
   }
