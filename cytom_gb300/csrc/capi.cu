@@ -113,7 +113,7 @@ int upload_store_desc(Ctx* c) {
   h.wts = c->wts;
   h.tile_ptr = c->tile_ptr;
   h.chunk_tile = c->chunk_tile;
-  h.out_deg = c->out_deg;
+  h.out_deg = c->est_deg ? c->est_deg + (uint64_t)c->est_at * c->n : c->out_deg;
   h.in_deg = c->in_deg;
   h.E = c->E;
   h.nchunks = (c->E + kChunk - 1) / kChunk;
@@ -130,7 +130,6 @@ int upload_store_desc(Ctx* c) {
   h.cmask = h.dir_ok ? c->cmask : nullptr;
   h.cshift = c->lT > 6 ? c->lT - 6 : 0u;
   h.traversal = (uint32_t)c->cfg.traversal;
-  h.small_ok = c->small_max ? 1u : 0u;
   h.xst = c->xs_stage;
   h.xcum = c->xs_cum;
   h.xcolcum = c->xs_colcum;
@@ -309,8 +308,34 @@ static int job_finish(Ctx* c, Job* j, const LoopState& ls, cudaEvent_t ev_a, cud
   return CYTOM_OK;
 }
 
+// Whether the runs about to be launched may take small rounds, and the degrees their estimates
+// read. Asynchronous runs need degrees that an insert beside them does not change; without
+// memory for those they take no small round.
+static int small_prepare(Ctx* c, bool async) {
+  if (!c->small_max && !c->hsd.small_ok) return CYTOM_OK;
+  bool changed = false;
+  if (c->small_max && async && !c->est_deg && small_vertices(c)) {
+    if (cy_malloc(&c->est_deg, 2 * c->n * 4) != cudaSuccess) {
+      cudaGetLastError();
+      c->est_deg = nullptr;
+    }
+    changed = c->est_deg != nullptr;
+  }
+  if (c->est_deg && c->est_version != c->version) {
+    cudaError_t e = cudaMemcpyAsync(c->est_deg + (uint64_t)c->est_at * c->n, c->out_deg, c->n * 4,
+                                    cudaMemcpyDeviceToDevice, c->stream);
+    if (e != cudaSuccess) return cuda_err(c, e, "degree copy");
+    c->est_version = c->version;
+  }
+  const uint32_t ok = (c->small_max && (!async || c->est_deg || !small_vertices(c))) ? 1u : 0u;
+  if (ok == c->hsd.small_ok && !changed) return CYTOM_OK;
+  c->hsd.small_ok = ok;
+  return upload_store_desc(c);
+}
+
 int job_run(Ctx* c, Job* j, cytom_run_stats* st) {
   int rc = job_prepare(c, j);
+  if (!rc && is_minprop(j->algo)) rc = small_prepare(c, false);
   if (rc) return rc;
   cudaEventRecord(c->run_a, c->stream);
   rc = is_minprop(j->algo) ? minprop_run(c, j) : pagerank_run(c, j);
@@ -346,9 +371,13 @@ void settle_runs(Ctx* c) {
 
 // Launches the jobs' loops on their streams after the shared preparation; the context's
 // stream is not made to wait for them (join_runs does that).
-static int launch_many(Ctx* c, Job** jobs, int count) {
+static int launch_many(Ctx* c, Job** jobs, int count, bool async) {
   for (int k = 0; k < count; ++k) {
     int rc = job_prepare(c, jobs[k]);
+    if (rc) return rc;
+  }
+  {
+    int rc = small_prepare(c, async);
     if (rc) return rc;
   }
   while ((int)c->conc.size() < count) {
@@ -426,7 +455,7 @@ int job_run_many(Ctx* c, Job** jobs, int count, cytom_run_stats* stats) {
     }
     return CYTOM_OK;
   }
-  int rc = launch_many(c, jobs, count);
+  int rc = launch_many(c, jobs, count, false);
   if (rc) return rc;
   return collect_runs(c, stats);
 }
@@ -576,7 +605,7 @@ int cytom_destroy(cytom_ctx* ctx) {
   void* ptrs[] = {c->dir, c->dir_alt, c->cmask, c->edges, c->wts, c->edges_alt, c->wts_alt, c->tile_ptr, c->tile_ptr_alt,
                   c->chunk_tile, c->chunk_tile_alt, c->app_keys, c->app_keys_alt, c->app_w, c->app_w_alt,
                   c->out_deg, c->in_deg, c->dsd, c->scratch, c->d_flag, c->xs_stage, c->xs_cum,
-                  c->xs_colcum, c->xs_tmp, c->pr_pair, c->dyn_pending, c->dyn_next};
+                  c->xs_colcum, c->xs_tmp, c->pr_pair, c->dyn_pending, c->dyn_next, c->est_deg};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
@@ -937,7 +966,7 @@ int cytom_run_many_async(cytom_ctx* ctx, const int* job_ids, int count) {
     c->sync_jobs = jobs;
     return CYTOM_OK;
   }
-  return launch_many(c, jobs.data(), count);
+  return launch_many(c, jobs.data(), count, true);
 }
 
 int cytom_run_many_wait(cytom_ctx* ctx, cytom_run_stats* stats) {

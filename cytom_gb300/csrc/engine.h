@@ -42,7 +42,7 @@ struct StoreDesc {
   const uint32_t* wts;
   const unsigned long long* tile_ptr;
   const uint32_t* chunk_tile;
-  const uint32_t* out_deg;
+  const uint32_t* out_deg;  // of the snapshot (Ctx::est_deg); read for small rounds' estimates only
   const uint32_t* in_deg;
   unsigned long long E;        // compacted edges (written on the device by compaction)
   unsigned long long nchunks;  // ceil(E / kChunk)
@@ -226,6 +226,12 @@ struct Ctx {
   // and the size found to fit per program (0: not asked yet)
   unsigned small_max = 16;
   unsigned small_cl[4] = {};
+  // Out-degrees of the installed snapshot for the estimates of small rounds, and those of the
+  // next one (est_at: the current half), kept once runs are launched asynchronously: an insert
+  // beside them raises out_deg. est_version: the snapshot the current half belongs to.
+  uint32_t* est_deg = nullptr;
+  int est_at = 0;
+  uint64_t est_version = ~0ULL;
   // batched executor: device tables kept by the first context of a batch
   void* batch = nullptr;
   uint64_t batch_units = 0;
@@ -349,6 +355,7 @@ int job_run(Ctx* c, Job* j, cytom_run_stats* st);
 int job_result(Ctx* c, Job* j, void* out, int where);
 int ensure_job_queue(Ctx* c, Job* j);
 int ensure_small(Ctx* c, Job* j);
+bool small_vertices(const Ctx* c);  // the vertex range allows small rounds
 int minprop_autotune(Ctx* c);
 void sg_shapes(int* ept, int* nst, int* minb, int* count);
 void batch_free(Ctx* c);

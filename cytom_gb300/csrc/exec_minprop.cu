@@ -1465,8 +1465,10 @@ int ensure_small(Ctx* c, Job* j) {
   if (cl) return CYTOM_OK;
   c->small_max = 0;
   c->tune_epoch++;  // captured loops are built again, without the cluster's node
-  return upload_store_desc(c);
+  return CYTOM_OK;
 }
+
+bool small_vertices(const Ctx* c) { return (c->n + 31) / 32 <= SMALL_WORDS; }
 
 static cudaError_t launch_small(Ctx* c, Job* j, int adaptive, unsigned max_rounds, int initial, unsigned max_iter) {
   void* fn = small_fn(j->algo);
@@ -1551,7 +1553,7 @@ static cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGr
 
 // A run on a graph of at most SMALL_E edges is one launch of the cluster, begin and seeding
 // apply included: pick_mode keeps every round of it small.
-static bool whole_run_small(const Ctx* c) { return c->small_max && c->E <= SMALL_E && (c->n + 31) / 32 <= SMALL_WORDS; }
+static bool whole_run_small(const Ctx* c) { return c->hsd.small_ok && c->E <= SMALL_E && small_vertices(c); }
 
 // Graph: begin -> seeding apply + control -> while(cont) { small rounds -> dense gather ->
 // sparse gather -> chunk pass -> apply + control }. The kind of round is picked on the device
@@ -1736,7 +1738,7 @@ int minprop_run(Ctx* c, Job* j) {
     }
     // launch a few rounds before checking: kernels are no-ops once the run ended
     for (int k = 0; k < 4 && round < max_iter; ++k, ++round) {
-      if (c->small_max) e = launch_small(c, j, adaptive, SM_ROUNDS, 0, max_iter);
+      if (c->hsd.small_ok) e = launch_small(c, j, adaptive, SM_ROUNDS, 0, max_iter);
       if (e != cudaSuccess) return cuda_err(c, e, "small rounds");
       int rc = launch_gather(c, j, adaptive);
       if (rc) return rc;

@@ -1215,6 +1215,9 @@ int compact(Ctx* c) {
     cudaFreeAsync(tmp, c->stream);
     return rc;
   }
+  if (c->est_deg)  // the degrees of the new snapshot, beside those that runs still read
+    cudaMemcpyAsync(c->est_deg + (uint64_t)(c->est_at ^ 1) * c->n, c->out_deg, c->n * 4, cudaMemcpyDeviceToDevice,
+                    c->stream);
   // Installing the merged snapshot: runs on the previous one must have finished (everything
   // above wrote to the new snapshot alone). The jobs are then seeded by the merged edges
   // (edgeChanged(INSERT)).
@@ -1246,6 +1249,10 @@ int compact(Ctx* c) {
   c->E += Kn;
   c->A = 0;
   c->version++;
+  if (c->est_deg) {
+    c->est_at ^= 1;
+    c->est_version = c->version;
+  }
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "merge");
   if (mdir) c->dir_version = c->version;

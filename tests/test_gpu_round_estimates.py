@@ -1,9 +1,19 @@
 """The out-edge estimate that picks the kind of a round depends on the snapshot alone: on small
-graphs it holds every listed word whichever kernel lists them."""
+graphs it holds every listed word whichever kernel lists them, and an insert beside
+asynchronous runs does not change it. The edges a run scans, which follow from the kinds of its
+rounds, are therefore the same in every repetition."""
+import json
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+ROOT = Path(__file__).resolve().parents[1]
 
 
 def test_small_graph_scans_the_same_edges_profiled(cg):
@@ -25,3 +35,72 @@ def test_small_graph_scans_the_same_edges_profiled(cg):
             eng.set_profiling(False)
             got.append((x["iterations"], x["count_edges"], x["edges_scanned"], cc.result().tobytes()))
     assert got[0] == got[1]
+
+
+CODE = """
+import sys, json, numpy as np
+sys.path.insert(0, {root!r})
+import torch, cytom_gb300 as cg
+side = 256
+n = side * side
+v = np.arange(n, dtype=np.uint32)
+r, d = v[v % side < side - 1], v[: side * (side - 1)]
+s = np.concatenate([r, d, r + 1, d + side]).astype(np.uint32)
+t = np.concatenate([r + 1, d + side, r, d]).astype(np.uint32)
+m = 1 << 25  # 512 out-edges a vertex: a frontier of 256 then holds more than a small round's
+bs = torch.randint(0, n, (m,), device="cuda", dtype=torch.int32)
+bt = torch.randint(0, n, (m,), device="cuda", dtype=torch.int32)
+torch.cuda.synchronize()
+want = (v // side + v % side).astype(np.uint32)
+out = []
+for beside in (False, True, True):
+    with cg.Engine(n, n) as eng:
+        eng.insert_edges(bs, bt)  # the append region has its size
+        eng.clear()
+        eng.insert_edges(s, t)
+        eng.do_global_compaction()
+        ps = [cg.BFS(eng, start_vertex=0, max_iterations=10000) for _ in range(2)]
+        eng.run_many_async(ps)
+        if beside:
+            eng.insert_edges(bs, bt)
+        x = eng.run_many_wait()
+        out.append([[q["iterations"], q["count_edges"], q["edges_scanned"]] for q in x])
+        if not beside:
+            assert all(np.array_equal(p.result(), want) for p in ps)
+print(json.dumps(out))
+"""
+
+
+def test_insert_beside_asynchronous_runs_changes_no_round():
+    """A lattice's small frontiers, while 2^25 edges are appended: dense rounds (forced by the
+    threshold) in place of small ones would scan the whole graph."""
+    env = dict(os.environ, CYTOM_SPARSE_DIV="1024")
+    r = subprocess.run([sys.executable, "-c", CODE.format(root=str(ROOT))], capture_output=True, text=True, env=env,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
+    out = json.loads(r.stdout.strip().splitlines()[-1])
+    assert out[0] == out[1] == out[2], out
+
+
+def test_without_memory_for_the_degrees(cg, orc):
+    """The first asynchronous launch cannot have its copy of the degrees: the runs give the same
+    values, later ones too."""
+    s, t = orc.rmat(12, 0, 1 << 16, 3)
+    n = 1 << 12
+    st = orc.Store(n, 1024)
+    st.insert(s, t)
+    st.compact()
+    with cg.Engine(n, 1024) as eng:
+        eng.insert_edges(s, t)
+        progs = [(cg.BFS(eng, start_vertex=0, max_iterations=1000), orc.BFS), (cg.CC(eng, max_iterations=1000), orc.CC)]
+        eng.run_many([p for p, _ in progs])
+        for fail in (1, 0):
+            for p, _ in progs:
+                p.init_algorithm()
+            eng.set_fault_injection(fail_alloc_after=fail)
+            eng.run_many_async([p for p, _ in progs])
+            stats = eng.run_many_wait()
+            eng.set_fault_injection()
+            for (p, a), x in zip(progs, stats):
+                ref, info = st.run_minprop(a, start=0, max_iter=1000)
+                assert np.array_equal(p.result(), ref) and x["iterations"] == info["iterations"]
