@@ -143,6 +143,7 @@ struct Job {
   int algo = 0;
   cytom_job_params params{};
   bool fresh = true;          // next run starts from scratch
+  bool lists_all = false;     // the next run's first frontier lists every word (CC from scratch)
   bool async = false;         // asynchronous program (CYTOM_ALGO_BFS_ASYNC / CC_ASYNC)
   JobDesc h{};                // host copy of the descriptor
   JobDesc* d = nullptr;       // device copy

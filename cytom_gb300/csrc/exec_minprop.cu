@@ -957,6 +957,7 @@ __global__ void __launch_bounds__(SM_T, 1)
   const uint32_t wtid = ((threadIdx.x >> 3) * ncta + rank) * 8 + (threadIdx.x & 7u);
   const uint32_t nwords = (uint32_t)((sd->n + 31) >> 5);
   const uint64_t E = sd->E, T = sd->T;
+  const uint32_t lT = sd->lT;
   const unsigned max_iter = initial ? max_iter_arg : vls->max_iter;
   const bool listed = sd->dir_ok && sd->adaptive;
   unsigned iter = initial ? 0u : vls->iter;
@@ -1040,7 +1041,12 @@ __global__ void __launch_bounds__(SM_T, 1)
             s_word[at] = i;
             s_bits[at] = w[k];
           } else {  // more changed words than the list holds: applied here
-            small_word(jd, sd, pw, i, w[k], atomicAdd(&tot->nact[pw], 1u), cnt, teps, est);
+            const unsigned m = __activemask();  // these lanes' slots with one atomic
+            const int lead = __ffs(m) - 1;
+            unsigned slot = 0;
+            if (lane == (unsigned)lead) slot = atomicAdd(&tot->nact[pw], (unsigned)__popc(m));
+            slot = __shfl_sync(m, slot, lead) + __popc(m & ((1u << lane) - 1u));
+            small_word(jd, sd, pw, i, w[k], slot, cnt, teps, est);
           }
         } else if (f[k]) {
           jd->fa[i] = 0;
@@ -1077,7 +1083,8 @@ __global__ void __launch_bounds__(SM_T, 1)
     const unsigned active = *(volatile unsigned*)&tot->active[pw];
     nact = *(volatile unsigned*)&tot->nact[pw];
     est0 = *(volatile unsigned*)&tot->est[pw];
-    mode = pick_mode(jd, sd, nact, est0, 1);
+    // (a whole run stays here; from values at hand first: pick_mode's loads take 0.15 us a round)
+    mode = initial || small_round(E, lT, listed, nact, est0) ? 2u : pick_mode(jd, sd, nact, est0, 0);
     active_total += active;
     cont = (active > 0 && iter < max_iter) ? 1u : 0u;
   } while (cont && mode == 2 && rounds < max_rounds);
@@ -1291,6 +1298,7 @@ int minprop_init(Ctx* c, Job* j) {
   int algo = j->algo;
   init_minprop_kernel<<<grid_persistent(c, 8), 256, 0, c->stream>>>(j->d, c->dsd, algo, j->params.start_vertex);
   c->launches++;
+  j->lists_all = algo == CYTOM_ALGO_CC;
   return cuda_err(c, cudaGetLastError(), "init_minprop");
 }
 
@@ -1552,8 +1560,12 @@ static cudaError_t add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGr
 }
 
 // A run on a graph of at most SMALL_E edges is one launch of the cluster, begin and seeding
-// apply included: pick_mode keeps every round of it small.
-static bool whole_run_small(const Ctx* c) { return c->hsd.small_ok && c->E <= SMALL_E && small_vertices(c); }
+// apply included, unless its first round lists more than SMALL_LISTED words (CC from scratch: all
+// of them). Later rounds list at most as many as the graph has edges.
+static bool whole_run_small(const Ctx* c, const Job* j) {
+  const bool listed = !j->lists_all || (c->n + 31) / 32 <= SMALL_LISTED;
+  return c->hsd.small_ok && c->E <= SMALL_E && small_vertices(c) && listed;
+}
 
 // Graph: begin -> seeding apply + control -> while(cont) { small rounds -> dense gather ->
 // sparse gather -> chunk pass -> apply + control }. The kind of round is picked on the device
@@ -1651,7 +1663,9 @@ static double round_bytes(const Ctx* c, const LoopState& a, const LoopState& b, 
 int minprop_run(Ctx* c, Job* j) {
   int adaptive = c->cfg.enable_adaptive_scheduling;
   unsigned max_iter = (unsigned)std::min<uint64_t>(j->params.max_iterations, 0xFFFFFFFFu);
-  if (!c->profiling && use_graphs() && whole_run_small(c)) {
+  const bool whole = whole_run_small(c, j);
+  j->lists_all = false;
+  if (!c->profiling && use_graphs() && whole) {
     j->last_run_graph = false;
     // a run converges within n rounds, each of them bounded
     cudaError_t e = launch_small(c, j, adaptive, 0xFFFFFFFFu, 1, max_iter);

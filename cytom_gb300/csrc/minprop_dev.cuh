@@ -129,11 +129,24 @@ __device__ __forceinline__ unsigned long long word_columns(const StoreDesc* __re
 
 // ---- small rounds --------------------------------------------------------
 // A round is small when one thread-block cluster finishes it sooner than the grid-wide
-// kernels, whose four launches cost about 20 us whatever the frontier holds: a graph of at
-// most SMALL_E edges, or a sparse round of at most SMALL_ITEMS (word, column) items whose
-// active vertices have at most SMALL_EDGES out-edges (LoopState::est). The cluster scans the
-// changed bitmap every round, which bounds the vertices (SMALL_WORDS).
+// kernels, whose launches cost about 20 us whatever the frontier holds: on a graph of at
+// most SMALL_E edges a round of at most SMALL_LISTED frontier words, else a sparse round of at
+// most SMALL_ITEMS (word, column) items whose active vertices have at most SMALL_EDGES
+// out-edges (LoopState::est). The cluster scans the changed bitmap every round, which bounds the
+// vertices (SMALL_WORDS).
+// Times of a round, cluster / grid-wide, in us, on graphs whose rounds all look alike:
+//   items (2^22 vertices)   1,024: 10.3 / 19.4   8,192: 10.8 / 19.4   65,536: 13.2 / 20.5
+//   out-edges (2^20)        4,600: 11.5 / 21.3   66,000: 18.9 / 28.2  263,000: 34 / 55
+//   vertices                2^20: 7.6 / 17.6     2^24: 15.6 / 20.9    2^25: 22.0 / 23.3
+//   edges, CC's whole run   65,500 (2^15 vertices): 348 / 754   131,000: 231 / 367   262,000: 249 / 289
+// so the limits of items, out-edges and edges lie below where the two meet on such graphs. Whole
+// workloads with one limit moved: 2^12 items, lattice of 2^18 vertices 19.5 ms, 2^13 17.9, 2^14 and
+// 2^16 as long (RMAT-22 stream 54.1, 53.8, 53.7, 53.0); 2^14 out-edges, lattice 23.0, 2^16 17.9, 2^18
+// 17.5; 2^14 edges, BFS on RMAT-12 167 us, 2^16 and 2^18 115; 2^16 words, stream 54.6, 2^19 53.8.
+// CC from scratch lists every word: with 60,000 edges 2^15 words take 123 us, grid-wide 139,
+// 2^16 words 165 / 141, 2^19 words 772 / 420 (three to five rounds).
 constexpr uint32_t SMALL_E = 1u << 16;
+constexpr uint32_t SMALL_LISTED = 1u << 15;
 constexpr uint32_t SMALL_ITEMS = 1u << 13;
 constexpr uint32_t SMALL_EDGES = 1u << 16;
 constexpr uint32_t SMALL_WORDS = 1u << 19;
@@ -143,7 +156,7 @@ constexpr uint32_t EST_MAX = 1u << 20;  // est saturates per block here
 // one whatever they hold. (On a graph of at most SMALL_E edges the estimate also chooses a small
 // round's gather.)
 __device__ __forceinline__ uint32_t est_words(const StoreDesc* __restrict__ sd) {
-  return sd->E <= SMALL_E ? 0xFFFFFFFFu : (SMALL_ITEMS >> sd->lT) + 1u;
+  return sd->E <= SMALL_E ? SMALL_LISTED : (SMALL_ITEMS >> sd->lT) + 1u;
 }
 
 // Out-edges of the active vertices of frontier word i (bits w), their degrees in flight
@@ -177,14 +190,18 @@ __device__ __forceinline__ unsigned word_edges(const StoreDesc* __restrict__ sd,
   return (unsigned)(e < EST_MAX ? e : EST_MAX);
 }
 
+// The limits of a small round of `nact` listed words on a graph whose vertex range allows them.
+__device__ __forceinline__ bool small_round(uint64_t E, uint32_t lT, bool listed, unsigned nact, unsigned est) {
+  return nact <= SMALL_LISTED &&
+         (E <= SMALL_E || (listed && ((uint64_t)nact << lT) <= SMALL_ITEMS && est <= SMALL_EDGES));
+}
+
 // The gather of a round with `nact` listed frontier words.
 __device__ __forceinline__ unsigned pick_mode(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
                                               unsigned nact, unsigned est, int allow_small) {
   const uint64_t nwords = (sd->n + 31) >> 5;
   const bool listed = sd->dir_ok && sd->adaptive;
-  if (allow_small && sd->small_ok && nwords <= SMALL_WORDS &&
-      (sd->E <= SMALL_E || (listed && ((uint64_t)nact << sd->lT) <= SMALL_ITEMS && est <= SMALL_EDGES)))
-    return 2u;
+  if (allow_small && sd->small_ok && nwords <= SMALL_WORDS && small_round(sd->E, sd->lT, listed, nact, est)) return 2u;
   const uint32_t div = jd->sparse_div ? jd->sparse_div : sd->sparse_div;
   return (listed && (uint64_t)nact * div <= nwords) ? 1u : 0u;
 }
