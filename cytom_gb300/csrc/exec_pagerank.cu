@@ -1527,7 +1527,8 @@ __global__ void dangling_sum_kernel(const T* __restrict__ r, const double* __res
 }
 
 // What dL/dw needs of vertex v, in vertex order: alpha r_v / s_v as a float pair and
-// (P^T lambda)_v in g, lambda_v. One FP64 division per vertex instead of one per edge.
+// (P^T lambda)_v in g, lambda_v. One FP64 division per vertex instead of one per edge. A factor
+// that a float pair cannot hold (ff_in_range) becomes NaN, and its edges are taken in FP64.
 __global__ void grad_prep_kernel(const uint32_t* __restrict__ perm, const float* __restrict__ r,
                                  const float* __restrict__ lam, const float* __restrict__ pt,
                                  const double* __restrict__ wsum, uint64_t n, double alpha, float4* __restrict__ g,
@@ -1535,7 +1536,9 @@ __global__ void grad_prep_kernel(const uint32_t* __restrict__ perm, const float*
   uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     const uint32_t q = perm[v];
-    const FF f = ff_from_double(alpha * (double)r[q] / wsum[q]);
+    const float rv = r[q];
+    FF f = ff_from_double(alpha * (double)rv / wsum[q]);
+    if (rv != 0.f && !ff_in_range(f.hi)) f.hi = __int_as_float(0x7FFFFFFF);
     g[v] = make_float4(f.hi, f.lo, pt[q], 0.f);
     lamv[v] = lam[q];
   }
@@ -1543,10 +1546,13 @@ __global__ void grad_prep_kernel(const uint32_t* __restrict__ perm, const float*
 
 // dL/dw of every stored edge u -> k, in store order:
 // alpha * r_u / s_u * (lambda_k - (P^T lambda)_u). FP32 form: the factor of u and the
-// difference as float pairs (each exact to about 44 bits), their product rounded once. Bound
+// difference as float pairs (the difference exact, the factor to 48 bits), their product rounded
+// once; where the factor or the product leaves their range the edge is taken in FP64. Bound
 // by the gather of lambda_k; in FP64 with a division per edge it was bound by the FP64 pipe.
 __global__ void grad_w32_kernel(const StoreDesc* __restrict__ sd, const float4* __restrict__ g,
-                                const float* __restrict__ lamv, float* __restrict__ gw) {
+                                const float* __restrict__ lamv, const uint32_t* __restrict__ perm,
+                                const float* __restrict__ r, const double* __restrict__ wsum, double alpha,
+                                float* __restrict__ gw) {
   const uint64_t E = sd->E;
   const uint32_t lT = sd->lT, lvpt = sd->lvpt;
   const uint32_t ymask = (uint32_t)(sd->T - 1);
@@ -1555,12 +1561,17 @@ __global__ void grad_w32_kernel(const StoreDesc* __restrict__ sd, const float4* 
     uint32_t t = sd->chunk_tile[e >> 7];
     while (sd->tile_ptr[t + 1] <= e) ++t;
     const uint32_t p = sd->edges[e];
-    const float4 gu = g[((t >> lT) << lvpt) | (p >> 16)];
+    const uint32_t u = ((t >> lT) << lvpt) | (p >> 16);
+    const float4 gu = g[u];
     const float lk = lamv[((t & ymask) << lvpt) | (p & 0xFFFFu)];
     const FF d = ff_two_sum(lk, -gu.z);
-    const float y = ff_mul(FF{gu.x, gu.y}, d).hi;
-    // an infinity makes the float pairs NaN; its plain product is what FP64 gives
-    gw[e] = isfinite(y) ? y : gu.x * (lk - gu.z);
+    float y = ff_mul(FF{gu.x, gu.y}, d).hi;
+    const bool zero = y == 0.f && (gu.x == 0.f || d.hi == 0.f);
+    if (!zero && !ff_in_range(y)) {
+      const uint32_t q = perm[u];
+      y = (float)(alpha * (double)r[q] / wsum[q] * ((double)lk - (double)gu.z));
+    }
+    gw[e] = y;
   }
 }
 
@@ -1699,7 +1710,8 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
     float* lamv = (float*)(tmp + 256 + wbytes + tbytes + gbytes);
     grad_prep_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(c->pr_perm, r32, lam, s->pt, g->wsum, n, a.alpha, gv, lamv);
     c->launches++;
-    if (E) grad_w32_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, gv, lamv, gw);
+    if (E)
+      grad_w32_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, gv, lamv, c->pr_perm, r32, g->wsum, a.alpha, gw);
     grad_t_kernel<float><<<grid_n(c, n), 256, 0, c->stream>>>(lam, c->pr_perm, n, dang, a.alpha, gt);
   } else {
     const double* lam = (pa == 0) ? s->lam64 : s->lam64 + n;

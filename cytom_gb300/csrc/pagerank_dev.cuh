@@ -155,6 +155,13 @@ __device__ __forceinline__ FF ff_div(FF a, FF b) {
   const FF r = ff_add(a, ff_mul(FF{-q, 0.f}, b));
   return ff_fast_two_sum(q, r.hi / b.hi);
 }
+// Float pairs have FP32's exponents: from 2^-96 down the low words of values, products and
+// quotients run out of them and the pair tends to plain FP32. A result that is not in this
+// range (nor exactly zero from zero factors) is taken in FP64 instead.
+constexpr float kFfMin = 0x1p-96f;  // 1.3e-29
+__device__ __forceinline__ bool ff_in_range(float hi) {
+  return fabsf(hi) >= kFfMin && fabsf(hi) <= 3.402823466e38f;  // false for NaN
+}
 __device__ __forceinline__ FF ff_abs(FF a) { return a.hi < 0.f ? FF{-a.hi, -a.lo} : a; }
 __host__ __device__ inline FF ff_from_double(double x) {
   const float hi = (float)x;

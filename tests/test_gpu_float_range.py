@@ -1,0 +1,56 @@
+"""FP32 forms of the weighted PageRank and its gradients where a value, a factor or a product of
+the update lies outside the range in which float pairs keep their low words. Against the FP64
+oracle on the same graph."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N, VPT = 1 << 12, 1024
+
+
+def solve(cg, orc, s, t, w, tele, c, n=N, vpt=VPT):
+    """(ranks, dL/dw, dL/dt) of the FP32 form and of the oracle, edges in store order."""
+    bits = w.astype(np.float32).view(np.uint32)
+    st = orc.Store(n, vpt, True)
+    st.insert(s, t, bits)
+    st.compact()
+    es, et, wb = orc.store_edges(st)
+    ew = wb.view(np.float32).astype(np.float64)
+    r, _ = orc.wpagerank(n, es, et, ew, t=tele, tol=1e-15)
+    lam, gw, gt, _ = orc.wpagerank_adjoint(n, es, et, ew, r, c, t=tele, tol=1e-15)
+    with cg.Engine(n, vpt, weight_type=cg.WEIGHT_F32) as eng:
+        eng.insert_edges(s, t, bits)
+        eng.do_global_compaction()
+        p = cg.WeightedPageRank(eng, max_iterations=2000, tolerance=1e-12, kahan=True)
+        p.set_teleport(tele)
+        p.execute_algorithm()
+        gw32, gt32, _ = p.adjoint(c)
+        r32 = p.result()
+    return (r32, gw32, gt32), (r, gw, gt), (es, et, ew, lam)
+
+
+@pytest.mark.parametrize("scale,c_scale", [(1e33, 1e3), (1e30, 1.0), (1e-30, 1.0), (1.0, 1e-32), (1.0, 1e30)])
+def test_gradients_of_extreme_weights_and_losses(cg, orc, scale, c_scale):
+    """Sources of one in-edge or none whose teleport mass is small and whose out-weights are scaled:
+    alpha r_u / s_u down to 1e-42, dL/dw still an FP32 normal. Every edge's gradient within 1e-5 of
+    |alpha r_u / s_u| max |lambda| (lambda and P^T lambda are FP32 values converged to a few 1e-7
+    of the largest), ranks within the family's bounds."""
+    rng = np.random.default_rng(8)
+    s, t = rng.integers(64, N, 40000, dtype=np.uint32), rng.integers(64, N, 40000, dtype=np.uint32)
+    w = rng.uniform(0.5, 1.0, len(s))
+    few = np.repeat(np.arange(64, dtype=np.uint32), 3)  # sources nobody points to
+    s, t = np.concatenate([s, few]), np.concatenate([t, rng.integers(64, N, len(few), dtype=np.uint32)])
+    w = np.concatenate([w, rng.uniform(0.5, 1.0, len(few)) * scale])
+    tele = rng.uniform(0.5, 1.5, N)
+    tele[:64] *= 1e-4
+    tele /= tele.sum()
+    c = rng.standard_normal(N) * c_scale
+    (r32, gw32, gt32), (r, gw, gt), (es, et, ew, lam) = solve(cg, orc, s, t, w, tele, c)
+    assert np.abs(r32 - r).sum() <= 1e-6 * r.sum()
+    out = np.bincount(es, ew, N)
+    assert np.isfinite(gw32).all()
+    bound = 0.85 * r[es] / out[es] * np.abs(lam).max() * 1e-5 + 1.5e-45  # and an FP32 denormal's step
+    err = np.abs(gw32.astype(np.float64) - gw)
+    assert (err <= bound).all(), (err / bound).max()
+    assert np.abs(gt32 - gt).max() <= 1e-5 * np.abs(gt).max()
