@@ -195,7 +195,7 @@ struct PrArgs {
   LoopState* ls;
   uint64_t n;
   double alpha, delta_param, base;
-  // alpha, base, 1/n, 1 - alpha and delta_param as float-float (pr_args_ff)
+  // alpha, base, 1/n (exact: n is a power of two), 1 - alpha and delta_param as float-float (pr_args_ff)
   FF alpha_ff, base_ff, inv_n_ff, rest_ff, delta_ff;
 };
 
@@ -381,7 +381,7 @@ __device__ __forceinline__ double pr_apply_w64(const PrArgs& a, uint64_t v, doub
 // (PageRank-delta: the rank changes; adjoint: t . lambda) and the vertices activated for the
 // next round (PageRank-delta). Flushed once per block (pr_tally_flush).
 struct PrTally {
-  double resid, rsum;  // FP64 forms; the FP32 forms' infinities
+  double resid, rsum;  // FP64 forms; of the FP32 forms what is out of a float pair's range
   FF fres, fsum;       // FP32 forms, in float-float
   unsigned nact;
   __device__ __forceinline__ void init() { resid = rsum = 0.0, fres = fsum = FF{0.f, 0.f}, nact = 0u; }
@@ -409,11 +409,23 @@ __device__ __forceinline__ void pr_apply_norm(const PrArgs& a, uint64_t v, pr_ff
   }
 }
 
+// What pr_apply_w32 takes in FP64; calls, so that the common path keeps its registers.
+// (lambda'_v, (P^T lambda)_v) of the adjoint:
+__device__ __forceinline__ float2 pr_adj_fp64(double s, FF sum, FF dang, float2 c, double alpha) {
+  const double ptd = s > 0.0 ? ((double)sum.hi + (double)sum.lo) / s : 0.0;
+  const double cd = isfinite(c.x) ? (double)c.x + (double)c.y : (double)c.x;
+  return make_float2((float)(cd + alpha * (ptd + (s > 0.0 ? 0.0 : (double)dang.hi + (double)dang.lo))), (float)ptd);
+}
+// r'_v of the forward form:
+__device__ __forceinline__ FF pr_w32_fp64(double tv, FF sum, FF dang, double alpha) {
+  return ff_from_double(tv * ((double)dang.hi + (double)dang.lo) + alpha * ((double)sum.hi + (double)sum.lo));
+}
+
 // The FP32 weighted forms' update of v in float-float.
 // PR_W32: r'_v = t_v ((1-alpha) + alpha D) + alpha sum (dang holds the bracket), kept as a
 // float pair. PR_ADJ32 (v is a source): lambda'_v = c_v + alpha ((P^T lambda)_v + a_v (t . lambda)),
-// kept as a float; its share of the next round's t . lambda joins the tally. Float pairs
-// turn an infinity into NaN, so a result that is not finite is taken in FP64 instead.
+// kept as a float; its share of the next round's t . lambda joins the tally. A result out of
+// the pairs' range (ff_in_range; they also turn an infinity into NaN) is taken in FP64 instead.
 template <int MODE, int PERSIST>
 __device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum, unsigned p, FF dang, PrTally& t) {
   FF tv = a.inv_n_ff;
@@ -427,11 +439,7 @@ __device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum
     float* rn = (p == 0) ? a.comp : a.rank;
     float* rnl = (p == 0) ? a.lo1 : a.lo0;
     FF nv = ff_add(ff_mul(tv, dang), ff_mul(a.alpha_ff, sum));
-    if (!isfinite(nv.hi)) {
-      const double d = (a.tele ? a.tele[v] : 1.0 / (double)a.n) * ((double)dang.hi + (double)dang.lo) +
-                       a.alpha * ((double)sum.hi + (double)sum.lo);
-      nv = ff_from_double(d);
-    }
+    if (!ff_in_range(nv.hi)) nv = pr_w32_fp64(a.tele ? a.tele[v] : (double)a.inv_n_ff.hi, sum, dang, a.alpha);
     rn[v] = nv.hi;
     rnl[v] = nv.lo;
     change = ff_add(nv, FF{-o.hi, -o.lo});
@@ -442,19 +450,19 @@ __device__ __forceinline__ void pr_apply_w32(const PrArgs& a, uint64_t v, FF sum
     FF ptv{0.f, 0.f}, add = dang;
     if (s.x > 0.f) ptv = add = ff_div(sum, FF{s.x, s.y});
     float nl = ff_add(FF{c.x, c.y}, ff_mul(a.alpha_ff, add)).hi, pv = ptv.hi;
-    if (!isfinite(nl) || !isfinite(pv)) {
-      const double sv = a.wsum[v];
-      const double ptd = sv > 0.0 ? ((double)sum.hi + (double)sum.lo) / sv : 0.0;
-      const double cd = isfinite(c.x) ? (double)c.x + (double)c.y : (double)c.x;
-      pv = (float)ptd;
-      nl = (float)(cd + a.alpha * (ptd + (sv > 0.0 ? 0.0 : (double)dang.hi + (double)dang.lo)));
+    const FF td = ff_mul(tv, FF{nl, 0.f});
+    const bool in = (ff_in_range(nl) && ff_in_range(td.hi)) || (nl == 0.f && add.hi == 0.f && c.x == 0.f);
+    if (in && (sum.hi == 0.f || (ff_in_range(sum.hi) && ff_in_range(pv)))) {
+      t.fsum = ff_add(t.fsum, td);
+    } else {
+      const float2 q = pr_adj_fp64(a.wsum[v], sum, dang, c, a.alpha);
+      nl = q.x;
+      pv = q.y;
+      t.rsum += (a.tele ? a.tele[v] : (double)a.inv_n_ff.hi) * (double)nl;
     }
     ((p == 0) ? a.comp : a.rank)[v] = nl;
     a.pt[v] = pv;
     change = isfinite(nl - old) ? ff_two_sum(nl, -old) : FF{nl - old, 0.f};
-    const FF td = ff_mul(tv, FF{nl, 0.f});
-    if (isfinite(td.hi)) t.fsum = ff_add(t.fsum, td);
-    else t.rsum += (double)(tv.hi * nl);
   }
   if (isfinite(change.hi)) t.fres = ff_add(t.fres, ff_abs(change));
   else t.resid += (double)fabsf(change.hi);
@@ -521,7 +529,7 @@ __device__ __forceinline__ void pr_tally_flush(LoopState* ls, unsigned p, PrTall
       if (kS)
         t.fsum = ff_add(t.fsum, FF{__shfl_xor_sync(0xFFFFFFFFu, t.fsum.hi, o), __shfl_xor_sync(0xFFFFFFFFu, t.fsum.lo, o)});
     }
-    if ((MODE == PR_W32 || MODE == PR_ADJ32) && __any_sync(0xFFFFFFFFu, t.resid != 0.0 || t.rsum != 0.0)) {  // infinities, NaN
+    if ((MODE == PR_W32 || MODE == PR_ADJ32) && __any_sync(0xFFFFFFFFu, t.resid != 0.0 || t.rsum != 0.0)) {  // out of range
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         t.resid += __shfl_xor_sync(0xFFFFFFFFu, t.resid, o);
@@ -757,7 +765,7 @@ __device__ __forceinline__ unsigned pr_control_step(LoopState* ls, int mode) {
   } else {
     more = more && resid > tol;
     // FP32 ranks cannot change by less than their rounding floor (about 6e-8 of the rank
-    // mass per round); once the FP64-measured change stops shrinking, the run is done
+    // mass per round); once the change, measured to 44 bits and more, stops shrinking, the run is done
     if (mode == PR_NORM32 || mode == PR_W32 || mode == PR_ADJ32) {
       if (resid < best * 0.999) {
         ls->best_resid = resid;

@@ -54,3 +54,36 @@ def test_gradients_of_extreme_weights_and_losses(cg, orc, scale, c_scale):
     err = np.abs(gw32.astype(np.float64) - gw)
     assert (err <= bound).all(), (err / bound).max()
     assert np.abs(gt32 - gt).max() <= 1e-5 * np.abs(gt).max()
+
+
+@pytest.mark.parametrize("c_scale,sparse", [(1e-37, False), (1e-33, False), (1e-33, True), (1.0, True), (1e30, False)])
+def test_adjoint_of_small_losses(cg, orc, c_scale, sparse):
+    """t . lambda of many small terms: 2^16 vertices, every second one dangling, loss weights equal
+    (the terms' roundings then do not cancel) or on 16 vertices only. dL/dt is proportional to
+    lambda: within 1e-6 of each entry (lambda is stored in FP32, 2^-24 a round, amplified by at
+    most 1 / (1 - alpha) = 6.7: 4e-7) and an FP32 denormal's step."""
+    n = 1 << 16
+    rng = np.random.default_rng(4)
+    s, t = rng.integers(0, n // 2, 1 << 18, dtype=np.uint32), rng.integers(0, n, 1 << 18, dtype=np.uint32)
+    w = rng.uniform(0.5, 1.0, len(s))
+    c = np.full(n, c_scale)
+    if sparse:
+        c[rng.permutation(n)[16:]] = 0.0
+    (r32, _, gt32), (r, _, gt), _ = solve(cg, orc, s, t, w, None, c, n=n, vpt=n)
+    err = np.abs(gt32.astype(np.float64) - gt)
+    bound = 1e-6 * np.abs(gt) + 1.5e-45
+    assert (err <= bound).all(), (err / bound).max()
+
+
+@pytest.mark.parametrize("low,high", [(1e-36, 1e-30), (1e-42, 1.0)])
+def test_ranks_of_extreme_teleports(cg, orc, low, high):
+    """Teleport vectors of small size and of wide span: ranks within 1e-5 relative of the oracle where an
+    FP32 normal holds them, within 1e-6 relative L1."""
+    rng = np.random.default_rng(6)
+    s, t = rng.integers(0, N // 2, 30000, dtype=np.uint32), rng.integers(0, N // 2, 30000, dtype=np.uint32)
+    w = rng.uniform(0.5, 1.0, len(s))
+    tele = np.exp(rng.uniform(np.log(low), np.log(high), N))
+    (r32, _, _), (r, _, _), _ = solve(cg, orc, s, t, w, tele, rng.standard_normal(N))
+    ok = r > 1e-35  # contributions r / s and their products are FP32 too
+    assert (np.abs(r32 - r)[ok] <= 1e-5 * r[ok]).all()
+    assert np.abs(r32 - r).sum() <= 1e-6 * r.sum()
