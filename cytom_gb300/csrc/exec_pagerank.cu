@@ -309,6 +309,15 @@ static PrBinLaunch bin_launch(Ctx* c, const uint64_t* nb);
 
 static int csc_settle(Ctx* c, Csc& q);
 
+// Allocates *p, or leaves it NULL.
+template <class T>
+static bool csx_alloc(T** p, size_t bytes) {
+  if (cy_malloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
 static int build_csx_stage(Ctx* c, Csc& q, int by_source, float** w, uint64_t* wcap) {
   int prc = pr_ensure_perm(c);
   if (prc) return prc;
@@ -318,19 +327,20 @@ static int build_csx_stage(Ctx* c, Csc& q, int by_source, float** w, uint64_t* w
   if (E > 0xFFFFFFFFULL - (1ULL << 20)) return set_err(c, CYTOM_ERR_RANGE, "PageRank CSC holds fewer than 2^32 - 2^20 edges");
   if (E > q.cap || !q.src) {
     cudaFree(q.src);
+    q.src = nullptr;
     q.cap = std::max<uint64_t>(E + E / 4, 1024);
-    if (cy_malloc(&q.src, q.cap * 4) != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "CSC");
+    if (!csx_alloc(&q.src, q.cap * 4)) return set_err(c, CYTOM_ERR_OOM, "CSC");
   }
   if (w && (E > *wcap || !*w)) {
     cudaFree(*w);
+    *w = nullptr;
     *wcap = std::max<uint64_t>(E + E / 4, 1024);
-    if (cy_malloc(w, *wcap * 4) != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "CSC weights");
+    if (!csx_alloc(w, *wcap * 4)) return set_err(c, CYTOM_ERR_OOM, "CSC weights");
   }
-  if (!q.ptr) {
-    if (cy_malloc(&q.ptr, (n + 1) * 4) != cudaSuccess || cy_malloc(&q.deg_out, n * 4) != cudaSuccess ||
-        cy_malloc(&q.bins, n * 4) != cudaSuccess)
-      return set_err(c, CYTOM_ERR_OOM, "CSC index");
-  }
+  // each by itself: a build that found room for some of them is repeated later
+  if ((!q.ptr && !csx_alloc(&q.ptr, (n + 1) * 4)) || (!q.deg_out && !csx_alloc(&q.deg_out, n * 4)) ||
+      (!q.bins && !csx_alloc(&q.bins, n * 4)))
+    return set_err(c, CYTOM_ERR_OOM, "CSC index");
   if ((!q.htot && cy_malloc_host(&q.htot, 64) != cudaSuccess) ||
       (!q.dbl && cy_malloc(&q.dbl, sizeof(PrBinLaunch)) != cudaSuccess))
     return set_err(c, CYTOM_ERR_OOM, "CSC bins");
@@ -357,7 +367,10 @@ static int build_csx_stage(Ctx* c, Csc& q, int by_source, float** w, uint64_t* w
     c->launches++;
     bool alt = false;
     rc = radix_sort_pairs(c, k0, k1, v0, v1, E, (int)(2 * lg_n), &alt);
-    if (rc) return rc;
+    if (rc) {
+      cudaFreeAsync(tmp, c->stream);
+      return rc;
+    }
     csc_src_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(alt ? k1 : k0, E, lg_n, q.src, seg_lo, seg_hi);
     c->launches++;
     if (w) cudaMemcpyAsync(*w, alt ? v1 : v0, E * 4, cudaMemcpyDeviceToDevice, c->stream);
@@ -367,10 +380,12 @@ static int build_csx_stage(Ctx* c, Csc& q, int by_source, float** w, uint64_t* w
   csc_cnt_bins_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(seg_lo, seg_hi, n, cnt, k0, seg_lo, tot, pr_warp_bin_hi(E));
   c->launches++;
   rc = exclusive_scan_u32(c, cnt, q.ptr, n, q.ptr + n);
-  if (rc) return rc;
   bool balt = false;
-  rc = radix_sort_pairs(c, k0, k1, seg_lo, q.bins, n, 3, &balt);
-  if (rc) return rc;
+  if (!rc) rc = radix_sort_pairs(c, k0, k1, seg_lo, q.bins, n, 3, &balt);
+  if (rc) {
+    cudaFreeAsync(tmp, c->stream);
+    return rc;
+  }
   if (!balt) cudaMemcpyAsync(q.bins, seg_lo, nbytes, cudaMemcpyDeviceToDevice, c->stream);
   cudaMemcpyAsync(q.htot, tot, kPrBins * 4, cudaMemcpyDeviceToHost, c->stream);
   cudaFreeAsync(tmp, c->stream);
@@ -524,7 +539,8 @@ static int update_csc_stage(Ctx* c, Csc& q) {
     rc = merge_csc_stage(c, q);
   else
     rc = build_csc_stage(c, q);
-  if (!rc) q.built_version = c->version;
+  // a merge that failed half way may have counted degrees already: built anew next time
+  q.built_version = rc ? ~0ULL : c->version;
   return rc;
 }
 
@@ -596,16 +612,24 @@ static int pr_ensure_perm(Ctx* c) {
     if (perm) cudaFree(perm);
     return set_err(c, CYTOM_ERR_OOM, "vertex renumbering");
   }
-  c->pr_perm = perm;
-  c->pr_inv = inv;
   perm_keys_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(c->out_deg, n, lg_n, k);
   bool alt = false;
   int rc = radix_sort_pairs(c, k, k + n, nullptr, nullptr, n, (int)(32 + lg_n), &alt);
-  if (rc) return rc;
-  perm_from_keys_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(alt ? k + n : k, n, lg_n, c->pr_perm, c->pr_inv);
+  if (!rc) {
+    perm_from_keys_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(alt ? k + n : k, n, lg_n, perm, inv);
+    rc = cuda_err(c, cudaGetLastError(), "vertex renumbering");
+  }
   c->launches += 2;
   cudaFreeAsync(k, c->stream);
-  return cuda_err(c, cudaGetLastError(), "vertex renumbering");
+  if (rc) {  // never left half made: later calls take it as it is
+    cudaStreamSynchronize(c->stream);
+    cudaFree(perm);
+    cudaFree(inv);
+    return rc;
+  }
+  c->pr_perm = perm;
+  c->pr_inv = inv;
+  return CYTOM_OK;
 }
 
 // Multiplicity out-degrees in the renumbering (PageRank-delta), per graph version.
@@ -1298,6 +1322,8 @@ int pagerank_batch_prep(Ctx* c, Job* j, PrArgs* out, uint64_t* nb, int* first_mo
 // Copies a renumbered vertex vector out in vertex order (host or device destination).
 template <typename T>
 static int unpermute_out(Ctx* c, const T* src, void* out, int where, const char* what) {
+  int rc = pr_ensure_perm(c);  // the job may never have run
+  if (rc) return rc;
   const uint64_t n = c->n;
   T* dst = (T*)out;
   T* tmp = nullptr;
