@@ -85,7 +85,7 @@ struct PrState {
   uint64_t seen_version = ~0ULL;
   // WPAGERANK
   double* tele = nullptr;     // teleport vector (NULL = uniform 1/n)
-  float2* tele2 = nullptr;    // the same as float pairs (FP32 form)
+  float2* tele2 = nullptr;    // the same as float pairs (FP32 form; from the pool, float_pairs)
   // WPAGERANK adjoint (allocated by the first adjoint call)
   float* lam = nullptr;       // FP32: lambda, double-buffered (2 x n)
   double* lam64 = nullptr;    // FP64: lambda, double-buffered (2 x n)
@@ -109,8 +109,9 @@ struct WGraph {
   float* out_w = nullptr;
   uint64_t in_wcap = 0, out_wcap = 0;
   double* wsum = nullptr;
-  float2* wsum2 = nullptr;  // the same as float pairs (FP32 forms)
+  float2* wsum2 = nullptr;  // the same as float pairs (FP32 forms; from the pool, float_pairs)
   uint64_t built_version = ~0ULL;
+  uint64_t pairs_version = ~0ULL;  // of wsum2
 };
 
 // --------------------------------------------------------------------------
@@ -1398,7 +1399,7 @@ int pagerank_result64(Ctx* c, Job* j, double* out, int where) {
 
 // s_u = sum of u's out-weights, one warp per source in CSR order (deterministic).
 __global__ void wsum_kernel(const uint32_t* __restrict__ ptr, const float* __restrict__ w, uint64_t n,
-                            double* __restrict__ wsum, float2* __restrict__ wsum2) {
+                            double* __restrict__ wsum) {
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -1407,12 +1408,30 @@ __global__ void wsum_kernel(const uint32_t* __restrict__ ptr, const float* __res
     for (uint32_t e = ptr[u] + lane; e < ptr[u + 1]; e += 32) s += (double)w[e];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) {
-      wsum[u] = s;
-      const FF f = ff_from_double(s);
-      wsum2[u] = make_float2(f.hi, f.lo);
-    }
+    if (lane == 0) wsum[u] = s;
   }
+}
+
+__global__ void float_pairs_kernel(const double* __restrict__ in, uint64_t n, float2* __restrict__ out) {
+  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+    const FF f = ff_from_double(in[v]);
+    out[v] = make_float2(f.hi, f.lo);
+  }
+}
+
+// The FP32 forms' copy of a vertex vector as float pairs, allocated on first use. It comes from the
+// stream-ordered pool and after the graph was built, whose temporaries (28 bytes a vertex and
+// more) the pool has just got back: it takes no memory that a run without it would leave free.
+static int float_pairs(Ctx* c, const double* in, float2** out) {
+  if (!*out && cy_malloc_async((void**)out, c->n * 8, c->stream) != cudaSuccess) {
+    cudaGetLastError();
+    *out = nullptr;
+    return set_err(c, CYTOM_ERR_OOM, "float pairs");
+  }
+  float_pairs_kernel<<<grid_n(c, c->n), 256, 0, c->stream>>>(in, c->n, *out);
+  c->launches++;
+  return cuda_err(c, cudaGetLastError(), "float pairs");
 }
 
 static int build_wgraph(Ctx* c, WGraph& g) {
@@ -1420,10 +1439,8 @@ static int build_wgraph(Ctx* c, WGraph& g) {
   int rc = build_csx(c, g.in, 0, &g.in_w, &g.in_wcap);
   if (!rc) rc = build_csx(c, g.out, 1, &g.out_w, &g.out_wcap);
   if (rc) return rc;
-  if ((!g.wsum && cy_malloc(&g.wsum, c->n * 8) != cudaSuccess) ||
-      (!g.wsum2 && cy_malloc(&g.wsum2, c->n * 8) != cudaSuccess))
-    return set_err(c, CYTOM_ERR_OOM, "weight sums");
-  wsum_kernel<<<grid_n(c, c->n * 32), 256, 0, c->stream>>>(g.out.ptr, g.out_w, c->n, g.wsum, g.wsum2);
+  if (!g.wsum && !csx_alloc(&g.wsum, c->n * 8)) return set_err(c, CYTOM_ERR_OOM, "weight sums");
+  wsum_kernel<<<grid_n(c, c->n * 32), 256, 0, c->stream>>>(g.out.ptr, g.out_w, c->n, g.wsum);
   c->launches++;
   g.built_version = c->version;
   return cuda_err(c, cudaGetLastError(), "weight sums");
@@ -1456,9 +1473,15 @@ static PrArgs wargs(Ctx* c, Job* j, const WGraph& g) {
 }
 
 static int wpagerank_run(Ctx* c, Job* j) {
+  PrState* s = prs(j);
   WGraph* g = ctx_wgraph(c);
   if (!g) return set_err(c, CYTOM_ERR_OOM, "weighted graph");
   int rc = build_wgraph(c, *g);
+  if (!rc && j->params.kahan) {
+    if (!g->wsum2 || g->pairs_version != c->version) rc = float_pairs(c, g->wsum, &g->wsum2);
+    if (!rc) g->pairs_version = c->version;
+    if (!rc && s->tele && !s->tele2) rc = float_pairs(c, s->tele, &s->tele2);
+  }
   if (rc) return rc;
   PrArgs a = wargs(c, j, *g);
   unsigned max_iter = (unsigned)std::min<uint64_t>(j->params.max_iterations, 0xFFFFFFFFu);
@@ -1484,27 +1507,22 @@ int pagerank_set_teleport(Ctx* c, Job* j, const double* t, int where) {
   }
   int prc = pr_ensure_perm(c);
   if (prc) return prc;
-  if (!s->tele) {
-    float2* t2 = nullptr;
-    double* t1 = nullptr;
-    if (cy_malloc(&t1, c->n * 8) != cudaSuccess || cy_malloc(&t2, c->n * 8) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(t1);
-      return set_err(c, CYTOM_ERR_OOM, "teleport");
-    }
-    s->tele = t1;
-    s->tele2 = t2;
-  }
   // kept in the renumbering
   double* tmp = nullptr;
-  if (cy_malloc_async((void**)&tmp, c->n * 8, c->stream) != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "teleport");
+  if (cy_malloc_async((void**)&tmp, c->n * 8, c->stream) != cudaSuccess ||
+      (!s->tele && !csx_alloc(&s->tele, c->n * 8))) {
+    cudaGetLastError();
+    if (tmp) cudaFreeAsync(tmp, c->stream);
+    return set_err(c, CYTOM_ERR_OOM, "teleport");
+  }
   cudaError_t e = cudaMemcpyAsync(tmp, t, c->n * 8,
                                   where == CYTOM_PTR_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                   c->stream);
   permute_kernel<double><<<grid_n(c, c->n), 256, 0, c->stream>>>(tmp, c->pr_perm, c->n, 1, s->tele);
-  permute_ff_kernel<<<grid_n(c, c->n), 256, 0, c->stream>>>(tmp, c->pr_perm, c->n, s->tele2);
-  c->launches += 2;
+  c->launches++;
+  if (s->tele2) prc = float_pairs(c, s->tele, &s->tele2);
   cudaFreeAsync(tmp, c->stream);
+  if (prc) return prc;
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   return cuda_err(c, e, "teleport upload");
 }
@@ -1601,10 +1619,12 @@ __global__ void grad_w32_kernel(const StoreDesc* __restrict__ sd, const float4* 
   }
 }
 
-// The FP64 form: every factor and the result's last rounding in FP64.
+// The FP64 form, and the FP32 form without memory for the vertices' factors: every factor and the
+// result's last rounding in FP64.
+template <typename T>
 __global__ void grad_w64_kernel(const StoreDesc* __restrict__ sd, const uint32_t* __restrict__ perm,
-                                const double* __restrict__ r, const double* __restrict__ lam,
-                                const double* __restrict__ pt, const double* __restrict__ wsum, double alpha,
+                                const T* __restrict__ r, const T* __restrict__ lam,
+                                const T* __restrict__ pt, const double* __restrict__ wsum, double alpha,
                                 float* __restrict__ gw) {
   const uint64_t E = sd->E;
   const uint32_t lT = sd->lT, lvpt = sd->lvpt;
@@ -1616,7 +1636,7 @@ __global__ void grad_w64_kernel(const StoreDesc* __restrict__ sd, const uint32_t
     const uint32_t p = sd->edges[e];
     const uint32_t u = perm[((t >> lT) << lvpt) | (p >> 16)];
     const uint32_t k = perm[((t & ymask) << lvpt) | (p & 0xFFFFu)];
-    gw[e] = (float)(alpha * r[u] / wsum[u] * (lam[k] - pt[u]));
+    gw[e] = (float)(alpha * (double)r[u] / wsum[u] * ((double)lam[k] - (double)pt[u]));
   }
 }
 
@@ -1657,6 +1677,10 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, CYTOM_ERR_OOM, "adjoint state");
+  }
+  if (f32 && s->tele && !s->tele2) {
+    int rc = float_pairs(c, s->tele, &s->tele2);
+    if (rc) return rc;
   }
   // the forward's newest ranks
   LoopState fls;
@@ -1722,8 +1746,13 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   char* tmp = nullptr;
   auto align256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t wbytes = align256(std::max<uint64_t>(E, 1) * 4), tbytes = align256(n * 4);
-  const size_t gbytes = f32 ? align256(n * 16) : 0;
-  if (cy_malloc_async((void**)&tmp, 256 + wbytes + tbytes + gbytes + (f32 ? n * 4 : 0), c->stream) != cudaSuccess)
+  const size_t gbytes = align256(n * 16);
+  bool factors = f32;
+  if (f32 && cy_malloc_async((void**)&tmp, 256 + wbytes + tbytes + gbytes + n * 4, c->stream) != cudaSuccess) {
+    cudaGetLastError();
+    factors = false;
+  }
+  if (!factors && cy_malloc_async((void**)&tmp, 256 + wbytes + tbytes, c->stream) != cudaSuccess)
     return set_err(c, CYTOM_ERR_OOM, "adjoint outputs");
   double* dang = (double*)tmp;
   float* gw = (owhere == CYTOM_PTR_DEVICE && d_w) ? d_w : (float*)(tmp + 256);
@@ -1732,18 +1761,22 @@ int pagerank_adjoint(Ctx* c, Job* j, const double* cv, int cwhere, float* d_w, f
   if (f32) {
     const float* lam = (pa == 0) ? s->lam : s->lam + n;
     dangling_sum_kernel<float><<<grid_n(c, n), 256, 0, c->stream>>>(r32, g->wsum, n, dang);
-    float4* gv = (float4*)(tmp + 256 + wbytes + tbytes);
-    float* lamv = (float*)(tmp + 256 + wbytes + tbytes + gbytes);
-    grad_prep_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(c->pr_perm, r32, lam, s->pt, g->wsum, n, a.alpha, gv, lamv);
-    c->launches++;
-    if (E)
-      grad_w32_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, gv, lamv, c->pr_perm, r32, g->wsum, a.alpha, gw);
+    if (factors) {
+      float4* gv = (float4*)(tmp + 256 + wbytes + tbytes);
+      float* lamv = (float*)(tmp + 256 + wbytes + tbytes + gbytes);
+      grad_prep_kernel<<<grid_n(c, n), 256, 0, c->stream>>>(c->pr_perm, r32, lam, s->pt, g->wsum, n, a.alpha, gv, lamv);
+      c->launches++;
+      if (E)
+        grad_w32_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, gv, lamv, c->pr_perm, r32, g->wsum, a.alpha, gw);
+    } else if (E) {
+      grad_w64_kernel<float><<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, c->pr_perm, r32, lam, s->pt, g->wsum, a.alpha, gw);
+    }
     grad_t_kernel<float><<<grid_n(c, n), 256, 0, c->stream>>>(lam, c->pr_perm, n, dang, a.alpha, gt);
   } else {
     const double* lam = (pa == 0) ? s->lam64 : s->lam64 + n;
     dangling_sum_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(r64, g->wsum, n, dang);
     if (E)
-      grad_w64_kernel<<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, c->pr_perm, r64, lam, s->pt64, g->wsum, a.alpha, gw);
+      grad_w64_kernel<double><<<grid_n(c, E), 256, 0, c->stream>>>(c->dsd, c->pr_perm, r64, lam, s->pt64, g->wsum, a.alpha, gw);
     grad_t_kernel<double><<<grid_n(c, n), 256, 0, c->stream>>>(lam, c->pr_perm, n, dang, a.alpha, gt);
   }
   c->launches += 3;
