@@ -228,9 +228,15 @@ __device__ __forceinline__ uint64_t make_key(uint32_t s, uint32_t t, uint32_t lv
 // end. Atomics on one sector go one after another, and in graphs numbered by degree or by a
 // generator the first take several per cent of the endpoints (12.5 M RMAT-22 edges 366 us
 // without, 326 with one such vertex, 253 with 64 or 512, 255 with 2,048, 236 with 4,096, which
-// leaves fewer blocks per SM).
+// leaves fewer blocks per SM). Where ids say nothing about degrees it costs the clearing and the
+// adding up. With / without, in us, on 4 M vertices:
+//   edges   RMAT ids       RMAT, ids shuffled   uniform
+//   2^17    8.4 / 9.4      8.0 / 7.3            8.4 / 7.1
+//   2^18    11.0 / 14.4    10.7 / 9.8           9.5 / 8.7
+//   2^20    24.4 / 31.3    20.7 / 20.6          17.2 / 16.2
+//   2^24    298 / 378      212 / 212            198 / 195
 constexpr uint32_t APPEND_HUBS = 2048;
-constexpr uint64_t kAppendHubsMin = 1ULL << 17;  // edges; below, a block's share is too small to pay the adding up
+constexpr uint64_t kAppendHubsMin = 1ULL << 18;  // edges: from here on the gain is three times the cost
 
 template <bool HUBS>
 __global__ void append_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ tgt,
