@@ -558,10 +558,12 @@ template <int IPT, bool VALS, class ST>
 static void onesweep_launch(Ctx* c, unsigned tiles, const uint64_t* kin, const uint32_t* vin, uint64_t n, int shift,
                             uint32_t mask, const uint32_t* doff, uint32_t* ticket, void* st, void* st_next,
                             uint64_t* kout, uint32_t* vout) {
+  const uint32_t polls = c->inj_idle_limit ? c->inj_idle_limit : OS_POLLS;
   auto fn = radix_onesweep_kernel<IPT, VALS, ST>;
   if (os_smem<IPT>() > 40 * 1024)  // with the static part past the 48 KB default
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)os_smem<IPT>());
-  fn<<<tiles, OS_T, os_smem<IPT>(), c->stream>>>(kin, vin, n, shift, mask, doff, ticket, (ST*)st, (ST*)st_next, kout, vout);
+  fn<<<tiles, OS_T, os_smem<IPT>(), c->stream>>>(kin, vin, n, shift, mask, doff, ticket, (ST*)st, (ST*)st_next, kout,
+                                             vout, polls);
 }
 
 template <int IPT, bool VALS>

@@ -109,7 +109,8 @@ __global__ void radix_downsweep_kernel(const uint64_t* __restrict__ keys, const 
 // before it (decoupled look-back, OS_LB status rows in flight per step) and writes the
 // tile's runs coalesced. Tiles are taken in order from a ticket, so a tile only ever looks
 // at tiles whose blocks are already running. A status row that stays empty for OS_POLLS
-// polls is not waited for any longer: the thread counts that tile's keys itself.
+// polls (fewer where a test says so) is not waited for any longer: the thread counts that
+// tile's keys itself.
 // Bound by instruction issue (the ballots of the ranking: issue slots 47 %, ALU pipe 60 %)
 // and its latency, DRAM 28 %. 12.5 M 44-bit keys with weights: 1,368 us (six passes of
 // count, three scan kernels, scatter) -> 629 us; without weights 511 us; 1 M with weights
@@ -223,7 +224,7 @@ template <int IPT, bool VALS, class ST>
 __global__ void __launch_bounds__(OS_T, 2) radix_onesweep_kernel(
     const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n, int shift, uint32_t mask,
     const uint32_t* __restrict__ doff, uint32_t* __restrict__ ticket, ST* status, ST* __restrict__ status_next,
-    uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
+    uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t max_polls) {
   extern __shared__ __align__(16) uint8_t os_raw[];
   __shared__ uint32_t s_tile, s_wsum[OS_WARPS];
   __shared__ uint32_t s_off[OS_BINS];  // digit's first place in the tile, then output place - tile place
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(OS_T, 2) radix_onesweep_kernel(
         const int f = (int)(w[b] >> (sizeof(ST) * 8 - 2));
         if (f == 0) {
           // not published yet: read again from here (and, past the limit, count it here)
-          if (++polls > OS_POLLS && t >= 0) {
+          if (++polls > max_polls && t >= 0) {
             const uint64_t tb = (uint64_t)t * TILE;
             for (uint32_t i = 0; i < TILE; ++i)
               before += ((uint32_t)(keys[tb + i] >> shift) & mask) == threadIdx.x ? 1 : 0;

@@ -329,7 +329,7 @@ class Engine:
     def set_fault_injection(self, fail_alloc_after: int = 0, idle_poll_limit: int = 0, phantom_jobs: int = 0):
         """Test hook (cytom_set_fault_injection): the fail_alloc_after-th allocation from now
         on fails once; the batched executor's idle wait gives up after idle_poll_limit
-        empty polls; phantom_jobs unfinished jobs without work keep its blocks waiting."""
+        empty polls, and this engine's sorts stop waiting for a tile's counts; phantom_jobs unfinished jobs without work keep its blocks waiting."""
         f = L.FaultInjection(fail_alloc_after, idle_poll_limit, phantom_jobs)
         self._check(self.lib.cytom_set_fault_injection(self.ctx, C.byref(f)))
 

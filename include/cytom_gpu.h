@@ -412,7 +412,8 @@ int cytom_get_tune_report(const cytom_ctx* ctx, cytom_tune_report* out);
  *    CYTOM_ERR_OOM; 0 turns it off.
  *  - idle_poll_limit: empty polls of the batched executor's bounded idle wait before a
  *    block gives up (CYTOM_ERR_TIMEOUT), for batches whose first context is ctx;
- *    0 = the default, 2^22.
+ *    0 = the default, 2^22. Also the polls after which a sort of ctx counts a tile itself
+ *    in place of waiting for its counts (the result is the same); default 2^18.
  *  - phantom_jobs: the batched executor counts this many further unfinished jobs that
  *    have no work, so its blocks find none until the idle wait gives up.
  * After a batched run that gave up, its jobs restart from scratch on their next run. */
