@@ -19,15 +19,17 @@
 // (radix sort of (tgt, src) keys): each target's in-edges are contiguous, so its sum is
 // accumulated in a fixed order with Neumaier compensation -- deterministic and
 // compensated, no float atomics. Targets are binned by in-degree: one thread (<= 4
-// in-edges), 4 lanes (<= 32), 8 lanes (<= 256), a warp (<= 4096) or a block (more) per
-// target, all bins in one launch. Residuals, dangling mass and rank sums are FP64
-// reductions.
+// in-edges), 4 lanes (<= 32), 8 lanes (<= 256), a warp (<= 512 to 4096, by the edges of the
+// graph: pr_warp_bin_hi) or a block (more) per target, all bins in one launch. Residuals,
+// dangling mass and rank sums are added in FP64 across warps, within a warp as float pairs in
+// the FP32 forms (pagerank_dev.cuh).
 //
 // A round of PageRank-delta is that one launch: each finished target also writes its
 // contribution to the next round (contributions by round parity), and the last block to
 // finish runs the control step and, in a captured loop, sets the loop condition. Only the
-// run's residual round has a contribution pass before the pull. The other forms run
-// contributions -> pull -> control.
+// run's residual round has a contribution pass before the pull. The adjoint of the weighted
+// form gathers lambda itself (pull -> control); the other forms run contributions -> pull ->
+// control.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -1097,7 +1099,7 @@ static cudaError_t pr_add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cud
 // rounds 18.1 / 16.0 / 15.6 / 15.5 ms; RMAT-20 adjoint with 1 / 2 / 4 / 8 13.6 / 13.3 / 13.4 /
 // 13.1, RMAT-22 FP64 11.9 / 11.8 / 12.0 / 11.7. (The five kernels of a BFS / CC / SSSP round
 // gain nothing by it.)
-constexpr int kPrBody = 8, kPrBodyFused = 8;
+constexpr int kPrBody = 8;
 template <int MODE>
 static int build_round_graph(Ctx* c, const PrArgs& base, const Csc& q, cudaGraphExec_t* out) {
   constexpr bool F = pr_fused<MODE>();
@@ -1131,7 +1133,7 @@ static int build_round_graph(Ctx* c, const PrArgs& base, const Csc& q, cudaGraph
     void* a_p0[] = {(void*)&a, (void*)&blp, (void*)&h, (void*)&zero};
     void* a_ctl[] = {(void*)&ls, (void*)&mode, (void*)&h, (void*)&one};
     const bool con = pr_opens_with_contrib<MODE>();
-    for (int k = 0; k < (F ? kPrBodyFused : kPrBody) && e == cudaSuccess; ++k) {
+    for (int k = 0; k < kPrBody && e == cudaSuccess; ++k) {
       if (F) {
         const cudaGraphNode_t before = k ? n_p : nullptr;
         e = pr_add_kernel(body, &n_p, k ? &before : nullptr, k ? 1 : 0, (void*)pr_pull_kernel<MODE>, pg, dim3(PR_T), a_p);

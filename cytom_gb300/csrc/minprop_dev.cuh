@@ -70,7 +70,6 @@ __device__ __forceinline__ uint32_t mp_cand(uint32_t c, uint32_t w) {
 // would do: next only decreases during a round and never exceeds current. Reading the
 // one-job kernels' pre-checks through L1 instead measured 2-3 % slower on the RMAT-22
 // stream's dense SSSP rounds.)
-template <int PERSIST>
 __device__ __forceinline__ uint32_t ld_next(const uint32_t* p) {
   return __ldcg(p);
 }
@@ -504,7 +503,7 @@ __device__ __forceinline__ void dense_stage(const JobDesc* __restrict__ jd, cons
       if (cand[idx] != kInf) cand[idx] = mp_cand<ALGO>(cand[idx], ww[idx]);
     uint32_t nv[EPT];
 #pragma unroll
-    for (int idx = 0; idx < EPT; ++idx) nv[idx] = (cand[idx] != kInf) ? ld_next<PERSIST>(next + vv[idx]) : 0u;
+    for (int idx = 0; idx < EPT; ++idx) nv[idx] = (cand[idx] != kInf) ? ld_next(next + vv[idx]) : 0u;
 #pragma unroll
     for (int idx = 0; idx < EPT; ++idx)
       if (cand[idx] != kInf && cand[idx] < nv[idx]) atomicMin(next + vv[idx], cand[idx]);
@@ -615,14 +614,14 @@ __device__ __forceinline__ void sp_batch(const JobDesc* __restrict__ jd, const S
     const bool act = ((valid >> k) & 1u) && ((bits[k] >> (sl & 31)) & 1u);
     cand[k] = act ? ld_src<PERSIST>(jd, async, ((xy[k] >> 16) << lvpt) | sl) : kInf;
     wv[k] = (mp_weighted<ALGO>() && act) ? sd->wts[pos[k]] : 0u;
-    if (LAT) nv[k] = act ? ld_next<PERSIST>(jd->next + (((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
+    if (LAT) nv[k] = act ? ld_next(jd->next + (((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
   }
 #pragma unroll
   for (int k = 0; k < ILP; ++k)
     if (cand[k] != kInf) cand[k] = mp_cand<ALGO>(cand[k], wv[k]);
 #pragma unroll
   for (int k = 0; k < ILP && !LAT; ++k)
-    nv[k] = (cand[k] != kInf) ? ld_next<PERSIST>(jd->next + (((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
+    nv[k] = (cand[k] != kInf) ? ld_next(jd->next + (((xy[k] & 0xFFFFu) << lvpt) | (pk[k] & 0xFFFFu))) : 0u;
 #pragma unroll
   for (int k = 0; k < ILP; ++k) {
     if (cand[k] != kInf && cand[k] < nv[k]) {

@@ -214,8 +214,8 @@ using pr_ff_t = typename std::conditional<pr_ff<MODE>(), FF, double>::type;
 
 template <int PERSIST, class T>
 __device__ __forceinline__ T pr_ld(const T* p) {
-  if constexpr (PERSIST == 1) return __ldcg(p);
-  else return *p;
+  static_assert(PERSIST != 1, "values written in the phase that reads them");
+  return *p;
 }
 
 // The contributions round p reads (fused form: half p; the adjoint: lambda before the round;
