@@ -138,7 +138,7 @@ __device__ void unit_apply(const BJob* J, bool initial, uint32_t unit) {
   const uint64_t base0 = (uint64_t)unit * BU_APPLY_WORDS;
   for (uint32_t k = 0; k < BU_APPLY_WORDS / BT; ++k) {
     const uint64_t base = base0 + (uint64_t)k * BT;
-    if (base < nwords) apply_step<2>(jd, sd, pw, base, cnt, teps, est);
+    if (base < nwords) apply_step<2>(jd, sd, pw, base, 0u, cnt, teps, est);
   }
   apply_flush<BT>(jd->ls, pw, cnt, teps, est);
 }

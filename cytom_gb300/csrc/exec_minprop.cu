@@ -69,11 +69,12 @@ __global__ void __launch_bounds__(APPLY_T) apply_minprop_kernel(const JobDesc* _
   if (!ls->cont || (!initial && ls->mode == 2)) return;
   const unsigned pw = initial ? 0u : ((ls->iter & 1u) ^ 1u);
   const uint64_t nwords = (sd->n + 31) >> 5;
+  const uint32_t est_lim = est_words(sd);
   unsigned cnt = 0, est = 0;
   unsigned long long teps = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nwords; base += stride)
-    apply_step<0>(jd, sd, pw, base, cnt, teps, est);
+    apply_step<0>(jd, sd, pw, base, est_lim, cnt, teps, est);
   apply_flush<APPLY_T>(ls, pw, cnt, teps, est);
   if (threadIdx.x == 0) {
     __threadfence();

@@ -212,11 +212,12 @@ __device__ __forceinline__ unsigned pick_mode(const JobDesc* __restrict__ jd, co
 // the next round (0 = the row is skipped; vpt = every source active, the frontier
 // test is skipped). A warp covers 32 consecutive words; when they share one row
 // (vpt >= 1024) it adds its row count with a single atomic. The non-zero frontier
-// words are listed (warp-ballot compaction) for sparse rounds.
+// words are listed (warp-ballot compaction) for sparse rounds; those listed first, est_lim
+// (est_words) of them, add to the estimate.
 template <int PERSIST>
 __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const StoreDesc* __restrict__ sd,
-                                           unsigned pw, uint64_t base, unsigned& cnt, unsigned long long& teps,
-                                           unsigned& est) {
+                                           unsigned pw, uint64_t base, uint32_t est_lim, unsigned& cnt,
+                                           unsigned long long& teps, unsigned& est) {
   LoopState* ls = jd->ls;
   const uint64_t n = sd->n, T = sd->T;
   const uint32_t lvpt = sd->lvpt;
@@ -269,7 +270,7 @@ __device__ __forceinline__ void apply_step(const JobDesc* __restrict__ jd, const
         const unsigned slot = slot0 + __popc(nz & ((1u << lane) - 1u));
         jd->aw[slot] = (uint32_t)i;
         jd->awm[slot] = word_columns(sd, i, w);
-        if (!PERSIST && slot < est_words(sd)) est = min(est + word_edges(sd, i, w), EST_MAX);
+        if (!PERSIST && slot < est_lim) est = min(est + word_edges(sd, i, w), EST_MAX);
       }
     }
   }
