@@ -113,7 +113,7 @@ int upload_store_desc(Ctx* c) {
   h.wts = c->wts;
   h.tile_ptr = c->tile_ptr;
   h.chunk_tile = c->chunk_tile;
-  h.out_deg = c->est_deg ? c->est_deg + (uint64_t)c->est_at * c->n : c->out_deg;
+  h.out_deg = c->est_deg ? c->est_deg : c->out_deg;
   h.in_deg = c->in_deg;
   h.E = c->E;
   h.nchunks = (c->E + kChunk - 1) / kChunk;
@@ -315,15 +315,14 @@ static int small_prepare(Ctx* c, bool async) {
   if (!c->small_max && !c->hsd.small_ok) return CYTOM_OK;
   bool changed = false;
   if (c->small_max && async && !c->est_deg && small_vertices(c)) {
-    if (cy_malloc(&c->est_deg, 2 * c->n * 4) != cudaSuccess) {
+    if (cy_malloc(&c->est_deg, c->n * 4) != cudaSuccess) {
       cudaGetLastError();
       c->est_deg = nullptr;
     }
     changed = c->est_deg != nullptr;
   }
   if (c->est_deg && c->est_version != c->version) {
-    cudaError_t e = cudaMemcpyAsync(c->est_deg + (uint64_t)c->est_at * c->n, c->out_deg, c->n * 4,
-                                    cudaMemcpyDeviceToDevice, c->stream);
+    cudaError_t e = cudaMemcpyAsync(c->est_deg, c->out_deg, c->n * 4, cudaMemcpyDeviceToDevice, c->stream);
     if (e != cudaSuccess) return cuda_err(c, e, "degree copy");
     c->est_version = c->version;
   }

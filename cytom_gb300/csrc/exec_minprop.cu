@@ -1215,16 +1215,29 @@ __device__ __forceinline__ uint32_t seed_cand(int algo, uint32_t uv, uint32_t w)
 }
 
 __global__ void seed_keys_multi_kernel(SeedJobs sj, const uint64_t* __restrict__ K, const uint32_t* __restrict__ W,
-                                       uint64_t count, uint32_t lvpt, uint32_t lT) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+                                       uint64_t count, uint32_t lvpt, uint32_t lT, uint32_t* est) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t m = (1ULL << lvpt) - 1ULL;
   const uint64_t tmask = (1ULL << lT) - 1ULL;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-    const uint64_t key = K[i];
-    const uint32_t w = W ? W[i] : 1u;
+  const unsigned lane = threadIdx.x & 31;
+  // whole warps go round the loop together
+  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < count; b += stride) {
+    const uint64_t i = b + lane;
+    const bool in = i < count;
+    const uint64_t key = in ? K[i] : 0ULL;
+    const uint32_t w = (W && in) ? W[i] : 1u;
     const uint64_t tile = key >> (2 * lvpt);
     const uint32_t u = (uint32_t)(((tile >> lT) << lvpt) | ((key >> lvpt) & m));
     const uint32_t v = (uint32_t)(((tile & tmask) << lvpt) | (key & m));
+    if (est) {  // keys of one source lie side by side: one add for the warp's
+      const uint32_t mine = in ? u : 0xFFFFFFFFu, before = __shfl_up_sync(0xFFFFFFFFu, mine, 1);
+      const bool head = lane == 0 || before != mine;
+      const unsigned heads = __ballot_sync(0xFFFFFFFFu, head);
+      const unsigned later = lane == 31 ? 0u : heads >> (lane + 1);
+      const unsigned len = later ? (unsigned)__ffs(later) : 32u - lane;
+      if (in && head) atomicAdd(est + u, len);
+    }
+    if (!in) continue;
     for (int k0 = 0; k0 < sj.count; k0 += SEED_JOBS) {
       uint32_t cand[SEED_JOBS], nv[SEED_JOBS];
 #pragma unroll
@@ -1246,7 +1259,7 @@ __global__ void seed_keys_multi_kernel(SeedJobs sj, const uint64_t* __restrict__
 }
 
 int minprop_seed_keys_many(Ctx* c, Job* const* jobs, int njobs, const uint64_t* K, const uint32_t* W,
-                           uint64_t count) {
+                           uint64_t count, uint32_t* est) {
   int g = std::max(1, std::min<int>(grid_persistent(c, 8), (int)((count + 255) / 256)));
   for (int base = 0; base < njobs; base += kMaxSeedJobs) {
     SeedJobs sj{};
@@ -1256,7 +1269,7 @@ int minprop_seed_keys_many(Ctx* c, Job* const* jobs, int njobs, const uint64_t* 
       sj.algo[k] = jobs[base + k]->algo;
     }
     int slot = prof_begin(c, KC_INSERT);
-    seed_keys_multi_kernel<<<g, 256, 0, c->stream>>>(sj, K, W, count, c->lvpt, c->lT);
+    seed_keys_multi_kernel<<<g, 256, 0, c->stream>>>(sj, K, W, count, c->lvpt, c->lT, base == 0 ? est : nullptr);
     c->launches++;
     prof_end(c, slot, (double)count * (12.0 + 8.0 * sj.count));
   }

@@ -1223,13 +1223,11 @@ int compact(Ctx* c) {
     cudaFreeAsync(tmp, c->stream);
     return rc;
   }
-  if (c->est_deg)  // the degrees of the new snapshot, beside those that runs still read
-    cudaMemcpyAsync(c->est_deg + (uint64_t)(c->est_at ^ 1) * c->n, c->out_deg, c->n * 4, cudaMemcpyDeviceToDevice,
-                    c->stream);
   // Installing the merged snapshot: runs on the previous one must have finished (everything
   // above wrote to the new snapshot alone). The jobs are then seeded by the merged edges
   // (edgeChanged(INSERT)).
   join_runs(c);
+  uint32_t* est = nullptr;  // the estimates' degrees, if the seeding pass brings them up to date
   {
     std::vector<Job*> mp;
     for (Job* j : c->jobs) {
@@ -1241,8 +1239,10 @@ int compact(Ctx* c) {
         rc = job_seed_keys(c, j, K, W, A);  // the PageRank family: a residual round next time
       if (rc) break;
     }
-    if (!rc && !mp.empty()) rc = minprop_seed_keys_many(c, mp.data(), (int)mp.size(), K, W, A);
+    if (c->est_deg && c->est_version == c->version && !mp.empty()) est = c->est_deg;
+    if (!rc && !mp.empty()) rc = minprop_seed_keys_many(c, mp.data(), (int)mp.size(), K, W, A, est);
     if (rc) {
+      if (est) c->est_version = ~0ULL;
       cudaFreeAsync(tmp, c->stream);
       return rc;
     }
@@ -1257,10 +1257,7 @@ int compact(Ctx* c) {
   c->E += Kn;
   c->A = 0;
   c->version++;
-  if (c->est_deg) {
-    c->est_at ^= 1;
-    c->est_version = c->version;
-  }
+  if (est) c->est_version = c->version;
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "merge");
   if (mdir) c->dir_version = c->version;

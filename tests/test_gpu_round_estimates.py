@@ -82,6 +82,55 @@ def test_insert_beside_asynchronous_runs_changes_no_round():
     assert out[0] == out[1] == out[2], out
 
 
+BATCHES = """
+import sys, json, numpy as np
+sys.path.insert(0, {root!r})
+import cytom_gb300 as cg
+side = 256
+n = side * side
+v = np.arange(n, dtype=np.uint32)
+r, d = v[v % side < side - 1], v[: side * (side - 1)]
+s = np.concatenate([r, d, r + 1, d + side]).astype(np.uint32)
+t = np.concatenate([r + 1, d + side, r, d]).astype(np.uint32)
+out, vals = [], []
+for asynchronous in (False, True):
+    rng = np.random.default_rng(1)
+    with cg.Engine(n, 4096, weight_type=cg.WEIGHT_U32) as eng:
+        eng.insert_edges(s, t, rng.integers(1, 100, len(s), dtype=np.uint32))
+        eng.do_global_compaction()
+        ps = [cg.BFS(eng, start_vertex=0, max_iterations=10000), cg.SSSP(eng, start_vertex=0, max_iterations=10000)]
+        rows = []
+        for k in range(6):
+            if asynchronous:
+                eng.run_many_async(ps)
+            else:
+                x = eng.run_many(ps)
+            m = (1 << 19) + 17 * k  # sources and targets among the last vertices, many of them repeated
+            a = (n - 1 - (rng.integers(0, n, m) >> rng.integers(0, 10, m))).astype(np.uint32)
+            b = (n - 1 - (rng.integers(0, n, m) >> rng.integers(0, 10, m))).astype(np.uint32)
+            eng.insert_edges(a, b, rng.integers(1000, 9000, m, dtype=np.uint32))
+            eng.do_global_compaction()
+            if asynchronous:
+                x = eng.run_many_wait()
+            rows.append([[q["iterations"], q["count_edges"], q["edges_scanned"]] for q in x])
+        out.append(rows)
+        vals.append([p.result().tobytes() for p in ps])
+assert vals[0] == vals[1]
+print(json.dumps(out))
+"""
+
+
+def test_estimates_follow_the_batches():
+    """A stream whose batches raise the degrees of the frontiers past a small round's limit, its runs
+    asynchronous and not: the same rounds, so the degrees that asynchronous runs keep follow."""
+    env = dict(os.environ, CYTOM_SPARSE_DIV="1024", CYTOM_AUTOTUNE="0")
+    r = subprocess.run([sys.executable, "-c", BATCHES.format(root=str(ROOT))], capture_output=True, text=True, env=env,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
+    out = json.loads(r.stdout.strip().splitlines()[-1])
+    assert out[0] == out[1], out
+
+
 def test_without_memory_for_the_degrees(cg, orc):
     """The first asynchronous launch cannot have its copy of the degrees: the runs give the same
     values, later ones too."""
