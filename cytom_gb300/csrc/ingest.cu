@@ -229,14 +229,19 @@ __device__ __forceinline__ uint64_t make_key(uint32_t s, uint32_t t, uint32_t lv
 // generator the first take several per cent of the endpoints (12.5 M RMAT-22 edges 366 us
 // without, 326 with one such vertex, 253 with 64 or 512, 255 with 2,048, 236 with 4,096, which
 // leaves fewer blocks per SM). Where ids say nothing about degrees it costs the clearing and the
-// adding up. With / without, in us, on 4 M vertices:
-//   edges   RMAT ids       RMAT, ids shuffled   uniform
-//   2^17    8.4 / 9.4      8.0 / 7.3            8.4 / 7.1
-//   2^18    11.0 / 14.4    10.7 / 9.8           9.5 / 8.7
-//   2^20    24.4 / 31.3    20.7 / 20.6          17.2 / 16.2
-//   2^24    298 / 378      212 / 212            198 / 195
+// adding up. With / without, in us:
+//   vertices  edges   RMAT ids       RMAT, ids shuffled   uniform
+//   2^12      2^17    12.0 / 20.8    12.1 / 11.7          9.9 / 8.3
+//   2^16      2^17    9.9 / 12.3     8.5 / 8.0            8.3 / 7.0
+//   2^16      2^18    12.2 / 20.8    11.2 / 10.2          9.9 / 8.3
+//   2^22      2^17    8.4 / 9.4      8.0 / 7.3            8.4 / 7.1
+//   2^22      2^18    11.0 / 14.4    10.7 / 9.8           9.5 / 8.7
+//   2^22      2^20    24.4 / 31.3    20.7 / 20.6          17.2 / 16.2
+//   2^22      2^24    298 / 378      212 / 212            198 / 195
+// (2^16 edges: 8.1 / 13.7 on 2^12 vertices, 8.1 / 8.9 on 2^16, 7.8 / 8.4 on 2^20 with RMAT ids,
+// 7.5 / 6.2, 7.0 / 6.1 and 6.5 / 6.1 uniform.)
 constexpr uint32_t APPEND_HUBS = 2048;
-constexpr uint64_t kAppendHubsMin = 1ULL << 18;  // edges: from here on the gain is three times the cost
+constexpr uint64_t kAppendHubsMin = 1ULL << 17;  // edges: from here on the gain is well above the cost
 
 template <bool HUBS>
 __global__ void append_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ tgt,
