@@ -87,3 +87,30 @@ def test_ranks_of_extreme_teleports(cg, orc, low, high):
     ok = r > 1e-35  # contributions r / s and their products are FP32 too
     assert (np.abs(r32 - r)[ok] <= 1e-5 * r[ok]).all()
     assert np.abs(r32 - r).sum() <= 1e-6 * r.sum()
+
+
+@pytest.mark.parametrize("what", ["loss", "teleport"])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_infinities_and_nan(cg, orc, what, value):
+    """One loss weight or teleport entry that is not finite: the FP32 form is finite exactly where the
+    FP64 form is, in ranks and gradients, and within the family's bounds there."""
+    rng = np.random.default_rng(9)
+    s, t = rng.integers(0, N - 64, 3000, dtype=np.uint32), rng.integers(0, N, 3000, dtype=np.uint32)
+    w = rng.uniform(0.5, 1.0, len(s)).astype(np.float32).view(np.uint32)
+    c, tele = rng.standard_normal(N), rng.uniform(0.5, 1.5, N) / N
+    (c if what == "loss" else tele)[700] = value
+    got = []
+    with cg.Engine(N, VPT, weight_type=cg.WEIGHT_F32) as eng:
+        eng.insert_edges(s, t, w)
+        eng.do_global_compaction()
+        for kahan in (True, False):
+            p = cg.WeightedPageRank(eng, max_iterations=4, tolerance=0.0, kahan=kahan)
+            p.set_teleport(tele)
+            p.execute_algorithm()
+            gw, gt, _ = p.adjoint(c)
+            got.append([np.asarray(x, np.float64) for x in (p.result(), gw, gt)])
+    for a, b in zip(*got):
+        ok = np.isfinite(b)
+        assert np.array_equal(np.isfinite(a), ok)
+        if ok.any():
+            assert np.abs(a - b)[ok].max() <= 1e-4 * np.abs(b[ok]).max()

@@ -131,6 +131,40 @@ def test_estimates_follow_the_batches():
     assert out[0] == out[1], out
 
 
+def test_rejected_insert_beside_asynchronous_runs(cg):
+    """The degrees a rejected batch raised and gave back are not seen by the runs beside it; the
+    degrees themselves and later runs are those of the graph without it."""
+    side = 256
+    n = side * side
+    v = np.arange(n, dtype=np.uint32)
+    r, d = v[v % side < side - 1], v[: side * (side - 1)]
+    s = np.concatenate([r, d, r + 1, d + side]).astype(np.uint32)
+    t = np.concatenate([r + 1, d + side, r, d]).astype(np.uint32)
+    rng = np.random.default_rng(2)
+    bs, bt = rng.integers(0, n, 1 << 22, dtype=np.uint32), rng.integers(0, n, 1 << 22, dtype=np.uint32)
+    bt[12345] = n
+    want = (v // side + v % side).astype(np.uint32)
+    got = []
+    for beside in (False, True):
+        with cg.Engine(n, n) as eng:
+            eng.insert_edges(s, t)
+            eng.do_global_compaction()
+            ps = [cg.BFS(eng, start_vertex=0, max_iterations=10000) for _ in range(2)]
+            eng.run_many_async(ps)
+            if beside:
+                with pytest.raises(cg.CytomError) as e:
+                    eng.insert_edges(bs, bt)
+                assert e.value.code == -3
+            x = eng.run_many_wait()
+            ps[0].init_algorithm()
+            x.append(ps[0].execute_algorithm())
+            got.append([[q["iterations"], q["count_edges"], q["edges_scanned"]] for q in x])
+            assert all(np.array_equal(p.result(), want) for p in ps)
+            out, inn = eng.degrees()
+            assert np.array_equal(out, np.bincount(s, minlength=n)) and np.array_equal(inn, np.bincount(t, minlength=n))
+    assert got[0] == got[1]
+
+
 def test_without_memory_for_the_degrees(cg, orc):
     """The first asynchronous launch cannot have its copy of the degrees: the runs give the same
     values, later ones too."""
