@@ -685,7 +685,8 @@ __device__ __forceinline__ double pr_shfl(double x, int lane) { return __shfl_sy
 // The FP32 PageRank's pull is bound by L2 requests, not by its update (22 instructions in
 // float pairs): its groups finish their targets alone, which needs 32 registers instead of
 // 48 and so keeps eight blocks per SM in flight (RMAT-24 26.4 ms, with shared updates 27.0 at
-// eight blocks per SM and 27.4 at five).
+// eight blocks per SM and 27.4 at five; RMAT-16 / 19 / 21 / 23 0.38 / 1.24 / 3.10 / 12.9, shared 0.39 /
+// 1.31 / 3.23 / 12.9).
 template <int MODE>
 __host__ __device__ constexpr bool pr_group_alone() {
   return MODE == PR_NORM32;
@@ -810,7 +811,12 @@ __device__ __forceinline__ void pull_vblocks(PrArgs& a, const pr_val_t<MODE>* cr
 
 // Resident blocks the pull is compiled for. Measured with 5 / 6 / 7 / 8: RMAT-22 FP64 11.8 /
 // 11.3 / 11.7 / 11.3 ms, RMAT-20 weighted forward and adjoint 15.0 / 14.0 / 13.4 / 13.4;
-// RMAT-16 PageRank-delta 20.3 with four, 21.1 with six, 21.7 with eight.
+// RMAT-16 PageRank-delta 20.3 with four, 21.1 with six, 21.7 with eight. Over other sizes, in ms, the
+// chosen number first: FP64 at RMAT-16 / 19 / 21 / 23 0.48 / 1.95 / 5.01 / 21.3 with six, 0.48 /
+// 2.01 / 5.08 / 21.5 with five, 0.48 / 1.97 / 5.03 / 21.4 with eight; FP32 0.38 / 1.24 / 3.10 / 12.9
+// with eight, 0.38 / 1.41 / 3.43 / 14.4 with five; weighted at 16 / 18 / 21 2.13 / 3.89 / 21.3 with
+// seven, 2.13 / 4.07 / 22.9 with five, 2.16 / 3.88 / 21.3 with eight; PageRank-delta streams at
+// 13 / 15 / 18 6.1 / 7.1 / 11.5 with four, 6.4 / 7.2 / 11.7 with six, 6.8 / 7.6 / 12.1 with eight.
 template <int MODE>
 __host__ __device__ constexpr int pr_min_blocks() {
   return MODE == PR_NORM32 ? 8 : MODE == PR_NORM64 ? 6 : (MODE == PR_W32 || MODE == PR_ADJ32) ? 7 : pr_fused<MODE>() ? 4 : 5;
