@@ -1060,23 +1060,30 @@ static int grow_store(Ctx* c, uint64_t need) {
   join_runs(c);  // the old buffers are freed below
   uint64_t ncap = std::max<uint64_t>(need + need / 2, 1 << 16);
   ncap = (ncap + kChunk - 1) / kChunk * kChunk + kChunk;
-  uint32_t *ne = nullptr, *nea = nullptr, *nw = nullptr, *nwa = nullptr;
+  // the chunk tables belong to the capacity: everything is there before anything is replaced
+  const uint64_t nch = ncap / kChunk + 2;
+  const bool chunks = nch > c->chunk_cap;
+  uint32_t *ne = nullptr, *nea = nullptr, *nw = nullptr, *nwa = nullptr, *ct = nullptr, *cta = nullptr;
   cudaError_t e = cy_malloc(&ne, ncap * 4);
   if (e == cudaSuccess) e = cy_malloc(&nea, ncap * 4);
   if (e == cudaSuccess && c->wtype) e = cy_malloc(&nw, ncap * 4);
   if (e == cudaSuccess && c->wtype) e = cy_malloc(&nwa, ncap * 4);
+  if (e == cudaSuccess && chunks) e = cy_malloc(&ct, nch * 4);
+  if (e == cudaSuccess && chunks) e = cy_malloc(&cta, nch * 4);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cudaFree(ne);
     cudaFree(nea);
     cudaFree(nw);
     cudaFree(nwa);
+    cudaFree(ct);
     return set_err(c, CYTOM_ERR_OOM, "tile store growth");
   }
   if (c->E) {
     cudaMemcpyAsync(ne, c->edges, c->E * 4, cudaMemcpyDeviceToDevice, c->stream);
     if (c->wtype) cudaMemcpyAsync(nw, c->wts, c->E * 4, cudaMemcpyDeviceToDevice, c->stream);
   }
+  if (chunks) cudaMemcpyAsync(ct, c->chunk_tile, c->chunk_cap * 4, cudaMemcpyDeviceToDevice, c->stream);
   cudaStreamSynchronize(c->stream);
   cudaFree(c->edges);
   cudaFree(c->edges_alt);
@@ -1087,23 +1094,14 @@ static int grow_store(Ctx* c, uint64_t need) {
   c->wts = nw;
   c->wts_alt = nwa;
   c->cap = ncap;
-  uint64_t nch = ncap / kChunk + 2;
-  if (nch > c->chunk_cap) {
-    uint32_t *ct = nullptr, *cta = nullptr;
-    if (cy_malloc(&ct, nch * 4) != cudaSuccess || cy_malloc(&cta, nch * 4) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(ct);
-      return set_err(c, CYTOM_ERR_OOM, "chunk table");
-    }
-    cudaMemcpyAsync(ct, c->chunk_tile, c->chunk_cap * 4, cudaMemcpyDeviceToDevice, c->stream);
-    cudaStreamSynchronize(c->stream);
+  if (chunks) {
     cudaFree(c->chunk_tile);
     cudaFree(c->chunk_tile_alt);
     c->chunk_tile = ct;
     c->chunk_tile_alt = cta;
     c->chunk_cap = nch;
   }
-  return CYTOM_OK;
+  return upload_store_desc(c);  // the compaction may yet fail
 }
 
 int ensure_app_capacity(Ctx* c, uint64_t need) {
