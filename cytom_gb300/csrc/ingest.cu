@@ -1543,8 +1543,9 @@ int delete_edges(Ctx* c, const uint32_t* src, const uint32_t* tgt, uint64_t coun
     if (j && !j->fresh && (j->algo == CYTOM_ALGO_BFS || j->algo == CYTOM_ALGO_CC || j->algo == CYTOM_ALGO_SSSP ||
                            j->algo == CYTOM_ALGO_SSWP))
       mp.push_back(j);
-  // temporaries: kill[nw+1], cnt[nw+1], P[nw+1], total, deleted list 3 x count, ndel, tight flags
-  const uint64_t words = 3 * (nw + 1) + 1 + 3 * count;
+  // temporaries: kill[nw+1], cnt[nw+1], P[nw+1], total, deleted list 3 x count, the scan's
+  // scratch (nothing is allocated once the degrees are lowered), ndel, tight flags
+  const uint64_t words = 3 * (nw + 1) + 1 + 3 * count + scan_scratch_words(nw + 1);
   const size_t bytes = ((words * 4 + 15) / 16) * 16 + 8 + (mp.size() + 1) * 4;
   char* tmp = nullptr;
   cudaError_t e = cy_malloc_async((void**)&tmp, bytes, c->stream);
@@ -1556,6 +1557,7 @@ int delete_edges(Ctx* c, const uint32_t* src, const uint32_t* tgt, uint64_t coun
   uint32_t* dsrc = total + 1;
   uint32_t* dtgt = dsrc + count;
   uint32_t* dw = dtgt + count;
+  uint32_t* sscan = dw + count;
   unsigned long long* ndel = (unsigned long long*)(tmp + ((words * 4 + 15) / 16) * 16);
   unsigned* tight = (unsigned*)(ndel + 1);
   cudaMemsetAsync(kill, 0, (nw + 1) * 4, c->stream);
@@ -1578,8 +1580,11 @@ int delete_edges(Ctx* c, const uint32_t* src, const uint32_t* tgt, uint64_t coun
   }
   keep_count_kernel<<<grid_for(c, nw + 1, 256), 256, 0, c->stream>>>(kill, E, nw, cnt);
   c->launches++;
-  rc = exclusive_scan_u32(c, cnt, P, nw + 1, total);
-  if (rc) return rc;
+  rc = scan_into(c, cnt, P, nw + 1, total, sscan);
+  if (rc) {
+    cudaFreeAsync(tmp, c->stream);
+    return rc;
+  }
   delete_gather_kernel<<<grid_for(c, E, 256, 16), 256, 0, c->stream>>>(c->edges, c->wts, E, kill, P, c->edges_alt,
                                                                        wt ? c->wts_alt : nullptr);
   c->launches++;
@@ -1588,7 +1593,10 @@ int delete_edges(Ctx* c, const uint32_t* src, const uint32_t* tgt, uint64_t coun
   c->launches++;
   for (size_t k = 0; k < mp.size(); ++k) {
     rc = minprop_delete_check(c, mp[k], dsrc, dtgt, wt ? dw : nullptr, nd, tight + k);
-    if (rc) return rc;
+    if (rc) {
+      cudaFreeAsync(tmp, c->stream);
+      return rc;
+    }
   }
   std::vector<unsigned> tflags(mp.size() + 1, 0);
   e = cudaMemcpyAsync(tflags.data(), tight, (mp.size() + 1) * 4, cudaMemcpyDeviceToHost, c->stream);

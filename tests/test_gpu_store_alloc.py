@@ -59,3 +59,30 @@ def test_compaction(cg, orc):
             if done:
                 break
         assert done, step
+
+
+def test_deletion(cg, orc):
+    """A deletion that runs out of memory has not lowered any degree."""
+    rng = np.random.default_rng(2)
+    s, t, w = batch(rng, 300000)  # its scan takes scratch of its own
+    gone = slice(1000, 90000)
+    for k in range(1, 20):
+        with cg.Engine(N, VPT, weight_type=cg.WEIGHT_U32) as eng:
+            eng.insert_edges(s, t, w)
+            eng.do_global_compaction()
+            before = eng.degrees()
+
+            def same():
+                assert all(np.array_equal(a, b) for a, b in zip(eng.degrees(), before))
+
+            more = disturbed(cg, eng, k, lambda: eng.delete_edges(s[gone], t[gone]), same)
+            pairs = lambda a, b: np.unique(a.astype(np.uint64) << np.uint64(32) | b)  # noqa: E731
+            left = np.setdiff1d(pairs(s, t), pairs(s[gone], t[gone]))
+            assert eng.count_edges()[0] == len(left)
+            killed = np.intersect1d(pairs(s, t), pairs(s[gone], t[gone]))
+            out, inn = eng.degrees()
+            assert np.array_equal(out, before[0] - np.bincount((killed >> np.uint64(32)).astype(np.int64), minlength=N))
+            assert np.array_equal(inn, before[1] - np.bincount((killed & np.uint64(0xFFFFFFFF)).astype(np.int64), minlength=N))
+        if not more:
+            break
+    assert not more
