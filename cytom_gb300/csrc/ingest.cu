@@ -322,24 +322,32 @@ __global__ void dyn_init_kernel(unsigned long long* __restrict__ next, uint64_t 
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += stride) next[t] = 4096;
 }
 
+// The counters, made before the first insert with dynamic compaction on changes anything.
+static int dynamic_counters(Ctx* c) {
+  if (c->dyn_pending) return CYTOM_OK;
+  const uint64_t nt = c->ntiles;
+  uint32_t* pending = nullptr;
+  if (cy_malloc(&pending, nt * 4) != cudaSuccess || cy_malloc(&c->dyn_next, nt * 8) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(pending);
+    c->dyn_next = nullptr;
+    return set_err(c, CYTOM_ERR_OOM, "dynamic compaction counters");
+  }
+  c->dyn_pending = pending;
+  cudaMemsetAsync(c->dyn_pending, 0, nt * 4, c->stream);
+  dyn_init_kernel<<<grid_for(c, nt, 256), 256, 0, c->stream>>>(c->dyn_next, nt);
+  c->launches++;
+  if (c->A) {  // edges appended before the counters existed
+    dyn_count_kernel<<<grid_for(c, c->A, 256), 256, 0, c->stream>>>(c->app_keys, c->A, c->lvpt, c->dyn_pending);
+    c->launches++;
+  }
+  return cuda_err(c, cudaGetLastError(), "dynamic compaction counters");
+}
+
 // After an insert with dynamic compaction on: counts the batch's edges per tile and
 // compacts the store when some tile reached its threshold.
 static int dynamic_compaction(Ctx* c, uint64_t first, uint64_t count) {
   const uint64_t nt = c->ntiles;
-  if (!c->dyn_pending) {
-    if (cy_malloc(&c->dyn_pending, nt * 4) != cudaSuccess || cy_malloc(&c->dyn_next, nt * 8) != cudaSuccess) {
-      cudaGetLastError();
-      return set_err(c, CYTOM_ERR_OOM, "dynamic compaction counters");
-    }
-    cudaMemsetAsync(c->dyn_pending, 0, nt * 4, c->stream);
-    dyn_init_kernel<<<grid_for(c, nt, 256), 256, 0, c->stream>>>(c->dyn_next, nt);
-    c->launches++;
-    // edges appended before the counters existed
-    if (first) {
-      dyn_count_kernel<<<grid_for(c, first, 256), 256, 0, c->stream>>>(c->app_keys, first, c->lvpt, c->dyn_pending);
-      c->launches++;
-    }
-  }
   dyn_count_kernel<<<grid_for(c, count, 256), 256, 0, c->stream>>>(c->app_keys + first, count, c->lvpt,
                                                                     c->dyn_pending);
   cudaMemsetAsync(c->d_flag, 0, sizeof(unsigned int), c->stream);
@@ -362,6 +370,7 @@ int insert_device(Ctx* c, const uint32_t* src, const uint32_t* tgt, const uint32
   cudaError_t e = cudaMemsetAsync(c->d_flag, 0, sizeof(unsigned int), c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "memset");
   int rc = ensure_app_capacity(c, c->A + count);
+  if (!rc && c->cfg.use_dynamic_compaction) rc = dynamic_counters(c);
   if (rc) return rc;
   const uint32_t* wuse = (c->wtype != CYTOM_UNWEIGHTED) ? w : nullptr;
   int slot = prof_begin(c, KC_INSERT);

@@ -86,3 +86,35 @@ def test_deletion(cg, orc):
         if not more:
             break
     assert not more
+
+
+def test_dynamic_compaction_counters(cg, orc):
+    """An insert whose counters found no room has inserted nothing."""
+    rng = np.random.default_rng(3)
+    parts = [batch(rng, 3000), batch(rng, 9000)]
+    st = orc.Store(N, VPT, True)
+    for p in parts:
+        st.insert(*p)
+    st.compact()
+    want = st.dump()
+    for k in range(1, 20):
+        with cg.Engine(N, VPT, weight_type=cg.WEIGHT_U32, dynamic_compaction=True) as eng:
+            more = False
+            for j, p in enumerate(parts):
+                if j == 0:
+                    empty = lambda: [x.sum() for x in eng.degrees()] == [0, 0] and eng.count_edges() == (0, 0)  # noqa: E731
+
+                    def nothing():
+                        assert empty()
+
+                    more = disturbed(cg, eng, k, lambda: eng.insert_edges(*p), nothing)
+                else:
+                    eng.insert_edges(*p)
+            out, _ = eng.degrees()
+            assert np.array_equal(out, np.bincount(np.concatenate([p[0] for p in parts]), minlength=N))
+            eng.do_global_compaction()
+            got = eng.dump_tiles(weights=True)
+            assert all(np.array_equal(a, b) for a, b in zip(got, want)), k
+        if not more:
+            break
+    assert not more
