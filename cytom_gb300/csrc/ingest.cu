@@ -1164,7 +1164,7 @@ int compact(Ctx* c) {
   if (rc) return rc;
   // temporaries
   const uint64_t nsp = (c->E + A + MERGE_SPAN - 1) / MERGE_SPAN;  // merge spans (upper bound)
-  size_t bytes = A * (4 + 4 + 8 + 4 + 8 + 4 + 4 + 4) + 64 + 2 * (nsp + 1) * 4;
+  size_t bytes = A * (4 + 4 + 8 + 4 + 8 + 4 + 4 + 4) + 64 + 2 * (nsp + 1) * 4 + scan_scratch_words(A) * 4;
   char* tmp = nullptr;
   cudaError_t e = cy_malloc_async((void**)&tmp, bytes, c->stream);
   if (e != cudaSuccess) return set_err(c, CYTOM_ERR_OOM, "compaction temporaries");
@@ -1179,14 +1179,18 @@ int compact(Ctx* c) {
   uint32_t* Kdev = ntile + A;
   uint32_t* sb = Kdev + 16;
   uint32_t* ts = sb + (nsp + 1);
+  uint32_t* sscan = ts + (nsp + 1);
   int slot = prof_begin(c, KC_MERGE);
   dedupe_lookup_kernel<<<grid_for(c, A, 256), 256, 0, c->stream>>>(
       K, W, A, c->edges, c->wts, c->tile_ptr,
       c->dir && !c->dir_disabled && c->dir_version == c->version ? c->dir : nullptr, (uint32_t)(c->vpt / 32), c->lvpt,
       keep, lb, wsel);
   c->launches++;
-  rc = exclusive_scan_u32(c, keep, P, A, Kdev);
-  if (rc) return rc;
+  rc = scan_into(c, keep, P, A, Kdev, sscan);
+  if (rc) {
+    cudaFreeAsync(tmp, c->stream);
+    return rc;
+  }
   pack_kept_kernel<<<grid_for(c, A, 256), 256, 0, c->stream>>>(K, A, keep, P, lb, wsel, c->lvpt, q,
                                                                nloc, wt ? nw : nullptr, ntile, c->cmask, c->lT,
                                                                c->lT > 6 ? c->lT - 6 : 0u);

@@ -118,3 +118,26 @@ def test_dynamic_compaction_counters(cg, orc):
         if not more:
             break
     assert not more
+
+
+def test_failed_compactions_give_their_memory_back(cg):
+    """A compaction that fails again and again, at each of its allocations, holds no more memory than
+    one that succeeds."""
+    import torch
+    n, m = 1 << 16, 1 << 21  # some 100 MB of temporaries each
+    rng = np.random.default_rng(4)
+    s, t = rng.integers(0, n, m, dtype=np.uint32), rng.integers(0, n, m, dtype=np.uint32)
+    free = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    with cg.Engine(n, 65536) as eng:
+        eng.insert_edges(s, t)
+        eng.do_global_compaction()
+        eng.insert_edges(s, t)  # the same edges: every buffer has its size
+        eng.do_global_compaction()
+        eng.sync()
+        before = free()
+        for k in range(1, 9):
+            for _ in range(4):
+                eng.insert_edges(s, t)
+                disturbed(cg, eng, k, eng.do_global_compaction)
+        eng.sync()
+        assert before - free() < 64 << 20
